@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/hpsi_gb300.h"
+#include "d64_gemm.cuh"
 #include "kernels.cuh"
 #include "tc_gemm.cuh"
 
@@ -34,6 +35,9 @@ struct KSlot {
     double* d_lam = nullptr;
     double2* pr64 = nullptr;
     bool pr64_grad = false;
+    int* d64_exp = nullptr;        // exponents of pr64's columns [npw] and rows for the digit split,
+                                   // in pr64's allocation
+    bool d64_exp_set = false;
     float2* pr32 = nullptr;
     bool pr32_grad = false;
     // tensor-core H|psi>: generator tables of the projector operands, one set
@@ -99,6 +103,11 @@ struct hpsi_ctx {
     std::map<int, KSlot> slots;
     unsigned char* ws = nullptr;
     size_t ws_size = 0;
+    // workspace of the FP64 GEMMs on the tensor cores, beside ws: a call that
+    // cannot have it runs the SIMT GEMMs
+    unsigned char* d64_ws = nullptr;
+    size_t d64_size = 0;
+    bool d64_ran = false;         // d_err is checked at the next synchronising call
     Prof prof;
     int* d_err = nullptr;         // device-side error flag of the bounded waits (tcgen05 GEMMs)
     // side stream of the tensor-core H|psi>: the projection chain runs there
@@ -170,6 +179,21 @@ inline int ws_reserve(hpsi_ctx* c, size_t bytes)
     return HPSI_OK;
 }
 
+// The FP64 GEMM workspace of at least bytes, or null when the device has no room.
+inline unsigned char* d64_reserve(hpsi_ctx* c, size_t bytes)
+{
+    if (bytes <= c->d64_size) return c->d64_ws;
+    if (c->d64_ws) cudaFree(c->d64_ws);
+    c->d64_ws = nullptr;
+    c->d64_size = 0;
+    if (cudaMalloc((void**)&c->d64_ws, bytes) != cudaSuccess) {
+        cudaGetLastError();  // not an error of the call
+        c->d64_ws = nullptr;
+        return nullptr;
+    }
+    c->d64_size = bytes;
+    return c->d64_ws;
+}
 
 // Build, once, what a precision needs on slot s (projector matrices, tensor-core
 // operands; with grad also the derivative operands).  Allocates.

@@ -1,0 +1,614 @@
+// d64_gemm.cu — complex128 GEMMs of the nonlocal term on the FP16 tensor cores.
+//
+// GB300 runs FP64 at 1/64 of the FP32 rate (0.6 T multiply-adds/s on the whole
+// part), so the FP64 projector sums were 94% of an FP64 H|psi> on the 64-atom
+// cell.  Here each operand is written as a sum of S = 7 slices of base-256
+// digits and the products of the slices run as exact integer arithmetic on the
+// tensor cores (the splitting scheme of Ozaki, Ogita, Oishi and Rump,
+// "Error-free transformations of matrix multiplication", Numer. Algorithms 59,
+// 2012):
+//   x 2^-(scales) = sum_i d_i 2^(-7 - 8 i),  i < 7, |d_i| <= 128 (FP16-exact),
+// a fixed-point number of 55 bits.  A slice product is at most 2^14, so FP32
+// accumulation of up to 1024 of them is exact; slice pairs (i, j) of one
+// diagonal d = i + j share an accumulator (at most 7 pairs), which is read out
+// every 128 of K.  Diagonals 0..7 are kept (34 of 49 pairs); the dropped ones
+// lie below the 2^-56 rounding of the digits.  The read-outs are added as 64-bit
+// integers and rounded to FP64 once per output.
+//
+// Scales: the columns of A (one per K index) are divided by a power of two to
+// at most one and B multiplied by it, then every row of A and of B is divided by
+// its own power of two.  The digits of an element are thus relative to the
+// largest *term* of the sums it enters, not to the largest element of its row:
+// projectors decay as exp(-q^2 rc^2/4) over the G-sphere, bands grow or decay
+// independently of that.  Error against 80-bit sums on the 8- and 16-atom cells
+// (projection / expansion, 2-norm): 4e-16 / 1e-16, where the FP64 SIMT GEMMs
+// have 1e-15 / 4e-16.
+//
+// What bounds it: 34 MMAs per K step of a 128 x 64 tile, so the tensor pipe on
+// large cells; operands come from L2 (84 KB of slices per 32 of K and tile).
+//
+// Layout: K-major tiles of (rows x 32) FP16 digits, slice after slice: an A tile
+// is 7 x 8 KB and a B tile 7 x NT x 64 bytes of contiguous memory, already in
+// the SWIZZLE_64B order of the MMA descriptors, so that a pipeline stage is two
+// bulk copies.
+#include <algorithm>
+#include <cuda_fp16.h>
+
+#include "d64_gemm.cuh"
+#include "tcgen05.cuh"
+
+namespace {
+
+constexpr int S = 7;                      // slices per operand
+constexpr int ND = 8;                     // diagonals kept: i + j < ND
+constexpr int TM = 128;                   // A rows per tile
+constexpr int KB = 32;                    // real K per pipeline stage
+constexpr int CHUNK = 4;                  // stages per read-out of the accumulators (128 of K)
+constexpr int FIX = 55;                   // bits of the fixed-point form
+constexpr int A_STAGE = S * TM * KB * 2;  // 56 KB
+constexpr int STAGES = 2;
+constexpr int DRAIN_WARPS = 16;
+constexpr int THREADS = 64 + 32 * DRAIN_WARPS;
+constexpr uint32_t TMEM_ALL = 512;
+constexpr size_t A_CAP = 768ull << 20;    // bytes of A slices resident at once
+constexpr int N_CAP = 256;                // bands per pass
+
+// Row and band exponents are stored with a bias, so that 0 means "no nonzero element".
+constexpr int F_BIAS = 8192;
+constexpr int F_BAD = 1 << 20;            // an infinity or NaN in the row
+
+__device__ uint32_t g_issue_wait_limit = WAIT_LIMIT;
+
+__device__ __forceinline__ int clean(int f) { return (f == 0 || f >= F_BAD) ? 0 : f - F_BIAS; }
+
+__device__ __forceinline__ int exp_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// biased exponent of the larger part, -1 for zero
+__device__ __forceinline__ int exp_of(double2 v)
+{
+    if (v.x == 0.0 && v.y == 0.0) return -1;
+    return max(exp_of(v.x), exp_of(v.y));
+}
+
+constexpr unsigned long long DIGIT_BIAS = 0x80808080808080ull;
+
+// rint(x 2^sh) + DIGIT_BIAS for |x 2^sh| < 2^55: byte i of the sum, minus
+// 128, is the base-256 digit of weight 2^(8 i); the top digit takes 9 bits.
+__device__ __forceinline__ unsigned long long fixed_digits(double x, int sh)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    const int e = (hi >> 20) & 0x7ff;
+    const unsigned long long m =
+        ((unsigned long long)((hi & 0xfffffu) | (e ? 0x100000u : 0u)) << 32 | lo) << 10;  // 63 bits
+    // value = m 2^(e' - 1085 + sh), e' the exponent of a normal number: shift right by r > 0, rounding
+    const int r = 1085 - sh - (e ? e : 1);
+    const unsigned long long t = m >> min(max(r - 1, 0), 63);
+    unsigned long long y = (t + 1) >> 1;
+    if (hi >> 31) y = 0ull - y;
+    return y + DIGIT_BIAS;
+}
+
+// slice i (0 the most significant) of two fixed-point values as an FP16 pair
+template <int I>
+__device__ __forceinline__ uint32_t slice_pair(unsigned long long u0, unsigned long long u1)
+{
+    constexpr int b = S - 1 - I;  // byte
+    uint32_t t;
+    if (b == S - 1) {
+        t = __byte_perm((uint32_t)(u0 >> 32), (uint32_t)(u1 >> 32), 0x7632) & 0x01ff01ffu;
+    } else {
+        const uint32_t w0 = b < 4 ? (uint32_t)u0 : (uint32_t)(u0 >> 32), w1 = b < 4 ? (uint32_t)u1 : (uint32_t)(u1 >> 32);
+        constexpr int c = b & 3;
+        t = __byte_perm(w0, w1, c | (c << 4) | ((4 + c) << 8) | ((4 + c) << 12)) & 0x00ff00ffu;
+    }
+    t |= 0x64006400u;  // FP16 1024 + digit + 128, exact
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&t), __floats2half2_rn(1152.f, 1152.f));
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// byte offset of 16-byte chunk c of row r within a slice (SWIZZLE_64B)
+__device__ __forceinline__ int slice_off(int r, int c) { return 64 * r + 16 * (c ^ ((r >> 1) & 3)); }
+
+template <int I>
+__device__ __forceinline__ void store_slices(unsigned char* at, size_t stride, const unsigned long long (&u)[8])
+{
+    uint4 v;
+    v.x = slice_pair<I>(u[0], u[1]);
+    v.y = slice_pair<I>(u[2], u[3]);
+    v.z = slice_pair<I>(u[4], u[5]);
+    v.w = slice_pair<I>(u[6], u[7]);
+    *reinterpret_cast<uint4*>(at + I * stride) = v;
+    if constexpr (I + 1 < S) store_slices<I + 1>(at, stride, u);
+}
+
+// ---- scales -----------------------------------------------------------------
+__global__ void col_exp_kernel(int M, int K, const double2* __restrict__ A, size_t lda, int mper, int* ek)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= K) return;
+    const int m0 = blockIdx.y * mper, m1 = min(M, m0 + mper);
+    int e = 0;
+#pragma unroll 4
+    for (int m = m0; m < m1; ++m) {
+        const double2 v = A[(size_t)m * lda + k];
+        const int x = exp_of(v.x), y = exp_of(v.y);
+        if (x != 0x7ff) e = max(e, x);
+        if (y != 0x7ff) e = max(e, y);
+    }
+    atomicMax(ek + k, e);
+}
+
+__global__ void row_exp_kernel(int K, const double2* __restrict__ A, size_t lda, const int* __restrict__ ek, int kper,
+                               int* fm)
+{
+    const int m = blockIdx.y, k0 = blockIdx.x * kper, k1 = min(K, k0 + kper);
+    int f = 0;
+    for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+        const int e = exp_of(A[(size_t)m * lda + k]);
+        if (e >= 0) f = max(f, e == 0x7ff ? F_BAD : e - ek[k] + F_BIAS);
+    }
+    f = __reduce_max_sync(0xffffffffu, f);
+    if ((threadIdx.x & 31) == 0 && f) atomicMax(fm + m, f);
+}
+
+// ---- slices -----------------------------------------------------------------
+// A rows [row0, row0 + gridDim.y * 64) of the GEMM operand, 16 complex K values
+// (one stage) per block.  TRANS = false: row r is A[r][.] (projection, scales
+// er = fm, ek); TRANS = true: row r is column r of A (expansion, er = ek, ek = fm).
+// A quad of lanes holds one row of a stage: 256-byte row reads (or 128-byte
+// column runs), and each slice store of a warp fills 512 contiguous bytes.
+template <bool TRANS>
+__global__ void __launch_bounds__(256) split_a_kernel(int R, int K, int row0, const double2* __restrict__ A, size_t lda,
+                                                      const int* __restrict__ er, const int* __restrict__ ek,
+                                                      unsigned char* __restrict__ out)
+{
+    const int kt = blockIdx.x, KT = gridDim.x;
+    const int rl = blockIdx.y * 64 + (threadIdx.x >> 2), r = row0 + rl, c = threadIdx.x & 3;
+    const int k0 = kt * 16 + c * 4;
+    unsigned long long u[8];
+    const int sr = r < R ? (TRANS ? 1022 - er[r] : -clean(er[r])) : 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int k = k0 + i;
+        double2 v = make_double2(0.0, 0.0);
+        int sk = 0;
+        if (r < R && k < K) {
+            v = TRANS ? A[(size_t)k * lda + r] : A[(size_t)r * lda + k];
+            sk = TRANS ? -clean(ek[k]) : 1022 - ek[k];
+        }
+        u[2 * i] = fixed_digits(v.x, FIX + sr + sk);
+        u[2 * i + 1] = fixed_digits(v.y, FIX + sr + sk);
+    }
+    unsigned char* tile = out + ((size_t)(rl >> 7) * KT + kt) * A_STAGE;
+    store_slices<0>(tile + slice_off(rl & 127, c), TM * KB * 2, u);
+}
+
+// B rows of one band per block: band b of tile t = b / BT sits in rows j = b % BT
+// (real part of the result) and BT + j (imaginary part).  TRANS = false: src[b][k],
+// the projection's rows (b_r, b_i) and (b_i, -b_r) for conj(A) B; TRANS = true:
+// src[k][b], the expansion's rows (W_r, -W_i) and (W_i, W_r).  First the band's
+// exponent fb, then the digits.  Bands past nb are zero.
+template <bool TRANS>
+__global__ void __launch_bounds__(512) split_b_kernel(int nb, int K, const double2* __restrict__ src, size_t ld,
+                                                      const int* __restrict__ ek, int KT, int BT,
+                                                      unsigned char* __restrict__ out, int* __restrict__ fb)
+{
+    __shared__ int red[16];
+    const int b = blockIdx.x, t = b / BT, j = b % BT;
+    int f = 0;
+    if (b < nb)
+        for (int k = threadIdx.x; k < K; k += blockDim.x) {
+            const int e = exp_of(TRANS ? src[(size_t)k * ld + b] : src[(size_t)b * ld + k]);
+            if (e >= 0) f = max(f, e == 0x7ff ? F_BAD : e - 1022 + (TRANS ? clean(ek[k]) : ek[k] - 1022) + F_BIAS);
+        }
+    f = __reduce_max_sync(0xffffffffu, f);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = f;
+    __syncthreads();
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) f = max(f, red[i]);
+    if (threadIdx.x == 0) fb[b] = f;
+    f = clean(f);
+    const size_t slice = (size_t)2 * BT * KB * 2;
+    for (int q = threadIdx.x; q < 4 * KT; q += blockDim.x) {
+        const int kt = q >> 2, c = q & 3;
+        unsigned long long re[8], im[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = kt * 16 + c * 4 + i;
+            double2 v = make_double2(0.0, 0.0);
+            int sh = 0;
+            if (b < nb && k < K) {
+                v = TRANS ? src[(size_t)k * ld + b] : src[(size_t)b * ld + k];
+                sh = FIX - f + (TRANS ? clean(ek[k]) : ek[k] - 1022);
+            }
+            const unsigned long long x = fixed_digits(v.x, sh), y = fixed_digits(v.y, sh);
+            re[2 * i] = x;
+            re[2 * i + 1] = TRANS ? 2 * DIGIT_BIAS - y : y;  // 2 bias - u: the digits of the negated value
+            im[2 * i] = y;
+            im[2 * i + 1] = TRANS ? x : 2 * DIGIT_BIAS - x;
+        }
+        unsigned char* tile = out + ((size_t)t * KT + kt) * S * slice;
+        store_slices<0>(tile + slice_off(j, c), slice, re);
+        store_slices<0>(tile + slice_off(BT + j, c), slice, im);
+    }
+}
+
+// ---- GEMM -------------------------------------------------------------------
+struct D64Smem {
+    uint64_t full[STAGES], empty[STAGES];
+    uint64_t dfull[2], dempty[2];  // accumulator set: a chunk's products final; read out
+    uint64_t done;
+    uint32_t tmem_base;
+    uint32_t abort_flag;
+};
+
+struct D64Out {
+    double2* part;   // projection: [z][M][ldn], first band of the pass
+    int ldn;
+    double2* out;    // expansion: [N][ldo], +=
+    size_t ldo;
+    const int* er;   // row exponents (fm, or ek with bias)
+    const int* fb;   // column exponents
+    int M, N, row0;  // result rows and bands; first row of this launch's A chunk
+};
+
+template <int CW>
+__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[CW])
+{
+    if constexpr (CW == 4)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(addr));
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+
+// (h 2^24 + l) 2^e rounded once to FP64, on the integer pipe
+__device__ __forceinline__ double round_sum(long long h, long long l, int e)
+{
+    const __int128 v = ((__int128)h << 24) + l;
+    if (v == 0) return 0.0;
+    const bool neg = v < 0;
+    const unsigned __int128 a = neg ? (unsigned __int128)-v : (unsigned __int128)v;
+    const unsigned long long ah = (unsigned long long)(a >> 64), al = (unsigned long long)a;
+    const int lz = ah ? __clzll((long long)ah) : 64 + __clzll((long long)al);
+    const unsigned __int128 n = a << lz;
+    const unsigned long long top = (unsigned long long)(n >> 64), rest = (unsigned long long)n;
+    unsigned long long m = top >> 11;
+    const unsigned long long dropped = top & 0x7ffu;
+    if (dropped > 0x400u || (dropped == 0x400u && (rest != 0 || (m & 1)))) ++m;
+    const int be = 127 - lz + e + 1023;  // biased exponent
+    const unsigned long long sign = neg ? 1ull << 63 : 0ull;
+    if (be >= 1 && be < 2046) return __longlong_as_double((long long)(sign + ((unsigned long long)(be - 1) << 52) + m));
+    const double x = __longlong_as_double((long long)(sign + (1022ull << 52) + m));  // [1, 2]
+    return scalbn(x, be - 1023);
+}
+
+// TMEM columns of one accumulator, and sets of ND accumulators in TMEM
+__host__ __device__ constexpr int acc_cols(int NT) { return NT <= 32 ? 32 : 64; }
+__host__ __device__ constexpr int acc_sets(int NT) { return (int)TMEM_ALL / (ND * acc_cols(NT)); }
+
+template <int NT, bool EXPAND>
+__global__ void __launch_bounds__(THREADS, 1)
+    d64_gemm_kernel(const unsigned char* __restrict__ A, const unsigned char* __restrict__ B, D64Out o, int KT,
+                    int chunks_per_split, uint32_t idesc, int* err)
+{
+    constexpr int B_STAGE = S * NT * KB * 2, STAGE = A_STAGE + B_STAGE, NBUF = acc_sets(NT);
+    constexpr int AC = acc_cols(NT);
+    constexpr int BT = NT / 2, BPW = BT / 4, CW = BPW % 4 == 0 ? 4 : 2;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    unsigned char* tiles = smem_raw + (((raw + 1023u) & ~1023u) - raw);
+    D64Smem* sh = reinterpret_cast<D64Smem*>(tiles + STAGES * STAGE);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int kt0 = blockIdx.z * chunks_per_split * CHUNK, kt1 = min(KT, kt0 + chunks_per_split * CHUNK);
+    const int nk = kt1 - kt0, nchunk = (nk + CHUNK - 1) / CHUNK;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&sh->full[s], 1);
+            mbar_init(&sh->empty[s], 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(&sh->dfull[a], 1);
+            mbar_init(&sh->dempty[a], DRAIN_WARPS);
+        }
+        mbar_init(&sh->done, 1);
+        sh->abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem_base)),
+                     "r"(TMEM_ALL));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh->tmem_base;
+    volatile uint32_t* abort = &sh->abort_flag;
+
+    if (warp == 0 && lane == 0) {
+        // ---- bulk copies: one A tile and one B tile per stage
+        const unsigned char* a = A + ((size_t)blockIdx.y * KT + kt0) * A_STAGE;
+        const unsigned char* b = B + ((size_t)blockIdx.x * KT + kt0) * B_STAGE;
+        int issued = 0;
+        for (int it = 0; it < nk; ++it) {
+            const int s = it % STAGES;
+            if (!mbar_wait_abort(&sh->empty[s], ((it / STAGES) & 1) ^ 1, &sh->abort_flag)) {
+                if (!*abort) { atomicExch(err, 11); *abort = 1; }
+                break;
+            }
+            if (*abort) break;
+            unsigned char* st = tiles + s * STAGE;
+            mbar_arrive_expect_tx(&sh->full[s], STAGE);
+            bulk_load(st, a + (size_t)it * A_STAGE, A_STAGE, &sh->full[s]);
+            bulk_load(st + A_STAGE, b + (size_t)it * B_STAGE, B_STAGE, &sh->full[s]);
+            issued = it + 1;
+        }
+        // drain: copies in flight must land before the CTA exits (bounded)
+        for (int it = max(0, issued - STAGES); it < issued; ++it) mbar_wait(&sh->full[it % STAGES], (it / STAGES) & 1);
+    } else if (warp == 1 && lane == 0) {
+        // ---- MMA issuer
+        const uint32_t lim = g_issue_wait_limit;
+        bool stop = false;
+        for (int c = 0; c < nchunk && !stop; ++c) {
+            const int buf = c % NBUF;
+            if (!mbar_wait_abort(&sh->dempty[buf], ((c / NBUF) & 1) ^ 1, &sh->abort_flag)) {
+                if (!*abort) { atomicExch(err, 12); *abort = 1; }
+                break;
+            }
+            tc_fence_after();
+            const uint32_t acc = tmem + buf * 256;
+            const int i1 = min(nk, (c + 1) * CHUNK);
+            for (int it = c * CHUNK; it < i1; ++it) {
+                const int s = it % STAGES;
+                if (!mbar_wait_n(&sh->full[s], (it / STAGES) & 1, lim)) {
+                    atomicExch(err, 13);
+                    *abort = 1;
+                    stop = true;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t st = smem_u32(tiles + s * STAGE);
+                const uint64_t ad = sdesc_sw64(st), bd = sdesc_sw64(st + A_STAGE);
+                const bool first = it == c * CHUNK;
+#pragma unroll
+                for (int kk = 0; kk < KB / 16; ++kk)
+#pragma unroll
+                    for (int i = 0; i < S; ++i)
+#pragma unroll
+                        for (int j = 0; j < S && i + j < ND; ++j) {
+                            // the first pair of a diagonal overwrites what the last read-out left
+                            const bool head = kk == 0 && (i == 0 || (i == 1 && j == S - 1));
+                            tc_mma(acc + (i + j) * AC, ad + ((i * TM * KB * 2 + kk * 32) >> 4),
+                                   bd + ((j * NT * KB * 2 + kk * 32) >> 4), idesc, head && first ? 0u : 1u);
+                        }
+                tc_commit(&sh->empty[s]);
+            }
+            if (!stop) tc_commit(&sh->dfull[buf]);
+        }
+        // every MMA issued has completed before the accumulators are freed (bounded)
+        tc_commit(&sh->done);
+        mbar_wait(&sh->done, 0);
+    } else if (warp >= 2) {
+        // ---- read-out: warp w holds TMEM lanes 32 (w % 4) .. +31 (rows) and
+        // bands sub BPW .. +BPW-1 of the tile, real and imaginary columns
+        const int q = warp & 3, sub = (warp - 2) >> 2;
+        long long h[2 * BPW], l[2 * BPW];
+#pragma unroll
+        for (int i = 0; i < 2 * BPW; ++i) h[i] = l[i] = 0;
+        bool go = true;
+        for (int c = 0; c < nchunk; ++c) {
+            const int buf = c % NBUF;
+            const bool ok = mbar_wait_abort(&sh->dfull[buf], (c / NBUF) & 1, &sh->abort_flag);
+            if (!ok && !*abort) { atomicExch(err, 14); *abort = 1; }
+            // warp-uniform: tcgen05.ld is a .sync.aligned warp instruction
+            go = __all_sync(0xffffffffu, ok && !*abort);
+            if (!go) break;
+            tc_fence_after();
+            const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + buf * 256 + sub * BPW;
+#pragma unroll
+            for (int p = 0; p < 2 * BPW; p += CW) {
+                const uint32_t at = base + (p < BPW ? p : BT + p - BPW);
+                uint32_t v[ND][CW];
+#pragma unroll
+                for (int d = 0; d < ND; ++d) tmem_ld<CW>(at + d * AC, v[d]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (p + CW >= 2 * BPW) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh->dempty[buf]);
+                }
+#pragma unroll
+                for (int i = 0; i < CW; ++i) {
+                    // exact integers: |diagonal d| <= 128 (d + 1) 2^14 < 2^24, the sums of
+                    // two adjacent low diagonals within 32 bits
+                    const int t01 = __float2int_rn(__uint_as_float(v[0][i])) * 256 + __float2int_rn(__uint_as_float(v[1][i]));
+                    const int t23 = __float2int_rn(__uint_as_float(v[2][i])) * 256 + __float2int_rn(__uint_as_float(v[3][i]));
+                    const int i4 = __float2int_rn(__uint_as_float(v[4][i])), i5 = __float2int_rn(__uint_as_float(v[5][i]));
+                    const int i67 = __float2int_rn(fmaf(__uint_as_float(v[7][i]), 1.f / 256.f, __uint_as_float(v[6][i])));
+                    h[p + i] += (long long)t01 * 65536 + t23;
+                    l[p + i] += (long long)i4 * 65536 + ((long long)i5 * 256 + i67);
+                }
+            }
+        }
+        const int row = o.row0 + blockIdx.y * TM + q * 32 + lane;
+        if (go && row < o.M) {
+            // h counts diagonal 3, l diagonal 6: weights 2^(72 - 110) and 2^(48 - 110)
+            const int fr = o.er[row];
+            const bool bad = !EXPAND && fr >= F_BAD;
+            const int er = (EXPAND ? fr - 1022 : clean(fr)) - 62;
+#pragma unroll
+            for (int i = 0; i < BPW; ++i) {
+                const int n = blockIdx.x * BT + sub * BPW + i;
+                if (n < o.N) {
+                    const int f = o.fb[n], e = er + clean(f);
+                    double2 v = make_double2(round_sum(h[i], l[i], e), round_sum(h[BPW + i], l[BPW + i], e));
+                    if (bad || f >= F_BAD) v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
+                    if (EXPAND) {
+                        double2* at = o.out + (size_t)n * o.ldo + row;
+                        double2 x = *at;
+                        x.x += v.x;
+                        x.y += v.y;
+                        *at = x;
+                    } else {
+                        o.part[((size_t)blockIdx.z * o.M + row) * o.ldn + n] = v;
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_ALL));
+    }
+}
+
+size_t smem_bytes(int NT) { return (size_t)STAGES * (A_STAGE + S * NT * KB * 2) + 1024 + sizeof(D64Smem); }
+
+template <int NT, bool EXPAND>
+cudaError_t launch_nt(dim3 grid, const unsigned char* A, const unsigned char* B, const D64Out& o, int KT, int cps,
+                      int* err, cudaStream_t st)
+{
+    const size_t smem = smem_bytes(NT);
+    const cudaError_t e = cudaFuncSetAttribute(d64_gemm_kernel<NT, EXPAND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem);
+    if (e) return e;
+    d64_gemm_kernel<NT, EXPAND><<<grid, THREADS, smem, st>>>(A, B, o, KT, cps, idesc_f16(TM, NT, 0), err);
+    return cudaGetLastError();
+}
+
+template <bool EXPAND>
+cudaError_t launch_gemm(int NT, dim3 grid, const unsigned char* A, const unsigned char* B, const D64Out& o, int KT,
+                        int cps, int* err, cudaStream_t st)
+{
+    if (NT == 16) return launch_nt<16, EXPAND>(grid, A, B, o, KT, cps, err, st);
+    if (NT == 32) return launch_nt<32, EXPAND>(grid, A, B, o, KT, cps, err, st);
+    if (NT == 48) return launch_nt<48, EXPAND>(grid, A, B, o, KT, cps, err, st);
+    return launch_nt<64, EXPAND>(grid, A, B, o, KT, cps, err, st);
+}
+
+int sms()
+{
+    static const int n = [] {
+        int dev = 0, v = 152;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+        return v;
+    }();
+    return n;
+}
+
+// Shape of one GEMM: R result rows (A operand), N bands, K complex terms.
+struct Plan {
+    int nt, BT, tiles_n;    // B rows per tile, bands per tile, tiles
+    int n_pass;             // bands per pass
+    int KT;                 // stages over K
+    int mt, mt_chunk;       // row tiles, row tiles per A chunk
+    int cps, nz;            // chunks per split, splits
+    size_t a_bytes, b_bytes, fb_bytes;
+};
+
+Plan plan(int R, int N, int K, bool split_k)
+{
+    Plan p;
+    p.n_pass = std::min(N, N_CAP);
+    // the fewest tiles of up to 32 bands, then the narrowest tile of 8, 16, 24
+    // or 32 that holds them: the MMAs of a tile cost in proportion to its width
+    const int tiles = ceil_div(p.n_pass, 32);
+    p.BT = std::max(1, ceil_div(ceil_div(p.n_pass, tiles), 8)) * 8;
+    p.nt = 2 * p.BT;
+    p.tiles_n = ceil_div(p.n_pass, p.BT);
+    p.KT = ceil_div(2l * K, KB);
+    p.mt = ceil_div(R, TM);
+    p.mt_chunk = (int)std::max<size_t>(1, std::min<size_t>(p.mt, A_CAP / ((size_t)p.KT * A_STAGE)));
+    const int nch = ceil_div(p.KT, CHUNK);
+    p.cps = nch;
+    if (split_k) {
+        // split K over the SMs: the split count that minimises waves x (chunks + the
+        // epilogue and set-up of a CTA, about two chunks)
+        const long tiles_mn = (long)p.mt_chunk * p.tiles_n;
+        double best = 1e300;
+        for (int nz = 1; nz <= std::min(nch, 256); ++nz) {
+            const int cps = ceil_div(nch, nz), z = ceil_div(nch, cps);
+            const double t = (double)ceil_div(tiles_mn * z, sms()) * (cps + 2.0) + 0.02 * z;
+            if (t < best) { best = t; p.cps = cps; }
+        }
+    }
+    p.nz = ceil_div(nch, p.cps);
+    p.a_bytes = (size_t)p.mt_chunk * p.KT * A_STAGE;
+    p.b_bytes = (size_t)p.tiles_n * p.KT * S * p.nt * KB * 2;
+    p.fb_bytes = ((size_t)p.tiles_n * p.BT * sizeof(int) + 255) / 256 * 256;
+    return p;
+}
+
+size_t plan_bytes(const Plan& p) { return p.a_bytes + p.b_bytes + p.fb_bytes; }
+
+// rows of A in chunks against all bands, the bands in passes of N_CAP
+template <bool EXPAND>
+cudaError_t run(int R, int N, int K, const double2* A, size_t lda, D64Scale s, const double2* B, size_t ldb,
+                double2* part, double2* out, size_t ldo, unsigned char* ws, int* err, cudaStream_t st)
+{
+    const Plan p = plan(R, N, K, !EXPAND);
+    unsigned char *a = ws, *b = ws + p.a_bytes;
+    int* fb = reinterpret_cast<int*>(b + p.b_bytes);
+    for (int n0 = 0; n0 < N; n0 += p.n_pass) {
+        const int n = std::min(p.n_pass, N - n0);
+        split_b_kernel<EXPAND><<<p.tiles_n * p.BT, 512, 0, st>>>(n, K, EXPAND ? B + n0 : B + (size_t)n0 * ldb, ldb,
+                                                                 EXPAND ? s.fm : s.ek, p.KT, p.BT, b, fb);
+        for (int m = 0; m < p.mt; m += p.mt_chunk) {
+            const int mt = std::min(p.mt_chunk, p.mt - m), row0 = m * TM;
+            if (n0 == 0 || p.mt > p.mt_chunk)
+                split_a_kernel<EXPAND><<<dim3(p.KT, 2 * mt), 256, 0, st>>>(R, K, row0, A, lda, EXPAND ? s.ek : s.fm,
+                                                                           EXPAND ? s.fm : s.ek, a);
+            D64Out o{EXPAND ? nullptr : part + n0, N, EXPAND ? out + (size_t)n0 * ldo : nullptr, ldo, EXPAND ? s.ek : s.fm, fb, R, n, row0};
+            const cudaError_t e =
+                launch_gemm<EXPAND>(p.nt, dim3(p.tiles_n, mt, p.nz), a, b, o, p.KT, p.cps, err, st);
+            if (e) return e;
+        }
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t d64_scales(int M, int K, const double2* A, size_t lda, D64Scale s, cudaStream_t st)
+{
+    if (M == 0 || K == 0) return cudaSuccess;
+    cudaError_t e;
+    if ((e = cudaMemsetAsync(s.ek, 0, ((size_t)K + M) * sizeof(int), st))) return e;
+    const int gx = ceil_div(K, 128), gy = std::max(1, std::min(ceil_div(M, 8), ceil_div(16 * sms(), gx)));
+    const int mper = ceil_div(M, gy);
+    col_exp_kernel<<<dim3(gx, ceil_div(M, mper)), 128, 0, st>>>(M, K, A, lda, mper, s.ek);
+    const int kper = 8192;
+    row_exp_kernel<<<dim3(ceil_div(K, kper), M), 256, 0, st>>>(K, A, lda, s.ek, kper, s.fm);
+    return cudaGetLastError();
+}
+
+int d64_proj_splits(int M, int N, int K) { return plan(M, N, K, true).nz; }
+
+size_t d64_proj_ws(int M, int N, int K) { return plan_bytes(plan(M, N, K, true)); }
+
+size_t d64_expand_ws(int M, int N, int K) { return plan_bytes(plan(K, N, M, false)); }
+
+cudaError_t d64_proj(int M, int N, int K, const double2* A, size_t lda, D64Scale s, const double2* B, size_t ldb,
+                     double2* part, unsigned char* ws, int* err, cudaStream_t st)
+{
+    if (M == 0 || N == 0 || K == 0) return cudaSuccess;
+    return run<false>(M, N, K, A, lda, s, B, ldb, part, nullptr, 0, ws, err, st);
+}
+
+cudaError_t d64_expand(int M, int N, int K, const double2* W, size_t ldw, const double2* A, size_t lda, D64Scale s,
+                       double2* out, size_t ldo, unsigned char* ws, int* err, cudaStream_t st)
+{
+    if (M == 0 || N == 0 || K == 0) return cudaSuccess;
+    return run<true>(K, N, M, A, lda, s, W, ldw, nullptr, out, ldo, ws, err, st);
+}
+
+cudaError_t d64_set_issue_wait_limit(long polls)
+{
+    const uint32_t v = polls < 0 ? WAIT_LIMIT : (uint32_t)std::min<long>(polls, (long)WAIT_LIMIT);
+    return cudaMemcpyToSymbol(g_issue_wait_limit, &v, sizeof(v));
+}

@@ -39,6 +39,7 @@ extern "C" int hpsi_ctx_destroy(hpsi_ctx* c)
     dfree(c->d_tables); dfree(c->d_rad_nq); dfree(c->d_rad_dq); dfree(c->d_tau); dfree(c->d_v64); dfree(c->d_v32); dfree(c->d_dv32);
     dfree(c->d_tw64); dfree(c->d_tw32); dfree(c->d_err); dfree(c->d_hess);
     if (c->ws) cudaFree(c->ws);
+    if (c->d64_ws) cudaFree(c->d64_ws);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
@@ -388,7 +389,15 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
     if (grad && !c->have_dbeta) return fail(c, HPSI_ERR_STATE, "gradient needs dbeta tables for every species");
     dfree(pr);
     const bool g = grad || c->have_dbeta;  // build the derivative rows together when tables allow
-    CUDA_TRY(c, dalloc(&pr, (size_t)(g ? 4 : 1) * s.P * s.npw));
+    const size_t rows = (size_t)(g ? 4 : 1) * s.P;
+    const bool f64 = std::is_same<C, double2>::value;
+    // FP64: the digit split's exponents behind the matrix (d64_scale)
+    const size_t tail = f64 ? ((rows + s.npw) * sizeof(int) + sizeof(C) - 1) / sizeof(C) : 0;
+    CUDA_TRY(c, dalloc(&pr, rows * s.npw + tail));
+    if (f64) {
+        s.d64_exp = reinterpret_cast<int*>(pr + rows * s.npw);
+        s.d64_exp_set = false;
+    }
     const int nlm = (c->lmax + 1) * (c->lmax + 1);
     const double* yth = c->have_dbeta ? s.d_ylm + (size_t)nlm * s.npw : nullptr;
     const double* yph = c->have_dbeta ? s.d_ylm + (size_t)2 * nlm * s.npw : nullptr;
@@ -425,6 +434,136 @@ static int nonlocal_apply(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, dou
     h = c->prof.open(PH_EXPAND, st);
     CUDA_TRY(c, launch_expand_gemm<C>(s.P, nb, s.npw, W, (size_t)nb, pr, (size_t)s.npw, hpsi, (size_t)s.npw, st));
     c->prof.close(h, st);
+    return HPSI_OK;
+}
+
+// ---- FP64 nonlocal term on the tensor cores ----------------------------------
+// The exponents of slot s's projector matrix (all its rows), once per matrix.
+static int d64_scale(hpsi_ctx* c, KSlot& s, D64Scale* out, cudaStream_t st)
+{
+    *out = D64Scale{s.d64_exp, s.d64_exp + s.npw};
+    if (s.d64_exp_set) return HPSI_OK;
+    int h = c->prof.open(PH_BUILD, st);
+    CUDA_TRY(c, d64_scales((s.pr64_grad ? 4 : 1) * s.P, s.npw, s.pr64, (size_t)s.npw, *out, st));
+    c->prof.close(h, st, 2);
+    s.d64_exp_set = true;
+    return HPSI_OK;
+}
+
+// Workspace of M projector rows against nb bands: partials, W, then the operands
+// of the projection and (after it) of the expansions of P rows each
+struct D64Ws {
+    size_t part, w, ops, bytes;
+    int nz;
+};
+
+static D64Ws d64_layout(int M, int P, int nb, int npw)
+{
+    D64Ws w;
+    w.nz = d64_proj_splits(M, nb, npw);
+    Carver cv;
+    w.part = cv.take<double2>((size_t)w.nz * M * nb);
+    w.w = cv.take<double2>((size_t)M * nb);
+    w.ops = cv.off;
+    w.bytes = cv.off + std::max(d64_proj_ws(M, nb, npw), d64_expand_ws(P, nb, npw));
+    return w;
+}
+
+// As nonlocal_apply in FP64, at every shape: the SIMT GEMMs are slower down to one
+// band of the smallest cell (16 projectors, 754 plane waves: 72 against 44 us).
+// *done = false (and nothing queued) when the device's free memory leaves the call to them.
+static int nonlocal_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* hpsi, cudaStream_t st,
+                        double* e_nl, bool* done)
+{
+    *done = false;
+    if (s.P == 0) return HPSI_OK;
+    const D64Ws w = d64_layout(s.P, s.P, nb, s.npw);
+    unsigned char* ws = d64_reserve(c, w.bytes);
+    if (!ws) return HPSI_OK;
+    *done = true;
+    D64Scale sc;
+    int rc = d64_scale(c, s, &sc, st);
+    if (rc) return rc;
+    c->d64_ran = true;
+    double2* part = reinterpret_cast<double2*>(ws + w.part);
+    double2* W = reinterpret_cast<double2*>(ws + w.w);
+    int h = c->prof.open(PH_PROJ, st);
+    CUDA_TRY(c, d64_proj(s.P, nb, s.npw, s.pr64, (size_t)s.npw, sc, psi, (size_t)s.npw, part, ws + w.ops, c->d_err, st));
+    c->prof.close(h, st, 3);
+    if (e_nl) CUDA_TRY(c, launch_nl_energy<double2>(s.P, nb, w.nz, part, s.d_lam, e_nl, st));
+    h = c->prof.open(PH_REDUCE, st);
+    CUDA_TRY(c, (launch_reduce_splits<double2, double2>(s.P, nb, w.nz, part, s.d_lam, s.P, W, (size_t)nb, st)));
+    c->prof.close(h, st);
+    h = c->prof.open(PH_EXPAND, st);
+    CUDA_TRY(c, d64_expand(s.P, nb, s.npw, W, (size_t)nb, s.pr64, (size_t)s.npw, sc, hpsi, (size_t)s.npw, ws + w.ops,
+                           c->d_err, st));
+    c->prof.close(h, st, 3);
+    return HPSI_OK;
+}
+
+// The projector part of grad_device in FP64 (all 4P rows of pr64); *done as above.
+static int grad_nonlocal_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* d[3], cudaStream_t st,
+                             bool* done)
+{
+    *done = false;
+    const int M = 4 * s.P;
+    const D64Ws w = d64_layout(M, s.P, nb, s.npw);
+    unsigned char* ws = d64_reserve(c, w.bytes);
+    if (!ws) return HPSI_OK;
+    *done = true;
+    D64Scale sc;
+    int rc = d64_scale(c, s, &sc, st);
+    if (rc) return rc;
+    c->d64_ran = true;
+    const size_t npw = (size_t)s.npw, PN = (size_t)s.P * npw;
+    double2* part = reinterpret_cast<double2*>(ws + w.part);
+    double2* W = reinterpret_cast<double2*>(ws + w.w);
+    int h = c->prof.open(PH_PROJ, st);
+    CUDA_TRY(c, d64_proj(M, nb, s.npw, s.pr64, npw, sc, psi, npw, part, ws + w.ops, c->d_err, st));
+    c->prof.close(h, st, 3);
+    h = c->prof.open(PH_REDUCE, st);
+    CUDA_TRY(c, (launch_reduce_splits<double2, double2>(M, nb, w.nz, part, s.d_lam, s.P, W, (size_t)nb, st)));
+    c->prof.close(h, st);
+    for (int a = 0; a < 3; ++a) {
+        if (!d[a]) continue;
+        h = c->prof.open(PH_EXPAND, st);
+        // lambda <dp_a|psi> p, then lambda <p|psi> dp_a
+        CUDA_TRY(c, d64_expand(s.P, nb, s.npw, W + (size_t)(a + 1) * s.P * nb, (size_t)nb, s.pr64, npw, sc, d[a], npw,
+                               ws + w.ops, c->d_err, st));
+        const D64Scale sa{sc.ek, sc.fm + (size_t)(a + 1) * s.P};
+        CUDA_TRY(c, d64_expand(s.P, nb, s.npw, W, (size_t)nb, s.pr64 + (size_t)(a + 1) * PN, npw, sa, d[a], npw,
+                               ws + w.ops, c->d_err, st));
+        c->prof.close(h, st, 6);
+    }
+    return HPSI_OK;
+}
+
+// m[a][i][j] = sum_G conj(psi_i) g_a,j for the three directions (g: [3][nb][npw]); *done as above.
+static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const double2* g, double2* m,
+                        cudaStream_t st, bool* done)
+{
+    *done = false;
+    const int nz = d64_proj_splits(nb, nb, s.npw);
+    Carver cv;
+    const size_t o_part = cv.take<double2>((size_t)nz * nb * nb);
+    const size_t o_exp = cv.take<int>((size_t)s.npw + nb);
+    const size_t o_ops = cv.off;
+    unsigned char* ws = d64_reserve(c, o_ops + d64_proj_ws(nb, nb, s.npw));
+    if (!ws) return HPSI_OK;
+    *done = true;
+    c->d64_ran = true;
+    double2* part = reinterpret_cast<double2*>(ws + o_part);
+    int* ex = reinterpret_cast<int*>(ws + o_exp);
+    const D64Scale sc{ex, ex + s.npw};
+    const size_t npw = (size_t)s.npw;
+    int h = c->prof.open(PH_OTHER, st);
+    CUDA_TRY(c, d64_scales(nb, s.npw, psi, npw, sc, st));
+    for (int a = 0; a < 3; ++a) {
+        CUDA_TRY(c, d64_proj(nb, nb, s.npw, psi, npw, sc, g + (size_t)a * nb * npw, npw, part, ws + o_ops, c->d_err, st));
+        CUDA_TRY(c, (launch_reduce_splits<double2, double2>(nb, nb, nz, part, nullptr, 0, m + (size_t)a * nb * nb,
+                                                            (size_t)nb, st)));
+    }
+    c->prof.close(h, st, 14);
     return HPSI_OK;
 }
 
@@ -785,6 +924,7 @@ static int tc_grad_nonlocal(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, d
 static int check_device_flag(hpsi_ctx* c)
 {
     int v = 0;
+    c->d64_ran = false;
     CUDA_TRY(c, cudaMemcpy(&v, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
     if (v) {
         cudaMemset(c->d_err, 0, sizeof(int));
@@ -815,7 +955,7 @@ __global__ void grad_kinetic_kernel(int npw, int nb, const double* __restrict__ 
 // d_alpha += dH/dk_alpha psi, all pointers on the device
 template <typename C, typename Acc>
 static int grad_device(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* d[3], unsigned char* work,
-                       cudaStream_t st)
+                       cudaStream_t st, bool d64)
 {
     const size_t nel = (size_t)nb * s.npw;
     int h = c->prof.open(PH_OTHER, st);
@@ -825,6 +965,11 @@ static int grad_device(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double
     if (s.P == 0) return HPSI_OK;
     int rc;
     if ((rc = ensure_proj<C>(c, s, true, st))) return rc;
+    if (std::is_same<C, double2>::value && d64) {
+        bool done;
+        rc = grad_nonlocal_d64(c, s, nb, psi, d, st, &done);
+        if (rc || done) return rc;
+    }
     const C* pr = std::is_same<C, double2>::value ? (const C*)s.pr64 : (const C*)s.pr32;
     const int M = 4 * s.P;
     const int ns = split_for(M, nb, s.npw);
@@ -904,6 +1049,8 @@ static size_t apply_ws_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int prec
 }
 
 // hpsi += H psi on device pointers with an explicit workspace (prepare_slot first)
+// d64: FP64 may use the context's tensor-core workspace (false on the server's
+// lanes, which run calls of one context at the same time)
 // hpsi_ready: an event after which hpsi holds its input (an H2D copy on
 // another stream); only the tensor-core expansion reads hpsi, so only it waits
 // hpsi_apply with host buffers: hpsi arrives in two G halves [0, mid) and
@@ -921,12 +1068,17 @@ struct HostHalves {
 
 static int apply_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* hpsi, int prec, unsigned char* work,
                      cudaStream_t st, double* epart = nullptr, double* e_nl = nullptr, bool fork = true,
-                     cudaEvent_t hpsi_ready = nullptr, const HostHalves* halves = nullptr)
+                     cudaEvent_t hpsi_ready = nullptr, const HostHalves* halves = nullptr, bool d64 = true)
 {
     int rc;
     if ((rc = prepare_slot(c, s, prec, false, st))) return rc;
     if (prec == HPSI_PREC_FP64) {
         if ((rc = local_apply<double2, double>(c, s, nb, psi, hpsi, work, c->d_v64, c->d_tw64, st, epart))) return rc;
+        if (d64) {
+            bool done;
+            rc = nonlocal_d64(c, s, nb, psi, hpsi, st, e_nl, &done);
+            if (rc || done) return rc;
+        }
         return nonlocal_apply<double2, double2>(c, s, nb, psi, hpsi, s.pr64, work, st, e_nl);
     }
     if (hpsi_ready && !(is_tc(prec) && s.P > 0 && nb > 0 && fork))
@@ -1055,13 +1207,13 @@ static size_t grad_ws_bytes(const KSlot& s, int nb, int prec)
 
 // d_a += dH/dk_a psi on device pointers (NULL d_a skipped)
 static int grad_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* d[3], int prec, unsigned char* work,
-                    cudaStream_t st)
+                    cudaStream_t st, bool d64 = true)
 {
     int rc;
     if ((rc = prepare_slot(c, s, prec, true, st))) return rc;
     if (is_tc(prec)) return grad_tc(c, s, nb, psi, d, work, prec == HPSI_PREC_TC ? 0 : 1, st);
-    return prec == HPSI_PREC_FP64 ? grad_device<double2, double2>(c, s, nb, psi, d, work, st)
-                                  : grad_device<float2, float2>(c, s, nb, psi, d, work, st);
+    return prec == HPSI_PREC_FP64 ? grad_device<double2, double2>(c, s, nb, psi, d, work, st, d64)
+                                  : grad_device<float2, float2>(c, s, nb, psi, d, work, st, false);
 }
 
 // velocity workspace: G_a (3 nb npw complex128), then either the gradient's
@@ -1113,7 +1265,7 @@ static size_t vel_ws_bytes(const KSlot& s, int nb, int prec)
 
 // m[a][i][j] = sum_G conj(psi_i) (dH_a psi_j), overwritten, device pointers
 static int velocity_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* m, int prec, unsigned char* ws,
-                        cudaStream_t st)
+                        cudaStream_t st, bool d64 = true)
 {
     const size_t nel = (size_t)nb * s.npw;
     const VelWs w = vel_layout(s, nb, prec);
@@ -1121,8 +1273,13 @@ static int velocity_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, doubl
     unsigned char* rest = ws + w.rest;
     CUDA_TRY(c, cudaMemsetAsync(g, 0, 3 * nel * sizeof(double2), st));
     double2* d[3] = {g, g + nel, g + 2 * nel};
-    int rc = grad_dev(c, s, nb, psi, d, prec, rest, st);
+    int rc = grad_dev(c, s, nb, psi, d, prec, rest, st, d64);
     if (rc) return rc;
+    if (prec == HPSI_PREC_FP64 && d64) {
+        bool done;
+        rc = velocity_d64(c, s, nb, psi, g, m, st, &done);
+        if (rc || done) return rc;
+    }
     if (is_tc(prec)) {
         // tensor cores: psi rows split once, each G_a as the band operand.  Both
         // tensor-core precisions use the scaled FP16 split here: a BF16 hi + lo
@@ -1251,7 +1408,7 @@ extern "C" int hpsi_apply(hpsi_ctx* c, int kid, int nb, const double* psi_, doub
     }
     if (!dev || (flags & HPSI_SYNC)) {
         CUDA_TRY(c, cudaStreamSynchronize(st));
-        if (is_tc(prec) && (rc = check_device_flag(c))) return rc;
+        if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
     }
     return HPSI_OK;
 }
@@ -1298,7 +1455,7 @@ extern "C" int hpsi_apply_energies(hpsi_ctx* c, int kid, int nb, const double* p
     }
     if (!dev || (flags & HPSI_SYNC)) {
         CUDA_TRY(c, cudaStreamSynchronize(st));
-        if (is_tc(prec) && (rc = check_device_flag(c))) return rc;
+        if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
     }
     return HPSI_OK;
 }
@@ -1439,7 +1596,7 @@ extern "C" int hpsi_sternheimer(hpsi_ctx* c, int kid, int nv, const double* psi_
         for (int b = 0; b < nv; ++b) residual[b] = hb[b] > 0.0 ? std::sqrt(hr[b] / hb[b]) : 0.0;
     if (!dev) CUDA_TRY(c, cudaMemcpyAsync(x_, x, nel * sizeof(double2), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(c, cudaStreamSynchronize(st));
-    if (is_tc(prec) && (rc = check_device_flag(c))) return rc;
+    if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
     if (n_active > 0)
         return fail(c, HPSI_ERR_TIMEOUT, "Sternheimer CG: %d of %d bands above tol after %d iterations", n_active, nv,
                     it);
@@ -1889,7 +2046,7 @@ extern "C" int hpsi_grad_apply(hpsi_ctx* c, int kid, int nb, const double* psi_,
             if (outs[a]) CUDA_TRY(c, cudaMemcpyAsync(outs[a], d[a], nel * sizeof(double2), cudaMemcpyDeviceToHost, st));
     if (!dev || (flags & HPSI_SYNC)) {
         CUDA_TRY(c, cudaStreamSynchronize(st));
-        if (is_tc(prec) && (rc = check_device_flag(c))) return rc;
+        if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
     }
     return HPSI_OK;
 }
@@ -1928,7 +2085,7 @@ extern "C" int hpsi_velocity_matrix(hpsi_ctx* c, int kid, int nb, const double* 
     if (!dev) CUDA_TRY(c, cudaMemcpyAsync(m_, m, nm * sizeof(double2), cudaMemcpyDeviceToHost, st));
     if (!dev || (flags & HPSI_SYNC)) {
         CUDA_TRY(c, cudaStreamSynchronize(st));
-        if (is_tc(prec) && (rc = check_device_flag(c))) return rc;
+        if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
     }
     return HPSI_OK;
 }
@@ -2389,8 +2546,8 @@ static int srv_issue_one(hpsi_server* S, SrvUnit* u, cudaStream_t st)
         r->err = cudaGetErrorString(e);
         return HPSI_ERR_CUDA;
     }
-    int rc = apply_dev(c, s, j.nb, psi, hpsi, S->prec, ws, st, nullptr, nullptr, false);
-    if (!rc && j.vel) rc = velocity_dev(c, s, j.nb, psi, m, S->prec, ws, st);
+    int rc = apply_dev(c, s, j.nb, psi, hpsi, S->prec, ws, st, nullptr, nullptr, false, nullptr, nullptr, false);
+    if (!rc && j.vel) rc = velocity_dev(c, s, j.nb, psi, m, S->prec, ws, st, false);
     if (rc) { r->err = c->err; return rc; }
     return srv_copy_back(r, j, nel, hpsi, m, st);
 }
@@ -2499,7 +2656,7 @@ static int srv_issue_merged(hpsi_server* S, SrvUnit* u, cudaStream_t st)
         const hpsi_job& j = t.req->jobs[t.job];
         KSlot& s = c->slots[j.kid];
         if (j.vel) {
-            const int rc = velocity_dev(c, s, j.nb, psi + off[i], mv, S->prec, base + m.o_ws, st);
+            const int rc = velocity_dev(c, s, j.nb, psi + off[i], mv, S->prec, base + m.o_ws, st, false);
             if (rc) { t.req->err = c->err; return rc; }
         }
         const int rc = srv_copy_back(t.req, j, (size_t)j.nb * s.npw, hpsi + off[i], mv, st);

@@ -4,6 +4,7 @@
 
 #include "hpsi_gb300.h"
 #include "common.cuh"
+#include "d64_gemm.cuh"
 #include "tc_gemm.cuh"
 
 namespace {
@@ -54,5 +55,6 @@ extern "C" int hpsi_selftest_convert(const double* x, long n, float* f_bits, flo
 // watch a wait run out and the error reach the caller as HPSI_ERR_TIMEOUT.
 extern "C" int hpsi_selftest_wait_limit(long polls)
 {
-    return tc_set_issue_wait_limit(polls) == cudaSuccess ? HPSI_OK : HPSI_ERR_CUDA;
+    return tc_set_issue_wait_limit(polls) == cudaSuccess && d64_set_issue_wait_limit(polls) == cudaSuccess
+               ? HPSI_OK : HPSI_ERR_CUDA;
 }
