@@ -287,12 +287,11 @@ static int tune_group(hpsi_batch* b, Group& g)
     set_xshape(g, bk, bbb);
     if ((rc = upload_xblk(b, g))) return rc;
     // plane blocks: a candidate replaces the default block size (timed in the
-    // x-pass search above, bpt = 0) only when it is faster
+    // x-pass search above, bpt = 0) only when it is faster; the FP64 plane
+    // kernels have one size per grid
     int bpt = 0;
-    static const int kPlaneThreads64[] = {64, 128, 256, 0}, kPlaneThreads32[] = {128, 256, 512, 768};
-    const int* cand = fp64(b) ? kPlaneThreads64 : kPlaneThreads32;
-    for (int ci = 0; ci < 4 && cand[ci] > 0; ++ci) {
-        const int pt = cand[ci];
+    for (int pt : {128, 256, 512, 768}) {
+        if (fp64(b)) break;
         g.la.plane_threads = pt;
         double ms = 0.0;
         if ((rc = time_ms(b, st, reps, [&] { return launch_group_local(b, g, st); }, &ms))) return rc;

@@ -97,7 +97,7 @@ struct hpsi_ctx {
     double* d_v64 = nullptr;
     float* d_v32 = nullptr;
     float* d_dv32 = nullptr;      // V64 - V32 per grid point (the energy sums' FP64 correction)
-    double2* d_tw64 = nullptr;    // twiddles x, y, z consecutive
+    int4* d_tw64 = nullptr;       // twiddles x, y, z consecutive (Q62 words)
     float2* d_tw32 = nullptr;
     FftLen L[3];
     std::map<int, KSlot> slots;

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "ctx.cuh"
+#include "fft_q64.cuh"
 
 thread_local std::string g_last_error;
 
@@ -156,18 +157,18 @@ static int ctx_init(hpsi_ctx* c, const hpsi_system* s)
         CUDA_TRY(c, cudaMemcpy(c->d_dv32, dv32.data(), N * sizeof(float), cudaMemcpyHostToDevice));
     }
     const int ntw = c->n1 + c->n2 + c->n3;
-    std::vector<double2> tw64(ntw);
+    std::vector<int4> tw64(ntw);
     std::vector<float2> tw32(ntw);
     int o = 0;
     for (int d = 0; d < 3; ++d)
         for (int j = 0; j < ns[d]; ++j, ++o) {
             double a = 6.283185307179586476925286766559 * (double)j / (double)ns[d];
-            tw64[o] = make_double2(std::cos(a), std::sin(a));
-            tw32[o] = make_float2((float)tw64[o].x, (float)tw64[o].y);
+            tw64[o] = q62_twiddle(j, ns[d]);
+            tw32[o] = make_float2((float)std::cos(a), (float)std::sin(a));
         }
     CUDA_TRY(c, dalloc(&c->d_tw64, ntw));
     CUDA_TRY(c, dalloc(&c->d_tw32, ntw));
-    CUDA_TRY(c, cudaMemcpy(c->d_tw64, tw64.data(), ntw * sizeof(double2), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, cudaMemcpy(c->d_tw64, tw64.data(), ntw * sizeof(int4), cudaMemcpyHostToDevice));
     CUDA_TRY(c, cudaMemcpy(c->d_tw32, tw32.data(), ntw * sizeof(float2), cudaMemcpyHostToDevice));
     if (c->natom > 0) {
         CUDA_TRY(c, dalloc(&c->d_tau, (size_t)3 * c->natom));
@@ -588,7 +589,7 @@ static int chunk_bands(const KSlot& s, const hpsi_ctx* c, int nb, size_t csize)
 
 template <typename C, typename V>
 static int local_apply(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* hpsi, unsigned char* ws,
-                       const V* vloc, const C* tw, cudaStream_t st, double* epart = nullptr,
+                       const V* vloc, const Tw<C>* tw, cudaStream_t st, double* epart = nullptr,
                        float2* out32 = nullptr, unsigned* rowmax = nullptr, cudaEvent_t after_g2r = nullptr,
                        const cudaEvent_t* psi_in = nullptr, int psi_mid = 0)
 {
@@ -637,7 +638,7 @@ static size_t local_ws(const hpsi_ctx* c, const KSlot& s, int nb, size_t csize);
 // rho += sum_b occ_b |psi_b(r)|^2 on device pointers (T chunks in ws)
 template <typename C>
 static int density_apply(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const double* occ, double* rho,
-                         unsigned char* ws, const C* tw, cudaStream_t st)
+                         unsigned char* ws, const Tw<C>* tw, cudaStream_t st)
 {
     if (nb == 0 || s.npw == 0) return HPSI_OK;
     const int* pl = s.d_plane;
@@ -2195,7 +2196,7 @@ static int noalloc_nl_chunk(const KSlot& s, int nb, size_t cap)
 
 template <typename C, typename Acc, typename V>
 static int apply_noalloc_impl(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* hpsi, const C* pr,
-                              const V* vloc, const C* tw, unsigned char* scratch, cudaStream_t st)
+                              const V* vloc, const Tw<C>* tw, unsigned char* scratch, cudaStream_t st)
 {
     const size_t cap = HPSI_NOALLOC_SCRATCH_BYTES;
     Prof off;  // never records: creating events is not allowed here
@@ -2554,7 +2555,7 @@ static int srv_issue_one(hpsi_server* S, SrvUnit* u, cudaStream_t st)
 
 template <typename C, typename V>
 static cudaError_t srv_merged_launches(hpsi_ctx* c, const LocalArgs& la, const MergePlan& m, unsigned char* base,
-                                       const BGemmItem* d_gi, int n_items, const V* vloc, const C* tw, cudaStream_t st)
+                                       const BGemmItem* d_gi, int n_items, const V* vloc, const Tw<C>* tw, cudaStream_t st)
 {
     cudaError_t e = launch_local_batch<C, V>(la, m.nbands, m.max_nxs, m.nxblk, reinterpret_cast<C*>(base + m.o_T), vloc,
                                              tw, tw + c->n1, tw + c->n1 + c->n2, st);

@@ -115,15 +115,23 @@ size_t local_smem_bytes(const LocalArgs& a, bool fp64);
 // choose kt/bb of the x pass for complex size csize (bytes)
 void local_xpass_shape(LocalArgs* a, size_t csize);
 
+// Twiddle tables exp(+2 pi i j / n): complex64, or for complex128 Q62 words
+// (cos l, cos h, sin l, sin h) of the fixed-point transforms (fft_q64.cuh)
+template <typename C> struct TwOf { using type = C; };
+template <> struct TwOf<double2> { using type = int4; };
+template <typename C> using Tw = typename TwOf<C>::type;
+
 template <typename C, typename V>
 cudaError_t launch_local(const LocalArgs& a, int nb, const double2* psi, double2* hpsi, const double* kinetic, C* T,
-                         const V* vloc, const C* twx, const C* twy, const C* twz, cudaStream_t st, Prof* prof);
+                         const V* vloc, const Tw<C>* twx, const Tw<C>* twy, const Tw<C>* twz, cudaStream_t st,
+                         Prof* prof);
 // rho[i][j][k] += sum_b occ_b |psi_b(r)|^2 over nb bands (FFT in C; FP64 band
 // sums, or on the complex64 register plans compensated FP32 sums per group of
 // bands added in FP64, with part: density_part_bytes of scratch, else null)
 template <typename C>
 cudaError_t launch_density(const LocalArgs& a, int nb, const double2* psi, const double* occ, double* rho, C* T,
-                           const C* twx, const C* twy, const C* twz, cudaStream_t st, double* part = nullptr);
+                           const Tw<C>* twx, const Tw<C>* twy, const Tw<C>* twz, cudaStream_t st,
+                           double* part = nullptr);
 // scratch of the register density x pass for nb bands (0: the plan has none)
 size_t density_part_bytes(const LocalArgs& a, int nb, size_t csize);
 // x-pass line buffer bytes of a given (kt, bb) shape
@@ -132,7 +140,22 @@ size_t local_xpass_smem(const LocalArgs& a, bool fp64);
 // batch, max_nxs = largest nxs, nxblk = x-pass band blocks (a.kt, a.bb set).
 template <typename C, typename V>
 cudaError_t launch_local_batch(const LocalArgs& a, int nbands, int max_nxs, int nxblk, C* T, const V* vloc,
-                               const C* twx, const C* twy, const C* twz, cudaStream_t st);
+                               const Tw<C>* twx, const Tw<C>* twy, const Tw<C>* twz, cudaStream_t st);
+// the FP64 forms (local64.cu)
+template <>
+cudaError_t launch_local<double2, double>(const LocalArgs& a, int nb, const double2* psi, double2* hpsi,
+                                          const double* kinetic, double2* T, const double* vloc, const int4* twx,
+                                          const int4* twy, const int4* twz, cudaStream_t st, Prof* prof);
+template <>
+cudaError_t launch_local_batch<double2, double>(const LocalArgs& a, int nbands, int max_nxs, int nxblk, double2* T,
+                                                const double* vloc, const int4* twx, const int4* twy, const int4* twz,
+                                                cudaStream_t st);
+template <>
+cudaError_t launch_density<double2>(const LocalArgs& a, int nb, const double2* psi, const double* occ, double* rho,
+                                    double2* T, const int4* twx, const int4* twy, const int4* twz, cudaStream_t st,
+                                    double* part);
+size_t local64_xpass_smem(const LocalArgs& a);
+void local64_xpass_shape(LocalArgs* a);
 
 // ---- projector build (projectors.cu) --------------------------------------
 // Per G: spherical coordinates, trig, Y_lm and its angular gradients.

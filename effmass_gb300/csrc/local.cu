@@ -1,4 +1,5 @@
-// local.cu — kinetic + local-potential term of H|psi>, batched over bands.
+// local.cu — kinetic + local-potential term of H|psi>, batched over bands, in
+// complex64 (complex128: local64.cu).
 //
 // Reference: src/H_psi/hamiltonian_callable.cpp:119-182 — kinetic loop,
 // scatter of psi(G) onto the grid at (g mod n), FFT3D G2R (unnormalised,
@@ -24,18 +25,14 @@
 #include "fft_reg.cuh"
 #include "kernels.cuh"
 
-// Launch shape per precision: complex64 kernels run two 768-thread plane
-// blocks per SM and four or five x-pass blocks per SM;
-// complex128 kernels keep the register budget of one block per SM.
+// Launch shape: two 768-thread plane blocks per SM and four or five x-pass
+// blocks per SM.
 template <typename C> struct Cfg;
 template <> struct Cfg<float2> {
     // 768-thread plane blocks, two per SM (48 warps): g2r_planes fits 40
     // registers without spills; r2g_planes spills 44 bytes there and still
     // measured faster than at 512 threads (0.139 vs 0.141 ms, 64-atom cell)
     static constexpr int plane_threads = 768, g2r_threads = 768, plane_min = 2, x_min = 4;
-};
-template <> struct Cfg<double2> {
-    static constexpr int plane_threads = 256, g2r_threads = 256, plane_min = 1, x_min = 1;
 };
 
 // Plan tag of the kernels that run the runtime FFT plans
@@ -49,7 +46,7 @@ template <typename C, bool WIDE, typename PL>
 constexpr int xpass_min()
 {
     if constexpr (WIDE) return (Cfg<C>::x_min + 1) / 2;
-    else if constexpr (std::is_same<C, float2>::value && !std::is_same<PL, NoPlan>::value) return 5;
+    else if constexpr (!std::is_same<PL, NoPlan>::value) return 5;
     else return Cfg<C>::x_min;
 }
 
@@ -133,9 +130,8 @@ __global__ void __launch_bounds__(Cfg<C>::g2r_threads, WIDE ? 1 : Cfg<C>::plane_
             int j = jk / n3, k = jk - j * n3;
             const C v = from_c128<C>(ps[ig]);
             b0[j * n3p + k] = v;
-            if constexpr (std::is_same<C, float2>::value)
-                mx = max(mx, max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu));
-        } else if constexpr (std::is_same<C, float2>::value) {
+            mx = max(mx, max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu));
+        } else {
             // a G that shares its grid point with a later one: not scattered,
             // but its coefficient is still a row element of the band operand
             if (a.rowmax && !a.items) {
@@ -144,13 +140,11 @@ __global__ void __launch_bounds__(Cfg<C>::g2r_threads, WIDE ? 1 : Cfg<C>::plane_
             }
         }
     }
-    if constexpr (std::is_same<C, float2>::value) {
-        // the band operand's row scale: every G of the band is in exactly one
-        // plane, so the blocks of band b together see all of its coefficients
-        if (a.rowmax && !a.items) {
-            for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            if ((threadIdx.x & 31) == 0 && mx) atomicMax(a.rowmax + b, mx);
-        }
+    // the band operand's row scale: every G of the band is in exactly one
+    // plane, so the blocks of band b together see all of its coefficients
+    if (a.rowmax && !a.items) {
+        for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if ((threadIdx.x & 31) == 0 && mx) atomicMax(a.rowmax + b, mx);
     }
     __syncthreads();
     // z (rows of b0): intermediates in b1 then b0; output to the buffer the last stage does not read
@@ -580,28 +574,17 @@ __global__ void __launch_bounds__(256, xpass_min<C, WIDE, PL>()) x_pass(LocalArg
         }
         __syncthreads();
         for (int L = threadIdx.x; L < NL; L += blockDim.x) {
-            if constexpr (std::is_same<R, float>::value) {
-                // compensated FP32 (two-sum) in part order: GB300's FP64 rate
-                // made the FP64 version of this loop a third of the pass
-                Sum2f s1, s0;
-                for (int part = 0; part < TPL; ++part) {
-                    const int t = part * NL + L;
-                    s1.add(psum[3 * t]);
-                    s1.add(psum[3 * t + 1]);
-                    s0.add(psum[3 * t + 2]);
-                }
-                lsum[2 * L] = f2d_bits(s1.s) + f2d_bits(s1.c);
-                lsum[2 * L + 1] = f2d_bits(s0.s) + f2d_bits(s0.c);
-            } else {
-                double s1 = 0.0, s0 = 0.0;
-                for (int part = 0; part < TPL; ++part) {
-                    const int t = part * NL + L;
-                    s1 += (double)psum[3 * t] + (double)psum[3 * t + 1];
-                    s0 += (double)psum[3 * t + 2];
-                }
-                lsum[2 * L] = s1;
-                lsum[2 * L + 1] = s0;
+            // compensated FP32 (two-sum) in part order: GB300's FP64 rate
+            // made the FP64 version of this loop a third of the pass
+            Sum2f s1, s0;
+            for (int part = 0; part < TPL; ++part) {
+                const int t = part * NL + L;
+                s1.add(psum[3 * t]);
+                s1.add(psum[3 * t + 1]);
+                s0.add(psum[3 * t + 2]);
             }
+            lsum[2 * L] = f2d_bits(s1.s) + f2d_bits(s1.c);
+            lsum[2 * L + 1] = f2d_bits(s0.s) + f2d_bits(s0.c);
         }
         __syncthreads();
         double* sums = lsum;
@@ -934,39 +917,24 @@ __global__ void __launch_bounds__(Cfg<C>::plane_threads, WIDE ? 1 : Cfg<C>::plan
     const double2* ps = psi + (size_t)b * npw;
     double2* hp = hpsi + (size_t)b * npw;
     const int e0 = plane_off[p], e1 = plane_off[p + 1];
-    if constexpr (std::is_same<C, float2>::value) {
-        // complex64: kinetic*psi + grid/N in FP32 (conversions on the integer
-        // pipe), one FP64 add per component into hpsi, or stored to out32
-        const float inv_n = (float)a.inv_n;
-        float2* o32 = (a.out32 && !a.items) ? a.out32 + (size_t)b * npw : nullptr;
-        for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-            int ig = ent_ig[e] & 0x7fffffff;
-            int jk = ent_jk[e];
-            int j = jk / n3, k = jk - j * n3;
-            const float2 g = res[j * n3p + k];
-            const float2 s = to_c64(ps[ig]);
-            const float kin = d2f_bits(kinetic[ig]);
-            const float2 t = make_float2(fmaf(kin, s.x, g.x * inv_n), fmaf(kin, s.y, g.y * inv_n));
-            if (o32) {
-                o32[ig] = t;  // the tensor-core expansion adds it into hpsi
-            } else {
-                double2 h = hp[ig];
-                h.x += f2d_bits(t.x);
-                h.y += f2d_bits(t.y);
-                hp[ig] = h;
-            }
-        }
-    } else {
-        for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-            int ig = ent_ig[e] & 0x7fffffff;
-            int jk = ent_jk[e];
-            int j = jk / n3, k = jk - j * n3;
-            double2 g = as_c128(res[j * n3p + k]);
-            double2 s = ps[ig];
-            double kin = kinetic[ig];
+    // complex64: kinetic*psi + grid/N in FP32 (conversions on the integer
+    // pipe), one FP64 add per component into hpsi, or stored to out32
+    const float inv_n = (float)a.inv_n;
+    float2* o32 = (a.out32 && !a.items) ? a.out32 + (size_t)b * npw : nullptr;
+    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+        int ig = ent_ig[e] & 0x7fffffff;
+        int jk = ent_jk[e];
+        int j = jk / n3, k = jk - j * n3;
+        const float2 g = res[j * n3p + k];
+        const float2 s = to_c64(ps[ig]);
+        const float kin = d2f_bits(kinetic[ig]);
+        const float2 t = make_float2(fmaf(kin, s.x, g.x * inv_n), fmaf(kin, s.y, g.y * inv_n));
+        if (o32) {
+            o32[ig] = t;  // the tensor-core expansion adds it into hpsi
+        } else {
             double2 h = hp[ig];
-            h.x += kin * s.x + g.x * a.inv_n;
-            h.y += kin * s.y + g.y * a.inv_n;
+            h.x += f2d_bits(t.x);
+            h.y += f2d_bits(t.y);
             hp[ig] = h;
         }
     }
@@ -997,30 +965,33 @@ size_t local_smem_bytes(const LocalArgs& a, bool fp64)
     LocalArgs b = a;
     local_xpass_shape(&b, fp64 ? sizeof(double2) : sizeof(float2));
     size_t p = fp64 ? plane_smem<double2>(b) : plane_smem<float2>(b);
-    size_t x = fp64 ? xpass_smem<double2, double>(b) : xpass_smem<float2, float>(b);
+    size_t x = local_xpass_smem(b, fp64);
     return p > x ? p : x;
 }
 
 // x-pass block shape: about 48 KB of complex64 line buffers (four blocks per
-// SM) or 96 KB of complex128 ones, at most 8 z-values per block, the rest
-// filled with bands.
+// SM), at most 8 z-values per block, the rest filled with bands; complex128 as
+// local64_xpass_shape has it.
 void local_xpass_shape(LocalArgs* a, size_t csize)
 {
-    const size_t budget = csize == 8 ? 48 * 1024 : 96 * 1024;
-    int nlmax = (int)(budget / (2 * (size_t)a->n1 * csize));
-    if (nlmax < 1) nlmax = 1;
-    if (csize == 8 && nlmax >= 8 && a->n3 >= 4) {
-        // complex64: 4 z-values and a power-of-two band group (<= 16) per block,
-        // the shape the batch plans' tuner picks for the 36^3 and 72^3 grids
-        a->kt = 4;
-        int bb = 1;
-        while (bb * 2 <= nlmax / 4 && bb * 2 <= 16) bb *= 2;
-        a->bb = bb;
+    if (csize == sizeof(double2)) {
+        local64_xpass_shape(a);
     } else {
-        a->kt = nlmax < 8 ? nlmax : 8;
-        if (a->kt > a->n3) a->kt = a->n3;
-        a->bb = nlmax / a->kt;
-        if (a->bb < 1) a->bb = 1;
+        int nlmax = (int)(48 * 1024 / (2 * (size_t)a->n1 * csize));
+        if (nlmax < 1) nlmax = 1;
+        if (nlmax >= 8 && a->n3 >= 4) {
+            // 4 z-values and a power-of-two band group (<= 16) per block, the
+            // shape the batch plans' tuner picks for the 36^3 and 72^3 grids
+            a->kt = 4;
+            int bb = 1;
+            while (bb * 2 <= nlmax / 4 && bb * 2 <= 16) bb *= 2;
+            a->bb = bb;
+        } else {
+            a->kt = nlmax < 8 ? nlmax : 8;
+            if (a->kt > a->n3) a->kt = a->n3;
+            a->bb = nlmax / a->kt;
+            if (a->bb < 1) a->bb = 1;
+        }
     }
     a->nl_z = make_fastdiv((uint32_t)a->n2);
     a->nl_y = make_fastdiv((uint32_t)a->n3);
@@ -1039,7 +1010,7 @@ void local_xpass_shape(LocalArgs* a, size_t csize)
 template <typename C, typename PL>
 constexpr bool xreg_plan()
 {
-    return std::is_same<C, float2>::value && !std::is_same<PL, NoPlan>::value;
+    return !std::is_same<PL, NoPlan>::value;
 }
 
 // launch of a lane-pair plane kernel: one n x (n+1) complex64 plane per block
@@ -1153,25 +1124,23 @@ static cudaError_t with_kernels(const LocalArgs& a, F&& f)
 {
     if (fft_needs_wide(a.Lx) || fft_needs_wide(a.Ly) || fft_needs_wide(a.Lz))
         return f(std::true_type{}, NoPlan{}, IntC<0>{});
-    if constexpr (std::is_same<C, float2>::value) {
-        const int id = fft_ct_id(a.Lx);
-        if (id != FFT_CT_NONE && fft_ct_id(a.Ly) == id && fft_ct_id(a.Lz) == id) {
-            const bool k4 = a.kt == 4;
-            switch (id) {
-                case FFT_CT_72:
-                    return k4 ? f(std::false_type{}, FftPlan2<8, 9>{}, IntC<4>{})
-                              : f(std::false_type{}, FftPlan2<8, 9>{}, IntC<0>{});
-                case FFT_CT_36:
-                    return k4 ? f(std::false_type{}, FftPlan2<9, 4>{}, IntC<4>{})
-                              : f(std::false_type{}, FftPlan2<9, 4>{}, IntC<0>{});
-                case FFT_CT_24:
-                    return k4 ? f(std::false_type{}, FftPlan2<8, 3>{}, IntC<4>{})
-                              : f(std::false_type{}, FftPlan2<8, 3>{}, IntC<0>{});
-                case FFT_CT_64:
-                    return k4 ? f(std::false_type{}, FftPlan2<8, 8>{}, IntC<4>{})
-                              : f(std::false_type{}, FftPlan2<8, 8>{}, IntC<0>{});
-                default: break;
-            }
+    const int id = fft_ct_id(a.Lx);
+    if (id != FFT_CT_NONE && fft_ct_id(a.Ly) == id && fft_ct_id(a.Lz) == id) {
+        const bool k4 = a.kt == 4;
+        switch (id) {
+            case FFT_CT_72:
+                return k4 ? f(std::false_type{}, FftPlan2<8, 9>{}, IntC<4>{})
+                          : f(std::false_type{}, FftPlan2<8, 9>{}, IntC<0>{});
+            case FFT_CT_36:
+                return k4 ? f(std::false_type{}, FftPlan2<9, 4>{}, IntC<4>{})
+                          : f(std::false_type{}, FftPlan2<9, 4>{}, IntC<0>{});
+            case FFT_CT_24:
+                return k4 ? f(std::false_type{}, FftPlan2<8, 3>{}, IntC<4>{})
+                          : f(std::false_type{}, FftPlan2<8, 3>{}, IntC<0>{});
+            case FFT_CT_64:
+                return k4 ? f(std::false_type{}, FftPlan2<8, 8>{}, IntC<4>{})
+                          : f(std::false_type{}, FftPlan2<8, 8>{}, IntC<0>{});
+            default: break;
         }
     }
     return f(std::false_type{}, NoPlan{}, IntC<0>{});
@@ -1179,7 +1148,7 @@ static cudaError_t with_kernels(const LocalArgs& a, F&& f)
 
 template <typename C, typename V>
 cudaError_t launch_local_batch(const LocalArgs& a, int nbands, int max_nxs, int nxblk, C* T, const V* vloc,
-                               const C* twx, const C* twy, const C* twz, cudaStream_t st)
+                               const Tw<C>* twx, const Tw<C>* twy, const Tw<C>* twz, cudaStream_t st)
 {
     if (!a.items || a.epart) return cudaErrorInvalidValue;
     if (a.plane_threads > Cfg<C>::plane_threads || a.plane_threads % 32) return cudaErrorInvalidValue;
@@ -1230,7 +1199,7 @@ static cudaError_t launch_density_t(const LocalArgs& a, int nb, const double2* p
 
 template <typename C>
 cudaError_t launch_density(const LocalArgs& a, int nb, const double2* psi, const double* occ, double* rho, C* T,
-                           const C* twx, const C* twy, const C* twz, cudaStream_t st, double* part)
+                           const Tw<C>* twx, const Tw<C>* twy, const Tw<C>* twz, cudaStream_t st, double* part)
 {
     if (a.items || a.epart) return cudaErrorInvalidValue;
     return with_kernels<C>(a, [&](auto wide, auto pl, auto) {
@@ -1257,12 +1226,13 @@ int local_energy_slots(const LocalArgs& a, size_t csize)
 
 size_t local_xpass_smem(const LocalArgs& a, bool fp64)
 {
-    return fp64 ? xpass_smem<double2, double>(a) : xpass_smem<float2, float>(a);
+    return fp64 ? local64_xpass_smem(a) : xpass_smem<float2, float>(a);
 }
 
 template <typename C, typename V>
 cudaError_t launch_local(const LocalArgs& a, int nb, const double2* psi, double2* hpsi, const double* kinetic, C* T,
-                         const V* vloc, const C* twx, const C* twy, const C* twz, cudaStream_t st, Prof* prof)
+                         const V* vloc, const Tw<C>* twx, const Tw<C>* twy, const Tw<C>* twz, cudaStream_t st,
+                         Prof* prof)
 {
     return with_kernels<C>(a, [&](auto wide, auto pl, auto ktc) {
         return launch_local_t<C, V, decltype(wide)::value, decltype(pl), decltype(ktc)::value>(
@@ -1270,17 +1240,10 @@ cudaError_t launch_local(const LocalArgs& a, int nb, const double2* psi, double2
     });
 }
 
-template cudaError_t launch_local<double2, double>(const LocalArgs&, int, const double2*, double2*, const double*,
-                                                   double2*, const double*, const double2*, const double2*,
-                                                   const double2*, cudaStream_t, Prof*);
 template cudaError_t launch_local<float2, float>(const LocalArgs&, int, const double2*, double2*, const double*,
                                                  float2*, const float*, const float2*, const float2*, const float2*,
                                                  cudaStream_t, Prof*);
-template cudaError_t launch_local_batch<double2, double>(const LocalArgs&, int, int, int, double2*, const double*,
-                                                         const double2*, const double2*, const double2*, cudaStream_t);
 template cudaError_t launch_local_batch<float2, float>(const LocalArgs&, int, int, int, float2*, const float*,
                                                        const float2*, const float2*, const float2*, cudaStream_t);
-template cudaError_t launch_density<double2>(const LocalArgs&, int, const double2*, const double*, double*, double2*,
-                                             const double2*, const double2*, const double2*, cudaStream_t, double*);
 template cudaError_t launch_density<float2>(const LocalArgs&, int, const double2*, const double*, double*, float2*,
                                             const float2*, const float2*, const float2*, cudaStream_t, double*);

@@ -5,9 +5,10 @@
 // then y, then x: G->r unnormalised with exp(+i..), r->G with exp(-i..) and
 // 1/n per axis.  This entry point applies the same three axis passes with the
 // transforms the H|psi> kernels are built from:
-//   * complex128, and complex64 without a compile-time plan: the runtime-plan
-//     Stockham stages of fft.cuh (fft_lines_io), one line per block in shared
-//     memory;
+//   * complex128: the 64-bit fixed-point transform of fft_q64.cuh, one line per
+//     block in shared memory;
+//   * complex64 without a compile-time plan: the runtime-plan Stockham stages of
+//     fft.cuh (fft_lines_io), one line per block in shared memory;
 //   * complex64 with a compile-time plan (n1 = n2 = n3 in {24, 36, 64, 72}):
 //     the lane-pair transform of the plane kernels (fftreg::fft_pair) along z
 //     and y, and the one-thread register transform of the x pass along x.
@@ -18,6 +19,7 @@
 
 #include "hpsi_gb300.h"
 #include "fft.cuh"
+#include "fft_q64.cuh"
 #include "fft_reg.cuh"
 
 namespace {
@@ -94,6 +96,40 @@ __global__ void line_fft_reg_kernel(float2* g, int es, int lines_inner, int stri
     }
 }
 
+// the same with the fixed-point transform of the FP64 kernels
+struct LineDouble {
+    const double2* b;
+    int unit;
+    HPSI_D longlong2 operator()(int, int e) const { return q64::from_double(b[e], unit); }
+};
+
+template <bool WIDE, int SIGN>
+__global__ void line_q64_kernel(double2* g, int n, int es, int lines_inner, int stride_inner, int stride_outer, FftLen L,
+                                const int4* __restrict__ tw_g, double scale)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    longlong2 *b0 = reinterpret_cast<longlong2*>(smem_raw), *b1 = b0 + n;
+    int4* tw = reinterpret_cast<int4*>(b1 + n);
+    __shared__ int e;
+    const int line = blockIdx.x;
+    double2* p = g + (size_t)(line % lines_inner) * stride_inner + (size_t)(line / lines_inner) * stride_outer;
+    if (threadIdx.x == 0) e = q64::EXP_NONE;
+    __syncthreads();
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        const double2 v = p[(size_t)t * es];
+        reinterpret_cast<double2*>(b1)[t] = v;
+        tw[t] = tw_g[t];
+        atomicMax(&e, q64::exp_of(v));
+    }
+    __syncthreads();
+    const int unit = q64::unit_of(e, q64::headroom(n));
+    const bool inb = q64::transform<WIDE, SIGN>(LineDouble{reinterpret_cast<const double2*>(b1), unit},
+                                                q64::Lines{b0, n, 1}, q64::Lines{b1, n, 1}, L, 1, tw);
+    const longlong2* r = inb ? b1 : b0;
+    for (int t = threadIdx.x; t < n; t += blockDim.x)
+        p[(size_t)t * es] = cscale(q64::to_double(r[t], unit, e >= q64::EXP_BAD), scale);
+}
+
 template <typename C>
 std::vector<C> twiddles(int n)
 {
@@ -143,6 +179,30 @@ cudaError_t run_runtime_axis(C* d, int d_axis, int n1, int n2, int n3, int sign,
     return e;
 }
 
+cudaError_t run_q64_axis(double2* d, int d_axis, int n1, int n2, int n3, int sign, cudaStream_t st)
+{
+    const int nn[3] = {n1, n2, n3}, n = nn[d_axis];
+    FftLen L;
+    if (!fft_factor(n, &L)) return cudaErrorInvalidValue;
+    std::vector<int4> tw(n);
+    for (int j = 0; j < n; ++j) tw[j] = q62_twiddle(j, n);
+    int4* dtw = nullptr;
+    cudaError_t e = cudaMalloc(&dtw, n * sizeof(int4));
+    if (e) return e;
+    cudaMemcpy(dtw, tw.data(), n * sizeof(int4), cudaMemcpyHostToDevice);
+    int es, li, si, so;
+    axis_walk(d_axis, n1, n2, n3, &es, &li, &si, &so);
+    const int nlines = n1 * n2 * n3 / n;
+    const size_t smem = 3 * sizeof(int4) * (size_t)n;
+    auto k = fft_needs_wide(L) ? (sign > 0 ? line_q64_kernel<true, +1> : line_q64_kernel<true, -1>)
+                               : (sign > 0 ? line_q64_kernel<false, +1> : line_q64_kernel<false, -1>);
+    k<<<nlines, 128, smem, st>>>(d, n, es, li, si, so, L, dtw, sign < 0 ? 1.0 / n : 1.0);
+    e = cudaGetLastError();
+    cudaStreamSynchronize(st);
+    cudaFree(dtw);
+    return e;
+}
+
 template <typename PL>
 cudaError_t run_plan_axes(float2* d, int sign, cudaStream_t st)
 {
@@ -183,7 +243,7 @@ extern "C" int hpsi_selftest_fft3d(int n1, int n2, int n3, double* grid, int dir
         if ((e = cudaMalloc(&d, total * sizeof(double2)))) return HPSI_ERR_OOM;
         cudaMemcpy(d, grid, total * sizeof(double2), cudaMemcpyHostToDevice);
         for (int ax : {2, 1, 0})
-            if (!e) e = run_runtime_axis<double2>(d, ax, n1, n2, n3, dir, st);
+            if (!e) e = run_q64_axis(d, ax, n1, n2, n3, dir, st);
         if (!e) e = cudaMemcpy(grid, d, total * sizeof(double2), cudaMemcpyDeviceToHost);
         cudaFree(d);
         return e ? HPSI_ERR_CUDA : HPSI_OK;
