@@ -24,12 +24,20 @@
 // (projection / expansion, 2-norm): 4e-16 / 1e-16, where the FP64 SIMT GEMMs
 // have 1e-15 / 4e-16.
 //
-// What bounds it: 34 MMAs per K step of a 128 x 64 tile, so the tensor pipe on
-// large cells; operands come from L2 (84 KB of slices per 32 of K and tile).
+// What bounds it: the tensor pipe on large cells (64-atom cell, 128 bands: 72% of
+// the measured bf16 rate in the GEMMs).  The seven slices of a B tile lie one
+// after the other in shared memory and the eight diagonals in TMEM, so one MMA of
+// N = 256 multiplies slice i of A with four slices of B into four diagonals: 12
+// MMAs per 16 of K instead of 34, which the issuing thread could not feed (70
+// clocks each; projection 1.81 -> 1.43 ms, expansion 1.75 -> 1.39 ms there).
+// Reading the accumulators out costs 15% (0.22 ms of the projection).  Measured
+// and not kept: releasing the accumulators diagonal by diagonal (1.45 / 1.37 ms),
+// integers by FP32 magic adds in place of F2I (1.47 / 1.42 ms), 32 of K per stage
+// (SWIZZLE_64B, two stages).
 //
-// Layout: K-major tiles of (rows x 32) FP16 digits, slice after slice: an A tile
-// is 7 x 8 KB and a B tile 7 x NT x 64 bytes of contiguous memory, already in
-// the SWIZZLE_64B order of the MMA descriptors, so that a pipeline stage is two
+// Layout: K-major tiles of (rows x 16) FP16 digits, slice after slice: an A tile
+// is 7 x 4 KB and a B tile 7 x NT x 32 bytes of contiguous memory, already in
+// the SWIZZLE_32B order of the MMA descriptors, so that a pipeline stage is two
 // bulk copies.
 #include <algorithm>
 #include <cuda_fp16.h>
@@ -42,15 +50,14 @@ namespace {
 constexpr int S = 7;                      // slices per operand
 constexpr int ND = 8;                     // diagonals kept: i + j < ND
 constexpr int TM = 128;                   // A rows per tile
-constexpr int KB = 32;                    // real K per pipeline stage
-constexpr int CHUNK = 4;                  // stages per read-out of the accumulators (128 of K)
+constexpr int KB = 16;                    // real K per pipeline stage (one MMA deep)
+constexpr int CHUNK = 8;                  // stages per read-out of the accumulators (128 of K)
 constexpr int FIX = 55;                   // bits of the fixed-point form
-constexpr int A_STAGE = S * TM * KB * 2;  // 56 KB
-constexpr int STAGES = 2;
+constexpr int A_STAGE = S * TM * KB * 2;  // 28 KB
 constexpr int DRAIN_WARPS = 16;
 constexpr int THREADS = 64 + 32 * DRAIN_WARPS;
 constexpr uint32_t TMEM_ALL = 512;
-constexpr size_t A_CAP = 768ull << 20;    // bytes of A slices resident at once
+constexpr size_t A_CAP = 1536ull << 20;    // bytes of A slices resident at once
 constexpr int N_CAP = 256;                // bands per pass
 
 // Row and band exponents are stored with a bias, so that 0 means "no nonzero element".
@@ -106,8 +113,21 @@ __device__ __forceinline__ uint32_t slice_pair(unsigned long long u0, unsigned l
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// byte offset of 16-byte chunk c of row r within a slice (SWIZZLE_64B)
-__device__ __forceinline__ int slice_off(int r, int c) { return 64 * r + 16 * (c ^ ((r >> 1) & 3)); }
+// byte offset of 16-byte chunk c of row r within a slice (SWIZZLE_32B)
+__device__ __forceinline__ int slice_off(int r, int c) { return 32 * r + 16 * (c ^ ((r >> 2) & 1)); }
+
+// SMEM descriptor of a K-major tile in the SWIZZLE_32B layout: 8-row x 32-byte
+// atoms stacked every 256 bytes
+__device__ __forceinline__ uint64_t sdesc_sw32(uint32_t saddr)
+{
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(256 >> 4) << 32 | (uint64_t)1 << 46 |
+           (uint64_t)6 << 61;
+}
+
+// pipeline stages that fit shared memory beside the barriers
+__host__ __device__ constexpr int stage_bytes(int NT) { return A_STAGE + S * NT * KB * 2; }
+__host__ __device__ constexpr int stages(int NT) { return 220 * 1024 / stage_bytes(NT); }
+constexpr int MAX_STAGES = 8;
 
 template <int I>
 __device__ __forceinline__ void store_slices(unsigned char* at, size_t stride, const unsigned long long (&u)[8])
@@ -153,18 +173,19 @@ __global__ void row_exp_kernel(int K, const double2* __restrict__ A, size_t lda,
 
 // ---- slices -----------------------------------------------------------------
 // A rows [row0, row0 + gridDim.y * 64) of the GEMM operand, 16 complex K values
-// (one stage) per block.  TRANS = false: row r is A[r][.] (projection, scales
+// (two stages) per block.  TRANS = false: row r is A[r][.] (projection, scales
 // er = fm, ek); TRANS = true: row r is column r of A (expansion, er = ek, ek = fm).
-// A quad of lanes holds one row of a stage: 256-byte row reads (or 128-byte
-// column runs), and each slice store of a warp fills 512 contiguous bytes.
+// A quad of lanes holds one row: 256-byte row reads (or 128-byte column runs), and
+// each slice store of a warp fills two runs of 256 bytes.
 template <bool TRANS>
-__global__ void __launch_bounds__(256) split_a_kernel(int R, int K, int row0, const double2* __restrict__ A, size_t lda,
+__global__ void __launch_bounds__(256) split_a_kernel(int R, int K, int KT, int row0, const double2* __restrict__ A, size_t lda,
                                                       const int* __restrict__ er, const int* __restrict__ ek,
                                                       unsigned char* __restrict__ out)
 {
-    const int kt = blockIdx.x, KT = gridDim.x;
-    const int rl = blockIdx.y * 64 + (threadIdx.x >> 2), r = row0 + rl, c = threadIdx.x & 3;
-    const int k0 = kt * 16 + c * 4;
+    const int rl = blockIdx.y * 64 + (threadIdx.x >> 2), r = row0 + rl;
+    const int kt = blockIdx.x * 2 + ((threadIdx.x >> 1) & 1), c = threadIdx.x & 1;
+    if (kt >= KT) return;
+    const int k0 = kt * 8 + c * 4;
     unsigned long long u[8];
     const int sr = r < R ? (TRANS ? 1022 - er[r] : -clean(er[r])) : 0;
 #pragma unroll
@@ -208,12 +229,12 @@ __global__ void __launch_bounds__(512) split_b_kernel(int nb, int K, const doubl
     if (threadIdx.x == 0) fb[b] = f;
     f = clean(f);
     const size_t slice = (size_t)2 * BT * KB * 2;
-    for (int q = threadIdx.x; q < 4 * KT; q += blockDim.x) {
-        const int kt = q >> 2, c = q & 3;
+    for (int q = threadIdx.x; q < 2 * KT; q += blockDim.x) {
+        const int kt = q >> 1, c = q & 1;
         unsigned long long re[8], im[8];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int k = kt * 16 + c * 4 + i;
+            const int k = kt * 8 + c * 4 + i;
             double2 v = make_double2(0.0, 0.0);
             int sh = 0;
             if (b < nb && k < K) {
@@ -234,7 +255,7 @@ __global__ void __launch_bounds__(512) split_b_kernel(int nb, int K, const doubl
 
 // ---- GEMM -------------------------------------------------------------------
 struct D64Smem {
-    uint64_t full[STAGES], empty[STAGES];
+    uint64_t full[MAX_STAGES], empty[MAX_STAGES];
     uint64_t dfull[2], dempty[2];  // accumulator set: a chunk's products final; read out
     uint64_t done;
     uint32_t tmem_base;
@@ -283,17 +304,16 @@ __device__ __forceinline__ double round_sum(long long h, long long l, int e)
     return scalbn(x, be - 1023);
 }
 
-// TMEM columns of one accumulator, and sets of ND accumulators in TMEM
-__host__ __device__ constexpr int acc_cols(int NT) { return NT <= 32 ? 32 : 64; }
-__host__ __device__ constexpr int acc_sets(int NT) { return (int)TMEM_ALL / (ND * acc_cols(NT)); }
+// sets of ND accumulators of NT columns in TMEM
+__host__ __device__ constexpr int acc_sets(int NT) { return (int)TMEM_ALL / (ND * NT); }
 
 template <int NT, bool EXPAND>
 __global__ void __launch_bounds__(THREADS, 1)
     d64_gemm_kernel(const unsigned char* __restrict__ A, const unsigned char* __restrict__ B, D64Out o, int KT,
-                    int chunks_per_split, uint32_t idesc, int* err)
+                    int chunks_per_split, int* err)
 {
-    constexpr int B_STAGE = S * NT * KB * 2, STAGE = A_STAGE + B_STAGE, NBUF = acc_sets(NT);
-    constexpr int AC = acc_cols(NT);
+    constexpr int B_STAGE = S * NT * KB * 2, STAGE = stage_bytes(NT), STAGES = stages(NT), NBUF = acc_sets(NT);
+
     constexpr int BT = NT / 2, BPW = BT / 4, CW = BPW % 4 == 0 ? 4 : 2;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -370,19 +390,25 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
                 tc_fence_after();
                 const uint32_t st = smem_u32(tiles + s * STAGE);
-                const uint64_t ad = sdesc_sw64(st), bd = sdesc_sw64(st + A_STAGE);
+                const uint64_t ad = sdesc_sw32(st), bd = sdesc_sw32(st + A_STAGE);
                 const bool first = it == c * CHUNK;
+                // Slice i of A against slices j0 .. j0 + n - 1 of B in one MMA: their
+                // rows follow each other in shared memory, and their diagonals
+                // i + j in TMEM.  The first products of a diagonal (i = 0, and
+                // i = 1 with the last j) overwrite what the last read-out left.
+                auto mma = [&](int i, int j0, int n, bool overwrite) {
+                    tc_mma(acc + (i + j0) * NT, ad + ((i * TM * KB * 2) >> 4), bd + ((j0 * NT * KB * 2) >> 4),
+                           idesc_f16(TM, n * NT, 0), overwrite ? 0u : 1u);
+                };
+                constexpr int W = 256 / NT < S ? 256 / NT : S;  // slices per MMA
 #pragma unroll
-                for (int kk = 0; kk < KB / 16; ++kk)
+                for (int i = 0; i < S; ++i) {
+                    const int nj = S < ND - i ? S : ND - i;  // j < nj
+                    const int whole = i == 1 ? nj - 1 : nj;
 #pragma unroll
-                    for (int i = 0; i < S; ++i)
-#pragma unroll
-                        for (int j = 0; j < S && i + j < ND; ++j) {
-                            // the first pair of a diagonal overwrites what the last read-out left
-                            const bool head = kk == 0 && (i == 0 || (i == 1 && j == S - 1));
-                            tc_mma(acc + (i + j) * AC, ad + ((i * TM * KB * 2 + kk * 32) >> 4),
-                                   bd + ((j * NT * KB * 2 + kk * 32) >> 4), idesc, head && first ? 0u : 1u);
-                        }
+                    for (int j = 0; j < whole; j += W) mma(i, j, whole - j < W ? whole - j : W, i == 0 && first);
+                    if (i == 1) mma(1, nj - 1, 1, first);
+                }
                 tc_commit(&sh->empty[s]);
             }
             if (!stop) tc_commit(&sh->dfull[buf]);
@@ -412,7 +438,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t at = base + (p < BPW ? p : BT + p - BPW);
                 uint32_t v[ND][CW];
 #pragma unroll
-                for (int d = 0; d < ND; ++d) tmem_ld<CW>(at + d * AC, v[d]);
+                for (int d = 0; d < ND; ++d) tmem_ld<CW>(at + d * NT, v[d]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (p + CW >= 2 * BPW) {
                     tc_fence_before();
@@ -466,7 +492,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
 }
 
-size_t smem_bytes(int NT) { return (size_t)STAGES * (A_STAGE + S * NT * KB * 2) + 1024 + sizeof(D64Smem); }
+size_t smem_bytes(int NT) { return (size_t)stages(NT) * stage_bytes(NT) + 1024 + sizeof(D64Smem); }
 
 template <int NT, bool EXPAND>
 cudaError_t launch_nt(dim3 grid, const unsigned char* A, const unsigned char* B, const D64Out& o, int KT, int cps,
@@ -476,7 +502,7 @@ cudaError_t launch_nt(dim3 grid, const unsigned char* A, const unsigned char* B,
     const cudaError_t e = cudaFuncSetAttribute(d64_gemm_kernel<NT, EXPAND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                (int)smem);
     if (e) return e;
-    d64_gemm_kernel<NT, EXPAND><<<grid, THREADS, smem, st>>>(A, B, o, KT, cps, idesc_f16(TM, NT, 0), err);
+    d64_gemm_kernel<NT, EXPAND><<<grid, THREADS, smem, st>>>(A, B, o, KT, cps, err);
     return cudaGetLastError();
 }
 
@@ -484,9 +510,7 @@ template <bool EXPAND>
 cudaError_t launch_gemm(int NT, dim3 grid, const unsigned char* A, const unsigned char* B, const D64Out& o, int KT,
                         int cps, int* err, cudaStream_t st)
 {
-    if (NT == 16) return launch_nt<16, EXPAND>(grid, A, B, o, KT, cps, err, st);
     if (NT == 32) return launch_nt<32, EXPAND>(grid, A, B, o, KT, cps, err, st);
-    if (NT == 48) return launch_nt<48, EXPAND>(grid, A, B, o, KT, cps, err, st);
     return launch_nt<64, EXPAND>(grid, A, B, o, KT, cps, err, st);
 }
 
@@ -515,15 +539,13 @@ Plan plan(int R, int N, int K, bool split_k)
 {
     Plan p;
     p.n_pass = std::min(N, N_CAP);
-    // the fewest tiles of up to 32 bands, then the narrowest tile of 8, 16, 24
-    // or 32 that holds them: the MMAs of a tile cost in proportion to its width
-    const int tiles = ceil_div(p.n_pass, 32);
-    p.BT = std::max(1, ceil_div(ceil_div(p.n_pass, tiles), 8)) * 8;
+    p.BT = p.n_pass <= 16 ? 16 : 32;
     p.nt = 2 * p.BT;
     p.tiles_n = ceil_div(p.n_pass, p.BT);
     p.KT = ceil_div(2l * K, KB);
     p.mt = ceil_div(R, TM);
-    p.mt_chunk = (int)std::max<size_t>(1, std::min<size_t>(p.mt, A_CAP / ((size_t)p.KT * A_STAGE)));
+    const int cap = (int)std::max<size_t>(1, std::min<size_t>(p.mt, A_CAP / ((size_t)p.KT * A_STAGE)));
+    p.mt_chunk = ceil_div(p.mt, ceil_div(p.mt, cap));  // chunks of equal size
     const int nch = ceil_div(p.KT, CHUNK);
     p.cps = nch;
     if (split_k) {
@@ -561,7 +583,7 @@ cudaError_t run(int R, int N, int K, const double2* A, size_t lda, D64Scale s, c
         for (int m = 0; m < p.mt; m += p.mt_chunk) {
             const int mt = std::min(p.mt_chunk, p.mt - m), row0 = m * TM;
             if (n0 == 0 || p.mt > p.mt_chunk)
-                split_a_kernel<EXPAND><<<dim3(p.KT, 2 * mt), 256, 0, st>>>(R, K, row0, A, lda, EXPAND ? s.ek : s.fm,
+                split_a_kernel<EXPAND><<<dim3(ceil_div(p.KT, 2), 2 * mt), 256, 0, st>>>(R, K, p.KT, row0, A, lda, EXPAND ? s.ek : s.fm,
                                                                            EXPAND ? s.fm : s.ek, a);
             D64Out o{EXPAND ? nullptr : part + n0, N, EXPAND ? out + (size_t)n0 * ldo : nullptr, ldo, EXPAND ? s.ek : s.fm, fb, R, n, row0};
             const cudaError_t e =
