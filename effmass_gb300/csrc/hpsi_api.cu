@@ -934,6 +934,8 @@ static int check_device_flag(hpsi_ctx* c)
     return HPSI_OK;
 }
 
+// d_a += K_a psi, or with SET d_a = K_a psi
+template <bool SET>
 __global__ void grad_kinetic_kernel(int npw, int nb, const double* __restrict__ kvec, const double2* __restrict__ psi,
                                     double2* dx, double2* dy, double2* dz)
 {
@@ -946,7 +948,7 @@ __global__ void grad_kinetic_kernel(int npw, int nb, const double* __restrict__ 
     for (int d = 0; d < 3; ++d) {
         if (!out[d]) continue;
         double k = kvec[3 * g + d];
-        double2 o = out[d][i];
+        double2 o = SET ? make_double2(0.0, 0.0) : out[d][i];
         o.x += k * p.x;
         o.y += k * p.y;
         out[d][i] = o;
@@ -956,11 +958,12 @@ __global__ void grad_kinetic_kernel(int npw, int nb, const double* __restrict__ 
 // d_alpha += dH/dk_alpha psi, all pointers on the device
 template <typename C, typename Acc>
 static int grad_device(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* d[3], unsigned char* work,
-                       cudaStream_t st, bool d64)
+                       cudaStream_t st, bool d64, bool set)
 {
     const size_t nel = (size_t)nb * s.npw;
     int h = c->prof.open(PH_OTHER, st);
-    grad_kinetic_kernel<<<ceil_div((long)nel, 256), 256, 0, st>>>(s.npw, nb, s.d_kvec, psi, d[0], d[1], d[2]);
+    if (set) grad_kinetic_kernel<true><<<ceil_div((long)nel, 256), 256, 0, st>>>(s.npw, nb, s.d_kvec, psi, d[0], d[1], d[2]);
+    else grad_kinetic_kernel<false><<<ceil_div((long)nel, 256), 256, 0, st>>>(s.npw, nb, s.d_kvec, psi, d[0], d[1], d[2]);
     c->prof.close(h, st);
     CUDA_TRY(c, cudaGetLastError());
     if (s.P == 0) return HPSI_OK;
@@ -1007,11 +1010,12 @@ static size_t grad_ws(const KSlot& s, int nb)
 }
 
 static int grad_tc(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* d[3], unsigned char* work, int fmt,
-                   cudaStream_t st)
+                   cudaStream_t st, bool set)
 {
     const size_t nel = (size_t)nb * s.npw;
     int h = c->prof.open(PH_OTHER, st);
-    grad_kinetic_kernel<<<ceil_div((long)nel, 256), 256, 0, st>>>(s.npw, nb, s.d_kvec, psi, d[0], d[1], d[2]);
+    if (set) grad_kinetic_kernel<true><<<ceil_div((long)nel, 256), 256, 0, st>>>(s.npw, nb, s.d_kvec, psi, d[0], d[1], d[2]);
+    else grad_kinetic_kernel<false><<<ceil_div((long)nel, 256), 256, 0, st>>>(s.npw, nb, s.d_kvec, psi, d[0], d[1], d[2]);
     c->prof.close(h, st);
     CUDA_TRY(c, cudaGetLastError());
     int rc;
@@ -1206,15 +1210,15 @@ static size_t grad_ws_bytes(const KSlot& s, int nb, int prec)
     return is_tc(prec) ? tc_grad_ws(s, nb) : grad_ws<float2, float2>(s, nb);
 }
 
-// d_a += dH/dk_a psi on device pointers (NULL d_a skipped)
+// d_a += dH/dk_a psi on device pointers (NULL d_a skipped); set: d_a = dH/dk_a psi
 static int grad_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* d[3], int prec, unsigned char* work,
-                    cudaStream_t st, bool d64 = true)
+                    cudaStream_t st, bool d64 = true, bool set = false)
 {
     int rc;
     if ((rc = prepare_slot(c, s, prec, true, st))) return rc;
-    if (is_tc(prec)) return grad_tc(c, s, nb, psi, d, work, prec == HPSI_PREC_TC ? 0 : 1, st);
-    return prec == HPSI_PREC_FP64 ? grad_device<double2, double2>(c, s, nb, psi, d, work, st, d64)
-                                  : grad_device<float2, float2>(c, s, nb, psi, d, work, st, false);
+    if (is_tc(prec)) return grad_tc(c, s, nb, psi, d, work, prec == HPSI_PREC_TC ? 0 : 1, st, set);
+    return prec == HPSI_PREC_FP64 ? grad_device<double2, double2>(c, s, nb, psi, d, work, st, d64, set)
+                                  : grad_device<float2, float2>(c, s, nb, psi, d, work, st, false, set);
 }
 
 // velocity workspace: G_a (3 nb npw complex128), then either the gradient's
@@ -1272,9 +1276,8 @@ static int velocity_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, doubl
     const VelWs w = vel_layout(s, nb, prec);
     double2* g = reinterpret_cast<double2*>(ws + w.g);
     unsigned char* rest = ws + w.rest;
-    CUDA_TRY(c, cudaMemsetAsync(g, 0, 3 * nel * sizeof(double2), st));
     double2* d[3] = {g, g + nel, g + 2 * nel};
-    int rc = grad_dev(c, s, nb, psi, d, prec, rest, st, d64);
+    int rc = grad_dev(c, s, nb, psi, d, prec, rest, st, d64, true);
     if (rc) return rc;
     if (prec == HPSI_PREC_FP64 && d64) {
         bool done;
@@ -1292,7 +1295,7 @@ static int velocity_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, doubl
         unsigned* rowmax = reinterpret_cast<unsigned*>(rest + w.rowmax);
         float* part = reinterpret_cast<float*>(rest + w.part);
         int h = c->prof.open(PH_OTHER, st);
-        CUDA_TRY(c, tc_rows_operand(psi, nb, s.npw, fp16, &A, st));
+        CUDA_TRY(c, tc_rows_operand(psi, nb, s.npw, &A, rowmax, st));
         for (int a = 0; a < 3; ++a) {
             CUDA_TRY(c, tc_band_operand(d[a], nb, s.npw, fp16, &B, rowmax, st));
             CUDA_TRY(c, tc_gemm_c128(A, nb, B, nb, w.ns_tc, fp16, part, m + (size_t)a * nb * nb, c->d_err, st));

@@ -742,33 +742,10 @@ __device__ __forceinline__ float block_max(float v, float* red)
     return r;
 }
 
-// split of an FP64 value: hi from its FP32 rounding, lo from the FP64 remainder
-template <typename T>
-__device__ __forceinline__ void split_store_d(double x, T* hi, T* lo);
-template <>
-__device__ __forceinline__ void split_store_d<__half>(double x, __half* hi, __half* lo)
-{
-    __half h = __float2half_rn((float)x);
-    *hi = h;
-    *lo = __float2half_rn((float)(x - (double)__half2float(h)));
-}
-template <>
-__device__ __forceinline__ void split_store_d<__nv_bfloat16>(double x, __nv_bfloat16* hi, __nv_bfloat16* lo)
-{
-    __nv_bfloat16 h = __float2bfloat16_rn((float)x);
-    *hi = h;
-    *lo = __float2bfloat16_rn((float)(x - (double)__bfloat162float(h)));
-}
-
 __device__ __forceinline__ void split_any(float x, float sc, __half* h, __half* l) { split_store<__half>(x * sc, h, l); }
 __device__ __forceinline__ void split_any(float x, float sc, __nv_bfloat16* h, __nv_bfloat16* l)
 {
     split_store<__nv_bfloat16>(x * sc, h, l);
-}
-__device__ __forceinline__ void split_any(double x, float sc, __half* h, __half* l) { split_store_d<__half>(x * sc, h, l); }
-__device__ __forceinline__ void split_any(double x, float sc, __nv_bfloat16* h, __nv_bfloat16* l)
-{
-    split_store_d<__nv_bfloat16>(x * sc, h, l);
 }
 
 // Projection A: row p of a complex matrix (complex64 Pr or complex128 psi,
@@ -868,17 +845,24 @@ __device__ __forceinline__ uint32_t abs_key(double x)
 }
 __device__ __forceinline__ uint32_t abs_key(float x) { return __float_as_uint(x) & 0x7fffffffu; }
 
+constexpr int MAX_PER = 8;  // elements per thread of the band maxima
+
 template <typename S, bool FROM_W>
-__global__ void band_max_kernel(const S* __restrict__ src, int nb, int len, unsigned* rowmax)
+__global__ void __launch_bounds__(256) band_max_kernel(const S* __restrict__ src, int nb, int len, unsigned* rowmax)
 {
     const int b = blockIdx.y;
+    const int i0 = blockIdx.x * (MAX_PER * 256) + threadIdx.x;
     uint32_t mx = 0u;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
-        const S v = FROM_W ? src[(size_t)i * nb + b] : src[(size_t)b * len + i];
-        mx = max(mx, max(abs_key(v.x), abs_key(v.y)));
+#pragma unroll
+    for (int u = 0; u < MAX_PER; ++u) {  // independent loads: the pass is bound by their latency otherwise
+        const int i = i0 + u * 256;
+        if (i < len) {
+            const S v = FROM_W ? src[(size_t)i * nb + b] : src[(size_t)b * len + i];
+            mx = max(mx, max(abs_key(v.x), abs_key(v.y)));
+        }
     }
     for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(rowmax + b, mx);
+    if ((threadIdx.x & 31) == 0 && mx) atomicMax(rowmax + b, mx);
 }
 
 template <typename T>
@@ -945,11 +929,76 @@ static void band_rows(const S* src, int nb, int len, size_t ldk, T* hi, T* lo, f
 {
     if (!have_max) {
         cudaMemsetAsync(rowmax, 0, sizeof(unsigned) * nb, st);
-        const int chunks = min(64, ceil_div(len, 256 * 4));
-        band_max_kernel<S, FROM_W><<<dim3(chunks, nb), 256, 0, st>>>(src, nb, len, rowmax);
+        band_max_kernel<S, FROM_W><<<dim3(ceil_div(len, 256 * MAX_PER), nb), 256, 0, st>>>(src, nb, len, rowmax);
     }
     band_write_kernel<T, S, FROM_W><<<dim3(ceil_div((long)(ldk / 4), 256), nb), 256, 0, st>>>(
         src, nb, len, ldk, hi, lo, inv_scale, rowmax, fp16);
+}
+
+// ---- complex128 row operand (the psi rows of the band-pair GEMMs) ------------
+// |x| rounded to float as its bits
+__device__ __forceinline__ uint32_t float_key(double x) { return __float_as_uint(d2f_bits(x)) & 0x7fffffffu; }
+
+__global__ void __launch_bounds__(256) row_max_kernel(const double2* __restrict__ src, int len, unsigned* rowmax)
+{
+    const double2* row = src + (size_t)blockIdx.y * len;
+    const int i0 = blockIdx.x * (MAX_PER * 256) + threadIdx.x;
+    uint32_t mx = 0u;
+#pragma unroll
+    for (int u = 0; u < MAX_PER; ++u) {
+        const int i = i0 + u * 256;
+        if (i < len) mx = max(mx, max(float_key(row[i].x), float_key(row[i].y)));
+    }
+    for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((threadIdx.x & 31) == 0 && mx) atomicMax(rowmax + blockIdx.y, mx);
+}
+
+// hi + lo pieces of y = x 2^s without FP64 instructions: hi from the FP32 rounding f
+// of y, lo from (f - hi) + (y - f), the second difference (the 29 bits that f
+// drops) taken from the bit pattern.  The same pieces as from y - hi in FP64
+// unless two roundings tie.
+__device__ __forceinline__ void split_row_value(double x, int s, __half& hi, __half& lo)
+{
+    uint32_t w = (uint32_t)__double2hiint(x);
+    const uint32_t l = (uint32_t)__double2loint(x);
+    const int ex = (int)((w >> 20) & 0x7ffu), e = ex + s;
+    if (e < 1023 - 60 || ex == 0x7ff) {  // below half of every FP16 value; infinities and NaN stay
+        hi = lo = __float2half_rn(ex == 0x7ff ? (float)x : 0.f);
+        return;
+    }
+    w = (w & 0x800fffffu) | ((uint32_t)e << 20);
+    const float f = d2f_bits(__hiloint2double((int)w, (int)l));
+    // the dropped bits, negative when f was rounded up: units 2^(e - 1023 - 52)
+    int r = (int)(l & 0x1fffffffu);
+    const uint32_t trunc = __funnelshift_l(l, w, 3) + 0x40000000u;
+    if (((__float_as_uint(f) ^ trunc) & 0x7fffffffu) != 0u) r -= 0x20000000;
+    const float unit = __uint_as_float((uint32_t)(e - 1023 - 52 + 127) << 23 | (w & 0x80000000u));
+    hi = __float2half_rn(f);
+    lo = __float2half_rn((f - __half2float(hi)) + (float)r * unit);
+}
+
+// row p of x, two complex elements (k = 4q .. 4q+3) per thread
+__global__ void __launch_bounds__(256) row_write_kernel(const double2* __restrict__ src, int len, size_t ldk, __half* hi,
+                                                        __half* lo, float* inv_scale,
+                                                        const unsigned* __restrict__ rowmax)
+{
+    const int p = blockIdx.y;
+    const float sc = row_scale(__uint_as_float(rowmax[p]), true);
+    if (blockIdx.x == 0 && threadIdx.x == 0) inv_scale[p] = 1.f / sc;
+    const int s = (int)((__float_as_uint(sc) >> 23) & 0xffu) - 127;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t k = 4 * (size_t)q;
+    if (k >= ldk) return;
+    __align__(8) __half h[4], l[4];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const double2 v = 2 * q + e < len ? src[(size_t)p * len + 2 * q + e] : make_double2(0.0, 0.0);
+        split_row_value(v.x, s, h[2 * e], l[2 * e]);
+        split_row_value(v.y, s, h[2 * e + 1], l[2 * e + 1]);
+    }
+    const size_t o = tile_off(p, k, ldk);
+    *reinterpret_cast<uint2*>(hi + o) = *reinterpret_cast<const uint2*>(h);
+    *reinterpret_cast<uint2*>(lo + o) = *reinterpret_cast<const uint2*>(l);
 }
 
 // rows of bands missing from the last 128-block: zero hi/lo, unit scale
@@ -1000,10 +1049,31 @@ __global__ void proj_reduce_kernel(int P, int nb, int N, int nsplit, const float
         }
         return;
     }
+    // complex128: two-float sums of 16 splits, folded in FP64 (an FP64 add per
+    // split was bound by the FP64 pipe: 168 -> 30 us for 256 x 256 over 290 splits)
     double sr = 0.0, si = 0.0;
-    for (int z = 0; z < nsplit; ++z) {
-        sr += pre[z * zs];
-        si += pim[z * zs];
+    for (int z0 = 0; z0 < nsplit; z0 += 16) {
+        Sum2f re, im;
+        if (z0 + 16 <= nsplit) {
+            float a[16], c[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                a[u] = pre[(z0 + u) * zs];
+                c[u] = pim[(z0 + u) * zs];
+            }
+#pragma unroll
+            for (int u = 0; u < 16; ++u) {
+                re.add(a[u]);
+                im.add(c[u]);
+            }
+        } else {
+            for (int z = z0; z < nsplit; ++z) {
+                re.add(pre[z * zs]);
+                im.add(pim[z * zs]);
+            }
+        }
+        sr += f2d_bits(re.s) + f2d_bits(re.c);
+        si += f2d_bits(im.s) + f2d_bits(im.c);
     }
     const double f = lam ? lam[p % period] : 1.0;
     W[idx] = from_c128<CW>(make_double2(f * sr, f * si));
@@ -1227,15 +1297,14 @@ cudaError_t tc_projection(const TcOperand& A, int P, const TcOperand& B, int nb,
     return cudaGetLastError();
 }
 
-cudaError_t tc_rows_operand(const double2* x, int rows, int npw, bool fp16, TcOperand* A, cudaStream_t st)
+cudaError_t tc_rows_operand(const double2* x, int rows, int npw, TcOperand* A, unsigned* rowmax, cudaStream_t st)
 {
     if (rows == 0) return cudaSuccess;
-    if (fp16)
-        split_rows_kernel<__half, double2><<<rows, 256, 0, st>>>(x, npw, A->ldk, (__half*)A->hi, (__half*)A->lo,
-                                                                 A->inv_scale, true);
-    else
-        split_rows_kernel<__nv_bfloat16, double2><<<rows, 256, 0, st>>>(x, npw, A->ldk, (__nv_bfloat16*)A->hi,
-                                                                        (__nv_bfloat16*)A->lo, A->inv_scale, false);
+    cudaError_t e = cudaMemsetAsync(rowmax, 0, sizeof(unsigned) * rows, st);
+    if (e) return e;
+    row_max_kernel<<<dim3(ceil_div(npw, 256 * MAX_PER), rows), 256, 0, st>>>(x, npw, rowmax);
+    row_write_kernel<<<dim3(ceil_div((long)(A->ldk / 4), 256), rows), 256, 0, st>>>(
+        x, npw, A->ldk, (__half*)A->hi, (__half*)A->lo, A->inv_scale, rowmax);
     return cudaGetLastError();
 }
 
@@ -1252,7 +1321,7 @@ cudaError_t tc_gemm_c128(const TcOperand& A, int M, const TcOperand& B, int nb, 
     const int ktiles = (int)(A.ldk / BK);
     const int per = ceil_div(ktiles, nsplit);
     const int nz = ceil_div(ktiles, per);
-    proj_reduce_kernel<double2><<<ceil_div((long)M * nb, 256), 256, 0, st>>>(M, nb, N, nz, part, nullptr, 1, out);
+    proj_reduce_kernel<double2><<<ceil_div((long)M * nb, 64), 64, 0, st>>>(M, nb, N, nz, part, nullptr, 1, out);
     return cudaGetLastError();
 }
 

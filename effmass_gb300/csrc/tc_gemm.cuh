@@ -80,8 +80,9 @@ cudaError_t tc_w_operand(const float2* W, int P, int nb, bool fp16, TcOperand* B
 cudaError_t tc_projection(const TcOperand& A, int P, const TcOperand& B, int nb, int nsplit, bool fp16, float* part,
                           const double* lam, int period, float2* W, int* err, cudaStream_t st, Prof* prof,
                           double* eterm = nullptr, double* e_nl = nullptr, const TcGen* gen = nullptr);
-// Row operand [rows][2npw] of a complex128 matrix (psi), for conj(A) B^T GEMMs
-cudaError_t tc_rows_operand(const double2* x, int rows, int npw, bool fp16, TcOperand* A, cudaStream_t st);
+// Row operand [rows][2npw] (FP16 split) of a complex128 matrix (psi), for conj(A) B^T
+// GEMMs; rowmax: rows scratch words
+cudaError_t tc_rows_operand(const double2* x, int rows, int npw, TcOperand* A, unsigned* rowmax, cudaStream_t st);
 // out[m][n] = sum_G conj(A[m][G]) B[n][G] in complex128 (B a band operand of nb rows)
 cudaError_t tc_gemm_c128(const TcOperand& A, int M, const TcOperand& B, int nb, int nsplit, bool fp16, float* part,
                          double2* out, int* err, cudaStream_t st);
