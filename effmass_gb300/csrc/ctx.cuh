@@ -110,7 +110,7 @@ struct hpsi_ctx {
     bool d64_ran = false;         // d_err is checked at the next synchronising call
     Prof prof;
     int* d_err = nullptr;         // device-side error flag of the bounded waits (tcgen05 GEMMs)
-    // side stream of the tensor-core H|psi>: the projection chain runs there
+    // side stream of the FP64 and tensor-core H|psi>: the projection chain runs there
     // beside the FFT passes (fork/join by events on the caller's stream)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

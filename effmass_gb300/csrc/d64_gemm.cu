@@ -142,6 +142,8 @@ __device__ __forceinline__ void store_slices(unsigned char* at, size_t stride, c
 }
 
 // ---- scales -----------------------------------------------------------------
+__device__ __forceinline__ int ceil_div_d(int a, int b) { return (a + b - 1) / b; }
+
 __global__ void col_exp_kernel(int M, int K, const double2* __restrict__ A, size_t lda, int mper, int* ek)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -172,64 +174,123 @@ __global__ void row_exp_kernel(int K, const double2* __restrict__ A, size_t lda,
 }
 
 // ---- slices -----------------------------------------------------------------
-// A rows [row0, row0 + gridDim.y * 64) of the GEMM operand, 16 complex K values
-// (two stages) per block.  TRANS = false: row r is A[r][.] (projection, scales
-// er = fm, ek); TRANS = true: row r is column r of A (expansion, er = ek, ek = fm).
-// A quad of lanes holds one row: 256-byte row reads (or 128-byte column runs), and
-// each slice store of a warp fills two runs of 256 bytes.
+// K index k of a GEMM -> row of A and row of W.  The expansion of dH/dk_a joins two
+// blocks of rows into one K: k < split: p rows against <d_a p|psi>, then d_a p
+// rows against <p|psi>.
+struct KMap {
+    int split, a1, w0, w1;
+    __device__ __forceinline__ int a(int k) const { return k < split ? k : k + a1; }
+    __device__ __forceinline__ int w(int k) const { return k < split ? k + w0 : k + w1; }
+};
+
+// Operands of nd GEMMs (the directions of an expansion; 1 for a projection)
+struct SplitArgs {
+    const double2 *A, *B;
+    size_t lda, ldb;
+    const int *ek, *fm;     // exponents of A's columns and rows
+    int R, row0;            // rows of the GEMM's A operand; first of this chunk
+    int nb, K, KT, BT;      // bands, complex K, stages, bands per tile
+    int a_x, a_blocks;      // A blocks per row of blocks, per GEMM
+    int b_seg, b_blocks;    // B blocks per band, per GEMM
+    unsigned char *a, *b;   // slices, nd times a_bytes / b_bytes
+    size_t a_bytes, b_bytes;
+    int* fb;                // [nd][bands padded to tiles]
+    KMap map[3];
+};
+
+// One stage holds 8 complex K values.  TRANS = false: the projection (A row r is
+// A[r][.], scales fm and ek; B row b is B[b][.]); TRANS = true: the expansion (A row
+// r is column r of A, scales ek and fm; band b is column b of W).
+
+// 64 rows x 16 K values of A.  A quad of lanes holds one row: 256-byte row reads (or
+// 128-byte column runs), and each slice store of a warp fills two runs of 256 bytes.
 template <bool TRANS>
-__global__ void __launch_bounds__(256) split_a_kernel(int R, int K, int KT, int row0, const double2* __restrict__ A, size_t lda,
-                                                      const int* __restrict__ er, const int* __restrict__ ek,
-                                                      unsigned char* __restrict__ out)
+__device__ __forceinline__ void split_a(const SplitArgs& s, int g, int block)
 {
-    const int rl = blockIdx.y * 64 + (threadIdx.x >> 2), r = row0 + rl;
-    const int kt = blockIdx.x * 2 + ((threadIdx.x >> 1) & 1), c = threadIdx.x & 1;
-    if (kt >= KT) return;
+    const int bx = block % s.a_x, by = block / s.a_x;
+    const int rl = by * 64 + (threadIdx.x >> 2), r = s.row0 + rl;
+    const int kt = bx * 2 + ((threadIdx.x >> 1) & 1), c = threadIdx.x & 1;
+    if (kt >= s.KT) return;
     const int k0 = kt * 8 + c * 4;
+    const KMap map = s.map[g];
     unsigned long long u[8];
-    const int sr = r < R ? (TRANS ? 1022 - er[r] : -clean(er[r])) : 0;
+    double2 v[4];
+    int sk[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int k = k0 + i;
-        double2 v = make_double2(0.0, 0.0);
-        int sk = 0;
-        if (r < R && k < K) {
-            v = TRANS ? A[(size_t)k * lda + r] : A[(size_t)r * lda + k];
-            sk = TRANS ? -clean(ek[k]) : 1022 - ek[k];
+        v[i] = make_double2(0.0, 0.0);
+        sk[i] = 0;
+        if (r < s.R && k < s.K) {
+            const int ka = TRANS ? map.a(k) : k;
+            v[i] = TRANS ? s.A[(size_t)ka * s.lda + r] : s.A[(size_t)r * s.lda + ka];
+            sk[i] = TRANS ? -clean(s.fm[ka]) : 1022 - s.ek[ka];
         }
-        u[2 * i] = fixed_digits(v.x, FIX + sr + sk);
-        u[2 * i + 1] = fixed_digits(v.y, FIX + sr + sk);
     }
-    unsigned char* tile = out + ((size_t)(rl >> 7) * KT + kt) * A_STAGE;
+    const int sr = FIX + (r < s.R ? (TRANS ? 1022 - s.ek[r] : -clean(s.fm[r])) : 0);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        u[2 * i] = fixed_digits(v[i].x, sr + sk[i]);
+        u[2 * i + 1] = fixed_digits(v[i].y, sr + sk[i]);
+    }
+    unsigned char* tile = s.a + g * s.a_bytes + ((size_t)(rl >> 7) * s.KT + kt) * A_STAGE;
     store_slices<0>(tile + slice_off(rl & 127, c), TM * KB * 2, u);
 }
 
-// B rows of one band per block: band b of tile t = b / BT sits in rows j = b % BT
-// (real part of the result) and BT + j (imaginary part).  TRANS = false: src[b][k],
-// the projection's rows (b_r, b_i) and (b_i, -b_r) for conj(A) B; TRANS = true:
-// src[k][b], the expansion's rows (W_r, -W_i) and (W_i, W_r).  First the band's
-// exponent fb, then the digits.  Bands past nb are zero.
 template <bool TRANS>
-__global__ void __launch_bounds__(512) split_b_kernel(int nb, int K, const double2* __restrict__ src, size_t ld,
-                                                      const int* __restrict__ ek, int KT, int BT,
-                                                      unsigned char* __restrict__ out, int* __restrict__ fb)
+__device__ __forceinline__ int band_exp(const SplitArgs& s, const KMap& map, int b, int k)
 {
-    __shared__ int red[16];
-    const int b = blockIdx.x, t = b / BT, j = b % BT;
+    const double2 v = TRANS ? s.B[(size_t)map.w(k) * s.ldb + b] : s.B[(size_t)b * s.ldb + k];
+    const int e = exp_of(v);
+    return e < 0 ? 0 : e == 0x7ff ? F_BAD : e - 1022 + (TRANS ? clean(s.fm[map.a(k)]) : s.ek[k] - 1022) + F_BIAS;
+}
+
+// Exponents fb of the bands of long K, over blocks of B_SEG values
+constexpr int B_SEG = 4096;
+template <bool TRANS>
+__global__ void __launch_bounds__(256) band_exp_kernel(SplitArgs s, int bands)
+{
+    const int b = blockIdx.y, g = blockIdx.z, k1 = min(s.K, (int)(blockIdx.x + 1) * B_SEG);
+    if (b >= s.nb) return;
     int f = 0;
-    if (b < nb)
-        for (int k = threadIdx.x; k < K; k += blockDim.x) {
-            const int e = exp_of(TRANS ? src[(size_t)k * ld + b] : src[(size_t)b * ld + k]);
-            if (e >= 0) f = max(f, e == 0x7ff ? F_BAD : e - 1022 + (TRANS ? clean(ek[k]) : ek[k] - 1022) + F_BIAS);
-        }
+#pragma unroll 4
+    for (int k = blockIdx.x * B_SEG + threadIdx.x; k < k1; k += 256) f = max(f, band_exp<TRANS>(s, s.map[g], b, k));
     f = __reduce_max_sync(0xffffffffu, f);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = f;
-    __syncthreads();
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) f = max(f, red[i]);
-    if (threadIdx.x == 0) fb[b] = f;
+    if ((threadIdx.x & 31) == 0 && f) atomicMax(s.fb + g * bands + b, f);
+}
+
+// B rows of one band (or B_SEG of its K values): band b of tile t = b / BT sits in
+// rows j = b % BT (real part of the result) and BT + j (imaginary part).  The
+// projection's rows are (b_r, b_i) and (b_i, -b_r), for conj(A) B; the expansion's
+// (W_r, -W_i) and (W_i, W_r).  Short K: the block takes the band's exponent
+// first.  Bands past nb are zero.
+template <bool TRANS>
+__device__ __forceinline__ void split_b(const SplitArgs& s, int g, int block)
+{
+    __shared__ int red[8];
+    const int bands = s.b_blocks / s.b_seg, b = block % bands, seg = block / bands, t = b / s.BT, j = b % s.BT;
+    const KMap map = s.map[g];
+    int f = 0;
+    if (s.b_seg == 1) {
+        if (b < s.nb) {
+#pragma unroll 4
+            for (int k = threadIdx.x; k < s.K; k += 256) f = max(f, band_exp<TRANS>(s, map, b, k));
+        }
+        f = __reduce_max_sync(0xffffffffu, f);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = f;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f = max(f, red[i]);
+        if (threadIdx.x == 0) s.fb[g * bands + b] = f;
+    } else if (b < s.nb) {
+        f = s.fb[g * bands + b];
+    }
     f = clean(f);
-    const size_t slice = (size_t)2 * BT * KB * 2;
-    for (int q = threadIdx.x; q < 2 * KT; q += blockDim.x) {
+    const size_t slice = (size_t)2 * s.BT * KB * 2;
+    unsigned char* out = s.b + g * s.b_bytes + (size_t)t * s.KT * S * slice;
+    const int per = s.b_seg == 1 ? 2 * s.KT : B_SEG / 4, q1 = min(2 * s.KT, (seg + 1) * per);
+#pragma unroll 2
+    for (int q = seg * per + threadIdx.x; q < q1; q += 256) {
         const int kt = q >> 1, c = q & 1;
         unsigned long long re[8], im[8];
 #pragma unroll
@@ -237,9 +298,9 @@ __global__ void __launch_bounds__(512) split_b_kernel(int nb, int K, const doubl
             const int k = kt * 8 + c * 4 + i;
             double2 v = make_double2(0.0, 0.0);
             int sh = 0;
-            if (b < nb && k < K) {
-                v = TRANS ? src[(size_t)k * ld + b] : src[(size_t)b * ld + k];
-                sh = FIX - f + (TRANS ? clean(ek[k]) : ek[k] - 1022);
+            if (b < s.nb && k < s.K) {
+                v = TRANS ? s.B[(size_t)map.w(k) * s.ldb + b] : s.B[(size_t)b * s.ldb + k];
+                sh = FIX - f + (TRANS ? clean(s.fm[map.a(k)]) : s.ek[k] - 1022);
             }
             const unsigned long long x = fixed_digits(v.x, sh), y = fixed_digits(v.y, sh);
             re[2 * i] = x;
@@ -247,10 +308,19 @@ __global__ void __launch_bounds__(512) split_b_kernel(int nb, int K, const doubl
             im[2 * i] = y;
             im[2 * i + 1] = TRANS ? x : 2 * DIGIT_BIAS - x;
         }
-        unsigned char* tile = out + ((size_t)t * KT + kt) * S * slice;
+        unsigned char* tile = out + (size_t)kt * S * slice;
         store_slices<0>(tile + slice_off(j, c), slice, re);
-        store_slices<0>(tile + slice_off(BT + j, c), slice, im);
+        store_slices<0>(tile + slice_off(s.BT + j, c), slice, im);
     }
+}
+
+// both operands of a GEMM in one launch, B's blocks first (they take longest)
+template <bool TRANS>
+__global__ void __launch_bounds__(256) split_kernel(SplitArgs s)
+{
+    const int block = blockIdx.x, g = blockIdx.y;
+    if (block < s.b_blocks) split_b<TRANS>(s, g, block);
+    else split_a<TRANS>(s, g, block - s.b_blocks);
 }
 
 // ---- GEMM -------------------------------------------------------------------
@@ -265,8 +335,10 @@ struct D64Smem {
 struct D64Out {
     double2* part;   // projection: [z][M][ldn], first band of the pass
     int ldn;
-    double2* out;    // expansion: [N][ldo], +=
+    double2* out[3]; // expansion: [N][ldo] of each GEMM, +=
     size_t ldo;
+    size_t a_bytes, b_bytes;  // operands of one GEMM
+    int bands;       // column exponents of one GEMM
     const int* er;   // row exponents (fm, or ek with bias)
     const int* fb;   // column exponents
     int M, N, row0;  // result rows and bands; first row of this launch's A chunk
@@ -320,7 +392,9 @@ __global__ void __launch_bounds__(THREADS, 1)
     unsigned char* tiles = smem_raw + (((raw + 1023u) & ~1023u) - raw);
     D64Smem* sh = reinterpret_cast<D64Smem*>(tiles + STAGES * STAGE);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kt0 = blockIdx.z * chunks_per_split * CHUNK, kt1 = min(KT, kt0 + chunks_per_split * CHUNK);
+    // blockIdx.z: the K split of a projection, the GEMM of an expansion
+    const int z = EXPAND ? 0 : blockIdx.z, gemm = EXPAND ? blockIdx.z : 0;
+    const int kt0 = z * chunks_per_split * CHUNK, kt1 = min(KT, kt0 + chunks_per_split * CHUNK);
     const int nk = kt1 - kt0, nchunk = (nk + CHUNK - 1) / CHUNK;
 
     if (threadIdx.x == 0) {
@@ -349,8 +423,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     if (warp == 0 && lane == 0) {
         // ---- bulk copies: one A tile and one B tile per stage
-        const unsigned char* a = A + ((size_t)blockIdx.y * KT + kt0) * A_STAGE;
-        const unsigned char* b = B + ((size_t)blockIdx.x * KT + kt0) * B_STAGE;
+        const unsigned char* a = A + gemm * o.a_bytes + ((size_t)blockIdx.y * KT + kt0) * A_STAGE;
+        const unsigned char* b = B + gemm * o.b_bytes + ((size_t)blockIdx.x * KT + kt0) * B_STAGE;
         int issued = 0;
         for (int it = 0; it < nk; ++it) {
             const int s = it % STAGES;
@@ -459,6 +533,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         }
         const int row = o.row0 + blockIdx.y * TM + q * 32 + lane;
+        double2* out = gemm == 0 ? o.out[0] : gemm == 1 ? o.out[1] : o.out[2];
         if (go && row < o.M) {
             // h counts diagonal 3, l diagonal 6: weights 2^(72 - 110) and 2^(48 - 110)
             const int fr = o.er[row];
@@ -468,11 +543,11 @@ __global__ void __launch_bounds__(THREADS, 1)
             for (int i = 0; i < BPW; ++i) {
                 const int n = blockIdx.x * BT + sub * BPW + i;
                 if (n < o.N) {
-                    const int f = o.fb[n], e = er + clean(f);
+                    const int f = o.fb[gemm * o.bands + n], e = er + clean(f);
                     double2 v = make_double2(round_sum(h[i], l[i], e), round_sum(h[BPW + i], l[BPW + i], e));
                     if (bad || f >= F_BAD) v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
                     if (EXPAND) {
-                        double2* at = o.out + (size_t)n * o.ldo + row;
+                        double2* at = out + (size_t)n * o.ldo + row;
                         double2 x = *at;
                         x.x += v.x;
                         x.y += v.y;
@@ -533,9 +608,10 @@ struct Plan {
     int mt, mt_chunk;       // row tiles, row tiles per A chunk
     int cps, nz;            // chunks per split, splits
     size_t a_bytes, b_bytes, fb_bytes;
+    int ng;                 // GEMMs run together
 };
 
-Plan plan(int R, int N, int K, bool split_k)
+Plan plan(int R, int N, int K, bool split_k, int ng)
 {
     Plan p;
     p.n_pass = std::min(N, N_CAP);
@@ -563,35 +639,101 @@ Plan plan(int R, int N, int K, bool split_k)
     p.a_bytes = (size_t)p.mt_chunk * p.KT * A_STAGE;
     p.b_bytes = (size_t)p.tiles_n * p.KT * S * p.nt * KB * 2;
     p.fb_bytes = ((size_t)p.tiles_n * p.BT * sizeof(int) + 255) / 256 * 256;
+    p.ng = ng;
     return p;
 }
 
-size_t plan_bytes(const Plan& p) { return p.a_bytes + p.b_bytes + p.fb_bytes; }
+size_t plan_bytes(const Plan& p) { return p.ng * (p.a_bytes + p.b_bytes + p.fb_bytes); }
+
+// The GEMMs of an expansion run together when their A slices fit the cap.
+Plan expand_plan(int M, int N, int K, int ng)
+{
+    const Plan p = plan(K, N, M, false, ng);
+    return ng > 1 && ng * p.a_bytes > A_CAP ? plan(K, N, M, false, 1) : p;
+}
 
 // rows of A in chunks against all bands, the bands in passes of N_CAP
 template <bool EXPAND>
-cudaError_t run(int R, int N, int K, const double2* A, size_t lda, D64Scale s, const double2* B, size_t ldb,
-                double2* part, double2* out, size_t ldo, unsigned char* ws, int* err, cudaStream_t st)
+cudaError_t run(const Plan& p, int R, int N, int K, const double2* A, size_t lda, D64Scale sc, const double2* B,
+                size_t ldb, double2* part, const KMap* maps, double2* const* out, size_t ldo, unsigned char* ws,
+                int* err, cudaStream_t st)
 {
-    const Plan p = plan(R, N, K, !EXPAND);
-    unsigned char *a = ws, *b = ws + p.a_bytes;
-    int* fb = reinterpret_cast<int*>(b + p.b_bytes);
+    SplitArgs s{};
+    s.A = A; s.lda = lda; s.ldb = ldb; s.ek = sc.ek; s.fm = sc.fm;
+    s.R = R; s.K = K; s.KT = p.KT; s.BT = p.BT;
+    s.a = ws; s.b = ws + p.ng * p.a_bytes;
+    s.a_bytes = p.a_bytes; s.b_bytes = p.b_bytes;
+    s.fb = reinterpret_cast<int*>(s.b + p.ng * p.b_bytes);
+    const int bands = p.tiles_n * p.BT;
+    s.b_seg = K > 2 * B_SEG ? ceil_div(p.KT, B_SEG / 8) : 1;
+    s.a_x = ceil_div(p.KT, 2);
+    for (int g = 0; g < p.ng; ++g) s.map[g] = maps[g];
     for (int n0 = 0; n0 < N; n0 += p.n_pass) {
-        const int n = std::min(p.n_pass, N - n0);
-        split_b_kernel<EXPAND><<<p.tiles_n * p.BT, 512, 0, st>>>(n, K, EXPAND ? B + n0 : B + (size_t)n0 * ldb, ldb,
-                                                                 EXPAND ? s.fm : s.ek, p.KT, p.BT, b, fb);
+        s.nb = std::min(p.n_pass, N - n0);
+        s.B = EXPAND ? B + n0 : B + (size_t)n0 * ldb;
+        if (s.b_seg > 1) {
+            const cudaError_t e = cudaMemsetAsync(s.fb, 0, (size_t)p.ng * bands * sizeof(int), st);
+            if (e) return e;
+            band_exp_kernel<EXPAND><<<dim3(ceil_div(K, B_SEG), s.nb, p.ng), 256, 0, st>>>(s, bands);
+        }
         for (int m = 0; m < p.mt; m += p.mt_chunk) {
-            const int mt = std::min(p.mt_chunk, p.mt - m), row0 = m * TM;
-            if (n0 == 0 || p.mt > p.mt_chunk)
-                split_a_kernel<EXPAND><<<dim3(ceil_div(p.KT, 2), 2 * mt), 256, 0, st>>>(R, K, p.KT, row0, A, lda, EXPAND ? s.ek : s.fm,
-                                                                           EXPAND ? s.fm : s.ek, a);
-            D64Out o{EXPAND ? nullptr : part + n0, N, EXPAND ? out + (size_t)n0 * ldo : nullptr, ldo, EXPAND ? s.ek : s.fm, fb, R, n, row0};
-            const cudaError_t e =
-                launch_gemm<EXPAND>(p.nt, dim3(p.tiles_n, mt, p.nz), a, b, o, p.KT, p.cps, err, st);
+            const int mt = std::min(p.mt_chunk, p.mt - m);
+            s.row0 = m * TM;
+            s.b_blocks = m == 0 ? bands * s.b_seg : 0;
+            s.a_blocks = n0 == 0 || p.mt > p.mt_chunk ? s.a_x * 2 * mt : 0;
+            if (s.a_blocks + s.b_blocks)
+                split_kernel<EXPAND><<<dim3(s.a_blocks + s.b_blocks, p.ng), 256, 0, st>>>(s);
+            D64Out o{};
+            o.part = EXPAND ? nullptr : part + n0;
+            o.ldn = N;
+            for (int g = 0; g < p.ng; ++g) o.out[g] = EXPAND ? out[g] + (size_t)n0 * ldo : nullptr;
+            o.ldo = ldo;
+            o.a_bytes = p.a_bytes; o.b_bytes = p.b_bytes; o.bands = bands;
+            o.er = EXPAND ? sc.ek : sc.fm;
+            o.fb = s.fb;
+            o.M = R; o.N = s.nb; o.row0 = s.row0;
+            const cudaError_t e = launch_gemm<EXPAND>(p.nt, dim3(p.tiles_n, mt, EXPAND ? p.ng : p.nz), s.a, s.b, o, p.KT,
+                                                      p.cps, err, st);
             if (e) return e;
         }
     }
     return cudaGetLastError();
+}
+
+// W[m][n] = scale[m % period] sum_z part[z][m][n]: 32 outputs per block, the splits
+// in SL slices that are added in order
+template <int SL>
+__global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total, int nz,
+                                                             const double2* __restrict__ part,
+                                                             const double* __restrict__ scale, int period,
+                                                             double2* __restrict__ W)
+{
+    __shared__ double2 sum[SL][32];
+    const size_t i = (size_t)blockIdx.x * 32 + threadIdx.x;
+    const int per = ceil_div_d(nz, SL), z1 = min(nz, (int)(threadIdx.y + 1) * per);
+    double re = 0.0, im = 0.0;
+    if (i < total) {
+#pragma unroll 4
+        for (int z = threadIdx.y * per; z < z1; ++z) {
+            const double2 v = part[(size_t)z * total + i];
+            re += v.x;
+            im += v.y;
+        }
+    }
+    if (SL > 1) {
+        sum[threadIdx.y][threadIdx.x] = make_double2(re, im);
+        __syncthreads();
+        if (threadIdx.y) return;
+#pragma unroll
+        for (int y = 1; y < SL; ++y) {
+            re += sum[y][threadIdx.x].x;
+            im += sum[y][threadIdx.x].y;
+        }
+    }
+    if (i < total) {
+        const double f = scale ? scale[(int)(i / N) % period] : 1.0;
+        W[i] = make_double2(f * re, f * im);
+    }
 }
 
 }  // namespace
@@ -609,24 +751,61 @@ cudaError_t d64_scales(int M, int K, const double2* A, size_t lda, D64Scale s, c
     return cudaGetLastError();
 }
 
-int d64_proj_splits(int M, int N, int K) { return plan(M, N, K, true).nz; }
+int d64_proj_splits(int M, int N, int K) { return plan(M, N, K, true, 1).nz; }
 
-size_t d64_proj_ws(int M, int N, int K) { return plan_bytes(plan(M, N, K, true)); }
+size_t d64_proj_ws(int M, int N, int K) { return plan_bytes(plan(M, N, K, true, 1)); }
 
-size_t d64_expand_ws(int M, int N, int K) { return plan_bytes(plan(K, N, M, false)); }
+size_t d64_expand_ws(int M, int N, int K) { return plan_bytes(expand_plan(M, N, K, 1)); }
+
+size_t d64_expand_grad_ws(int P, int N, int K, int nd) { return plan_bytes(expand_plan(2 * P, N, K, nd)); }
 
 cudaError_t d64_proj(int M, int N, int K, const double2* A, size_t lda, D64Scale s, const double2* B, size_t ldb,
                      double2* part, unsigned char* ws, int* err, cudaStream_t st)
 {
     if (M == 0 || N == 0 || K == 0) return cudaSuccess;
-    return run<false>(M, N, K, A, lda, s, B, ldb, part, nullptr, 0, ws, err, st);
+    const KMap map{K, 0, 0, 0};
+    return run<false>(plan(M, N, K, true, 1), M, N, K, A, lda, s, B, ldb, part, &map, nullptr, 0, ws, err, st);
+}
+
+cudaError_t d64_reduce(int M, int N, int nz, const double2* part, const double* scale, int period, double2* W,
+                       cudaStream_t st)
+{
+    const size_t total = (size_t)M * N;
+    if (total == 0) return cudaSuccess;
+    const int blocks = ceil_div((long)total, 32);
+    if (nz >= 16) d64_reduce_kernel<8><<<blocks, dim3(32, 8), 0, st>>>(N, total, nz, part, scale, period, W);
+    else d64_reduce_kernel<1><<<blocks, dim3(32, 1), 0, st>>>(N, total, nz, part, scale, period, W);
+    return cudaGetLastError();
 }
 
 cudaError_t d64_expand(int M, int N, int K, const double2* W, size_t ldw, const double2* A, size_t lda, D64Scale s,
                        double2* out, size_t ldo, unsigned char* ws, int* err, cudaStream_t st)
 {
     if (M == 0 || N == 0 || K == 0) return cudaSuccess;
-    return run<true>(K, N, M, A, lda, s, W, ldw, nullptr, out, ldo, ws, err, st);
+    const KMap map{M, 0, 0, 0};
+    return run<true>(expand_plan(M, N, K, 1), K, N, M, A, lda, s, W, ldw, nullptr, &map, &out, ldo, ws, err, st);
+}
+
+cudaError_t d64_expand_grad(int P, int N, int K, const double2* W, size_t ldw, const double2* A, size_t lda, D64Scale s,
+                            double2* const out[3], size_t ldo, unsigned char* ws, int* err, cudaStream_t st)
+{
+    if (P == 0 || N == 0 || K == 0) return cudaSuccess;
+    KMap map[3];
+    double2* to[3];
+    int nd = 0;
+    for (int a = 0; a < 3; ++a)
+        if (out[a]) {
+            map[nd] = KMap{P, a * P, (a + 1) * P, -P};
+            to[nd++] = out[a];
+        }
+    if (nd == 0) return cudaSuccess;
+    const Plan p = expand_plan(2 * P, N, K, nd);
+    for (int g = 0; g < nd; g += p.ng) {
+        const cudaError_t e =
+            run<true>(p, K, N, 2 * P, A, lda, s, W, ldw, nullptr, map + g, to + g, ldo, ws, err, st);
+        if (e) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t d64_set_issue_wait_limit(long polls)

@@ -451,91 +451,64 @@ static int d64_scale(hpsi_ctx* c, KSlot& s, D64Scale* out, cudaStream_t st)
     return HPSI_OK;
 }
 
-// Workspace of M projector rows against nb bands: partials, W, then the operands
-// of the projection and (after it) of the expansions of P rows each
-struct D64Ws {
-    size_t part, w, ops, bytes;
-    int nz;
+// The FP64 GEMMs of one call: workspace pieces and the projector matrix's scales.
+struct D64Call {
+    double2 *part, *W;  // partials of the projection [nz][M][nb]; W [M][nb]
+    unsigned char* ops; // operands of the projection, then of the expansion
+    D64Scale sc;
+    int M, nz;
 };
 
-static D64Ws d64_layout(int M, int P, int nb, int npw)
+// Plan a call that projects M rows and expands with expand_ws bytes of operands.
+// *ok = false (and nothing queued) when the device has no room for the workspace:
+// the call then runs the SIMT GEMMs.  These are slower at every shape, down to one
+// band of the smallest cell (16 projectors, 754 plane waves: 72 against 44 us).
+static int d64_begin(hpsi_ctx* c, KSlot& s, int M, int nb, size_t expand_ws, D64Call* d, bool* ok, cudaStream_t st)
 {
-    D64Ws w;
-    w.nz = d64_proj_splits(M, nb, npw);
+    *ok = false;
+    if (s.P == 0) return HPSI_OK;
+    d->M = M;
+    d->nz = d64_proj_splits(M, nb, s.npw);
     Carver cv;
-    w.part = cv.take<double2>((size_t)w.nz * M * nb);
-    w.w = cv.take<double2>((size_t)M * nb);
-    w.ops = cv.off;
-    w.bytes = cv.off + std::max(d64_proj_ws(M, nb, npw), d64_expand_ws(P, nb, npw));
-    return w;
+    const size_t o_part = cv.take<double2>((size_t)d->nz * M * nb), o_w = cv.take<double2>((size_t)M * nb);
+    unsigned char* ws = d64_reserve(c, cv.off + std::max(d64_proj_ws(M, nb, s.npw), expand_ws));
+    if (!ws) return HPSI_OK;
+    d->part = reinterpret_cast<double2*>(ws + o_part);
+    d->W = reinterpret_cast<double2*>(ws + o_w);
+    d->ops = ws + cv.off;
+    *ok = true;
+    c->d64_ran = true;
+    return d64_scale(c, s, &d->sc, st);
 }
 
-// As nonlocal_apply in FP64, at every shape: the SIMT GEMMs are slower down to one
-// band of the smallest cell (16 projectors, 754 plane waves: 72 against 44 us).
-// *done = false (and nothing queued) when the device's free memory leaves the call to them.
-static int nonlocal_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* hpsi, cudaStream_t st,
-                        double* e_nl, bool* done)
+// W = lambda <p|psi> for the first M rows of pr64 (and the nonlocal energies)
+static int d64_project(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const D64Call& d, double* e_nl,
+                       cudaStream_t st)
 {
-    *done = false;
-    if (s.P == 0) return HPSI_OK;
-    const D64Ws w = d64_layout(s.P, s.P, nb, s.npw);
-    unsigned char* ws = d64_reserve(c, w.bytes);
-    if (!ws) return HPSI_OK;
-    *done = true;
-    D64Scale sc;
-    int rc = d64_scale(c, s, &sc, st);
-    if (rc) return rc;
-    c->d64_ran = true;
-    double2* part = reinterpret_cast<double2*>(ws + w.part);
-    double2* W = reinterpret_cast<double2*>(ws + w.w);
+    const size_t npw = (size_t)s.npw;
     int h = c->prof.open(PH_PROJ, st);
-    CUDA_TRY(c, d64_proj(s.P, nb, s.npw, s.pr64, (size_t)s.npw, sc, psi, (size_t)s.npw, part, ws + w.ops, c->d_err, st));
-    c->prof.close(h, st, 3);
-    if (e_nl) CUDA_TRY(c, launch_nl_energy<double2>(s.P, nb, w.nz, part, s.d_lam, e_nl, st));
+    CUDA_TRY(c, d64_proj(d.M, nb, s.npw, s.pr64, npw, d.sc, psi, npw, d.part, d.ops, c->d_err, st));
+    c->prof.close(h, st, 2);
+    if (e_nl) CUDA_TRY(c, launch_nl_energy<double2>(s.P, nb, d.nz, d.part, s.d_lam, e_nl, st));
     h = c->prof.open(PH_REDUCE, st);
-    CUDA_TRY(c, (launch_reduce_splits<double2, double2>(s.P, nb, w.nz, part, s.d_lam, s.P, W, (size_t)nb, st)));
+    CUDA_TRY(c, d64_reduce(d.M, nb, d.nz, d.part, s.d_lam, s.P, d.W, st));
     c->prof.close(h, st);
-    h = c->prof.open(PH_EXPAND, st);
-    CUDA_TRY(c, d64_expand(s.P, nb, s.npw, W, (size_t)nb, s.pr64, (size_t)s.npw, sc, hpsi, (size_t)s.npw, ws + w.ops,
-                           c->d_err, st));
-    c->prof.close(h, st, 3);
     return HPSI_OK;
 }
 
-// The projector part of grad_device in FP64 (all 4P rows of pr64); *done as above.
+// The projector part of grad_device in FP64 (all 4P rows of pr64); *done as *ok above.
 static int grad_nonlocal_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* d[3], cudaStream_t st,
                              bool* done)
 {
-    *done = false;
-    const int M = 4 * s.P;
-    const D64Ws w = d64_layout(M, s.P, nb, s.npw);
-    unsigned char* ws = d64_reserve(c, w.bytes);
-    if (!ws) return HPSI_OK;
-    *done = true;
-    D64Scale sc;
-    int rc = d64_scale(c, s, &sc, st);
-    if (rc) return rc;
-    c->d64_ran = true;
-    const size_t npw = (size_t)s.npw, PN = (size_t)s.P * npw;
-    double2* part = reinterpret_cast<double2*>(ws + w.part);
-    double2* W = reinterpret_cast<double2*>(ws + w.w);
-    int h = c->prof.open(PH_PROJ, st);
-    CUDA_TRY(c, d64_proj(M, nb, s.npw, s.pr64, npw, sc, psi, npw, part, ws + w.ops, c->d_err, st));
-    c->prof.close(h, st, 3);
-    h = c->prof.open(PH_REDUCE, st);
-    CUDA_TRY(c, (launch_reduce_splits<double2, double2>(M, nb, w.nz, part, s.d_lam, s.P, W, (size_t)nb, st)));
-    c->prof.close(h, st);
-    for (int a = 0; a < 3; ++a) {
-        if (!d[a]) continue;
-        h = c->prof.open(PH_EXPAND, st);
-        // lambda <dp_a|psi> p, then lambda <p|psi> dp_a
-        CUDA_TRY(c, d64_expand(s.P, nb, s.npw, W + (size_t)(a + 1) * s.P * nb, (size_t)nb, s.pr64, npw, sc, d[a], npw,
-                               ws + w.ops, c->d_err, st));
-        const D64Scale sa{sc.ek, sc.fm + (size_t)(a + 1) * s.P};
-        CUDA_TRY(c, d64_expand(s.P, nb, s.npw, W, (size_t)nb, s.pr64 + (size_t)(a + 1) * PN, npw, sa, d[a], npw,
-                               ws + w.ops, c->d_err, st));
-        c->prof.close(h, st, 6);
-    }
+    const int nd = (d[0] != nullptr) + (d[1] != nullptr) + (d[2] != nullptr);
+    const size_t npw = (size_t)s.npw;
+    D64Call k;
+    int rc = d64_begin(c, s, 4 * s.P, nb, d64_expand_grad_ws(s.P, nb, s.npw, nd), &k, done, st);
+    if (rc || !*done) return rc;
+    if ((rc = d64_project(c, s, nb, psi, k, nullptr, st))) return rc;
+    int h = c->prof.open(PH_EXPAND, st);
+    CUDA_TRY(c, d64_expand_grad(s.P, nb, s.npw, k.W, (size_t)nb, s.pr64, npw, k.sc, d, npw, k.ops, c->d_err, st));
+    c->prof.close(h, st, 2);
     return HPSI_OK;
 }
 
@@ -561,10 +534,9 @@ static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const
     CUDA_TRY(c, d64_scales(nb, s.npw, psi, npw, sc, st));
     for (int a = 0; a < 3; ++a) {
         CUDA_TRY(c, d64_proj(nb, nb, s.npw, psi, npw, sc, g + (size_t)a * nb * npw, npw, part, ws + o_ops, c->d_err, st));
-        CUDA_TRY(c, (launch_reduce_splits<double2, double2>(nb, nb, nz, part, nullptr, 0, m + (size_t)a * nb * nb,
-                                                            (size_t)nb, st)));
+        CUDA_TRY(c, d64_reduce(nb, nb, nz, part, nullptr, nb, m + (size_t)a * nb * nb, st));
     }
-    c->prof.close(h, st, 14);
+    c->prof.close(h, st, 11);
     return HPSI_OK;
 }
 
@@ -1078,11 +1050,30 @@ static int apply_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2*
     int rc;
     if ((rc = prepare_slot(c, s, prec, false, st))) return rc;
     if (prec == HPSI_PREC_FP64) {
-        if ((rc = local_apply<double2, double>(c, s, nb, psi, hpsi, work, c->d_v64, c->d_tw64, st, epart))) return rc;
-        if (d64) {
-            bool done;
-            rc = nonlocal_d64(c, s, nb, psi, hpsi, st, e_nl, &done);
-            if (rc || done) return rc;
+        // the projection chain on the side stream beside the FFT passes (tensor
+        // cores against the integer pipes); the expansion joins after both
+        D64Call k;
+        bool ok = false;
+        if (d64 && (rc = d64_begin(c, s, s.P, nb, d64_expand_ws(s.P, nb, s.npw), &k, &ok, st))) return rc;
+        if (ok && fork) {
+            CUDA_TRY(c, cudaEventRecord(c->ev_fork, st));
+            CUDA_TRY(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
+            rc = d64_project(c, s, nb, psi, k, e_nl, c->side);
+            const cudaError_t e = cudaEventRecord(c->ev_join, c->side);  // join even after an error
+            const int rl = local_apply<double2, double>(c, s, nb, psi, hpsi, work, c->d_v64, c->d_tw64, st, epart);
+            CUDA_TRY(c, e);
+            CUDA_TRY(c, cudaStreamWaitEvent(st, c->ev_join, 0));
+            if (rc || rl) return rc ? rc : rl;
+        } else {
+            if ((rc = local_apply<double2, double>(c, s, nb, psi, hpsi, work, c->d_v64, c->d_tw64, st, epart))) return rc;
+            if (ok && (rc = d64_project(c, s, nb, psi, k, e_nl, st))) return rc;
+        }
+        if (ok) {
+            const size_t npw = (size_t)s.npw;
+            int h = c->prof.open(PH_EXPAND, st);
+            CUDA_TRY(c, d64_expand(s.P, nb, s.npw, k.W, (size_t)nb, s.pr64, npw, k.sc, hpsi, npw, k.ops, c->d_err, st));
+            c->prof.close(h, st, 2);
+            return HPSI_OK;
         }
         return nonlocal_apply<double2, double2>(c, s, nb, psi, hpsi, s.pr64, work, st, e_nl);
     }

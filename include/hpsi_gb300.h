@@ -63,7 +63,9 @@ extern "C" {
 #define HPSI_ERR_STATE    -6   /* k-point not set, missing table (runtime_error) */
 
 /* flags: precision in bits 0-3 */
-#define HPSI_PREC_FP64      0  /* complex128 FFTs, FP64 projector sums: parity path */
+#define HPSI_PREC_FP64      0  /* FP64-accurate 64-bit fixed-point FFTs and digit-sliced tensor-core
+                                  projector GEMMs (SIMT FP64 ones where a call has no workspace for
+                                  them): parity path */
 #define HPSI_PREC_FP32      1  /* complex64 FFTs, FP32 projector GEMMs, FP64 phases */
 #define HPSI_PREC_TC        2  /* complex64 FFTs, tcgen05 tensor-core projector GEMMs on split FP16
                                   (x*2^s = hi + lo per row, 3 products, FP32 accumulation) */
@@ -71,8 +73,8 @@ extern "C" {
 #define HPSI_PREC_MASK    0xF
 #define HPSI_DEVICE_PTRS  0x10 /* psi/outputs are device pointers (else host memory) */
 #define HPSI_SYNC         0x20 /* synchronise `stream` before returning */
-#define HPSI_ONE_STREAM   0x40 /* tensor-core hpsi_apply / hpsi_apply_energies: run the
-                                * projection chain on `stream` too instead of on the
+#define HPSI_ONE_STREAM   0x40 /* FP64 and tensor-core hpsi_apply / hpsi_apply_energies: run
+                                * the projection chain on `stream` too instead of on the
                                 * context's side stream beside the FFT passes */
 
 /* One pseudopotential species after the per-l diagonalisation of D
