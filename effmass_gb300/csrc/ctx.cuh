@@ -13,10 +13,22 @@
 #include "kernels.cuh"
 #include "tc_gemm.cuh"
 
+// A device buffer kept by a slot when it is rebound, for the next binding
+struct Spare {
+    void* p = nullptr;
+    size_t bytes = 0;
+};
+// Larger buffers go back to the device at once (their builds take longer than
+// cudaMalloc and cudaFree).
+constexpr size_t kSpareMax = 64ull << 20;
+
 struct KSlot {
     bool valid = false;
     int npw = 0;
     double kf[3] = {0, 0, 0};
+    // the binding's tables, d_kin to d_lam, in one allocation
+    unsigned char* mem = nullptr;
+    size_t mem_cap = 0;
     double* d_kin = nullptr;
     double* d_kvec = nullptr;
     int* d_g = nullptr;
@@ -33,13 +45,19 @@ struct KSlot {
     std::vector<ProjRow> rows;     // host copy of d_rows
     ProjRow* d_rows = nullptr;
     double* d_lam = nullptr;
+    // projector matrices: rows [0, P), and with dbeta tables room for the 3 P
+    // derivative rows behind them (filled on first use: pr*_grad)
     double2* pr64 = nullptr;
     bool pr64_grad = false;
-    int* d64_exp = nullptr;        // exponents of pr64's columns [npw] and rows for the digit split,
-                                   // in pr64's allocation
-    bool d64_exp_set = false;
+    // exponents of pr64's columns and rows for the digit split, of the first P rows
+    // (H) and of all 4 P (gradient), in pr64's allocation
+    int* d64_exp[2] = {nullptr, nullptr};
+    bool d64_exp_set[2] = {false, false};
     float2* pr32 = nullptr;
     bool pr32_grad = false;
+    size_t pr_bytes[2] = {0, 0};   // allocation sizes of pr64, pr32
+    size_t tc_bytes[2] = {0, 0};   // and of tc_mem
+    Spare spare_pr[2], spare_tc[2];
     // tensor-core H|psi>: generator tables of the projector operands, one set
     // per split format (0 FP16, 1 BF16), built from the FP64 tables on first
     // use and kept until the slot is rebound (batch plans hold pointers into
@@ -75,11 +93,52 @@ inline void dfree(T*& p)
 
 inline void slot_free(KSlot& s)
 {
-    dfree(s.d_kin); dfree(s.d_kvec); dfree(s.d_g); dfree(s.d_q); dfree(s.d_trig); dfree(s.d_ylm);
-    dfree(s.d_beta); dfree(s.d_dbeta0); dfree(s.d_sf); dfree(s.d_plane); dfree(s.d_rows); dfree(s.d_lam);
+    dfree(s.mem);
+    for (Spare* p : {&s.spare_pr[0], &s.spare_pr[1], &s.spare_tc[0], &s.spare_tc[1]}) dfree(p->p);
     dfree(s.pr64); dfree(s.pr32); dfree(s.tc_mem[0]); dfree(s.tc_mem[1]); dfree(s.tcg_mem); dfree(s.hess64);
     dfree(s.hess32);
     s = KSlot();
+}
+
+// Empty slot s for a new binding.  The tables' allocation stays, and projector
+// buffers of up to kSpareMax stay as spares.  The caller has synchronised the device.
+inline void slot_reset(KSlot& s)
+{
+    KSlot n;
+    n.mem = s.mem;
+    n.mem_cap = s.mem_cap;
+    s.mem = nullptr;
+    auto keep = [](void* p, size_t bytes, Spare& old, Spare& to) {
+        if (p && bytes <= kSpareMax) {
+            dfree(old.p);
+            to = Spare{p, bytes};
+            return true;
+        }
+        to = old;
+        old = Spare{};
+        return false;
+    };
+    if (keep(s.pr64, s.pr_bytes[0], s.spare_pr[0], n.spare_pr[0])) s.pr64 = nullptr;
+    if (keep(s.pr32, s.pr_bytes[1], s.spare_pr[1], n.spare_pr[1])) s.pr32 = nullptr;
+    for (int f = 0; f < 2; ++f)
+        if (keep(s.tc_mem[f], s.tc_bytes[f], s.spare_tc[f], n.spare_tc[f])) s.tc_mem[f] = nullptr;
+    for (int f = 0; f < 2; ++f) s.spare_pr[f] = s.spare_tc[f] = Spare{};  // moved or freed above
+    slot_free(s);
+    s = n;
+}
+
+// *p = a buffer of at least bytes: the spare when it fits, else a new one
+inline cudaError_t spare_alloc(Spare& spare, void** p, size_t* bytes)
+{
+    if (spare.p && spare.bytes >= *bytes && spare.bytes / 2 <= *bytes) {
+        *p = spare.p;
+        *bytes = spare.bytes;
+        spare = Spare{};
+        return cudaSuccess;
+    }
+    dfree(spare.p);
+    spare = Spare{};
+    return cudaMalloc(p, *bytes);
 }
 
 struct hpsi_ctx {
@@ -101,10 +160,17 @@ struct hpsi_ctx {
     float2* d_tw32 = nullptr;
     FftLen L[3];
     std::map<int, KSlot> slots;
+    // projector rows and strengths (the same for every k-point), and the largest q
+    // that every radial table covers
+    std::vector<ProjRow> proj_rows;
+    std::vector<double> proj_lam;
+    double q_safe = 0;
+    unsigned char* stage = nullptr;  // pinned staging of hpsi_set_kpoint
+    size_t stage_size = 0;
     unsigned char* ws = nullptr;
     size_t ws_size = 0;
-    // workspace of the FP64 GEMMs on the tensor cores, beside ws: a call that
-    // cannot have it runs the SIMT GEMMs
+    // workspace of the FP64 GEMMs on the tensor cores, within ws (set per call): a
+    // call that cannot have it runs the SIMT GEMMs
     unsigned char* d64_ws = nullptr;
     size_t d64_size = 0;
     bool d64_ran = false;         // d_err is checked at the next synchronising call
@@ -173,26 +239,33 @@ inline int ws_reserve(hpsi_ctx* c, size_t bytes)
     if (c->ws) cudaFree(c->ws);
     c->ws = nullptr;
     c->ws_size = 0;
+    c->d64_ws = nullptr;
     size_t want = bytes + bytes / 8;
     CUDA_TRY(c, cudaMalloc((void**)&c->ws, want));
     c->ws_size = want;
     return HPSI_OK;
 }
 
-// The FP64 GEMM workspace of at least bytes, or null when the device has no room.
-inline unsigned char* d64_reserve(hpsi_ctx* c, size_t bytes)
+// Reserve base bytes, and extra bytes behind them for the FP64 GEMMs on the tensor
+// cores (d64_ws).  Without room for extra the call goes on with base alone.
+inline int ws_reserve_d64(hpsi_ctx* c, size_t base, size_t extra)
 {
-    if (bytes <= c->d64_size) return c->d64_ws;
-    if (c->d64_ws) cudaFree(c->d64_ws);
+    const size_t off = (base + 255) / 256 * 256;
     c->d64_ws = nullptr;
     c->d64_size = 0;
-    if (cudaMalloc((void**)&c->d64_ws, bytes) != cudaSuccess) {
+    if (extra) {
+        const std::string err = c->err;
+        const int rc = ws_reserve(c, off + extra);
+        if (rc == HPSI_OK) {
+            c->d64_ws = c->ws + off;
+            c->d64_size = extra;
+            return HPSI_OK;
+        }
+        if (rc != HPSI_ERR_OOM) return rc;
         cudaGetLastError();  // not an error of the call
-        c->d64_ws = nullptr;
-        return nullptr;
+        c->err = err;
     }
-    c->d64_size = bytes;
-    return c->d64_ws;
+    return ws_reserve(c, base);
 }
 
 // Build, once, what a precision needs on slot s (projector matrices, tensor-core

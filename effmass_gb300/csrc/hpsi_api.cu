@@ -40,7 +40,7 @@ extern "C" int hpsi_ctx_destroy(hpsi_ctx* c)
     dfree(c->d_tables); dfree(c->d_rad_nq); dfree(c->d_rad_dq); dfree(c->d_tau); dfree(c->d_v64); dfree(c->d_v32); dfree(c->d_dv32);
     dfree(c->d_tw64); dfree(c->d_tw32); dfree(c->d_err); dfree(c->d_hess);
     if (c->ws) cudaFree(c->ws);
-    if (c->d64_ws) cudaFree(c->d64_ws);
+    if (c->stage) cudaFreeHost(c->stage);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
@@ -124,6 +124,23 @@ static int ctx_init(hpsi_ctx* c, const hpsi_system* s)
             c->nrad++;
         }
     }
+    for (int a = 0; a < c->natom; ++a) {
+        const int sp = c->atom_species[a], r0 = c->rad_off[sp];
+        const int r1 = (sp + 1 < (int)c->rad_off.size()) ? c->rad_off[sp + 1] : c->nrad;
+        for (int r = r0; r < r1; ++r) {
+            if (std::fabs(c->rad_lam[r]) < 1e-15) continue;  // src/H_psi/hamiltonian_callable.cpp:226-227
+            const int l = c->rad_l[r];
+            for (int m = -l; m <= l; ++m) {
+                c->proj_rows.push_back(ProjRow{a, r, l, m});
+                c->proj_lam.push_back(c->rad_lam[r]);
+            }
+        }
+    }
+    // below q_safe no radial table is left: floor(q / dq) + 2 < nq holds with a node to spare
+    c->q_safe = 1e300;
+    for (int r = 0; r < c->nrad; ++r)
+        if (!(std::fabs(c->rad_lam[r]) < 1e-15))
+            c->q_safe = std::min({c->q_safe, c->rad_qmax[r], c->rad_dq[r] * (c->rad_nq[r] - 3) * (1.0 - 1e-12)});
     // plane FFT kernels keep two n2*n3 planes in shared memory
     LocalArgs la{};
     la.n1 = c->n1; la.n2 = c->n2; la.n3 = c->n3;
@@ -140,6 +157,9 @@ static int ctx_init(hpsi_ctx* c, const hpsi_system* s)
     for (cudaEvent_t* e : {&c->ev_half_in[0], &c->ev_half_in[1], &c->ev_half_exp, &c->ev_half_out, &c->ev_psi_in[0],
                            &c->ev_psi_in[1]})
         CUDA_TRY(c, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    // the workspace of a small cell's calls, so that the first one does not wait for it
+    int rc = ws_reserve(c, 4u << 20);
+    if (rc) return rc;
     CUDA_TRY(c, dalloc(&c->d_err, (size_t)1));
     CUDA_TRY(c, cudaMemset(c->d_err, 0, sizeof(int)));
     const size_t N = (size_t)c->n1 * c->n2 * c->n3;
@@ -238,132 +258,142 @@ extern "C" int hpsi_set_kpoint(hpsi_ctx* c, int kid, const hpsi_kpoint* kp)
     CUDA_TRY(c, cudaSetDevice(c->dev));
     const int n[3] = {c->n1, c->n2, c->n3};
 
-    // --- host-side validation: the reference's domain_error / assert cases
+    // --- host-side validation (the reference's domain_error / assert cases) and
+    // the plane decomposition of the sphere on the FFT grid
+    std::vector<int> gi(npw), jk(npw);
+    std::vector<int> plane_of_x(c->n1, -1);
     for (int ig = 0; ig < npw; ++ig) {
+        int at[3];
         for (int d = 0; d < 3; ++d) {
-            int gd = kp->g_idx[3 * ig + d];
-            int idx = gd + n[d] / 2 + 4;  // structure-factor cache index, src/H_psi/structure_factor.cppm:68-72
+            const int gd = kp->g_idx[3 * ig + d];
+            const int idx = gd + n[d] / 2 + 4;  // structure-factor cache index, src/H_psi/structure_factor.cppm:68-72
             if (idx < 0 || idx >= n[d] + 8)
                 return fail(c, HPSI_ERR_RANGE, "G %d: g[%d]=%d outside [-n/2-4, n/2+3] for n=%d", ig, d, gd, n[d]);
+            at[d] = gd >= 0 && gd < n[d] ? gd : gd < 0 && gd + n[d] >= 0 ? gd + n[d] : ((gd % n[d]) + n[d]) % n[d];
         }
         const double kx = kp->kvec[3 * ig], ky = kp->kvec[3 * ig + 1], kz = kp->kvec[3 * ig + 2];
         const double q = std::sqrt(kx * kx + ky * ky + kz * kz);
-        for (int r = 0; r < c->nrad; ++r) {
-            if (std::fabs(c->rad_lam[r]) < 1e-15) continue;
-            if (q > c->rad_qmax[r])
-                return fail(c, HPSI_ERR_RANGE, "G %d: q=%.17g exceeds q_max=%.17g", ig, q, c->rad_qmax[r]);
-            if (q > 0 && (int)std::floor(q / c->rad_dq[r]) + 2 >= c->rad_nq[r])
-                return fail(c, HPSI_ERR_RANGE, "G %d: q=%.17g beyond the table (nq=%d)", ig, q, c->rad_nq[r]);
-        }
+        if (!(q <= c->q_safe))
+            for (int r = 0; r < c->nrad; ++r) {
+                if (std::fabs(c->rad_lam[r]) < 1e-15) continue;
+                if (q > c->rad_qmax[r])
+                    return fail(c, HPSI_ERR_RANGE, "G %d: q=%.17g exceeds q_max=%.17g", ig, q, c->rad_qmax[r]);
+                if (q > 0 && (int)std::floor(q / c->rad_dq[r]) + 2 >= c->rad_nq[r])
+                    return fail(c, HPSI_ERR_RANGE, "G %d: q=%.17g beyond the table (nq=%d)", ig, q, c->rad_nq[r]);
+            }
+        gi[ig] = at[0];
+        jk[ig] = at[1] * n[2] + at[2];
+        plane_of_x[at[0]] = 1;
     }
-
-    // --- plane decomposition of the sphere on the FFT grid
-    std::vector<int> gi(npw), jk(npw);
-    std::vector<int> plane_of_x(c->n1, -1);
-    std::map<long, int> last;
-    for (int ig = 0; ig < npw; ++ig) {
-        int i = ((kp->g_idx[3 * ig] % n[0]) + n[0]) % n[0];
-        int j = ((kp->g_idx[3 * ig + 1] % n[1]) + n[1]) % n[1];
-        int k = ((kp->g_idx[3 * ig + 2] % n[2]) + n[2]) % n[2];
-        gi[ig] = i;
-        jk[ig] = j * n[2] + k;
-        last[(long)i * n[1] * n[2] + jk[ig]] = ig;  // the reference's scatter: the last write wins
-        plane_of_x[i] = 1;
-    }
-    std::vector<int> plane_x;
+    int nxs = 0;
     for (int i = 0; i < c->n1; ++i)
-        if (plane_of_x[i] > 0) { plane_of_x[i] = (int)plane_x.size(); plane_x.push_back(i); }
-    const int nxs = (int)plane_x.size();
-    std::vector<int> plane_off(nxs + 1, 0);
+        if (plane_of_x[i] > 0) plane_of_x[i] = nxs++;
+    // plane_x [nxs], plane_off [nxs + 1], ent_ig [npw], ent_jk [npw], plane_jr [nxs]
+    std::vector<int> pl((size_t)3 * nxs + 1 + 2 * (size_t)npw, 0);
+    int *plane_x = pl.data(), *plane_off = plane_x + nxs, *ent_ig = plane_off + nxs + 1, *ent_jk = ent_ig + npw;
+    int* plane_jr = ent_jk + npw;
+    for (int i = 0; i < c->n1; ++i)
+        if (plane_of_x[i] >= 0) plane_x[plane_of_x[i]] = i;
     for (int ig = 0; ig < npw; ++ig) plane_off[plane_of_x[gi[ig]] + 1]++;
     for (int p = 0; p < nxs; ++p) plane_off[p + 1] += plane_off[p];
-    std::vector<int> fill(plane_off.begin(), plane_off.end() - 1);
-    std::vector<int> ent_ig(npw), ent_jk(npw);
-    bool aliased = false;
-    for (int ig = 0; ig < npw; ++ig) {
-        int p = plane_of_x[gi[ig]];
-        int e = fill[p]++;
-        bool scatter = last[(long)gi[ig] * n[1] * n[2] + jk[ig]] == ig;
-        ent_ig[e] = scatter ? ig : (int)((unsigned)ig | 0x80000000u);
-        ent_jk[e] = jk[ig];
-        aliased = aliased || !scatter;
+    {
+        std::vector<int> fill(plane_off, plane_off + nxs);
+        for (int ig = 0; ig < npw; ++ig) {
+            const int e = fill[plane_of_x[gi[ig]]]++;
+            ent_ig[e] = ig;
+            ent_jk[e] = jk[ig];
+        }
     }
-    // rows in use per plane: |G_y| <= plane_jr[p], i.e. j <= jr or j >= n2 - jr
-    std::vector<int> plane_jr(nxs, 0);
-    for (int p = 0; p < nxs; ++p)
-        for (int e = plane_off[p]; e < plane_off[p + 1]; ++e) {
-            const int j = ent_jk[e] / n[2];
-            plane_jr[p] = std::max(plane_jr[p], std::min(j, n[1] - j));
-        }
-
-    // --- projector rows
-    std::vector<ProjRow> rows;
-    std::vector<double> lam;
-    for (int a = 0; a < c->natom; ++a) {
-        int sp = c->atom_species[a];
-        int r0 = c->rad_off[sp];
-        int r1 = (sp + 1 < (int)c->rad_off.size()) ? c->rad_off[sp + 1] : c->nrad;
-        for (int r = r0; r < r1; ++r) {
-            if (std::fabs(c->rad_lam[r]) < 1e-15) continue;  // src/H_psi/hamiltonian_callable.cpp:226-227
-            int l = c->rad_l[r];
-            for (int m = -l; m <= l; ++m) {
-                rows.push_back(ProjRow{a, r, l, m});
-                lam.push_back(c->rad_lam[r]);
+    // of several G on one grid point the last is scattered (the reference's scatter:
+    // the last write wins); cell: the point's latest entry, of this plane if not
+    // before its range.  Rows in use per plane: |G_y| <= plane_jr[p], i.e. j <= jr
+    // or j >= n2 - jr.
+    bool aliased = false;
+    {
+        std::vector<int> cell((size_t)n[1] * n[2], -1);
+        for (int p = 0; p < nxs; ++p)
+            for (int e = plane_off[p]; e < plane_off[p + 1]; ++e) {
+                int& last = cell[ent_jk[e]];
+                if (last >= plane_off[p]) {
+                    ent_ig[last] = (int)((unsigned)ent_ig[last] | 0x80000000u);
+                    aliased = true;
+                }
+                last = e;
+                const int j = ent_jk[e] / n[2];
+                plane_jr[p] = std::max(plane_jr[p], std::min(j, n[1] - j));
             }
-        }
     }
 
     KSlot& s = c->slots[kid];
-    slot_free(s);
+    // work queued on any stream may still read the old tables
+    if (s.mem) CUDA_TRY(c, cudaDeviceSynchronize());
+    slot_reset(s);
     s.gen = ++c->gen_counter;
     s.npw = npw;
     for (int d = 0; d < 3; ++d) s.kf[d] = kp->k_frac[d];
     s.nxs = nxs;
     s.aliased = aliased;
-    s.P = (int)rows.size();
+    s.P = (int)c->proj_rows.size();
     if (npw > 0) {
         const int nlm = (c->lmax + 1) * (c->lmax + 1);
         const bool grads = c->have_dbeta;
-        CUDA_TRY(c, dalloc(&s.d_kin, (size_t)npw));
-        CUDA_TRY(c, dalloc(&s.d_kvec, (size_t)3 * npw));
-        CUDA_TRY(c, dalloc(&s.d_g, (size_t)3 * npw));
-        CUDA_TRY(c, dalloc(&s.d_q, (size_t)npw));
-        CUDA_TRY(c, dalloc(&s.d_trig, (size_t)4 * npw));
-        CUDA_TRY(c, dalloc(&s.d_ylm, (size_t)(grads ? 3 : 1) * nlm * npw));
-        CUDA_TRY(c, dalloc(&s.d_plane, (size_t)3 * nxs + 1 + 2 * (size_t)npw));
-        CUDA_TRY(c, cudaMemcpy(s.d_kin, kp->kinetic, npw * sizeof(double), cudaMemcpyHostToDevice));
-        CUDA_TRY(c, cudaMemcpy(s.d_kvec, kp->kvec, 3 * npw * sizeof(double), cudaMemcpyHostToDevice));
-        CUDA_TRY(c, cudaMemcpy(s.d_g, kp->g_idx, 3 * npw * sizeof(int), cudaMemcpyHostToDevice));
-        std::vector<int> pl;
-        pl.insert(pl.end(), plane_x.begin(), plane_x.end());
-        pl.insert(pl.end(), plane_off.begin(), plane_off.end());
-        pl.insert(pl.end(), ent_ig.begin(), ent_ig.end());
-        pl.insert(pl.end(), ent_jk.begin(), ent_jk.end());
-        pl.insert(pl.end(), plane_jr.begin(), plane_jr.end());
-        CUDA_TRY(c, cudaMemcpy(s.d_plane, pl.data(), pl.size() * sizeof(int), cudaMemcpyHostToDevice));
+        // one allocation: the uploaded arrays first (one copy), then the derived tables
+        Carver cv;
+        const size_t o_kin = cv.take<double>((size_t)npw), o_kvec = cv.take<double>((size_t)3 * npw);
+        const size_t o_lam = cv.take<double>((size_t)s.P), o_rows = cv.take<ProjRow>((size_t)s.P);
+        const size_t o_g = cv.take<int>((size_t)3 * npw), o_pl = cv.take<int>(pl.size());
+        const size_t upload = cv.off;
+        const size_t o_q = cv.take<double>((size_t)npw), o_trig = cv.take<double>((size_t)4 * npw);
+        const size_t o_ylm = cv.take<double>((size_t)(grads ? 3 : 1) * nlm * npw);
+        const size_t o_beta = cv.take<double>((size_t)(grads ? 2 : 1) * c->nrad * npw);
+        const size_t o_db0 = cv.take<double>((size_t)c->nrad), o_sf = cv.take<double2>((size_t)c->natom * npw);
+        if (s.mem && (s.mem_cap < cv.off || (s.mem_cap > kSpareMax && s.mem_cap / 2 > cv.off))) dfree(s.mem);
+        if (!s.mem) {
+            CUDA_TRY(c, dalloc(&s.mem, cv.off));
+            s.mem_cap = cv.off;
+        }
+        if (c->stage_size < upload) {
+            if (c->stage) cudaFreeHost(c->stage);
+            c->stage = nullptr;
+            c->stage_size = 0;
+            CUDA_TRY(c, cudaMallocHost((void**)&c->stage, upload + upload / 8));
+            c->stage_size = upload + upload / 8;
+        }
+        std::memcpy(c->stage + o_kin, kp->kinetic, npw * sizeof(double));
+        std::memcpy(c->stage + o_kvec, kp->kvec, 3 * (size_t)npw * sizeof(double));
+        if (s.P > 0) {
+            std::memcpy(c->stage + o_lam, c->proj_lam.data(), s.P * sizeof(double));
+            std::memcpy(c->stage + o_rows, c->proj_rows.data(), s.P * sizeof(ProjRow));
+        }
+        std::memcpy(c->stage + o_g, kp->g_idx, 3 * (size_t)npw * sizeof(int));
+        std::memcpy(c->stage + o_pl, pl.data(), pl.size() * sizeof(int));
+        CUDA_TRY(c, cudaMemcpyAsync(s.mem, c->stage, upload, cudaMemcpyHostToDevice, 0));
+        s.d_kin = reinterpret_cast<double*>(s.mem + o_kin);
+        s.d_kvec = reinterpret_cast<double*>(s.mem + o_kvec);
+        s.d_lam = reinterpret_cast<double*>(s.mem + o_lam);
+        s.d_rows = reinterpret_cast<ProjRow*>(s.mem + o_rows);
+        s.d_g = reinterpret_cast<int*>(s.mem + o_g);
+        s.d_plane = reinterpret_cast<int*>(s.mem + o_pl);
+        s.d_q = reinterpret_cast<double*>(s.mem + o_q);
+        s.d_trig = reinterpret_cast<double*>(s.mem + o_trig);
+        s.d_ylm = reinterpret_cast<double*>(s.mem + o_ylm);
+        s.d_beta = reinterpret_cast<double*>(s.mem + o_beta);
+        s.d_dbeta0 = reinterpret_cast<double*>(s.mem + o_db0);
+        s.d_sf = reinterpret_cast<double2*>(s.mem + o_sf);
+        s.rows = c->proj_rows;
 
         GTabArgs ga{npw, c->lmax, s.d_kvec, s.d_q, s.d_trig, s.d_ylm, grads ? s.d_ylm + (size_t)nlm * npw : nullptr,
                     grads ? s.d_ylm + (size_t)2 * nlm * npw : nullptr};
         CUDA_TRY(c, launch_gtab(ga, 0));
         if (c->nrad > 0) {
-            CUDA_TRY(c, dalloc(&s.d_beta, (size_t)(grads ? 2 : 1) * c->nrad * npw));
-            CUDA_TRY(c, dalloc(&s.d_dbeta0, (size_t)c->nrad));
             BetaArgs ba{npw, c->nrad, s.d_q, c->d_tables, grads ? c->d_tables + (size_t)c->nrad * c->nq_max : nullptr,
                         c->d_rad_nq, c->d_rad_dq, c->nq_max, 1.0 / std::sqrt(c->omega), s.d_beta,
                         grads ? s.d_beta + (size_t)c->nrad * npw : nullptr, grads ? s.d_dbeta0 : nullptr};
             CUDA_TRY(c, launch_beta(ba, 0));
         }
         if (c->natom > 0) {
-            CUDA_TRY(c, dalloc(&s.d_sf, (size_t)c->natom * npw));
             SfArgs sa{npw, c->natom, s.d_g, c->d_tau, s.kf[0], s.kf[1], s.kf[2], s.d_sf};
             CUDA_TRY(c, launch_sf(sa, 0));
-        }
-        if (s.P > 0) {
-            CUDA_TRY(c, dalloc(&s.d_rows, (size_t)s.P));
-            CUDA_TRY(c, dalloc(&s.d_lam, (size_t)s.P));
-            CUDA_TRY(c, cudaMemcpy(s.d_rows, rows.data(), s.P * sizeof(ProjRow), cudaMemcpyHostToDevice));
-            s.rows.assign(rows.begin(), rows.begin() + s.P);
-            CUDA_TRY(c, cudaMemcpy(s.d_lam, lam.data(), s.P * sizeof(double), cudaMemcpyHostToDevice));
         }
         CUDA_TRY(c, cudaDeviceSynchronize());
     }
@@ -379,25 +409,31 @@ template <typename C> static C*& slot_hess(KSlot& s);
 template <> double2*& slot_hess<double2>(KSlot& s) { return s.hess64; }
 template <> float2*& slot_hess<float2>(KSlot& s) { return s.hess32; }
 
-// Build (once) the projector matrices of slot s in complex type C.
+// Build (once) the projector matrix of slot s in complex type C, with grad also its
+// derivative rows (room for them is there from the start when the tables allow).
 template <typename C>
 static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
 {
+    constexpr bool f64 = std::is_same<C, double2>::value;
     C*& pr = slot_pr<C>(s);
-    bool& has_grad = std::is_same<C, double2>::value ? s.pr64_grad : s.pr32_grad;
+    bool& has_grad = f64 ? s.pr64_grad : s.pr32_grad;
     if (s.P == 0 || s.npw == 0) return HPSI_OK;
     if (pr && (has_grad || !grad)) return HPSI_OK;
     if (grad && !c->have_dbeta) return fail(c, HPSI_ERR_STATE, "gradient needs dbeta tables for every species");
-    dfree(pr);
-    const bool g = grad || c->have_dbeta;  // build the derivative rows together when tables allow
-    const size_t rows = (size_t)(g ? 4 : 1) * s.P;
-    const bool f64 = std::is_same<C, double2>::value;
-    // FP64: the digit split's exponents behind the matrix (d64_scale)
-    const size_t tail = f64 ? ((rows + s.npw) * sizeof(int) + sizeof(C) - 1) / sizeof(C) : 0;
-    CUDA_TRY(c, dalloc(&pr, rows * s.npw + tail));
-    if (f64) {
-        s.d64_exp = reinterpret_cast<int*>(pr + rows * s.npw);
-        s.d64_exp_set = false;
+    const bool fresh = !pr;
+    if (fresh) {
+        const size_t rows = (size_t)(c->have_dbeta ? 4 : 1) * s.P;
+        // FP64: the digit split's exponents behind the matrix (d64_scale)
+        const size_t n_exp = f64 ? 2 * (size_t)s.npw + s.P + rows : 0;
+        size_t bytes = rows * s.npw * sizeof(C) + n_exp * sizeof(int);
+        const int k = f64 ? 0 : 1;
+        CUDA_TRY(c, spare_alloc(s.spare_pr[k], (void**)&pr, &bytes));
+        s.pr_bytes[k] = bytes;
+        if (f64) {
+            s.d64_exp[0] = reinterpret_cast<int*>(pr + rows * s.npw);
+            s.d64_exp[1] = s.d64_exp[0] + s.npw + s.P;
+            s.d64_exp_set[0] = s.d64_exp_set[1] = false;
+        }
     }
     const int nlm = (c->lmax + 1) * (c->lmax + 1);
     const double* yth = c->have_dbeta ? s.d_ylm + (size_t)nlm * s.npw : nullptr;
@@ -405,9 +441,9 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
     const double* dbeta = c->have_dbeta ? s.d_beta + (size_t)c->nrad * s.npw : nullptr;
     int h = c->prof.open(PH_BUILD, st);
     CUDA_TRY(c, launch_assemble<C>(s.P, s.npw, s.d_rows, s.d_beta, dbeta, s.d_dbeta0, s.d_q, s.d_trig, s.d_ylm, yth,
-                                   yph, s.d_sf, g, pr, (size_t)s.npw, st));
+                                   yph, s.d_sf, fresh, grad, pr, (size_t)s.npw, st));
     c->prof.close(h, st);
-    has_grad = g;
+    has_grad = grad;
     return HPSI_OK;
 }
 
@@ -439,15 +475,15 @@ static int nonlocal_apply(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, dou
 }
 
 // ---- FP64 nonlocal term on the tensor cores ----------------------------------
-// The exponents of slot s's projector matrix (all its rows), once per matrix.
-static int d64_scale(hpsi_ctx* c, KSlot& s, D64Scale* out, cudaStream_t st)
+// The exponents of the first P rows of slot s's projector matrix, or of all 4 P, once.
+static int d64_scale(hpsi_ctx* c, KSlot& s, bool all, D64Scale* out, cudaStream_t st)
 {
-    *out = D64Scale{s.d64_exp, s.d64_exp + s.npw};
-    if (s.d64_exp_set) return HPSI_OK;
+    *out = D64Scale{s.d64_exp[all], s.d64_exp[all] + s.npw};
+    if (s.d64_exp_set[all]) return HPSI_OK;
     int h = c->prof.open(PH_BUILD, st);
-    CUDA_TRY(c, d64_scales((s.pr64_grad ? 4 : 1) * s.P, s.npw, s.pr64, (size_t)s.npw, *out, st));
+    CUDA_TRY(c, d64_scales((all ? 4 : 1) * s.P, s.npw, s.pr64, (size_t)s.npw, *out, st));
     c->prof.close(h, st, 2);
-    s.d64_exp_set = true;
+    s.d64_exp_set[all] = true;
     return HPSI_OK;
 }
 
@@ -458,6 +494,24 @@ struct D64Call {
     D64Scale sc;
     int M, nz;
 };
+
+// Workspace of a call that projects M rows and expands with expand_ws bytes of operands
+static size_t d64_bytes(const KSlot& s, int M, int nb, size_t expand_ws)
+{
+    if (s.P == 0 || nb == 0) return 0;
+    Carver cv;
+    cv.take<double2>((size_t)d64_proj_splits(M, nb, s.npw) * M * nb);
+    cv.take<double2>((size_t)M * nb);
+    return cv.off + std::max(d64_proj_ws(M, nb, s.npw), expand_ws);
+}
+static size_t d64_apply_bytes(const KSlot& s, int nb, int prec)
+{
+    return prec == HPSI_PREC_FP64 ? d64_bytes(s, s.P, nb, d64_expand_ws(s.P, nb, s.npw)) : 0;
+}
+static size_t d64_grad_bytes(const KSlot& s, int nb, int nd, int prec)
+{
+    return prec == HPSI_PREC_FP64 ? d64_bytes(s, 4 * s.P, nb, d64_expand_grad_ws(s.P, nb, s.npw, nd)) : 0;
+}
 
 // Plan a call that projects M rows and expands with expand_ws bytes of operands.
 // *ok = false (and nothing queued) when the device has no room for the workspace:
@@ -471,14 +525,14 @@ static int d64_begin(hpsi_ctx* c, KSlot& s, int M, int nb, size_t expand_ws, D64
     d->nz = d64_proj_splits(M, nb, s.npw);
     Carver cv;
     const size_t o_part = cv.take<double2>((size_t)d->nz * M * nb), o_w = cv.take<double2>((size_t)M * nb);
-    unsigned char* ws = d64_reserve(c, cv.off + std::max(d64_proj_ws(M, nb, s.npw), expand_ws));
-    if (!ws) return HPSI_OK;
+    unsigned char* ws = c->d64_ws;
+    if (!ws || c->d64_size < d64_bytes(s, M, nb, expand_ws)) return HPSI_OK;
     d->part = reinterpret_cast<double2*>(ws + o_part);
     d->W = reinterpret_cast<double2*>(ws + o_w);
     d->ops = ws + cv.off;
     *ok = true;
     c->d64_ran = true;
-    return d64_scale(c, s, &d->sc, st);
+    return d64_scale(c, s, M > s.P, &d->sc, st);
 }
 
 // W = lambda <p|psi> for the first M rows of pr64 (and the nonlocal energies)
@@ -512,6 +566,15 @@ static int grad_nonlocal_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, 
     return HPSI_OK;
 }
 
+static size_t d64_velocity_bytes(const KSlot& s, int nb, int prec)
+{
+    if (prec != HPSI_PREC_FP64 || nb == 0) return 0;
+    Carver cv;
+    cv.take<double2>((size_t)d64_proj_splits(nb, nb, s.npw) * nb * nb);
+    cv.take<int>((size_t)s.npw + nb);
+    return std::max(cv.off + d64_proj_ws(nb, nb, s.npw), d64_grad_bytes(s, nb, 3, prec));
+}
+
 // m[a][i][j] = sum_G conj(psi_i) g_a,j for the three directions (g: [3][nb][npw]); *done as above.
 static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const double2* g, double2* m,
                         cudaStream_t st, bool* done)
@@ -522,8 +585,8 @@ static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const
     const size_t o_part = cv.take<double2>((size_t)nz * nb * nb);
     const size_t o_exp = cv.take<int>((size_t)s.npw + nb);
     const size_t o_ops = cv.off;
-    unsigned char* ws = d64_reserve(c, o_ops + d64_proj_ws(nb, nb, s.npw));
-    if (!ws) return HPSI_OK;
+    unsigned char* ws = c->d64_ws;
+    if (!ws || c->d64_size < o_ops + d64_proj_ws(nb, nb, s.npw)) return HPSI_OK;
     *done = true;
     c->d64_ran = true;
     double2* part = reinterpret_cast<double2*>(ws + o_part);
@@ -686,7 +749,9 @@ static int ensure_tc(hpsi_ctx* c, KSlot& s, int fmt, cudaStream_t st)
         prow[(size_t)p] = make_int2(r.atom, it->second);
     }
     const int nby = (int)byinfo.size();
-    CUDA_TRY(c, dalloc(&s.tc_mem[fmt], tc_gen_bytes(s.P, s.npw, nby, c->natom)));
+    size_t bytes = tc_gen_bytes(s.P, s.npw, nby, c->natom);
+    CUDA_TRY(c, spare_alloc(s.spare_tc[fmt], (void**)&s.tc_mem[fmt], &bytes));
+    s.tc_bytes[fmt] = bytes;
     int h = c->prof.open(PH_BUILD, st);
     CUDA_TRY(c, tc_build_gen(s.tc_mem[fmt], s.P, s.npw, prow.data(), byinfo.data(), nby, c->natom, s.d_beta,
                              s.d_ylm, s.d_sf, fmt == 0, &s.tcgen[fmt], st));
@@ -1330,7 +1395,7 @@ extern "C" int hpsi_apply(hpsi_ctx* c, int kid, int nb, const double* psi_, doub
     size_t o_psi = dev ? 0 : cv.take<double2>(nel);
     size_t o_hpsi = dev ? 0 : cv.take<double2>(nel);
     size_t o_work = cv.off;
-    if ((rc = ws_reserve(c, o_work + apply_ws_bytes(c, *s, nb, prec)))) return rc;
+    if ((rc = ws_reserve_d64(c, o_work + apply_ws_bytes(c, *s, nb, prec), d64_apply_bytes(*s, nb, prec)))) return rc;
     const double2* psi = (const double2*)psi_;
     double2* hpsi = (double2*)hpsi_;
     const bool fork = !(flags & HPSI_ONE_STREAM);
@@ -1431,7 +1496,9 @@ extern "C" int hpsi_apply_energies(hpsi_ctx* c, int kid, int nb, const double* p
     size_t o_e = dev ? 0 : cv.take<double>((size_t)nb);
     size_t o_work = cv.off;
     const EnergyWs w = energy_layout(c, nb, prec);
-    if ((rc = ws_reserve(c, o_work + w.work + apply_ws_bytes(c, *s, nb, prec, true)))) return rc;
+    if ((rc = ws_reserve_d64(c, o_work + w.work + apply_ws_bytes(c, *s, nb, prec, true),
+                             d64_apply_bytes(*s, nb, prec))))
+        return rc;
     const double2* psi = (const double2*)psi_;
     double2* hpsi = (double2*)hpsi_;
     double* e = eout;
@@ -1505,7 +1572,8 @@ extern "C" int hpsi_sternheimer(hpsi_ctx* c, int kid, int nv, const double* psi_
     const size_t o_act = cv.take<int>((size_t)nv);
     const size_t o_work = cv.off;
     const size_t work = std::max(apply_ws_bytes(c, *s, nv, prec), grad_ws_bytes(*s, nv, prec));
-    if ((rc = ws_reserve(c, o_work + work))) return rc;
+    const size_t d64 = std::max(d64_apply_bytes(*s, nv, prec), d64_grad_bytes(*s, nv, 1, prec));
+    if ((rc = ws_reserve_d64(c, o_work + work, d64))) return rc;
     unsigned char* ws = c->ws;
     const double2* psi = dev ? (const double2*)psi_ : reinterpret_cast<const double2*>(ws + o_psi);
     const double* eps = dev ? eps_ : reinterpret_cast<const double*>(ws + o_eps);
@@ -2023,7 +2091,8 @@ extern "C" int hpsi_grad_apply(hpsi_ctx* c, int kid, int nb, const double* psi_,
     for (int a = 0; a < 3; ++a)
         if (!dev && outs[a]) o_out[a] = cv.take<double2>(nel);
     size_t o_work = cv.off;
-    if ((rc = ws_reserve(c, o_work + grad_ws_bytes(*s, nb, prec)))) return rc;
+    const int nd = (dx != nullptr) + (dy != nullptr) + (dz != nullptr);
+    if ((rc = ws_reserve_d64(c, o_work + grad_ws_bytes(*s, nb, prec), d64_grad_bytes(*s, nb, nd, prec)))) return rc;
     const double2* psi = (const double2*)psi_;
     double2* d[3] = {(double2*)dx, (double2*)dy, (double2*)dz};
     if (!dev) {
@@ -2068,7 +2137,7 @@ extern "C" int hpsi_velocity_matrix(hpsi_ctx* c, int kid, int nb, const double* 
     size_t o_psi = dev ? 0 : cv.take<double2>(nel);
     size_t o_m = dev ? 0 : cv.take<double2>(nm);
     size_t o_work = cv.off;
-    if ((rc = ws_reserve(c, o_work + vel_ws_bytes(*s, nb, prec)))) return rc;
+    if ((rc = ws_reserve_d64(c, o_work + vel_ws_bytes(*s, nb, prec), d64_velocity_bytes(*s, nb, prec)))) return rc;
     const double2* psi = (const double2*)psi_;
     double2* m = (double2*)m_;
     if (!dev) {

@@ -201,13 +201,13 @@ struct ProjRow {
     int atom, rad, l, m;
 };
 
-// Projector matrices Pr[row][G] = beta*Y*S and, with grad, dPr_alpha rows at
-// row offsets (1+alpha)*P.
+// Projector matrices: with value rows Pr[row][G] = beta*Y*S, with grad dPr_alpha
+// rows at row offsets (1+alpha)*P.
 template <typename C>
 cudaError_t launch_assemble(int P, int npw, const ProjRow* rows, const double* beta, const double* dbeta,
                             const double* dbeta0, const double* q, const double* trig, const double* ylm,
-                            const double* yth, const double* yph, const double2* sf, bool grad, C* out,
-                            size_t ld, cudaStream_t st);
+                            const double* yth, const double* yph, const double2* sf, bool value, bool grad,
+                            C* out, size_t ld, cudaStream_t st);
 
 // ---- SIMT complex GEMMs (gemm.cu) -----------------------------------------
 // Projection, split over K: part[s][m][n] = sum_{k in split s} conj(A[m][k]) * B[n][k]

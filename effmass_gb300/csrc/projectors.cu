@@ -226,7 +226,7 @@ __global__ void assemble_kernel(int P, int npw, const ProjRow* __restrict__ rows
                                 const double* __restrict__ dbeta, const double* __restrict__ dbeta0,
                                 const double* __restrict__ q, const double* __restrict__ trig,
                                 const double* __restrict__ ylm, const double* __restrict__ yth,
-                                const double* __restrict__ yph, const double2* __restrict__ sf, bool grad,
+                                const double* __restrict__ yph, const double2* __restrict__ sf, bool value, bool grad,
                                 C* __restrict__ out, size_t ld)
 {
     const int ig = blockIdx.x * blockDim.x + threadIdx.x;
@@ -238,7 +238,7 @@ __global__ void assemble_kernel(int P, int npw, const ProjRow* __restrict__ rows
     const double y = ylm[lm];
     const double2 S = sf[(size_t)r.atom * npw + ig];
     const double by = b * y;
-    out[(size_t)row * ld + ig] = from_c128<C>(make_double2(by * S.x, by * S.y));
+    if (value) out[(size_t)row * ld + ig] = from_c128<C>(make_double2(by * S.x, by * S.y));
     if (grad) {
         const double qq = q[ig];
         const double boq = (qq > 1e-12) ? b / qq : dbeta0[r.rad];
@@ -257,18 +257,21 @@ __global__ void assemble_kernel(int P, int npw, const ProjRow* __restrict__ rows
 template <typename C>
 cudaError_t launch_assemble(int P, int npw, const ProjRow* rows, const double* beta, const double* dbeta,
                             const double* dbeta0, const double* q, const double* trig, const double* ylm,
-                            const double* yth, const double* yph, const double2* sf, bool grad, C* out, size_t ld,
-                            cudaStream_t st)
+                            const double* yth, const double* yph, const double2* sf, bool value, bool grad, C* out,
+                            size_t ld, cudaStream_t st)
 {
     if (P == 0 || npw == 0) return cudaSuccess;
     dim3 g(ceil_div(npw, 256), P);
-    assemble_kernel<C><<<g, 256, 0, st>>>(P, npw, rows, beta, dbeta, dbeta0, q, trig, ylm, yth, yph, sf, grad, out, ld);
+    assemble_kernel<C><<<g, 256, 0, st>>>(P, npw, rows, beta, dbeta, dbeta0, q, trig, ylm, yth, yph, sf, value, grad,
+                                               out, ld);
     return cudaGetLastError();
 }
 
 template cudaError_t launch_assemble<double2>(int, int, const ProjRow*, const double*, const double*, const double*,
                                               const double*, const double*, const double*, const double*,
-                                              const double*, const double2*, bool, double2*, size_t, cudaStream_t);
+                                              const double*, const double2*, bool, bool, double2*, size_t,
+                                              cudaStream_t);
 template cudaError_t launch_assemble<float2>(int, int, const ProjRow*, const double*, const double*, const double*,
                                              const double*, const double*, const double*, const double*,
-                                             const double*, const double2*, bool, float2*, size_t, cudaStream_t);
+                                             const double*, const double2*, bool, bool, float2*, size_t,
+                                             cudaStream_t);
