@@ -24,16 +24,20 @@
 // (projection / expansion, 2-norm): 4e-16 / 1e-16, where the FP64 SIMT GEMMs
 // have 1e-15 / 4e-16.
 //
-// What bounds it: the tensor pipe on large cells (64-atom cell, 128 bands: 72% of
+// What bounds it: the tensor pipe on large cells (64-atom cell, 128 bands: 80% of
 // the measured bf16 rate in the GEMMs).  The seven slices of a B tile lie one
-// after the other in shared memory and the eight diagonals in TMEM, so one MMA of
-// N = 256 multiplies slice i of A with four slices of B into four diagonals: 12
-// MMAs per 16 of K instead of 34, which the issuing thread could not feed (70
-// clocks each; projection 1.81 -> 1.43 ms, expansion 1.75 -> 1.39 ms there).
-// Reading the accumulators out costs 15% (0.22 ms of the projection).  Measured
-// and not kept: releasing the accumulators diagonal by diagonal (1.45 / 1.37 ms),
-// integers by FP32 magic adds in place of F2I (1.47 / 1.42 ms), 32 of K per stage
-// (SWIZZLE_64B, two stages).
+// after the other in shared memory and the eight diagonals in TMEM, so one MMA
+// of up to N = 224 multiplies slice i of A with all its slices of B into their
+// diagonals: 7 MMAs per 16 of K instead of 34, which the issuing thread could not
+// feed (70 clocks each).  Tiles of 16 bands (32 rows of B) leave TMEM room for two
+// sets of accumulators, so that one is read out under the next chunk's MMAs;
+// against tiles of 32 bands with one set, H|psi> us before -> now: 8-atom cell,
+// 48 bands 187 -> 173; 16 atoms, 37 bands 266 -> 234; 64 atoms, 128 bands
+// 5542 -> 5404; gradient, 8 atoms 129 -> 101.  What is left beside
+// the MMAs is writing the slices of A: 0.66 ms of the 64-atom call, at the rate
+// of the memory.  Tiles of A fetched by half or by a quarter do not change the
+// GEMMs' time, so A is not multicast.  Measured and not kept: integers by FP32
+// magic adds in place of F2I, 32 of K per stage (SWIZZLE_64B).
 //
 // Layout: K-major tiles of (rows x 16) FP16 digits, slice after slice: an A tile
 // is 7 x 4 KB and a B tile 7 x NT x 32 bytes of contiguous memory, already in
@@ -50,10 +54,15 @@ namespace {
 constexpr int S = 7;                      // slices per operand
 constexpr int ND = 8;                     // diagonals kept: i + j < ND
 constexpr int TM = 128;                   // A rows per tile
+constexpr int BT = 16;                    // bands per tile
+constexpr int NT = 2 * BT;                // B rows per tile: two sets of ND accumulators fill TMEM
 constexpr int KB = 16;                    // real K per pipeline stage (one MMA deep)
 constexpr int CHUNK = 8;                  // stages per read-out of the accumulators (128 of K)
 constexpr int FIX = 55;                   // bits of the fixed-point form
 constexpr int A_STAGE = S * TM * KB * 2;  // 28 KB
+constexpr int B_STAGE = S * NT * KB * 2;  // 7 KB
+constexpr int STAGE = A_STAGE + B_STAGE;
+constexpr int STAGES = 220 * 1024 / STAGE;  // that fit shared memory beside the barriers
 constexpr int DRAIN_WARPS = 16;
 constexpr int THREADS = 64 + 32 * DRAIN_WARPS;
 constexpr uint32_t TMEM_ALL = 512;
@@ -124,11 +133,6 @@ __device__ __forceinline__ uint64_t sdesc_sw32(uint32_t saddr)
            (uint64_t)6 << 61;
 }
 
-// pipeline stages that fit shared memory beside the barriers
-__host__ __device__ constexpr int stage_bytes(int NT) { return A_STAGE + S * NT * KB * 2; }
-__host__ __device__ constexpr int stages(int NT) { return 220 * 1024 / stage_bytes(NT); }
-constexpr int MAX_STAGES = 8;
-
 template <int I>
 __device__ __forceinline__ void store_slices(unsigned char* at, size_t stride, const unsigned long long (&u)[8])
 {
@@ -189,7 +193,7 @@ struct SplitArgs {
     size_t lda, ldb;
     const int *ek, *fm;     // exponents of A's columns and rows
     int R, row0;            // rows of the GEMM's A operand; first of this chunk
-    int nb, K, KT, BT;      // bands, complex K, stages, bands per tile
+    int nb, K, KT;          // bands, complex K, stages
     int a_x, a_blocks;      // A blocks per row of blocks, per GEMM
     int b_seg, b_blocks;    // B blocks per band, per GEMM
     unsigned char *a, *b;   // slices, nd times a_bytes / b_bytes
@@ -268,7 +272,7 @@ template <bool TRANS>
 __device__ __forceinline__ void split_b(const SplitArgs& s, int g, int block)
 {
     __shared__ int red[8];
-    const int bands = s.b_blocks / s.b_seg, b = block % bands, seg = block / bands, t = b / s.BT, j = b % s.BT;
+    const int bands = s.b_blocks / s.b_seg, b = block % bands, seg = block / bands, t = b / BT, j = b % BT;
     const KMap map = s.map[g];
     int f = 0;
     if (s.b_seg == 1) {
@@ -286,7 +290,7 @@ __device__ __forceinline__ void split_b(const SplitArgs& s, int g, int block)
         f = s.fb[g * bands + b];
     }
     f = clean(f);
-    const size_t slice = (size_t)2 * s.BT * KB * 2;
+    const size_t slice = (size_t)2 * BT * KB * 2;
     unsigned char* out = s.b + g * s.b_bytes + (size_t)t * s.KT * S * slice;
     const int per = s.b_seg == 1 ? 2 * s.KT : B_SEG / 4, q1 = min(2 * s.KT, (seg + 1) * per);
 #pragma unroll 2
@@ -310,7 +314,7 @@ __device__ __forceinline__ void split_b(const SplitArgs& s, int g, int block)
         }
         unsigned char* tile = out + (size_t)kt * S * slice;
         store_slices<0>(tile + slice_off(j, c), slice, re);
-        store_slices<0>(tile + slice_off(s.BT + j, c), slice, im);
+        store_slices<0>(tile + slice_off(BT + j, c), slice, im);
     }
 }
 
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs s)
 
 // ---- GEMM -------------------------------------------------------------------
 struct D64Smem {
-    uint64_t full[MAX_STAGES], empty[MAX_STAGES];
+    uint64_t full[STAGES], empty[STAGES];
     uint64_t dfull[2], dempty[2];  // accumulator set: a chunk's products final; read out
     uint64_t done;
     uint32_t tmem_base;
@@ -344,15 +348,11 @@ struct D64Out {
     int M, N, row0;  // result rows and bands; first row of this launch's A chunk
 };
 
-template <int CW>
-__device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&r)[CW])
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t (&r)[4])
 {
-    if constexpr (CW == 4)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                     : "r"(addr));
-    else
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
 }
 
 // (h 2^24 + l) 2^e rounded once to FP64, on the integer pipe
@@ -376,17 +376,12 @@ __device__ __forceinline__ double round_sum(long long h, long long l, int e)
     return scalbn(x, be - 1023);
 }
 
-// sets of ND accumulators of NT columns in TMEM
-__host__ __device__ constexpr int acc_sets(int NT) { return (int)TMEM_ALL / (ND * NT); }
-
-template <int NT, bool EXPAND>
+template <bool EXPAND>
 __global__ void __launch_bounds__(THREADS, 1)
     d64_gemm_kernel(const unsigned char* __restrict__ A, const unsigned char* __restrict__ B, D64Out o, int KT,
                     int chunks_per_split, int* err)
 {
-    constexpr int B_STAGE = S * NT * KB * 2, STAGE = stage_bytes(NT), STAGES = stages(NT), NBUF = acc_sets(NT);
-
-    constexpr int BT = NT / 2, BPW = BT / 4, CW = BPW % 4 == 0 ? 4 : 2;
+    constexpr int NBUF = TMEM_ALL / (ND * NT), BPW = BT / 4;  // accumulator sets, bands per warp
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     unsigned char* tiles = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -452,7 +447,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 break;
             }
             tc_fence_after();
-            const uint32_t acc = tmem + buf * 256;
+            const uint32_t acc = tmem + buf * (ND * NT);
             const int i1 = min(nk, (c + 1) * CHUNK);
             for (int it = c * CHUNK; it < i1; ++it) {
                 const int s = it % STAGES;
@@ -474,15 +469,15 @@ __global__ void __launch_bounds__(THREADS, 1)
                     tc_mma(acc + (i + j0) * NT, ad + ((i * TM * KB * 2) >> 4), bd + ((j0 * NT * KB * 2) >> 4),
                            idesc_f16(TM, n * NT, 0), overwrite ? 0u : 1u);
                 };
-                constexpr int W = 256 / NT < S ? 256 / NT : S;  // slices per MMA
-#pragma unroll
-                for (int i = 0; i < S; ++i) {
-                    const int nj = S < ND - i ? S : ND - i;  // j < nj
-                    const int whole = i == 1 ? nj - 1 : nj;
-#pragma unroll
-                    for (int j = 0; j < whole; j += W) mma(i, j, whole - j < W ? whole - j : W, i == 0 && first);
-                    if (i == 1) mma(1, nj - 1, 1, first);
+                mma(0, 0, S, first);
+                if (first) {
+                    mma(1, 0, ND - 2, false);
+                    mma(1, ND - 2, 1, true);
+                } else {
+                    mma(1, 0, ND - 1, false);
                 }
+#pragma unroll
+                for (int i = 2; i < S; ++i) mma(i, 0, ND - i, false);
                 tc_commit(&sh->empty[s]);
             }
             if (!stop) tc_commit(&sh->dfull[buf]);
@@ -506,21 +501,21 @@ __global__ void __launch_bounds__(THREADS, 1)
             go = __all_sync(0xffffffffu, ok && !*abort);
             if (!go) break;
             tc_fence_after();
-            const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + buf * 256 + sub * BPW;
+            const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + buf * (ND * NT) + sub * BPW;
 #pragma unroll
-            for (int p = 0; p < 2 * BPW; p += CW) {
+            for (int p = 0; p < 2 * BPW; p += BPW) {
                 const uint32_t at = base + (p < BPW ? p : BT + p - BPW);
-                uint32_t v[ND][CW];
+                uint32_t v[ND][BPW];
 #pragma unroll
-                for (int d = 0; d < ND; ++d) tmem_ld<CW>(at + d * NT, v[d]);
+                for (int d = 0; d < ND; ++d) tmem_ld4(at + d * NT, v[d]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (p + CW >= 2 * BPW) {
+                if (p + BPW >= 2 * BPW) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sh->dempty[buf]);
                 }
 #pragma unroll
-                for (int i = 0; i < CW; ++i) {
+                for (int i = 0; i < BPW; ++i) {
                     // exact integers: |diagonal d| <= 128 (d + 1) 2^14 < 2^24, the sums of
                     // two adjacent low diagonals within 32 bits
                     const int t01 = __float2int_rn(__uint_as_float(v[0][i])) * 256 + __float2int_rn(__uint_as_float(v[1][i]));
@@ -567,26 +562,16 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
 }
 
-size_t smem_bytes(int NT) { return (size_t)stages(NT) * stage_bytes(NT) + 1024 + sizeof(D64Smem); }
-
-template <int NT, bool EXPAND>
-cudaError_t launch_nt(dim3 grid, const unsigned char* A, const unsigned char* B, const D64Out& o, int KT, int cps,
-                      int* err, cudaStream_t st)
-{
-    const size_t smem = smem_bytes(NT);
-    const cudaError_t e = cudaFuncSetAttribute(d64_gemm_kernel<NT, EXPAND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem);
-    if (e) return e;
-    d64_gemm_kernel<NT, EXPAND><<<grid, THREADS, smem, st>>>(A, B, o, KT, cps, err);
-    return cudaGetLastError();
-}
-
 template <bool EXPAND>
-cudaError_t launch_gemm(int NT, dim3 grid, const unsigned char* A, const unsigned char* B, const D64Out& o, int KT,
-                        int cps, int* err, cudaStream_t st)
+cudaError_t launch_gemm(dim3 grid, const unsigned char* A, const unsigned char* B, const D64Out& o, int KT, int cps,
+                        int* err, cudaStream_t st)
 {
-    if (NT == 32) return launch_nt<32, EXPAND>(grid, A, B, o, KT, cps, err, st);
-    return launch_nt<64, EXPAND>(grid, A, B, o, KT, cps, err, st);
+    constexpr size_t smem = (size_t)STAGES * STAGE + 1024 + sizeof(D64Smem);
+    const cudaError_t e =
+        cudaFuncSetAttribute(d64_gemm_kernel<EXPAND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e) return e;
+    d64_gemm_kernel<EXPAND><<<grid, THREADS, smem, st>>>(A, B, o, KT, cps, err);
+    return cudaGetLastError();
 }
 
 int sms()
@@ -602,7 +587,7 @@ int sms()
 
 // Shape of one GEMM: R result rows (A operand), N bands, K complex terms.
 struct Plan {
-    int nt, BT, tiles_n;    // B rows per tile, bands per tile, tiles
+    int tiles_n;            // band tiles
     int n_pass;             // bands per pass
     int KT;                 // stages over K
     int mt, mt_chunk;       // row tiles, row tiles per A chunk
@@ -615,9 +600,7 @@ Plan plan(int R, int N, int K, bool split_k, int ng)
 {
     Plan p;
     p.n_pass = std::min(N, N_CAP);
-    p.BT = p.n_pass <= 16 ? 16 : 32;
-    p.nt = 2 * p.BT;
-    p.tiles_n = ceil_div(p.n_pass, p.BT);
+    p.tiles_n = ceil_div(p.n_pass, BT);
     p.KT = ceil_div(2l * K, KB);
     p.mt = ceil_div(R, TM);
     const int cap = (int)std::max<size_t>(1, std::min<size_t>(p.mt, A_CAP / ((size_t)p.KT * A_STAGE)));
@@ -637,8 +620,8 @@ Plan plan(int R, int N, int K, bool split_k, int ng)
     }
     p.nz = ceil_div(nch, p.cps);
     p.a_bytes = (size_t)p.mt_chunk * p.KT * A_STAGE;
-    p.b_bytes = (size_t)p.tiles_n * p.KT * S * p.nt * KB * 2;
-    p.fb_bytes = ((size_t)p.tiles_n * p.BT * sizeof(int) + 255) / 256 * 256;
+    p.b_bytes = (size_t)p.tiles_n * p.KT * B_STAGE;
+    p.fb_bytes = ((size_t)p.tiles_n * BT * sizeof(int) + 255) / 256 * 256;
     p.ng = ng;
     return p;
 }
@@ -660,11 +643,11 @@ cudaError_t run(const Plan& p, int R, int N, int K, const double2* A, size_t lda
 {
     SplitArgs s{};
     s.A = A; s.lda = lda; s.ldb = ldb; s.ek = sc.ek; s.fm = sc.fm;
-    s.R = R; s.K = K; s.KT = p.KT; s.BT = p.BT;
+    s.R = R; s.K = K; s.KT = p.KT;
     s.a = ws; s.b = ws + p.ng * p.a_bytes;
     s.a_bytes = p.a_bytes; s.b_bytes = p.b_bytes;
     s.fb = reinterpret_cast<int*>(s.b + p.ng * p.b_bytes);
-    const int bands = p.tiles_n * p.BT;
+    const int bands = p.tiles_n * BT;
     s.b_seg = K > 2 * B_SEG ? ceil_div(p.KT, B_SEG / 8) : 1;
     s.a_x = ceil_div(p.KT, 2);
     for (int g = 0; g < p.ng; ++g) s.map[g] = maps[g];
@@ -692,7 +675,7 @@ cudaError_t run(const Plan& p, int R, int N, int K, const double2* A, size_t lda
             o.er = EXPAND ? sc.ek : sc.fm;
             o.fb = s.fb;
             o.M = R; o.N = s.nb; o.row0 = s.row0;
-            const cudaError_t e = launch_gemm<EXPAND>(p.nt, dim3(p.tiles_n, mt, EXPAND ? p.ng : p.nz), s.a, s.b, o, p.KT,
+            const cudaError_t e = launch_gemm<EXPAND>(dim3(p.tiles_n, mt, EXPAND ? p.ng : p.nz), s.a, s.b, o, p.KT,
                                                       p.cps, err, st);
             if (e) return e;
         }
