@@ -1,5 +1,5 @@
-// gemm.cu — register-tiled SIMT complex GEMMs for the nonlocal term
-// (FP64 parity path and FP32 path).
+// gemm.cu — register-tiled SIMT complex GEMMs for the nonlocal term: the FP32
+// path, and FP64 where the digit-sliced GEMMs (d64_gemm.cu) have no workspace.
 //
 // The reference applies each projector separately with two passes over the
 // G-sphere per (atom, l, m, i) (src/H_psi/hamiltonian_callable.cpp:259-297):
@@ -8,9 +8,15 @@
 // matrix Pr[P][npw]:
 //   projection  W[P][nb]   = conj(Pr) psi^T       (K = npw, split over K)
 //   expansion   hpsi[nb][G] += (lambda W)^T Pr     (K = P)
-// Tiles: 64 x 64 outputs per 256-thread block, 16-deep K slices staged in
-// shared memory; each thread owns a 4 x 4 block of outputs at stride 16 so
-// that shared-memory reads of a warp are bank-conflict free.
+// Tiles: up to 64 x 64 outputs per 256-thread block, 16-deep K slices staged in
+// shared memory; each thread owns up to a 4 x 4 block of outputs at stride 16 so
+// that shared-memory reads of a warp are bank-conflict free.  What bounds them on
+// the smaller cells is the latency of a block's loads and too few blocks, so the
+// next slice is fetched while one is multiplied, and tiles shrink while blocks do
+// not fill the SMs.  FP32, us before -> now: H|psi> of 2 atoms, 32 bands 41 -> 34;
+// 8 atoms, 48 bands 85 -> 58 (projection 26 -> 13, expansion 26 -> 13); 16 atoms,
+// 37 bands 197 -> 156; 64 atoms, 16 bands 878 -> 646; gradient, 8 atoms, 48 bands
+// 194 -> 109.  All sums keep their order: the results are the same bits.
 #include <type_traits>
 #include "kernels.cuh"
 
@@ -21,14 +27,29 @@ template <> HPSI_D float2 load_as<float2, double2>(const double2& v) { return to
 template <> HPSI_D float2 load_as<float2, float2>(const float2& v) { return v; }
 template <> HPSI_D double2 load_as<double2, float2>(const float2& v) { return to_c128(v); }
 
+// r + i s += conj(a) b.  In FP32 the roundings are written out, so that a result
+// does not depend on the tile that computes it: the product of the imaginary
+// parts is the one rounded by itself, with YFIRST that of the real parts.
+template <bool YFIRST>
+HPSI_D void mac_conj(double& r, double& s, double2 a, double2 b)
+{
+    r += a.x * b.x + a.y * b.y;
+    s += a.x * b.y - a.y * b.x;
+}
+template <bool YFIRST>
+HPSI_D void mac_conj(float& r, float& s, float2 a, float2 b)
+{
+    r = __fadd_rn(r, YFIRST ? __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)) : __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+    s = __fadd_rn(s, __fmaf_rn(a.x, b.y, -__fmul_rn(a.y, b.x)));
+}
+
 constexpr int GB_K = 16;  // K slice staged per iteration
 
 // Projection tile: (16 TM) x (16 TN) outputs per 256-thread block, each thread
 // TM x TN at stride 16 (conflict-free shared-memory reads).  The launcher picks
 // the tile from M and N so that small problems (a few bands, few projectors)
-// do not spend the block on padding — FP64 runs at a small fraction of the
-// FP32 rate on this part, so wasted FP64 work shows directly.
-template <typename TA, typename TB, typename Acc, int TM, int TN>
+// do not spend the block on padding.
+template <typename TA, typename TB, typename Acc, int TM, int TN, bool YFIRST>
 __global__ void __launch_bounds__(256) proj_gemm_kernel(int M, int N, int K, const TA* __restrict__ A, size_t lda,
                                                         const TB* __restrict__ B, size_t ldb, Acc* __restrict__ part,
                                                         int kchunk)
@@ -47,16 +68,31 @@ __global__ void __launch_bounds__(256) proj_gemm_kernel(int M, int N, int K, con
 #pragma unroll
         for (int j = 0; j < TN; ++j) accr[i][j] = acci[i][j] = 0;
 
+    // The next slice's elements travel in registers while a slice is multiplied:
+    // a block of a short split is bound by the latency of its loads.
+    const int kk0 = threadIdx.x % GB_K, r0 = threadIdx.x / GB_K;
+    Acc av[TM], bv[TN];
+    auto fetch = [&](int k0) {
+        const int gk = k0 + kk0;
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int r = m0 + r0 + 16 * i;
+            av[i] = (r < M && gk < kend) ? load_as<Acc>(A[(size_t)r * lda + gk]) : cmake<Acc>(0, 0);
+        }
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int r = n0 + r0 + 16 * j;
+            bv[j] = (r < N && gk < kend) ? load_as<Acc>(B[(size_t)r * ldb + gk]) : cmake<Acc>(0, 0);
+        }
+    };
+    if (kbeg < kend) fetch(kbeg);
     for (int k0 = kbeg; k0 < kend; k0 += GB_K) {
-        for (int e = threadIdx.x; e < BM * GB_K; e += 256) {
-            const int r = e / GB_K, kk = e % GB_K, gk = k0 + kk;
-            As[kk][r] = (m0 + r < M && gk < kend) ? load_as<Acc>(A[(size_t)(m0 + r) * lda + gk]) : cmake<Acc>(0, 0);
-        }
-        for (int e = threadIdx.x; e < BN * GB_K; e += 256) {
-            const int r = e / GB_K, kk = e % GB_K, gk = k0 + kk;
-            Bs[kk][r] = (n0 + r < N && gk < kend) ? load_as<Acc>(B[(size_t)(n0 + r) * ldb + gk]) : cmake<Acc>(0, 0);
-        }
+#pragma unroll
+        for (int i = 0; i < TM; ++i) As[kk0][r0 + 16 * i] = av[i];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) Bs[kk0][r0 + 16 * j] = bv[j];
         __syncthreads();
+        if (k0 + GB_K < kend) fetch(k0 + GB_K);
 #pragma unroll
         for (int kk = 0; kk < GB_K; ++kk) {
             Acc a[TM], b[TN];
@@ -68,9 +104,7 @@ __global__ void __launch_bounds__(256) proj_gemm_kernel(int M, int N, int K, con
             for (int i = 0; i < TM; ++i)
 #pragma unroll
                 for (int j = 0; j < TN; ++j) {
-                    // conj(a) * b
-                    accr[i][j] += a[i].x * b[j].x + a[i].y * b[j].y;
-                    acci[i][j] += a[i].x * b[j].y - a[i].y * b[j].x;
+                    mac_conj<YFIRST>(accr[i][j], acci[i][j], a[i], b[j]);
                 }
         }
         __syncthreads();
@@ -89,11 +123,11 @@ __global__ void __launch_bounds__(256) proj_gemm_kernel(int M, int N, int K, con
 
 static inline int tile_mult(int extent) { return extent <= 16 ? 1 : (extent <= 32 ? 2 : 4); }
 
-template <typename TA, typename TB, typename Acc, int TM, int TN>
+template <typename TA, typename TB, typename Acc, int TM, int TN, bool YFIRST = false>
 static void proj_launch(dim3 g, int M, int N, int K, const TA* A, size_t lda, const TB* B, size_t ldb, Acc* part,
                         int kchunk, cudaStream_t st)
 {
-    proj_gemm_kernel<TA, TB, Acc, TM, TN><<<g, 256, 0, st>>>(M, N, K, A, lda, B, ldb, part, kchunk);
+    proj_gemm_kernel<TA, TB, Acc, TM, TN, YFIRST><<<g, 256, 0, st>>>(M, N, K, A, lda, B, ldb, part, kchunk);
 }
 
 template <typename TA, typename TB, typename Acc>
@@ -103,10 +137,17 @@ cudaError_t launch_proj_gemm(int M, int N, int K, const TA* A, size_t lda, const
     if (M == 0 || N == 0) return cudaSuccess;
     int kchunk = ceil_div(K, nsplit);
     kchunk = ceil_div(kchunk, GB_K) * GB_K;
-    const int tm = tile_mult(M), tn = tile_mult(N);
+    int tm = tile_mult(M), tn = tile_mult(N);
+    const bool one_tile = tm == 1 && tn == 1;
+    // smaller tiles while the blocks do not fill the SMs (P = 64, K = 3000, 48 bands: 26 -> 17 us);
+    // the splits stay, and with them the order of the sums
+    const auto blocks = [&] { return ceil_div(M, 16 * tm) * ceil_div(N, 16 * tn) * nsplit; };
+    while (tn > 1 && blocks() < 152) tn /= 2;
+    while (tm > 1 && blocks() < 152) tm /= 2;
     dim3 g(ceil_div(M, 16 * tm), ceil_div(N, 16 * tn), nsplit);
     // nsplit partial slabs are written even when K is split finer than needed (empty chunks write zeros)
-    if (tm == 1 && tn == 1) proj_launch<TA, TB, Acc, 1, 1>(g, M, N, K, A, lda, B, ldb, part, kchunk, st);
+    if (one_tile) proj_launch<TA, TB, Acc, 1, 1, true>(g, M, N, K, A, lda, B, ldb, part, kchunk, st);
+    else if (tm == 1 && tn == 1) proj_launch<TA, TB, Acc, 1, 1>(g, M, N, K, A, lda, B, ldb, part, kchunk, st);
     else if (tm == 1 && tn == 2) proj_launch<TA, TB, Acc, 1, 2>(g, M, N, K, A, lda, B, ldb, part, kchunk, st);
     else if (tm == 2 && tn == 1) proj_launch<TA, TB, Acc, 2, 1>(g, M, N, K, A, lda, B, ldb, part, kchunk, st);
     else if (tm == 2 && tn == 2) proj_launch<TA, TB, Acc, 2, 2>(g, M, N, K, A, lda, B, ldb, part, kchunk, st);
@@ -184,16 +225,41 @@ __global__ void __launch_bounds__(256) expand_gemm_kernel(int M, int N, int K, c
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) accr[i][j] = acci[i][j] = 0;
+    // small tiles fetch their outputs beside the first slice
+    constexpr bool EARLY = TM * TN <= 8;
+    double2 o[TM][TN];
+    auto fetch_out = [&]() {
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int n = n0 + ty + 16 * i, k = k0 + tx + 16 * j;
+                o[i][j] = (n < N && k < K) ? out[(size_t)n * ldo + k] : make_double2(0.0, 0.0);
+            }
+    };
+    // the next slice travels in registers while a slice is multiplied
+    C wv[TM], av[TN];
+    auto fetch = [&](int m0) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int e = threadIdx.x + 256 * i, gm = m0 + e / BN, c = n0 + e % BN;
+            wv[i] = (gm < M && c < N) ? W[(size_t)gm * ldw + c] : cmake<C>(0, 0);
+        }
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int e = threadIdx.x + 256 * j, gm = m0 + e / BK, c = k0 + e % BK;
+            av[j] = (gm < M && c < K) ? A[(size_t)gm * lda + c] : cmake<C>(0, 0);
+        }
+    };
+    if (M > 0) fetch(0);
+    if (EARLY) fetch_out();
     for (int m0 = 0; m0 < M; m0 += GB_K) {
-        for (int e = threadIdx.x; e < GB_K * BN; e += 256) {
-            const int mm = e / BN, c = e % BN, gm = m0 + mm;
-            Ws[mm][c] = (gm < M && n0 + c < N) ? W[(size_t)gm * ldw + n0 + c] : cmake<C>(0, 0);
-        }
-        for (int e = threadIdx.x; e < GB_K * BK; e += 256) {
-            const int mm = e / BK, c = e % BK, gm = m0 + mm;
-            As[mm][c] = (gm < M && k0 + c < K) ? A[(size_t)gm * lda + k0 + c] : cmake<C>(0, 0);
-        }
+#pragma unroll
+        for (int i = 0; i < TM; ++i) Ws[(threadIdx.x + 256 * i) / BN][(threadIdx.x + 256 * i) % BN] = wv[i];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) As[(threadIdx.x + 256 * j) / BK][(threadIdx.x + 256 * j) % BK] = av[j];
         __syncthreads();
+        if (m0 + GB_K < M) fetch(m0 + GB_K);
 #pragma unroll
         for (int mm = 0; mm < GB_K; ++mm) {
             C w[TM], a[TN];
@@ -212,14 +278,7 @@ __global__ void __launch_bounds__(256) expand_gemm_kernel(int M, int N, int K, c
         __syncthreads();
     }
     // all loads of the read-modify-write first, so that they overlap
-    double2 o[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int n = n0 + ty + 16 * i, k = k0 + tx + 16 * j;
-            o[i][j] = (n < N && k < K) ? out[(size_t)n * ldo + k] : make_double2(0.0, 0.0);
-        }
+    if (!EARLY) fetch_out();
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -238,17 +297,15 @@ cudaError_t launch_expand_gemm(int M, int N, int K, const C* W, size_t ldw, cons
                                size_t ldo, cudaStream_t st)
 {
     if (N == 0 || K == 0 || M == 0) return cudaSuccess;
-    // few bands: a narrow band tile and four G-columns per thread
-    if (N <= 16) {
-        dim3 g(ceil_div(K, 64), ceil_div(N, 16));
-        expand_gemm_kernel<C, 1, 4><<<g, 256, 0, st>>>(M, N, K, W, ldw, A, lda, out, ldo);
-    } else if (N <= 32) {
-        dim3 g(ceil_div(K, 64), ceil_div(N, 32));
-        expand_gemm_kernel<C, 2, 4><<<g, 256, 0, st>>>(M, N, K, W, ldw, A, lda, out, ldo);
-    } else {
-        dim3 g(ceil_div(K, 64), ceil_div(N, 64));
-        expand_gemm_kernel<C, 4, 4><<<g, 256, 0, st>>>(M, N, K, W, ldw, A, lda, out, ldo);
-    }
+    // few bands: a narrow band tile; four G-columns per thread, or one where that
+    // would leave SMs without a block (P = 64, K = 3000, 48 bands: 26 -> 12 us)
+    const bool small = ceil_div(K, 64) * ceil_div(N, 64) < 152;
+    auto go = [&](auto kernel, int bn, int bk) {
+        kernel<<<dim3(ceil_div(K, bk), ceil_div(N, bn)), 256, 0, st>>>(M, N, K, W, ldw, A, lda, out, ldo);
+    };
+    if (N <= 16) small ? go(expand_gemm_kernel<C, 1, 1>, 16, 16) : go(expand_gemm_kernel<C, 1, 4>, 16, 64);
+    else if (N <= 32 || small) small ? go(expand_gemm_kernel<C, 2, 1>, 32, 16) : go(expand_gemm_kernel<C, 2, 4>, 32, 64);
+    else go(expand_gemm_kernel<C, 4, 4>, 64, 64);
     return cudaGetLastError();
 }
 
