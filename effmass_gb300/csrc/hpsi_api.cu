@@ -449,12 +449,11 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
 
 static int split_for(int M, int N, int K) { return proj_gemm_splits(M, N, K); }
 
-// hpsi_out[nb][npw] += nonlocal(psi) using projector matrix pr (complex C)
+// W = lambda Pr^* psi^T in ws, with projector matrix pr (complex C)
 template <typename C, typename Acc>
-static int nonlocal_apply(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* hpsi, const C* pr,
-                          unsigned char* ws, cudaStream_t st, double* e_nl = nullptr)
+static int nonlocal_project(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const C* pr, unsigned char* ws,
+                            cudaStream_t st, double* e_nl, C** W_out)
 {
-    if (s.P == 0 || nb == 0) return HPSI_OK;
     const int ns = split_for(s.P, nb, s.npw);
     Carver cv;
     size_t o_part = cv.take<Acc>((size_t)ns * s.P * nb);
@@ -468,10 +467,29 @@ static int nonlocal_apply(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, dou
     h = c->prof.open(PH_REDUCE, st);
     CUDA_TRY(c, (launch_reduce_splits<Acc, C>(s.P, nb, ns, part, s.d_lam, s.P, W, (size_t)nb, st)));
     c->prof.close(h, st);
-    h = c->prof.open(PH_EXPAND, st);
+    *W_out = W;
+    return HPSI_OK;
+}
+
+// hpsi[nb][npw] += Pr^T W
+template <typename C>
+static int nonlocal_expand(hpsi_ctx* c, KSlot& s, int nb, const C* W, double2* hpsi, const C* pr, cudaStream_t st)
+{
+    int h = c->prof.open(PH_EXPAND, st);
     CUDA_TRY(c, launch_expand_gemm<C>(s.P, nb, s.npw, W, (size_t)nb, pr, (size_t)s.npw, hpsi, (size_t)s.npw, st));
     c->prof.close(h, st);
     return HPSI_OK;
+}
+
+// hpsi[nb][npw] += nonlocal(psi)
+template <typename C, typename Acc>
+static int nonlocal_apply(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2* hpsi, const C* pr,
+                          unsigned char* ws, cudaStream_t st, double* e_nl = nullptr)
+{
+    if (s.P == 0 || nb == 0) return HPSI_OK;
+    C* W = nullptr;
+    const int rc = nonlocal_project<C, Acc>(c, s, nb, psi, pr, ws, st, e_nl, &W);
+    return rc ? rc : nonlocal_expand<C>(c, s, nb, W, hpsi, pr, st);
 }
 
 // ---- FP64 nonlocal term on the tensor cores ----------------------------------
@@ -1075,6 +1093,19 @@ int prepare_slot(hpsi_ctx* c, KSlot& s, int prec, bool grad, cudaStream_t st)
     return ensure_proj<float2>(c, s, grad, st);
 }
 
+// FP32: whether the projection chain goes beside the FFT passes.  Both ends
+// measured (us, one stream -> side stream): below, the two events cost more than
+// they hide (2 atoms, 16 projectors, 756 plane waves: 48 bands 34.8 -> 37.0, 64
+// bands 36.9 -> 35.8; 8 atoms: 1 band 40 -> 37, 48 bands 58 -> 43; 16 atoms, 37
+// bands 156 -> 126); above, the GEMM fills the SMs by itself and the passes
+// only push its last blocks back (16 atoms, 128 bands 347 -> 320; 64 atoms: 1
+// band 591 -> 563, 16 bands 646 -> 705).
+static bool fork_fp32(const KSlot& s, int nb)
+{
+    const double work = (double)s.P * s.npw * (nb + 8);
+    return work > 0.8e6 && work < 250e6;
+}
+
 // workspace of one H|psi> on device pointers
 static size_t apply_ws_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int prec, bool energy = false)
 {
@@ -1086,8 +1117,8 @@ static size_t apply_ws_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int prec
         cv.take<float2>((size_t)nb * s.npw);
         return wl + tc_ws(s, nb, energy) + (s.P > 0 ? cv.off : 0);
     }
-    size_t wn = fp64 ? nonlocal_ws<double2, double2>(s, nb, 1) : nonlocal_ws<float2, float2>(s, nb, 1);
-    return std::max(wl, wn);
+    if (fp64) return std::max(wl, nonlocal_ws<double2, double2>(s, nb, 1));
+    return wl + nonlocal_ws<float2, float2>(s, nb, 1);  // disjoint: they run concurrently
 }
 
 // hpsi += H psi on device pointers with an explicit workspace (prepare_slot first)
@@ -1198,6 +1229,20 @@ static int apply_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2*
         }
         if (hpsi_ready) CUDA_TRY(c, cudaStreamWaitEvent(st, hpsi_ready, 0));
         return tc_nonlocal_expand(c, s, nb, hpsi, wnl, st, e_nl != nullptr, loc32);
+    }
+    if (fork && fork_fp32(s, nb)) {
+        // the projection chain beside the FFT passes as well, in the workspace behind theirs
+        float2* W = nullptr;
+        CUDA_TRY(c, cudaEventRecord(c->ev_fork, st));
+        CUDA_TRY(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
+        rc = nonlocal_project<float2, float2>(c, s, nb, psi, s.pr32, work + local_ws(c, s, nb, sizeof(float2)), c->side,
+                                              e_nl, &W);
+        const cudaError_t e = cudaEventRecord(c->ev_join, c->side);  // join even after an error
+        const int rl = local_apply<float2, float>(c, s, nb, psi, hpsi, work, c->d_v32, c->d_tw32, st, epart);
+        CUDA_TRY(c, e);
+        CUDA_TRY(c, cudaStreamWaitEvent(st, c->ev_join, 0));
+        if (rc || rl) return rc ? rc : rl;
+        return nonlocal_expand<float2>(c, s, nb, W, hpsi, s.pr32, st);
     }
     if ((rc = local_apply<float2, float>(c, s, nb, psi, hpsi, work, c->d_v32, c->d_tw32, st, epart))) return rc;
     return nonlocal_apply<float2, float2>(c, s, nb, psi, hpsi, s.pr32, work, st, e_nl);

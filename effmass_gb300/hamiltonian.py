@@ -143,8 +143,8 @@ class Hamiltonian:
 
     # -- raw calls --
     def apply(self, kid: int, nb: int, psi, hpsi, precision: Optional[str] = None, one_stream: bool = False):
-        """hpsi += H psi.  one_stream: keep the (FP64 or tensor-core) projection chain on
-        the caller's stream (HPSI_ONE_STREAM) instead of the side stream."""
+        """hpsi += H psi.  one_stream: keep the projection chain on the caller's
+        stream (HPSI_ONE_STREAM) instead of the side stream."""
         npw = self.dim(kid)
         p, dev_p = _ptr(psi, npw, nb, "psi")
         h, dev_h = _ptr(hpsi, npw, nb, "hpsi")

@@ -73,7 +73,7 @@ extern "C" {
 #define HPSI_PREC_MASK    0xF
 #define HPSI_DEVICE_PTRS  0x10 /* psi/outputs are device pointers (else host memory) */
 #define HPSI_SYNC         0x20 /* synchronise `stream` before returning */
-#define HPSI_ONE_STREAM   0x40 /* FP64 and tensor-core hpsi_apply / hpsi_apply_energies: run
+#define HPSI_ONE_STREAM   0x40 /* hpsi_apply / hpsi_apply_energies at any precision: run
                                 * the projection chain on `stream` too instead of on the
                                 * context's side stream beside the FFT passes */
 

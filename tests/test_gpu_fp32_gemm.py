@@ -1,8 +1,10 @@
-"""FP32 projector GEMMs (csrc/gemm.cu) at the edges of their tiles.
+"""FP32 projector GEMMs (csrc/gemm.cu) at the edges of their tiles, and the side stream of FP32 calls.
 
 H|psi> in FP32 is compared with FP64 per band.  Tolerance: sums of K <= 3000
 terms, each rounded to 24 bits, are off by sqrt(K) 2^-24 = 3e-6 of their
-2-norm; ten times that, 3e-5, allows for cancellation in the expansion.
+2-norm; ten times that, 3e-5, allows for cancellation in the expansion.  The
+projection chain on the side stream adds the same terms in the same order as
+on the caller's, so both give the same bits.
 """
 import numpy as np
 import pytest
@@ -29,11 +31,12 @@ def test_fp32_apply(name, nb):
     psi = rng.standard_normal((nb, kp.npw)) + 1j * rng.standard_normal((nb, kp.npw))
     psi = torch.from_numpy(psi / (1.0 + kp.kinetic)).cuda()
     outs = []
-    for prec in ("fp64", "fp32"):
+    for prec, one in (("fp64", False), ("fp32", False), ("fp32", True)):
         out = torch.zeros_like(psi)
-        H.apply(0, nb, psi, out, prec)
+        H.apply(0, nb, psi, out, prec, one_stream=one)
         torch.cuda.synchronize()
         outs.append(out)
-    ref, out = outs
-    assert float((torch.linalg.norm(out - ref, dim=1) / torch.linalg.norm(ref, dim=1)).max()) <= TOL
+    ref, side, one = outs
+    assert float((torch.linalg.norm(side - ref, dim=1) / torch.linalg.norm(ref, dim=1)).max()) <= TOL
+    assert torch.equal(side, one)
     H.close()
