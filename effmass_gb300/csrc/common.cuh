@@ -55,6 +55,10 @@ __device__ __forceinline__ double f2d_bits(float x)
     const uint32_t lo = normal ? u << 29 : 0u;
     return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
+
+// to FP64 off the FP64 pipe
+__device__ __forceinline__ double widen(float x) { return f2d_bits(x); }
+__device__ __forceinline__ double widen(double x) { return x; }
 #endif
 
 HPSI_HD float2 to_c64(double2 a)

@@ -285,8 +285,8 @@ __global__ void __launch_bounds__(256) expand_gemm_kernel(int M, int N, int K, c
         for (int j = 0; j < TN; ++j) {
             const int n = n0 + ty + 16 * i, k = k0 + tx + 16 * j;
             if (n < N && k < K) {
-                o[i][j].x += (double)accr[i][j];
-                o[i][j].y += (double)acci[i][j];
+                o[i][j].x += widen(accr[i][j]);
+                o[i][j].y += widen(acci[i][j]);
                 out[(size_t)n * ldo + k] = o[i][j];
             }
         }
