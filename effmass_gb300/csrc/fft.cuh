@@ -292,16 +292,20 @@ HPSI_D void fft_stage_io_p(int p, const LD& ld, const ST& st, int n, const FastD
     }
 }
 
-// ---- compile-time two-stage transforms --------------------------------------
+// ---- compile-time two- and three-stage transforms ----------------------------
 // For the grid lengths of the common cells (72 = 8*9, 36 = 9*4, 24 = 8*3,
-// 64 = 8*8) the stage shapes are template constants: the per-element index
+// 64 = 8*8, 60 = 4*3*5, ...) the stage shapes are template constants: the per-element index
 // arithmetic (butterfly -> group and offset, twiddle index, output position)
 // folds into constant multiplies and shifts instead of runtime divisions.
 // The radix order is the one fft_factor picks: the same arithmetic as the
 // runtime-plan path.
 template <int R0, int R1>
 struct FftPlan2 {
-    static constexpr int r0 = R0, r1 = R1, n = R0 * R1;
+    static constexpr int r0 = R0, r1 = R1, r2 = 1, n = R0 * R1;
+};
+template <int R0, int R1, int R2>
+struct FftPlan3 {
+    static constexpr int r0 = R0, r1 = R1, r2 = R2, n = R0 * R1 * R2;
 };
 
 // Line accessor with compile-time strides: element e of line L at b[L*LS + e*ES]
@@ -339,29 +343,40 @@ HPSI_D void fft_stage_ct(const LD& ld, const ST& st, const FastDiv& nlf, const C
     }
 }
 
-// Two-stage transform of nl lines: stage 0 reads through ld and writes bufA
-// (line stride ls, element stride es), stage 1 reads bufA and writes through
-// st (the same buffer contract as fft_lines_io with nst == 2: the last stage
-// reads bufA).
+// Transform of nl lines: stage 0 reads through ld and writes bufA (line stride ls,
+// element stride es), the last stage writes through st (the same buffer contract
+// as fft_lines_io: the last of two stages reads bufA, of three bufB).
 template <typename C, typename PL, typename LD, typename ST>
-HPSI_D void fft_lines_ct(const LD& ld, const ST& st, C* bufA, const FastDiv& nlf, int ls, int es, const C* tw,
+HPSI_D void fft_lines_ct(const LD& ld, const ST& st, C* bufA, C* bufB, const FastDiv& nlf, int ls, int es, const C* tw,
                          int sign)
 {
-    const SmemLines<C> A{bufA, ls, es};
+    const SmemLines<C> A{bufA, ls, es}, B{bufB, ls, es};
     fft_stage_ct<C, PL::n, PL::r0, 1, 0>(ld, A, nlf, tw, sign);
     __syncthreads();
-    fft_stage_ct<C, PL::n, PL::r1, PL::r0, 0>(A, st, nlf, tw, sign);
+    if constexpr (PL::r2 == 1) {
+        fft_stage_ct<C, PL::n, PL::r1, PL::r0, 0>(A, st, nlf, tw, sign);
+    } else {
+        fft_stage_ct<C, PL::n, PL::r1, PL::r0, 0>(A, B, nlf, tw, sign);
+        __syncthreads();
+        fft_stage_ct<C, PL::n, PL::r2, PL::r0 * PL::r1, 0>(B, st, nlf, tw, sign);
+    }
 }
 
-// The same with a compile-time line count NLC and intermediate accessor A
+// The same with a compile-time line count NLC and intermediate accessors A, B
 // (constant strides): no runtime index arithmetic left but the loop.
 template <typename C, typename PL, int NLC, typename AB, typename LD, typename ST>
-HPSI_D void fft_lines_cc(const LD& ld, const ST& st, const AB& A, const C* tw, int sign)
+HPSI_D void fft_lines_cc(const LD& ld, const ST& st, const AB& A, const AB& B, const C* tw, int sign)
 {
     const FastDiv unused{};
     fft_stage_ct<C, PL::n, PL::r0, 1, NLC>(ld, A, unused, tw, sign);
     __syncthreads();
-    fft_stage_ct<C, PL::n, PL::r1, PL::r0, NLC>(A, st, unused, tw, sign);
+    if constexpr (PL::r2 == 1) {
+        fft_stage_ct<C, PL::n, PL::r1, PL::r0, NLC>(A, st, unused, tw, sign);
+    } else {
+        fft_stage_ct<C, PL::n, PL::r1, PL::r0, NLC>(A, B, unused, tw, sign);
+        __syncthreads();
+        fft_stage_ct<C, PL::n, PL::r2, PL::r0 * PL::r1, NLC>(B, st, unused, tw, sign);
+    }
 }
 
 // ---- pruned plane transforms --------------------------------------------
@@ -407,8 +422,9 @@ HPSI_D void fft_stage_rows(const LD& ld, const ST& st, int nl, float rinv, const
     }
 }
 
-// Two-stage transform of the rows in use (jr as above; 2 jr + 1 < n) of a
-// plane with line stride LS and element stride ES: in -> A -> out (in may be out)
+// Transform of the rows in use (jr as above; 2 jr + 1 < n) of a plane with line
+// stride LS and element stride ES: two stages in -> A -> out (in may be out),
+// three in -> A -> in -> out (A may be out)
 template <typename C, typename PL, int LS, int ES>
 HPSI_D void fft_rows_cc(C* in, C* out, C* A, int jr, const C* tw, int sign)
 {
@@ -417,8 +433,14 @@ HPSI_D void fft_rows_cc(C* in, C* out, C* A, int jr, const C* tw, int sign)
     fft_stage_rows<C, PL::n, PL::r0, 1>(SmemRowsC<C, LS, ES>{in, jr, gap}, SmemRowsC<C, LS, ES>{A, jr, gap}, nl, rinv,
                                         tw, sign);
     __syncthreads();
-    fft_stage_rows<C, PL::n, PL::r1, PL::r0>(SmemRowsC<C, LS, ES>{A, jr, gap}, SmemRowsC<C, LS, ES>{out, jr, gap}, nl,
-                                             rinv, tw, sign);
+    constexpr bool two = PL::r2 == 1;
+    fft_stage_rows<C, PL::n, PL::r1, PL::r0>(SmemRowsC<C, LS, ES>{A, jr, gap},
+                                             SmemRowsC<C, LS, ES>{two ? out : in, jr, gap}, nl, rinv, tw, sign);
+    if constexpr (!two) {
+        __syncthreads();
+        fft_stage_rows<C, PL::n, PL::r2, PL::r0 * PL::r1>(SmemRowsC<C, LS, ES>{in, jr, gap},
+                                                          SmemRowsC<C, LS, ES>{out, jr, gap}, nl, rinv, tw, sign);
+    }
 }
 
 // Plan ids the host selects (0 = runtime plan)

@@ -51,13 +51,13 @@ constexpr int xpass_min()
 }
 
 // Transform of a kernel's lines: the runtime plan (NoPlan) or a compile-time
-// two-stage plan (FftPlan2) chosen by the host for common grid lengths.
+// plan (FftPlan2, FftPlan3) chosen by the host for common grid lengths.
 template <typename C, bool WIDE, typename PL, typename LD, typename ST>
 HPSI_D void lines(const LD& ld, const ST& st, C* bufA, C* bufB, const FftLen& L, const FastDiv& nlf, int ls, int es,
                   const C* tw, int sign)
 {
     if constexpr (std::is_same<PL, NoPlan>::value) fft_lines_io<C, true, WIDE>(ld, st, bufA, bufB, L, nlf, ls, es, tw, sign);
-    else fft_lines_ct<C, PL>(ld, st, bufA, nlf, ls, es, tw, sign);
+    else fft_lines_ct<C, PL>(ld, st, bufA, bufB, nlf, ls, es, tw, sign);
 }
 
 // Shared-memory planes use a padded row stride n3p = n3 + 1 (odd) so that
@@ -84,8 +84,8 @@ struct PlaneGlobalC {
     HPSI_D void operator()(int L, int e, C v) const { p[e * N3 + L] = v; }
 };
 
-// grid length of an axis: the compile-time plan's when there is one (then all
-// three axes share it), else the runtime value
+// grid length of a plane's axes: the compile-time plan's when there is one (then
+// both share it), else the runtime value
 template <typename PL>
 HPSI_D int plan_n(int runtime)
 {
@@ -119,6 +119,9 @@ __global__ void __launch_bounds__(Cfg<C>::g2r_threads, WIDE ? 1 : Cfg<C>::plane_
     for (int t = threadIdx.x; t < n2; t += blockDim.x) twy[t] = tw_y_g[t];
     for (int t = threadIdx.x; t < n3; t += blockDim.x) twz[t] = tw_z_g[t];
     for (int t = threadIdx.x; t < n23p; t += blockDim.x) b0[t] = cmake<C>(0, 0);
+    if constexpr (!std::is_same<PL, NoPlan>::value)
+        if (PL::r2 > 1)  // three stages end in b1: its rows not in use are zero too
+            for (int t = threadIdx.x; t < n23p; t += blockDim.x) b1[t] = cmake<C>(0, 0);
     __syncthreads();
     const double2* ps = psi + (size_t)b * npw;
     const int e0 = plane_off[p], e1 = plane_off[p + 1];
@@ -161,17 +164,17 @@ __global__ void __launch_bounds__(Cfg<C>::g2r_threads, WIDE ? 1 : Cfg<C>::plane_
                            +1);
     } else {
         constexpr int N = PL::n, NP = PL::n + 1;  // n2 = n3 = N lines per axis
-        // z-lines of the rows in use only: the other rows of b0 are zero and
-        // stay zero in zo (= b0 for these two-stage plans)
+        // z-lines of the rows in use only: the other rows are zero in zo (b0 for
+        // two stages, b1 for three)
         const int jr = plane_jr ? plane_jr[p] : N;
-        if (2 * jr + 1 < N && zo == b0)
+        if (2 * jr + 1 < N)
             fft_rows_cc<C, PL, NP, 1>(b0, zo, b1, jr, twz, +1);
         else
-            fft_lines_cc<C, PL, N>(SmemLinesC<C, NP, 1>{b0}, SmemLinesC<C, NP, 1>{zo}, SmemLinesC<C, NP, 1>{b1}, twz,
-                                   +1);
+            fft_lines_cc<C, PL, N>(SmemLinesC<C, NP, 1>{b0}, SmemLinesC<C, NP, 1>{zo}, SmemLinesC<C, NP, 1>{b1},
+                                   SmemLinesC<C, NP, 1>{b0}, twz, +1);
         __syncthreads();
-        fft_lines_cc<C, PL, N>(SmemLinesC<C, 1, NP>{zo}, PlaneGlobalC<C, N>{Tp}, SmemLinesC<C, 1, NP>{zother}, twy,
-                               +1);
+        fft_lines_cc<C, PL, N>(SmemLinesC<C, 1, NP>{zo}, PlaneGlobalC<C, N>{Tp}, SmemLinesC<C, 1, NP>{zother},
+                               SmemLinesC<C, 1, NP>{zo}, twy, +1);
     }
 }
 
@@ -902,7 +905,8 @@ __global__ void __launch_bounds__(Cfg<C>::plane_threads, WIDE ? 1 : Cfg<C>::plan
                            -1);
     } else {
         constexpr int N = PL::n, NP = PL::n + 1;
-        fft_lines_cc<C, PL, N>(PlaneGlobalC<C, N>{Tp}, SmemLinesC<C, 1, NP>{yo}, SmemLinesC<C, 1, NP>{b0}, twy, -1);
+        fft_lines_cc<C, PL, N>(PlaneGlobalC<C, N>{Tp}, SmemLinesC<C, 1, NP>{yo}, SmemLinesC<C, 1, NP>{b0},
+                               SmemLinesC<C, 1, NP>{b1}, twy, -1);
         __syncthreads();
         // z-lines of the rows in use only: the gather reads no other row
         const int jr = plane_jr ? plane_jr[p] : N;
@@ -910,7 +914,7 @@ __global__ void __launch_bounds__(Cfg<C>::plane_threads, WIDE ? 1 : Cfg<C>::plan
             fft_rows_cc<C, PL, NP, 1>(yo, zo, yother, jr, twz, -1);
         else
             fft_lines_cc<C, PL, N>(SmemLinesC<C, NP, 1>{yo}, SmemLinesC<C, NP, 1>{zo}, SmemLinesC<C, NP, 1>{yother},
-                                   twz, -1);
+                                   SmemLinesC<C, NP, 1>{yo}, twz, -1);
     }
     __syncthreads();
     const C* res = zo;
@@ -1027,16 +1031,80 @@ constexpr int pair_block()
     else return pair_threads<PL::n>();
 }
 
-template <typename C, typename V, bool WIDE, typename PL, int KTC>
+// Kernels of the shared-memory passes.  Each takes a compile-time plan when its own
+// axes have one: the plane passes when y and z have the same, the x pass by x alone
+// (supercells rarely have the same length on all axes).  The arithmetic is that of
+// the runtime plans, so the results are the same bits.  The passes are bound by
+// instruction issue, and the runtime plans spend about half of it on index
+// arithmetic and on rows without sphere points.  Runtime -> compile-time plan, us:
+// 36 x 64 x 64 grid, 64 bands: G->r 43 -> 31, x 63 -> 43, r->G 45 -> 35; 60^3 grid,
+// 128 bands: 195 -> 132, 278 -> 179, 208 -> 142 (H|psi> on the tensor cores 881 ->
+// 655); 30^3 grid, 48 bands: H|psi> in FP32 86 -> 59.  An x tile other than four
+// columns keeps the runtime plan (batch plans may choose one).
+template <typename F>
+static auto with_plan(const FftLen& L, F&& f)
+{
+    if (L.nst == 2) {
+        const int p = L.rad[0], q = L.rad[1];
+        if (p == 8 && q == 9) return f(FftPlan2<8, 9>{});
+        if (p == 9 && q == 4) return f(FftPlan2<9, 4>{});
+        if (p == 8 && q == 3) return f(FftPlan2<8, 3>{});
+        if (p == 8 && q == 8) return f(FftPlan2<8, 8>{});
+        if (p == 8 && q == 4) return f(FftPlan2<8, 4>{});
+        if (p == 8 && q == 5) return f(FftPlan2<8, 5>{});
+    }
+    if (L.nst == 3) {
+        const int p = L.rad[0], q = L.rad[1], t = L.rad[2];
+        if (p == 4 && q == 3 && t == 5) return f(FftPlan3<4, 3, 5>{});
+        if (p == 2 && q == 3 && t == 5) return f(FftPlan3<2, 3, 5>{});
+        if (p == 8 && q == 2 && t == 3) return f(FftPlan3<8, 2, 3>{});
+    }
+    return f(NoPlan{});
+}
+template <typename C>
+using G2rFn = void (*)(LocalArgs, const double2*, C*, const C*, const C*);
+template <typename C>
+using R2gFn = void (*)(LocalArgs, const C*, const double2*, double2*, const double*, const C*, const C*);
+template <typename C, typename V>
+using XFn = void (*)(LocalArgs, int, C*, const V*, const C*);
+
+template <typename C, bool WIDE>
+static G2rFn<C> g2r_kernel(const LocalArgs& a)
+{
+    if constexpr (!WIDE)
+        if (a.n2 == a.n3) return with_plan(a.Ly, [](auto pl) -> G2rFn<C> { return g2r_planes<C, false, decltype(pl)>; });
+    return g2r_planes<C, WIDE, NoPlan>;
+}
+template <typename C, bool WIDE>
+static R2gFn<C> r2g_kernel(const LocalArgs& a)
+{
+    if constexpr (!WIDE)
+        if (a.n2 == a.n3) return with_plan(a.Ly, [](auto pl) -> R2gFn<C> { return r2g_planes<C, false, decltype(pl)>; });
+    return r2g_planes<C, WIDE, NoPlan>;
+}
+template <typename C, typename V, bool WIDE, bool ENERGY>
+static XFn<C, V> x_kernel(const LocalArgs& a)
+{
+    if constexpr (!WIDE)
+        return with_plan(a.Lx, [&](auto pl) -> XFn<C, V> {
+            using PL = decltype(pl);
+            if constexpr (!std::is_same<PL, NoPlan>::value)
+                if (a.kt == 4) return x_pass<C, V, false, ENERGY, PL, 4>;
+            return x_pass<C, V, false, ENERGY, NoPlan, 0>;
+        });
+    return x_pass<C, V, true, ENERGY, NoPlan, 0>;
+}
+
+template <typename C, typename V, bool WIDE, typename PL>
 static cudaError_t launch_local_t(const LocalArgs& a, int nb, const double2* psi, double2* hpsi, const double* kinetic,
                                   C* T, const V* vloc, const C* twx, const C* twy, const C* twz, cudaStream_t st,
                                   Prof* prof)
 {
     const size_t sp = plane_smem<C>(a), sx = xpass_smem<C, V>(a);
     cudaError_t e;
-    auto g2r = g2r_planes<C, WIDE, PL>;
-    auto r2g = r2g_planes<C, WIDE, PL>;
-    auto xp = a.epart ? x_pass<C, V, WIDE, true, PL, KTC> : x_pass<C, V, WIDE, false, PL, KTC>;
+    const auto g2r = g2r_kernel<C, WIDE>(a);
+    const auto r2g = r2g_kernel<C, WIDE>(a);
+    const auto xp = a.epart ? x_kernel<C, V, WIDE, true>(a) : x_kernel<C, V, WIDE, false>(a);
     if ((e = cudaFuncSetAttribute(g2r, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp))) return e;
     if ((e = cudaFuncSetAttribute(r2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp))) return e;
     if ((e = cudaFuncSetAttribute(xp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx))) return e;
@@ -1086,15 +1154,15 @@ static cudaError_t launch_local_t(const LocalArgs& a, int nb, const double2* psi
     return cudaGetLastError();
 }
 
-template <typename C, typename V, bool WIDE, typename PL, int KTC>
+template <typename C, typename V, bool WIDE, typename PL>
 static cudaError_t launch_local_batch_t(const LocalArgs& a, int nbands, int max_nxs, int nxblk, C* T, const V* vloc,
                                         const C* twx, const C* twy, const C* twz, cudaStream_t st)
 {
     const size_t sp = plane_smem<C>(a), sx = xpass_smem<C, V>(a);
     cudaError_t e;
-    auto g2r = g2r_planes<C, WIDE, PL>;
-    auto r2g = r2g_planes<C, WIDE, PL>;
-    auto xp = x_pass<C, V, WIDE, false, PL, KTC>;
+    const auto g2r = g2r_kernel<C, WIDE>(a);
+    const auto r2g = r2g_kernel<C, WIDE>(a);
+    const auto xp = x_kernel<C, V, WIDE, false>(a);
     if ((e = cudaFuncSetAttribute(g2r, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp))) return e;
     if ((e = cudaFuncSetAttribute(r2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp))) return e;
     if ((e = cudaFuncSetAttribute(xp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx))) return e;
@@ -1115,35 +1183,24 @@ static cudaError_t launch_local_batch_t(const LocalArgs& a, int nbands, int max_
     return cudaGetLastError();
 }
 
-// Kernel set of a launch: the wide-radix set, a compile-time two-stage plan
-// (complex64, the same plan on all three axes; with KT = 4 also a
-// compile-time z-tile in the x pass), or the runtime-plan set.
-template <int K> using IntC = std::integral_constant<int, K>;
+// Kernel set of a launch: the register passes (complex64, the same compile-time
+// plan on all three axes), or the shared-memory passes, with the wide radices
+// where an axis needs them.
 template <typename C, typename F>
 static cudaError_t with_kernels(const LocalArgs& a, F&& f)
 {
-    if (fft_needs_wide(a.Lx) || fft_needs_wide(a.Ly) || fft_needs_wide(a.Lz))
-        return f(std::true_type{}, NoPlan{}, IntC<0>{});
+    if (fft_needs_wide(a.Lx) || fft_needs_wide(a.Ly) || fft_needs_wide(a.Lz)) return f(std::true_type{}, NoPlan{});
     const int id = fft_ct_id(a.Lx);
     if (id != FFT_CT_NONE && fft_ct_id(a.Ly) == id && fft_ct_id(a.Lz) == id) {
-        const bool k4 = a.kt == 4;
         switch (id) {
-            case FFT_CT_72:
-                return k4 ? f(std::false_type{}, FftPlan2<8, 9>{}, IntC<4>{})
-                          : f(std::false_type{}, FftPlan2<8, 9>{}, IntC<0>{});
-            case FFT_CT_36:
-                return k4 ? f(std::false_type{}, FftPlan2<9, 4>{}, IntC<4>{})
-                          : f(std::false_type{}, FftPlan2<9, 4>{}, IntC<0>{});
-            case FFT_CT_24:
-                return k4 ? f(std::false_type{}, FftPlan2<8, 3>{}, IntC<4>{})
-                          : f(std::false_type{}, FftPlan2<8, 3>{}, IntC<0>{});
-            case FFT_CT_64:
-                return k4 ? f(std::false_type{}, FftPlan2<8, 8>{}, IntC<4>{})
-                          : f(std::false_type{}, FftPlan2<8, 8>{}, IntC<0>{});
+            case FFT_CT_72: return f(std::false_type{}, FftPlan2<8, 9>{});
+            case FFT_CT_36: return f(std::false_type{}, FftPlan2<9, 4>{});
+            case FFT_CT_24: return f(std::false_type{}, FftPlan2<8, 3>{});
+            case FFT_CT_64: return f(std::false_type{}, FftPlan2<8, 8>{});
             default: break;
         }
     }
-    return f(std::false_type{}, NoPlan{}, IntC<0>{});
+    return f(std::false_type{}, NoPlan{});
 }
 
 template <typename C, typename V>
@@ -1152,8 +1209,8 @@ cudaError_t launch_local_batch(const LocalArgs& a, int nbands, int max_nxs, int 
 {
     if (!a.items || a.epart) return cudaErrorInvalidValue;
     if (a.plane_threads > Cfg<C>::plane_threads || a.plane_threads % 32) return cudaErrorInvalidValue;
-    return with_kernels<C>(a, [&](auto wide, auto pl, auto ktc) {
-        return launch_local_batch_t<C, V, decltype(wide)::value, decltype(pl), decltype(ktc)::value>(
+    return with_kernels<C>(a, [&](auto wide, auto pl) {
+        return launch_local_batch_t<C, V, decltype(wide)::value, decltype(pl)>(
             a, nbands, max_nxs, nxblk, T, vloc, twx, twy, twz, st);
     });
 }
@@ -1173,7 +1230,7 @@ static cudaError_t launch_density_t(const LocalArgs& a, int nb, const double2* p
 {
     const size_t sp = plane_smem<C>(a), sx = density_smem<C>(a);
     cudaError_t e;
-    auto g2r = g2r_planes<C, WIDE, PL>;
+    const auto g2r = g2r_kernel<C, WIDE>(a);
     auto xd = x_density<C, WIDE>;
     if ((e = cudaFuncSetAttribute(g2r, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp))) return e;
     if ((e = cudaFuncSetAttribute(xd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx))) return e;
@@ -1202,7 +1259,7 @@ cudaError_t launch_density(const LocalArgs& a, int nb, const double2* psi, const
                            const Tw<C>* twx, const Tw<C>* twy, const Tw<C>* twz, cudaStream_t st, double* part)
 {
     if (a.items || a.epart) return cudaErrorInvalidValue;
-    return with_kernels<C>(a, [&](auto wide, auto pl, auto) {
+    return with_kernels<C>(a, [&](auto wide, auto pl) {
         return launch_density_t<C, decltype(wide)::value, decltype(pl)>(a, nb, psi, occ, rho, T, twx, twy, twz, st,
                                                                          part);
     });
@@ -1234,8 +1291,8 @@ cudaError_t launch_local(const LocalArgs& a, int nb, const double2* psi, double2
                          const V* vloc, const Tw<C>* twx, const Tw<C>* twy, const Tw<C>* twz, cudaStream_t st,
                          Prof* prof)
 {
-    return with_kernels<C>(a, [&](auto wide, auto pl, auto ktc) {
-        return launch_local_t<C, V, decltype(wide)::value, decltype(pl), decltype(ktc)::value>(
+    return with_kernels<C>(a, [&](auto wide, auto pl) {
+        return launch_local_t<C, V, decltype(wide)::value, decltype(pl)>(
             a, nb, psi, hpsi, kinetic, T, vloc, twx, twy, twz, st, prof);
     });
 }
