@@ -169,6 +169,10 @@ struct hpsi_ctx {
     size_t stage_size = 0;
     unsigned char* ws = nullptr;
     size_t ws_size = 0;
+    // the first workspace stays with the context: freeing it when a call needs more
+    // would cost that call the time of a cudaFree (50-80 us)
+    unsigned char* ws_first = nullptr;
+    size_t ws_first_size = 0;
     // workspace of the FP64 GEMMs on the tensor cores, within ws (set per call): a
     // call that cannot have it runs the SIMT GEMMs
     unsigned char* d64_ws = nullptr;
@@ -236,13 +240,19 @@ struct Carver {
 inline int ws_reserve(hpsi_ctx* c, size_t bytes)
 {
     if (bytes <= c->ws_size) return HPSI_OK;
-    if (c->ws) cudaFree(c->ws);
-    c->ws = nullptr;
-    c->ws_size = 0;
+    if (c->ws != c->ws_first) cudaFree(c->ws);
+    c->ws = c->ws_first;
+    c->ws_size = c->ws_first_size;
     c->d64_ws = nullptr;
-    size_t want = bytes + bytes / 8;
-    CUDA_TRY(c, cudaMalloc((void**)&c->ws, want));
+    const size_t want = bytes + bytes / 8;
+    unsigned char* p = nullptr;
+    CUDA_TRY(c, cudaMalloc((void**)&p, want));
+    c->ws = p;
     c->ws_size = want;
+    if (!c->ws_first) {
+        c->ws_first = p;
+        c->ws_first_size = want;
+    }
     return HPSI_OK;
 }
 

@@ -39,7 +39,8 @@ extern "C" int hpsi_ctx_destroy(hpsi_ctx* c)
     for (auto& kv : c->slots) slot_free(kv.second);
     dfree(c->d_tables); dfree(c->d_rad_nq); dfree(c->d_rad_dq); dfree(c->d_tau); dfree(c->d_v64); dfree(c->d_v32); dfree(c->d_dv32);
     dfree(c->d_tw64); dfree(c->d_tw32); dfree(c->d_err); dfree(c->d_hess);
-    if (c->ws) cudaFree(c->ws);
+    if (c->ws != c->ws_first) cudaFree(c->ws);
+    if (c->ws_first) cudaFree(c->ws_first);
     if (c->stage) cudaFreeHost(c->stage);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
