@@ -422,13 +422,13 @@ HPSI_D void fft_stage_rows(const LD& ld, const ST& st, int nl, float rinv, const
     }
 }
 
-// Transform of the rows in use (jr as above; 2 jr + 1 < n) of a plane with line
-// stride LS and element stride ES: two stages in -> A -> out (in may be out),
+// Transform of the rows in use (jr as above; 2 jr + 1 < ROWS) of a plane of ROWS
+// rows with line stride LS and element stride ES: two stages in -> A -> out (in may be out),
 // three in -> A -> in -> out (A may be out)
-template <typename C, typename PL, int LS, int ES>
+template <typename C, typename PL, int ROWS, int LS, int ES>
 HPSI_D void fft_rows_cc(C* in, C* out, C* A, int jr, const C* tw, int sign)
 {
-    const int nl = 2 * jr + 1, gap = PL::n - nl;
+    const int nl = 2 * jr + 1, gap = ROWS - nl;
     const float rinv = 1.0f / (float)nl;
     fft_stage_rows<C, PL::n, PL::r0, 1>(SmemRowsC<C, LS, ES>{in, jr, gap}, SmemRowsC<C, LS, ES>{A, jr, gap}, nl, rinv,
                                         tw, sign);

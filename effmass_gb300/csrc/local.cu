@@ -84,8 +84,8 @@ struct PlaneGlobalC {
     HPSI_D void operator()(int L, int e, C v) const { p[e * N3 + L] = v; }
 };
 
-// grid length of a plane's axes: the compile-time plan's when there is one (then
-// both share it), else the runtime value
+// grid length of an axis: the compile-time plan's when there is one, else the
+// runtime value
 template <typename PL>
 HPSI_D int plan_n(int runtime)
 {
@@ -93,12 +93,13 @@ HPSI_D int plan_n(int runtime)
     else return PL::n;
 }
 
-template <typename C, bool WIDE, typename PL>
+// PL, PZ: plans of y and z (both compile-time plans, or neither)
+template <typename C, bool WIDE, typename PL, typename PZ = PL>
 __global__ void __launch_bounds__(Cfg<C>::g2r_threads, WIDE ? 1 : Cfg<C>::plane_min) g2r_planes(LocalArgs a, const double2* __restrict__ psi, C* __restrict__ T,
                                                   const C* __restrict__ tw_y_g, const C* __restrict__ tw_z_g)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n2 = plan_n<PL>(a.n2), n3 = plan_n<PL>(a.n3), n3p = n3 + 1, n23 = n2 * n3, n23p = n2 * n3p;
+    const int n2 = plan_n<PL>(a.n2), n3 = plan_n<PZ>(a.n3), n3p = n3 + 1, n23 = n2 * n3, n23p = n2 * n3p;
     C* b0 = reinterpret_cast<C*>(smem_raw);
     C* b1 = b0 + n23p;
     C* twy = b1 + n23p;
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(Cfg<C>::g2r_threads, WIDE ? 1 : Cfg<C>::plane_
     for (int t = threadIdx.x; t < n3; t += blockDim.x) twz[t] = tw_z_g[t];
     for (int t = threadIdx.x; t < n23p; t += blockDim.x) b0[t] = cmake<C>(0, 0);
     if constexpr (!std::is_same<PL, NoPlan>::value)
-        if (PL::r2 > 1)  // three stages end in b1: its rows not in use are zero too
+        if (PZ::r2 > 1)  // three stages end in b1: its rows not in use are zero too
             for (int t = threadIdx.x; t < n23p; t += blockDim.x) b1[t] = cmake<C>(0, 0);
     __syncthreads();
     const double2* ps = psi + (size_t)b * npw;
@@ -163,18 +164,18 @@ __global__ void __launch_bounds__(Cfg<C>::g2r_threads, WIDE ? 1 : Cfg<C>::plane_
         lines<C, WIDE, PL>(SmemLines<C>{zo, 1, n3p}, PlaneGlobal<C>{Tp, n3}, zother, zo, a.Ly, a.nl_y, 1, n3p, twy,
                            +1);
     } else {
-        constexpr int N = PL::n, NP = PL::n + 1;  // n2 = n3 = N lines per axis
+        constexpr int NY = PL::n, NZ = PZ::n, NP = NZ + 1;
         // z-lines of the rows in use only: the other rows are zero in zo (b0 for
         // two stages, b1 for three)
-        const int jr = plane_jr ? plane_jr[p] : N;
-        if (2 * jr + 1 < N)
-            fft_rows_cc<C, PL, NP, 1>(b0, zo, b1, jr, twz, +1);
+        const int jr = plane_jr ? plane_jr[p] : NY;
+        if (2 * jr + 1 < NY)
+            fft_rows_cc<C, PZ, NY, NP, 1>(b0, zo, b1, jr, twz, +1);
         else
-            fft_lines_cc<C, PL, N>(SmemLinesC<C, NP, 1>{b0}, SmemLinesC<C, NP, 1>{zo}, SmemLinesC<C, NP, 1>{b1},
-                                   SmemLinesC<C, NP, 1>{b0}, twz, +1);
+            fft_lines_cc<C, PZ, NY>(SmemLinesC<C, NP, 1>{b0}, SmemLinesC<C, NP, 1>{zo}, SmemLinesC<C, NP, 1>{b1},
+                                    SmemLinesC<C, NP, 1>{b0}, twz, +1);
         __syncthreads();
-        fft_lines_cc<C, PL, N>(SmemLinesC<C, 1, NP>{zo}, PlaneGlobalC<C, N>{Tp}, SmemLinesC<C, 1, NP>{zother},
-                               SmemLinesC<C, 1, NP>{zo}, twy, +1);
+        fft_lines_cc<C, PL, NZ>(SmemLinesC<C, 1, NP>{zo}, PlaneGlobalC<C, NZ>{Tp}, SmemLinesC<C, 1, NP>{zother},
+                                SmemLinesC<C, 1, NP>{zo}, twy, +1);
     }
 }
 
@@ -863,13 +864,13 @@ __global__ void __launch_bounds__(256, WIDE ? (Cfg<C>::x_min + 1) / 2 : Cfg<C>::
     }
 }
 
-template <typename C, bool WIDE, typename PL>
+template <typename C, bool WIDE, typename PL, typename PZ = PL>
 __global__ void __launch_bounds__(Cfg<C>::plane_threads, WIDE ? 1 : Cfg<C>::plane_min) r2g_planes(LocalArgs a, const C* __restrict__ T, const double2* __restrict__ psi,
                                                   double2* __restrict__ hpsi, const double* __restrict__ kinetic,
                                                   const C* __restrict__ tw_y_g, const C* __restrict__ tw_z_g)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int n2 = plan_n<PL>(a.n2), n3 = plan_n<PL>(a.n3), n3p = n3 + 1, n23 = n2 * n3, n23p = n2 * n3p;
+    const int n2 = plan_n<PL>(a.n2), n3 = plan_n<PZ>(a.n3), n3p = n3 + 1, n23 = n2 * n3, n23p = n2 * n3p;
     C* b0 = reinterpret_cast<C*>(smem_raw);
     C* b1 = b0 + n23p;
     C* twy = b1 + n23p;
@@ -904,17 +905,17 @@ __global__ void __launch_bounds__(Cfg<C>::plane_threads, WIDE ? 1 : Cfg<C>::plan
         lines<C, WIDE, PL>(SmemLines<C>{yo, n3p, 1}, SmemLines<C>{zo, n3p, 1}, yother, yo, a.Lz, a.nl_z, n3p, 1, twz,
                            -1);
     } else {
-        constexpr int N = PL::n, NP = PL::n + 1;
-        fft_lines_cc<C, PL, N>(PlaneGlobalC<C, N>{Tp}, SmemLinesC<C, 1, NP>{yo}, SmemLinesC<C, 1, NP>{b0},
-                               SmemLinesC<C, 1, NP>{b1}, twy, -1);
+        constexpr int NY = PL::n, NZ = PZ::n, NP = NZ + 1;
+        fft_lines_cc<C, PL, NZ>(PlaneGlobalC<C, NZ>{Tp}, SmemLinesC<C, 1, NP>{yo}, SmemLinesC<C, 1, NP>{b0},
+                                SmemLinesC<C, 1, NP>{b1}, twy, -1);
         __syncthreads();
         // z-lines of the rows in use only: the gather reads no other row
-        const int jr = plane_jr ? plane_jr[p] : N;
-        if (2 * jr + 1 < N)
-            fft_rows_cc<C, PL, NP, 1>(yo, zo, yother, jr, twz, -1);
+        const int jr = plane_jr ? plane_jr[p] : NY;
+        if (2 * jr + 1 < NY)
+            fft_rows_cc<C, PZ, NY, NP, 1>(yo, zo, yother, jr, twz, -1);
         else
-            fft_lines_cc<C, PL, N>(SmemLinesC<C, NP, 1>{yo}, SmemLinesC<C, NP, 1>{zo}, SmemLinesC<C, NP, 1>{yother},
-                                   SmemLinesC<C, NP, 1>{yo}, twz, -1);
+            fft_lines_cc<C, PZ, NY>(SmemLinesC<C, NP, 1>{yo}, SmemLinesC<C, NP, 1>{zo}, SmemLinesC<C, NP, 1>{yother},
+                                    SmemLinesC<C, NP, 1>{yo}, twz, -1);
     }
     __syncthreads();
     const C* res = zo;
@@ -1032,7 +1033,7 @@ constexpr int pair_block()
 }
 
 // Kernels of the shared-memory passes.  Each takes a compile-time plan when its own
-// axes have one: the plane passes when y and z have the same, the x pass by x alone
+// axes have one: the plane passes by y and z (with_planes), the x pass by x alone
 // (supercells rarely have the same length on all axes).  The arithmetic is that of
 // the runtime plans, so the results are the same bits.  The passes are bound by
 // instruction issue, and the runtime plans spend about half of it on index
@@ -1061,6 +1062,19 @@ static auto with_plan(const FftLen& L, F&& f)
     }
     return f(NoPlan{});
 }
+// plane plans (y, z): the same length, or z twice as long (a cell doubled along z:
+// 32 x 64 planes, 128 bands, G->r 50 -> 35 us; H|psi> on the tensor cores 201 -> 177;
+// 30 x 60, 37 bands 145 -> 130; 36 x 72, 37 bands 153 -> 141)
+template <typename F>
+static auto with_planes(const LocalArgs& a, F&& f)
+{
+    if (a.n2 == a.n3) return with_plan(a.Ly, [&](auto pl) { return f(pl, pl); });
+    if (a.n2 == 32 && a.n3 == 64) return f(FftPlan2<8, 4>{}, FftPlan2<8, 8>{});
+    if (a.n2 == 30 && a.n3 == 60) return f(FftPlan3<2, 3, 5>{}, FftPlan3<4, 3, 5>{});
+    if (a.n2 == 36 && a.n3 == 72) return f(FftPlan2<9, 4>{}, FftPlan2<8, 9>{});
+    if (a.n2 == 24 && a.n3 == 48) return f(FftPlan2<8, 3>{}, FftPlan3<8, 2, 3>{});
+    return f(NoPlan{}, NoPlan{});
+}
 template <typename C>
 using G2rFn = void (*)(LocalArgs, const double2*, C*, const C*, const C*);
 template <typename C>
@@ -1072,14 +1086,18 @@ template <typename C, bool WIDE>
 static G2rFn<C> g2r_kernel(const LocalArgs& a)
 {
     if constexpr (!WIDE)
-        if (a.n2 == a.n3) return with_plan(a.Ly, [](auto pl) -> G2rFn<C> { return g2r_planes<C, false, decltype(pl)>; });
+        return with_planes(a, [](auto py, auto pz) -> G2rFn<C> {
+            return g2r_planes<C, false, decltype(py), decltype(pz)>;
+        });
     return g2r_planes<C, WIDE, NoPlan>;
 }
 template <typename C, bool WIDE>
 static R2gFn<C> r2g_kernel(const LocalArgs& a)
 {
     if constexpr (!WIDE)
-        if (a.n2 == a.n3) return with_plan(a.Ly, [](auto pl) -> R2gFn<C> { return r2g_planes<C, false, decltype(pl)>; });
+        return with_planes(a, [](auto py, auto pz) -> R2gFn<C> {
+            return r2g_planes<C, false, decltype(py), decltype(pz)>;
+        });
     return r2g_planes<C, WIDE, NoPlan>;
 }
 template <typename C, typename V, bool WIDE, bool ENERGY>

@@ -14,7 +14,7 @@ from effmass_gb300 import system as S
 pytestmark = pytest.mark.gpu
 TOL = 5e-6
 GRIDS = [(36, 64, 64), (64, 36, 36), (24, 32, 32), (32, 32, 64), (40, 40, 40), (30, 30, 30), (30, 60, 60), (60, 30, 30),
-         (48, 48, 48), (72, 60, 60), (60, 72, 72), (7, 48, 48), (20, 24, 24)]
+         (48, 48, 48), (72, 60, 60), (60, 72, 72), (7, 48, 48), (20, 24, 24), (30, 30, 60), (36, 36, 72), (24, 24, 48)]
 
 
 @pytest.mark.parametrize("full", [False, True])
