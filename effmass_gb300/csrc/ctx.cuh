@@ -48,13 +48,13 @@ struct KSlot {
     // projector matrices: rows [0, P), and with dbeta tables room for the 3 P
     // derivative rows behind them (filled on first use: pr*_grad)
     double2* pr64 = nullptr;
-    bool pr64_grad = false;
+    bool pr64_built = false, pr64_grad = false;  // rows [0, P) and the derivative rows hold their values
     // exponents of pr64's columns and rows for the digit split, of the first P rows
     // (H) and of all 4 P (gradient), in pr64's allocation
     int* d64_exp[2] = {nullptr, nullptr};
     bool d64_exp_set[2] = {false, false};
     float2* pr32 = nullptr;
-    bool pr32_grad = false;
+    bool pr32_built = false, pr32_grad = false;
     size_t pr_bytes[2] = {0, 0};   // allocation sizes of pr64, pr32
     size_t tc_bytes[2] = {0, 0};   // and of tc_mem
     Spare spare_pr[2], spare_tc[2];
@@ -69,12 +69,27 @@ struct KSlot {
     TcGen tcgen[2];
     TcOperand tc_proj[2], tc_expand[2];
     int tcg_fmt = -1;              // gradient operands (4P-row projection, per-direction expansion)
+    bool tcg_built = false;
     unsigned char* tcg_mem = nullptr;
     TcOperand tcg_proj, tcg_exp[3];
     long gen = 0;                  // binding generation: changes when the slot is rebound
     double2* hess64 = nullptr;     // projector second derivatives [6][P][npw] (Hessian), per precision
     float2* hess32 = nullptr;
+    bool hess64_built = false, hess32_built = false;
 };
+
+// Whether work queued on st is recorded into a graph instead of run.  A first-use
+// build that is recorded is not marked as built: the next eager call cannot know
+// whether the graph has been launched, and builds again.
+inline bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {
+        cudaGetLastError();  // the legacy stream while another one captures
+        return false;
+    }
+    return s != cudaStreamCaptureStatusNone;
+}
 
 template <typename T>
 inline cudaError_t dalloc(T** p, size_t count)

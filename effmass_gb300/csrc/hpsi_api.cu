@@ -417,18 +417,21 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
 {
     constexpr bool f64 = std::is_same<C, double2>::value;
     C*& pr = slot_pr<C>(s);
+    bool& has_value = f64 ? s.pr64_built : s.pr32_built;
     bool& has_grad = f64 ? s.pr64_grad : s.pr32_grad;
     if (s.P == 0 || s.npw == 0) return HPSI_OK;
-    if (pr && (has_grad || !grad)) return HPSI_OK;
+    if (has_value && (has_grad || !grad)) return HPSI_OK;
     if (grad && !c->have_dbeta) return fail(c, HPSI_ERR_STATE, "gradient needs dbeta tables for every species");
-    const bool fresh = !pr;
-    if (fresh) {
+    const bool record = capturing(st), value = !has_value;
+    if (!pr) {
         const size_t rows = (size_t)(c->have_dbeta ? 4 : 1) * s.P;
         // FP64: the digit split's exponents behind the matrix (d64_scale)
         const size_t n_exp = f64 ? 2 * (size_t)s.npw + s.P + rows : 0;
         size_t bytes = rows * s.npw * sizeof(C) + n_exp * sizeof(int);
         const int k = f64 ? 0 : 1;
-        CUDA_TRY(c, spare_alloc(s.spare_pr[k], (void**)&pr, &bytes));
+        // a spare would let a capture record a build that it otherwise refuses
+        if (record) CUDA_TRY(c, cudaMalloc((void**)&pr, bytes));
+        else CUDA_TRY(c, spare_alloc(s.spare_pr[k], (void**)&pr, &bytes));
         s.pr_bytes[k] = bytes;
         if (f64) {
             s.d64_exp[0] = reinterpret_cast<int*>(pr + rows * s.npw);
@@ -442,9 +445,12 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
     const double* dbeta = c->have_dbeta ? s.d_beta + (size_t)c->nrad * s.npw : nullptr;
     int h = c->prof.open(PH_BUILD, st);
     CUDA_TRY(c, launch_assemble<C>(s.P, s.npw, s.d_rows, s.d_beta, dbeta, s.d_dbeta0, s.d_q, s.d_trig, s.d_ylm, yth,
-                                   yph, s.d_sf, fresh, grad, pr, (size_t)s.npw, st));
+                                   yph, s.d_sf, value, grad, pr, (size_t)s.npw, st));
     c->prof.close(h, st);
-    has_grad = grad;
+    if (!record) {
+        has_value = true;
+        has_grad = grad;
+    }
     return HPSI_OK;
 }
 
@@ -502,7 +508,7 @@ static int d64_scale(hpsi_ctx* c, KSlot& s, bool all, D64Scale* out, cudaStream_
     int h = c->prof.open(PH_BUILD, st);
     CUDA_TRY(c, d64_scales((all ? 4 : 1) * s.P, s.npw, s.pr64, (size_t)s.npw, *out, st));
     c->prof.close(h, st, 2);
-    s.d64_exp_set[all] = true;
+    s.d64_exp_set[all] = !capturing(st);
     return HPSI_OK;
 }
 
@@ -754,6 +760,10 @@ static int ensure_tc(hpsi_ctx* c, KSlot& s, int fmt, cudaStream_t st)
         s.tc_fmt = fmt;
         return HPSI_OK;
     }
+    // the build copies from host tables that do not outlive this call
+    if (capturing(st))
+        return fail(c, HPSI_ERR_STATE, "the projector tables of this k-point are not built yet: one eager call before "
+                                       "the capture builds them");
     // by rows: the distinct (radial function, lm) pairs of the projectors
     std::vector<int2> prow((size_t)s.P), byinfo;
     std::map<std::pair<int, int>, int> at;
@@ -887,11 +897,12 @@ static int tc_nonlocal_expand(hpsi_ctx* c, KSlot& s, int nb, double2* hpsi, unsi
 static int ensure_tc_grad(hpsi_ctx* c, KSlot& s, int fmt, cudaStream_t st)
 {
     if (s.P == 0 || s.npw == 0) return HPSI_OK;
-    if (s.tcg_fmt == fmt && s.tcg_mem) return HPSI_OK;
+    if (s.tcg_fmt == fmt && s.tcg_mem && s.tcg_built) return HPSI_OK;
     int rc;
     if ((rc = ensure_proj<float2>(c, s, true, st))) return rc;
-    dfree(s.tcg_mem);
+    if (s.tcg_fmt != fmt) dfree(s.tcg_mem);
     s.tcg_fmt = -1;
+    s.tcg_built = false;
     const size_t k1 = tc_round_k(2 * (size_t)s.npw), k2 = tc_round_k(4 * (size_t)s.P);
     Carver cv;
     const size_t rp = tc_rows_pad(4 * (size_t)s.P), rg = tc_rows_pad(s.npw);
@@ -904,7 +915,7 @@ static int ensure_tc_grad(hpsi_ctx* c, KSlot& s, int fmt, cudaStream_t st)
         os[a] = cv.take<float>((size_t)s.npw);
     }
     const size_t ocm = cv.take<float>((size_t)s.npw);
-    CUDA_TRY(c, dalloc(&s.tcg_mem, cv.off));
+    if (!s.tcg_mem) CUDA_TRY(c, dalloc(&s.tcg_mem, cv.off));
     CUDA_TRY(c, cudaMemsetAsync(s.tcg_mem, 0, cv.off, st));  // padding rows and K padding read as zero
     s.tcg_proj = TcOperand{s.tcg_mem + o1h, s.tcg_mem + o1l, reinterpret_cast<float*>(s.tcg_mem + o1s), k1};
     for (int a = 0; a < 3; ++a)
@@ -914,6 +925,7 @@ static int ensure_tc_grad(hpsi_ctx* c, KSlot& s, int fmt, cudaStream_t st)
                                        reinterpret_cast<float*>(s.tcg_mem + ocm), st));
     c->prof.close(h, st);
     s.tcg_fmt = fmt;
+    s.tcg_built = !capturing(st);
     return HPSI_OK;
 }
 
@@ -1917,7 +1929,11 @@ extern "C" int hpsi_set_hessian_tables(hpsi_ctx* c, int species, int nq, double 
                            cudaMemcpyHostToDevice));
     for (int r = r0; r < r1; ++r) c->hess_set[r] = 1;
     // slots bound before: their second-derivative rows are rebuilt on next use
-    for (auto& kv : c->slots) { dfree(kv.second.hess64); dfree(kv.second.hess32); }
+    for (auto& kv : c->slots) {
+        dfree(kv.second.hess64);
+        dfree(kv.second.hess32);
+        kv.second.hess64_built = kv.second.hess32_built = false;
+    }
     return HPSI_OK;
 }
 
@@ -1925,7 +1941,8 @@ template <typename C>
 static int ensure_hess(hpsi_ctx* c, KSlot& s, cudaStream_t st)
 {
     C*& d2 = slot_hess<C>(s);
-    if (d2 || s.P == 0 || s.npw == 0) return HPSI_OK;
+    bool& built = std::is_same<C, double2>::value ? s.hess64_built : s.hess32_built;
+    if (built || s.P == 0 || s.npw == 0) return HPSI_OK;
     for (int r = 0; r < c->nrad; ++r)
         if (std::fabs(c->rad_lam[r]) >= 1e-15 && (c->hess_set.empty() || !c->hess_set[r]))
             return fail(c, HPSI_ERR_STATE, "Hessian tables missing for radial function %d (hpsi_set_hessian_tables)", r);
@@ -1935,9 +1952,10 @@ static int ensure_hess(hpsi_ctx* c, KSlot& s, cudaStream_t st)
     CUDA_TRY(c, cudaMemcpy(q.data(), s.d_q, s.npw * sizeof(double), cudaMemcpyDeviceToHost));
     for (double v : q)
         if (v > qtop) return fail(c, HPSI_ERR_RANGE, "q=%.17g beyond the Hessian tables (%.17g)", v, qtop);
-    CUDA_TRY(c, dalloc(&d2, (size_t)6 * s.P * s.npw));
+    if (!d2) CUDA_TRY(c, dalloc(&d2, (size_t)6 * s.P * s.npw));
     CUDA_TRY(c, launch_hess_assemble<C>(s.P, s.npw, s.d_rows, c->d_hess, c->hess_nq, c->hess_dq,
                                         1.0 / std::sqrt(c->omega), s.d_kvec, s.d_sf, d2, st));
+    built = !capturing(st);
     return HPSI_OK;
 }
 
@@ -2382,7 +2400,7 @@ extern "C" int hpsi_apply_noalloc(hpsi_ctx* c, int kid, int nb, const double* ps
     if (nb > 0 && (!psi_ || !hpsi_)) return fail(c, HPSI_ERR_BAD_ARG, "psi/hpsi NULL");
     if (nb == 0 || s->npw == 0) return HPSI_OK;
     const bool fp64 = prec == HPSI_PREC_FP64;
-    if (s->P > 0 && !(fp64 ? (void*)s->pr64 : (void*)s->pr32))
+    if (s->P > 0 && !(fp64 ? s->pr64_built : s->pr32_built))
         return fail(c, HPSI_ERR_STATE,
                     "hpsi_apply_noalloc: projector matrices of this precision are not built yet; one hpsi_apply or "
                     "hpsi_grad_apply at this precision on k-point %d builds them", kid);
