@@ -122,6 +122,19 @@ static int bfail(hpsi_batch* b, int code, const char* fmt, ...)
                          #expr, cudaGetErrorString(e_), __FILE__, __LINE__);                            \
     } while (0)
 
+// dalloc that asks the contexts for their optional memory before it reports that there is no room
+template <typename T>
+static cudaError_t balloc(hpsi_batch* b, T** p, size_t count)
+{
+    cudaError_t e = dalloc(p, count);
+    if (e != cudaErrorMemoryAllocation) return e;
+    bool freed = false;
+    for (const BItem& it : b->items) freed = release_optional(it.ctx) || freed;
+    if (!freed) return e;
+    cudaGetLastError();
+    return dalloc(p, count);
+}
+
 static void batch_free(hpsi_batch* b)
 {
     if (!b) return;
@@ -452,7 +465,7 @@ static int build_rag(hpsi_batch* b, Group& g)
     cv.take<unsigned>(nrm);
     if (g.rag.size() > 65535 || rows.size() > 65535 || bands.size() > 65535)
         return bfail(b, HPSI_ERR_BAD_ARG, "a tensor-core plan holds at most 65535 bands of one cell");
-    BCUDA(b, dalloc(&g.rag_mem, cv.off));
+    BCUDA(b, balloc(b, &g.rag_mem, cv.off));
     BCUDA(b, cudaMemset(g.rag_mem, 0, cv.off));
     g.rag_rowmax = reinterpret_cast<unsigned*>(g.rag_mem + rm0);
     g.rag_nrowmax = nrm;
@@ -474,10 +487,10 @@ static int build_rag(hpsi_batch* b, Group& g)
     g.rag_bands = (int)bands.size();
     g.rag_rows = (int)rows.size();
     g.rag_tiles = (int)tiles.size();
-    BCUDA(b, dalloc(&g.d_rag, g.rag.size()));
-    BCUDA(b, dalloc(&g.d_rag_bands, bands.size()));
-    BCUDA(b, dalloc(&g.d_rag_rows, rows.size()));
-    BCUDA(b, dalloc(&g.d_rag_tiles, tiles.size()));
+    BCUDA(b, balloc(b, &g.d_rag, g.rag.size()));
+    BCUDA(b, balloc(b, &g.d_rag_bands, bands.size()));
+    BCUDA(b, balloc(b, &g.d_rag_rows, rows.size()));
+    BCUDA(b, balloc(b, &g.d_rag_tiles, tiles.size()));
     BCUDA(b, cudaMemcpy(g.d_rag, g.rag.data(), g.rag.size() * sizeof(TcRagItem), cudaMemcpyHostToDevice));
     BCUDA(b, cudaMemcpy(g.d_rag_bands, bands.data(), bands.size() * sizeof(int2), cudaMemcpyHostToDevice));
     BCUDA(b, cudaMemcpy(g.d_rag_rows, rows.data(), rows.size() * sizeof(int2), cudaMemcpyHostToDevice));
@@ -541,13 +554,13 @@ static int build_group(hpsi_batch* b, Group& g)
     g.t_elems = t_off;
     BCUDA(b, cudaDeviceSynchronize());
     // device tables and buffers
-    BCUDA(b, dalloc(&g.d_litems, g.litems.size()));
-    BCUDA(b, dalloc(&g.d_band_item, band_item.size()));
-    BCUDA(b, dalloc(&g.d_xblk, (size_t)g.nbands));
-    BCUDA(b, dalloc(&g.d_gitems, g.gitems.size()));
+    BCUDA(b, balloc(b, &g.d_litems, g.litems.size()));
+    BCUDA(b, balloc(b, &g.d_band_item, band_item.size()));
+    BCUDA(b, balloc(b, &g.d_xblk, (size_t)g.nbands));
+    BCUDA(b, balloc(b, &g.d_gitems, g.gitems.size()));
     BCUDA(b, cudaMemcpy(g.d_litems, g.litems.data(), g.litems.size() * sizeof(LocalItem), cudaMemcpyHostToDevice));
     BCUDA(b, cudaMemcpy(g.d_band_item, band_item.data(), band_item.size() * sizeof(int), cudaMemcpyHostToDevice));
-    BCUDA(b, cudaMalloc(&g.T, std::max<size_t>(g.t_elems, 1) * cs));
+    BCUDA(b, balloc(b, (unsigned char**)&g.T, std::max<size_t>(g.t_elems, 1) * cs));
     g.max_split = 1;
     if (g.P > 0 && tc(b)) {
         int rc = build_rag(b, g);
@@ -555,8 +568,8 @@ static int build_group(hpsi_batch* b, Group& g)
     } else if (g.P > 0) {
         for (int ns : kSplits)
             if ((size_t)ns * g.P * g.nbands * cs <= kPartBudget) g.max_split = ns;
-        BCUDA(b, cudaMalloc(&g.part, (size_t)g.max_split * g.P * g.nbands * cs));
-        BCUDA(b, cudaMalloc(&g.W, (size_t)g.P * g.nbands * cs));
+        BCUDA(b, balloc(b, (unsigned char**)&g.part, (size_t)g.max_split * g.P * g.nbands * cs));
+        BCUDA(b, balloc(b, (unsigned char**)&g.W, (size_t)g.P * g.nbands * cs));
     }
     // local arguments shared by every launch of the cell
     LocalArgs& a = g.la;
@@ -604,8 +617,8 @@ static int batch_init(hpsi_batch* b, const hpsi_batch_item* items, int n_items, 
         }
     }
     BCUDA(b, cudaSetDevice(b->dev));
-    BCUDA(b, dalloc(&b->psi, std::max<size_t>(b->n_complex, 1)));
-    BCUDA(b, dalloc(&b->hpsi, std::max<size_t>(b->n_complex, 1)));
+    BCUDA(b, balloc(b, &b->psi, std::max<size_t>(b->n_complex, 1)));
+    BCUDA(b, balloc(b, &b->hpsi, std::max<size_t>(b->n_complex, 1)));
     BCUDA(b, cudaMemset(b->psi, 0, std::max<size_t>(b->n_complex, 1) * sizeof(double2)));
     BCUDA(b, cudaStreamCreateWithFlags(&b->s_cap, cudaStreamNonBlocking));
     BCUDA(b, cudaEventCreateWithFlags(&b->ev_start, cudaEventDisableTiming));

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <map>
 #include <string>
@@ -142,20 +143,6 @@ inline void slot_reset(KSlot& s)
     s = n;
 }
 
-// *p = a buffer of at least bytes: the spare when it fits, else a new one
-inline cudaError_t spare_alloc(Spare& spare, void** p, size_t* bytes)
-{
-    if (spare.p && spare.bytes >= *bytes && spare.bytes / 2 <= *bytes) {
-        *p = spare.p;
-        *bytes = spare.bytes;
-        spare = Spare{};
-        return cudaSuccess;
-    }
-    dfree(spare.p);
-    spare = Spare{};
-    return cudaMalloc(p, *bytes);
-}
-
 struct hpsi_ctx {
     int dev = 0;
     int n1 = 0, n2 = 0, n3 = 0;
@@ -188,10 +175,21 @@ struct hpsi_ctx {
     // would cost that call the time of a cudaFree (50-80 us)
     unsigned char* ws_first = nullptr;
     size_t ws_first_size = 0;
-    // workspace of the FP64 GEMMs on the tensor cores, within ws (set per call): a
-    // call that cannot have it runs the SIMT GEMMs
+    // workspace of the FP64 GEMMs on the tensor cores (set per call): behind the call's
+    // own in ws where that has room, else d64_mem.  A call that cannot have it runs the
+    // SIMT GEMMs, and d64_mem goes back to the device when anything else finds no room.
     unsigned char* d64_ws = nullptr;
     size_t d64_size = 0;
+    unsigned char* d64_mem = nullptr;
+    size_t d64_cap = 0;
+    // the smallest workspace that the device had no room for, and its free bytes then:
+    // not asked for again before more is free
+    size_t d64_refused = SIZE_MAX, d64_refused_free = 0;
+    // test hooks (hpsi_selftest_memory): largest d64_mem granted, allocations that are
+    // to find no room, and allocations of d64_mem tried
+    size_t test_d64_room = SIZE_MAX;
+    int test_oom = 0;
+    long d64_tries = 0;
     bool d64_ran = false;         // d_err is checked at the next synchronising call
     Prof prof;
     int* d_err = nullptr;         // device-side error flag of the bounded waits (tcgen05 GEMMs)
@@ -252,16 +250,52 @@ struct Carver {
     }
 };
 
+// Give memory that only makes calls faster back to the device; false if there is none.
+inline bool release_optional(hpsi_ctx* c)
+{
+    if (!c->d64_mem) return false;
+    if (c->d64_ws == c->d64_mem) c->d64_ws = nullptr;
+    dfree(c->d64_mem);
+    c->d64_cap = 0;
+    return true;
+}
+
+// cudaMalloc that asks for optional memory back before it reports that there is no room
+template <typename T>
+inline cudaError_t dev_malloc(hpsi_ctx* c, T** p, size_t bytes)
+{
+    *p = nullptr;
+    cudaError_t e = c->test_oom > 0 ? cudaErrorMemoryAllocation : cudaMalloc((void**)p, bytes);
+    if (c->test_oom > 0) --c->test_oom;
+    if (e != cudaErrorMemoryAllocation || !release_optional(c)) return e;
+    cudaGetLastError();
+    return cudaMalloc((void**)p, bytes);
+}
+
+// *p = a buffer of at least bytes: the spare when it fits, else a new one
+inline cudaError_t spare_alloc(hpsi_ctx* c, Spare& spare, void** p, size_t* bytes)
+{
+    if (spare.p && spare.bytes >= *bytes && spare.bytes / 2 <= *bytes) {
+        *p = spare.p;
+        *bytes = spare.bytes;
+        spare = Spare{};
+        return cudaSuccess;
+    }
+    dfree(spare.p);
+    spare = Spare{};
+    return dev_malloc(c, p, *bytes);
+}
+
 inline int ws_reserve(hpsi_ctx* c, size_t bytes)
 {
+    c->d64_ws = nullptr;
     if (bytes <= c->ws_size) return HPSI_OK;
     if (c->ws != c->ws_first) cudaFree(c->ws);
     c->ws = c->ws_first;
     c->ws_size = c->ws_first_size;
-    c->d64_ws = nullptr;
     const size_t want = bytes + bytes / 8;
     unsigned char* p = nullptr;
-    CUDA_TRY(c, cudaMalloc((void**)&p, want));
+    CUDA_TRY(c, dev_malloc(c, &p, want));
     c->ws = p;
     c->ws_size = want;
     if (!c->ws_first) {
@@ -271,26 +305,47 @@ inline int ws_reserve(hpsi_ctx* c, size_t bytes)
     return HPSI_OK;
 }
 
-// Reserve base bytes, and extra bytes behind them for the FP64 GEMMs on the tensor
-// cores (d64_ws).  Without room for extra the call goes on with base alone.
-inline int ws_reserve_d64(hpsi_ctx* c, size_t base, size_t extra)
+// d64_mem of at least bytes; false when the device has no room, or under capture
+// (an allocation would end it)
+inline bool d64_reserve(hpsi_ctx* c, size_t bytes, cudaStream_t st)
 {
-    const size_t off = (base + 255) / 256 * 256;
-    c->d64_ws = nullptr;
-    c->d64_size = 0;
-    if (extra) {
-        const std::string err = c->err;
-        const int rc = ws_reserve(c, off + extra);
-        if (rc == HPSI_OK) {
-            c->d64_ws = c->ws + off;
-            c->d64_size = extra;
-            return HPSI_OK;
+    if (bytes <= c->d64_cap) return true;
+    if (capturing(st)) return false;
+    size_t free_bytes = 0, total = 0;
+    if (bytes >= c->d64_refused &&
+        (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes <= c->d64_refused_free))
+        return false;
+    release_optional(c);
+    ++c->d64_tries;
+    for (size_t want : {bytes + bytes / 8, bytes}) {
+        if (want <= c->test_d64_room && cudaMalloc((void**)&c->d64_mem, want) == cudaSuccess) {
+            c->d64_cap = want;
+            c->d64_refused = SIZE_MAX;
+            return true;
         }
-        if (rc != HPSI_ERR_OOM) return rc;
         cudaGetLastError();  // not an error of the call
-        c->err = err;
     }
-    return ws_reserve(c, base);
+    c->d64_mem = nullptr;
+    c->d64_refused = bytes;
+    if (cudaMemGetInfo(&c->d64_refused_free, &total) != cudaSuccess) c->d64_refused_free = 0;
+    return false;
+}
+
+// Reserve base bytes, and extra bytes for the FP64 GEMMs on the tensor cores
+// (d64_ws).  Without room for extra the call goes on with base alone.
+inline int ws_reserve_d64(hpsi_ctx* c, size_t base, size_t extra, cudaStream_t st)
+{
+    const int rc = ws_reserve(c, base);
+    if (rc || extra == 0) return rc;
+    const size_t off = (base + 255) / 256 * 256;
+    if (off + extra <= c->ws_size && extra <= c->test_d64_room) {
+        c->d64_ws = c->ws + off;
+    } else {
+        if (!d64_reserve(c, extra, st)) return HPSI_OK;
+        c->d64_ws = c->d64_mem;
+    }
+    c->d64_size = extra;
+    return HPSI_OK;
 }
 
 // Build, once, what a precision needs on slot s (projector matrices, tensor-core

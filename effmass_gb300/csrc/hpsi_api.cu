@@ -41,6 +41,7 @@ extern "C" int hpsi_ctx_destroy(hpsi_ctx* c)
     dfree(c->d_tw64); dfree(c->d_tw32); dfree(c->d_err); dfree(c->d_hess);
     if (c->ws != c->ws_first) cudaFree(c->ws);
     if (c->ws_first) cudaFree(c->ws_first);
+    dfree(c->d64_mem);
     if (c->stage) cudaFreeHost(c->stage);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -350,7 +351,7 @@ extern "C" int hpsi_set_kpoint(hpsi_ctx* c, int kid, const hpsi_kpoint* kp)
         const size_t o_db0 = cv.take<double>((size_t)c->nrad), o_sf = cv.take<double2>((size_t)c->natom * npw);
         if (s.mem && (s.mem_cap < cv.off || (s.mem_cap > kSpareMax && s.mem_cap / 2 > cv.off))) dfree(s.mem);
         if (!s.mem) {
-            CUDA_TRY(c, dalloc(&s.mem, cv.off));
+            CUDA_TRY(c, dev_malloc(c, &s.mem, cv.off));
             s.mem_cap = cv.off;
         }
         if (c->stage_size < upload) {
@@ -430,8 +431,8 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
         size_t bytes = rows * s.npw * sizeof(C) + n_exp * sizeof(int);
         const int k = f64 ? 0 : 1;
         // a spare would let a capture record a build that it otherwise refuses
-        if (record) CUDA_TRY(c, cudaMalloc((void**)&pr, bytes));
-        else CUDA_TRY(c, spare_alloc(s.spare_pr[k], (void**)&pr, &bytes));
+        if (record) CUDA_TRY(c, dev_malloc(c, &pr, bytes));
+        else CUDA_TRY(c, spare_alloc(c, s.spare_pr[k], (void**)&pr, &bytes));
         s.pr_bytes[k] = bytes;
         if (f64) {
             s.d64_exp[0] = reinterpret_cast<int*>(pr + rows * s.npw);
@@ -779,7 +780,7 @@ static int ensure_tc(hpsi_ctx* c, KSlot& s, int fmt, cudaStream_t st)
     }
     const int nby = (int)byinfo.size();
     size_t bytes = tc_gen_bytes(s.P, s.npw, nby, c->natom);
-    CUDA_TRY(c, spare_alloc(s.spare_tc[fmt], (void**)&s.tc_mem[fmt], &bytes));
+    CUDA_TRY(c, spare_alloc(c, s.spare_tc[fmt], (void**)&s.tc_mem[fmt], &bytes));
     s.tc_bytes[fmt] = bytes;
     int h = c->prof.open(PH_BUILD, st);
     CUDA_TRY(c, tc_build_gen(s.tc_mem[fmt], s.P, s.npw, prow.data(), byinfo.data(), nby, c->natom, s.d_beta,
@@ -915,7 +916,7 @@ static int ensure_tc_grad(hpsi_ctx* c, KSlot& s, int fmt, cudaStream_t st)
         os[a] = cv.take<float>((size_t)s.npw);
     }
     const size_t ocm = cv.take<float>((size_t)s.npw);
-    if (!s.tcg_mem) CUDA_TRY(c, dalloc(&s.tcg_mem, cv.off));
+    if (!s.tcg_mem) CUDA_TRY(c, dev_malloc(c, &s.tcg_mem, cv.off));
     CUDA_TRY(c, cudaMemsetAsync(s.tcg_mem, 0, cv.off, st));  // padding rows and K padding read as zero
     s.tcg_proj = TcOperand{s.tcg_mem + o1h, s.tcg_mem + o1l, reinterpret_cast<float*>(s.tcg_mem + o1s), k1};
     for (int a = 0; a < 3; ++a)
@@ -1453,7 +1454,9 @@ extern "C" int hpsi_apply(hpsi_ctx* c, int kid, int nb, const double* psi_, doub
     size_t o_psi = dev ? 0 : cv.take<double2>(nel);
     size_t o_hpsi = dev ? 0 : cv.take<double2>(nel);
     size_t o_work = cv.off;
-    if ((rc = ws_reserve_d64(c, o_work + apply_ws_bytes(c, *s, nb, prec), d64_apply_bytes(*s, nb, prec)))) return rc;
+    if ((rc = ws_reserve_d64(c, o_work + apply_ws_bytes(c, *s, nb, prec), d64_apply_bytes(*s, nb, prec),
+                             st)))
+        return rc;
     const double2* psi = (const double2*)psi_;
     double2* hpsi = (double2*)hpsi_;
     const bool fork = !(flags & HPSI_ONE_STREAM);
@@ -1555,7 +1558,7 @@ extern "C" int hpsi_apply_energies(hpsi_ctx* c, int kid, int nb, const double* p
     size_t o_work = cv.off;
     const EnergyWs w = energy_layout(c, nb, prec);
     if ((rc = ws_reserve_d64(c, o_work + w.work + apply_ws_bytes(c, *s, nb, prec, true),
-                             d64_apply_bytes(*s, nb, prec))))
+                             d64_apply_bytes(*s, nb, prec), st)))
         return rc;
     const double2* psi = (const double2*)psi_;
     double2* hpsi = (double2*)hpsi_;
@@ -1631,7 +1634,7 @@ extern "C" int hpsi_sternheimer(hpsi_ctx* c, int kid, int nv, const double* psi_
     const size_t o_work = cv.off;
     const size_t work = std::max(apply_ws_bytes(c, *s, nv, prec), grad_ws_bytes(*s, nv, prec));
     const size_t d64 = std::max(d64_apply_bytes(*s, nv, prec), d64_grad_bytes(*s, nv, 1, prec));
-    if ((rc = ws_reserve_d64(c, o_work + work, d64))) return rc;
+    if ((rc = ws_reserve_d64(c, o_work + work, d64, st))) return rc;
     unsigned char* ws = c->ws;
     const double2* psi = dev ? (const double2*)psi_ : reinterpret_cast<const double2*>(ws + o_psi);
     const double* eps = dev ? eps_ : reinterpret_cast<const double*>(ws + o_eps);
@@ -1952,7 +1955,7 @@ static int ensure_hess(hpsi_ctx* c, KSlot& s, cudaStream_t st)
     CUDA_TRY(c, cudaMemcpy(q.data(), s.d_q, s.npw * sizeof(double), cudaMemcpyDeviceToHost));
     for (double v : q)
         if (v > qtop) return fail(c, HPSI_ERR_RANGE, "q=%.17g beyond the Hessian tables (%.17g)", v, qtop);
-    if (!d2) CUDA_TRY(c, dalloc(&d2, (size_t)6 * s.P * s.npw));
+    if (!d2) CUDA_TRY(c, dev_malloc(c, &d2, (size_t)6 * s.P * s.npw * sizeof(C)));
     CUDA_TRY(c, launch_hess_assemble<C>(s.P, s.npw, s.d_rows, c->d_hess, c->hess_nq, c->hess_dq,
                                         1.0 / std::sqrt(c->omega), s.d_kvec, s.d_sf, d2, st));
     built = !capturing(st);
@@ -2156,7 +2159,8 @@ extern "C" int hpsi_grad_apply(hpsi_ctx* c, int kid, int nb, const double* psi_,
         if (!dev && outs[a]) o_out[a] = cv.take<double2>(nel);
     size_t o_work = cv.off;
     const int nd = (dx != nullptr) + (dy != nullptr) + (dz != nullptr);
-    if ((rc = ws_reserve_d64(c, o_work + grad_ws_bytes(*s, nb, prec), d64_grad_bytes(*s, nb, nd, prec)))) return rc;
+    if ((rc = ws_reserve_d64(c, o_work + grad_ws_bytes(*s, nb, prec), d64_grad_bytes(*s, nb, nd, prec), st)))
+        return rc;
     const double2* psi = (const double2*)psi_;
     double2* d[3] = {(double2*)dx, (double2*)dy, (double2*)dz};
     if (!dev) {
@@ -2201,7 +2205,8 @@ extern "C" int hpsi_velocity_matrix(hpsi_ctx* c, int kid, int nb, const double* 
     size_t o_psi = dev ? 0 : cv.take<double2>(nel);
     size_t o_m = dev ? 0 : cv.take<double2>(nm);
     size_t o_work = cv.off;
-    if ((rc = ws_reserve_d64(c, o_work + vel_ws_bytes(*s, nb, prec), d64_velocity_bytes(*s, nb, prec)))) return rc;
+    if ((rc = ws_reserve_d64(c, o_work + vel_ws_bytes(*s, nb, prec), d64_velocity_bytes(*s, nb, prec), st)))
+        return rc;
     const double2* psi = (const double2*)psi_;
     double2* m = (double2*)m_;
     if (!dev) {
@@ -2415,6 +2420,29 @@ extern "C" int hpsi_apply_noalloc(hpsi_ctx* c, int kid, int nb, const double* ps
                                                            st);
     if (rc) return rc;
     if (flags & HPSI_SYNC) CUDA_TRY(c, cudaStreamSynchronize(st));
+    return HPSI_OK;
+}
+
+// Test hooks.  room: the largest tensor-core workspace of FP64 calls that is granted
+// (< 0: any); oom: so many of the context's next allocations find no room at first.
+// out: workspace address and bytes, bytes of d64_mem, allocations of it tried.
+extern "C" int hpsi_selftest_memory(hpsi_ctx* c, long long room, int oom)
+{
+    if (!c) return HPSI_ERR_BAD_ARG;
+    c->test_d64_room = room < 0 ? SIZE_MAX : (size_t)room;
+    c->test_oom = oom;
+    if (room < 0) c->d64_refused = SIZE_MAX;
+    else if (c->d64_cap > (size_t)room) release_optional(c);
+    return HPSI_OK;
+}
+
+extern "C" int hpsi_selftest_memory_state(const hpsi_ctx* c, long long* out)
+{
+    if (!c || !out) return HPSI_ERR_BAD_ARG;
+    out[0] = (long long)(uintptr_t)c->ws;
+    out[1] = (long long)c->ws_size;
+    out[2] = (long long)c->d64_cap;
+    out[3] = c->d64_tries;
     return HPSI_OK;
 }
 
@@ -2940,8 +2968,14 @@ extern "C" int hpsi_server_create(hpsi_ctx* const* systems, int n_systems, const
                 return srv_fail(nullptr, rc, m);
             }
         }
-    if (cudaDeviceSynchronize() != cudaSuccess ||
-        cudaMalloc((void**)&S->arena_mem, cfg->device_budget_bytes) != cudaSuccess) {
+    cudaError_t e = cudaDeviceSynchronize();
+    if (!e) e = cudaMalloc((void**)&S->arena_mem, cfg->device_budget_bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        for (hpsi_ctx* c : S->sys) release_optional(c);
+        e = cudaMalloc((void**)&S->arena_mem, cfg->device_budget_bytes);
+    }
+    if (e) {
         delete S;
         return srv_fail(nullptr, HPSI_ERR_OOM, "server: cannot allocate the device budget");
     }

@@ -410,6 +410,13 @@ int hpsi_selftest_kpoint_tables(hpsi_ctx* ctx, int kid, double* ylm, double* sf)
  * and the next synchronising call returns HPSI_ERR_TIMEOUT. */
 int hpsi_selftest_wait_limit(long polls);
 
+/* Test hooks for device memory that runs out.  room: the largest workspace of the
+ * FP64 tensor-core GEMMs that the context is granted (< 0: any); oom: so many of
+ * its next allocations find no room at first.  _state: out[4] = workspace address
+ * and bytes, bytes held for the FP64 GEMMs, allocations of those tried so far. */
+int hpsi_selftest_memory(hpsi_ctx* ctx, long long room, int oom);
+int hpsi_selftest_memory_state(const hpsi_ctx* ctx, long long* out);
+
 /* Message of the last failed call on ctx (never NULL); with ctx == NULL the
  * message of the calling thread's last failed hpsi_ctx_create. */
 const char* hpsi_last_error(const hpsi_ctx* ctx);
