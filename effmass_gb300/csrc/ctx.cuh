@@ -14,13 +14,14 @@
 #include "kernels.cuh"
 #include "tc_gemm.cuh"
 
-// A device buffer kept by a slot when it is rebound, for the next binding
+// A device buffer kept when a slot is rebound, for the next binding
 struct Spare {
     void* p = nullptr;
     size_t bytes = 0;
 };
-// Larger buffers go back to the device at once (their builds take longer than
-// cudaMalloc and cudaFree).
+// What a context keeps at most, all spares together.  Larger buffers go back to the
+// device at once (their builds take longer than cudaMalloc and cudaFree), and so
+// does a spare that no call took between two rebindings.
 constexpr size_t kSpareMax = 64ull << 20;
 
 struct KSlot {
@@ -58,7 +59,6 @@ struct KSlot {
     bool pr32_built = false, pr32_grad = false;
     size_t pr_bytes[2] = {0, 0};   // allocation sizes of pr64, pr32
     size_t tc_bytes[2] = {0, 0};   // and of tc_mem
-    Spare spare_pr[2], spare_tc[2];
     // tensor-core H|psi>: generator tables of the projector operands, one set
     // per split format (0 FP16, 1 BF16), built from the FP64 tables on first
     // use and kept until the slot is rebound (batch plans hold pointers into
@@ -110,37 +110,9 @@ inline void dfree(T*& p)
 inline void slot_free(KSlot& s)
 {
     dfree(s.mem);
-    for (Spare* p : {&s.spare_pr[0], &s.spare_pr[1], &s.spare_tc[0], &s.spare_tc[1]}) dfree(p->p);
     dfree(s.pr64); dfree(s.pr32); dfree(s.tc_mem[0]); dfree(s.tc_mem[1]); dfree(s.tcg_mem); dfree(s.hess64);
     dfree(s.hess32);
     s = KSlot();
-}
-
-// Empty slot s for a new binding.  The tables' allocation stays, and projector
-// buffers of up to kSpareMax stay as spares.  The caller has synchronised the device.
-inline void slot_reset(KSlot& s)
-{
-    KSlot n;
-    n.mem = s.mem;
-    n.mem_cap = s.mem_cap;
-    s.mem = nullptr;
-    auto keep = [](void* p, size_t bytes, Spare& old, Spare& to) {
-        if (p && bytes <= kSpareMax) {
-            dfree(old.p);
-            to = Spare{p, bytes};
-            return true;
-        }
-        to = old;
-        old = Spare{};
-        return false;
-    };
-    if (keep(s.pr64, s.pr_bytes[0], s.spare_pr[0], n.spare_pr[0])) s.pr64 = nullptr;
-    if (keep(s.pr32, s.pr_bytes[1], s.spare_pr[1], n.spare_pr[1])) s.pr32 = nullptr;
-    for (int f = 0; f < 2; ++f)
-        if (keep(s.tc_mem[f], s.tc_bytes[f], s.spare_tc[f], n.spare_tc[f])) s.tc_mem[f] = nullptr;
-    for (int f = 0; f < 2; ++f) s.spare_pr[f] = s.spare_tc[f] = Spare{};  // moved or freed above
-    slot_free(s);
-    s = n;
 }
 
 struct hpsi_ctx {
@@ -162,6 +134,8 @@ struct hpsi_ctx {
     float2* d_tw32 = nullptr;
     FftLen L[3];
     std::map<int, KSlot> slots;
+    // projector buffers of the last binding that was replaced: pr64, pr32, tc_mem[0], [1]
+    Spare spare[4];
     // projector rows and strengths (the same for every k-point), and the largest q
     // that every radial table covers
     std::vector<ProjRow> proj_rows;
@@ -253,11 +227,16 @@ struct Carver {
 // Give memory that only makes calls faster back to the device; false if there is none.
 inline bool release_optional(hpsi_ctx* c)
 {
-    if (!c->d64_mem) return false;
+    bool any = c->d64_mem != nullptr;
     if (c->d64_ws == c->d64_mem) c->d64_ws = nullptr;
     dfree(c->d64_mem);
     c->d64_cap = 0;
-    return true;
+    for (Spare& p : c->spare) {
+        any = any || p.p;
+        dfree(p.p);
+        p.bytes = 0;
+    }
+    return any;
 }
 
 // cudaMalloc that asks for optional memory back before it reports that there is no room
@@ -272,11 +251,37 @@ inline cudaError_t dev_malloc(hpsi_ctx* c, T** p, size_t bytes)
     return cudaMalloc((void**)p, bytes);
 }
 
+// Empty slot s for a new binding.  The tables' allocation stays with it, its projector
+// buffers stay with the context as spares.  The caller has synchronised the device.
+inline void slot_reset(hpsi_ctx* c, KSlot& s)
+{
+    size_t kept = 0;
+    auto keep = [&](Spare& to, auto*& p, size_t bytes) {
+        dfree(to.p);
+        to.bytes = 0;
+        if (!p || kept + bytes > kSpareMax) return;
+        to = Spare{p, bytes};
+        kept += bytes;
+        p = nullptr;
+    };
+    keep(c->spare[0], s.pr64, s.pr_bytes[0]);
+    keep(c->spare[1], s.pr32, s.pr_bytes[1]);
+    keep(c->spare[2], s.tc_mem[0], s.tc_bytes[0]);
+    keep(c->spare[3], s.tc_mem[1], s.tc_bytes[1]);
+    unsigned char* mem = s.mem;
+    const size_t cap = s.mem_cap;
+    s.mem = nullptr;
+    slot_free(s);
+    s.mem = mem;
+    s.mem_cap = cap;
+}
+
 // *p = a buffer of at least bytes: the spare when it fits, else a new one
-inline cudaError_t spare_alloc(hpsi_ctx* c, Spare& spare, void** p, size_t* bytes)
+template <typename T>
+inline cudaError_t spare_alloc(hpsi_ctx* c, Spare& spare, T** p, size_t* bytes)
 {
     if (spare.p && spare.bytes >= *bytes && spare.bytes / 2 <= *bytes) {
-        *p = spare.p;
+        *p = static_cast<T*>(spare.p);
         *bytes = spare.bytes;
         spare = Spare{};
         return cudaSuccess;

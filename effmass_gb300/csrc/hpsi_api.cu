@@ -41,7 +41,7 @@ extern "C" int hpsi_ctx_destroy(hpsi_ctx* c)
     dfree(c->d_tw64); dfree(c->d_tw32); dfree(c->d_err); dfree(c->d_hess);
     if (c->ws != c->ws_first) cudaFree(c->ws);
     if (c->ws_first) cudaFree(c->ws_first);
-    dfree(c->d64_mem);
+    release_optional(c);
     if (c->stage) cudaFreeHost(c->stage);
     if (c->side) cudaStreamDestroy(c->side);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -329,7 +329,7 @@ extern "C" int hpsi_set_kpoint(hpsi_ctx* c, int kid, const hpsi_kpoint* kp)
     KSlot& s = c->slots[kid];
     // work queued on any stream may still read the old tables
     if (s.mem) CUDA_TRY(c, cudaDeviceSynchronize());
-    slot_reset(s);
+    slot_reset(c, s);
     s.gen = ++c->gen_counter;
     s.npw = npw;
     for (int d = 0; d < 3; ++d) s.kf[d] = kp->k_frac[d];
@@ -432,7 +432,7 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
         const int k = f64 ? 0 : 1;
         // a spare would let a capture record a build that it otherwise refuses
         if (record) CUDA_TRY(c, dev_malloc(c, &pr, bytes));
-        else CUDA_TRY(c, spare_alloc(c, s.spare_pr[k], (void**)&pr, &bytes));
+        else CUDA_TRY(c, spare_alloc(c, c->spare[k], &pr, &bytes));
         s.pr_bytes[k] = bytes;
         if (f64) {
             s.d64_exp[0] = reinterpret_cast<int*>(pr + rows * s.npw);
@@ -780,7 +780,7 @@ static int ensure_tc(hpsi_ctx* c, KSlot& s, int fmt, cudaStream_t st)
     }
     const int nby = (int)byinfo.size();
     size_t bytes = tc_gen_bytes(s.P, s.npw, nby, c->natom);
-    CUDA_TRY(c, spare_alloc(c, s.spare_tc[fmt], (void**)&s.tc_mem[fmt], &bytes));
+    CUDA_TRY(c, spare_alloc(c, c->spare[2 + fmt], &s.tc_mem[fmt], &bytes));
     s.tc_bytes[fmt] = bytes;
     int h = c->prof.open(PH_BUILD, st);
     CUDA_TRY(c, tc_build_gen(s.tc_mem[fmt], s.P, s.npw, prow.data(), byinfo.data(), nby, c->natom, s.d_beta,
@@ -2425,7 +2425,8 @@ extern "C" int hpsi_apply_noalloc(hpsi_ctx* c, int kid, int nb, const double* ps
 
 // Test hooks.  room: the largest tensor-core workspace of FP64 calls that is granted
 // (< 0: any); oom: so many of the context's next allocations find no room at first.
-// out: workspace address and bytes, bytes of d64_mem, allocations of it tried.
+// out: workspace address and bytes, bytes of d64_mem, allocations of it tried, bytes
+// of spares.
 extern "C" int hpsi_selftest_memory(hpsi_ctx* c, long long room, int oom)
 {
     if (!c) return HPSI_ERR_BAD_ARG;
@@ -2443,6 +2444,8 @@ extern "C" int hpsi_selftest_memory_state(const hpsi_ctx* c, long long* out)
     out[1] = (long long)c->ws_size;
     out[2] = (long long)c->d64_cap;
     out[3] = c->d64_tries;
+    out[4] = 0;
+    for (const Spare& p : c->spare) out[4] += (long long)p.bytes;
     return HPSI_OK;
 }
 

@@ -412,8 +412,9 @@ int hpsi_selftest_wait_limit(long polls);
 
 /* Test hooks for device memory that runs out.  room: the largest workspace of the
  * FP64 tensor-core GEMMs that the context is granted (< 0: any); oom: so many of
- * its next allocations find no room at first.  _state: out[4] = workspace address
- * and bytes, bytes held for the FP64 GEMMs, allocations of those tried so far. */
+ * its next allocations find no room at first.  _state: out[5] = workspace address
+ * and bytes, bytes held for the FP64 GEMMs, allocations of those tried so far,
+ * bytes kept of replaced bindings. */
 int hpsi_selftest_memory(hpsi_ctx* ctx, long long room, int oom);
 int hpsi_selftest_memory_state(const hpsi_ctx* ctx, long long* out);
 

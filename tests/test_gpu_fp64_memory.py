@@ -36,7 +36,7 @@ class Case:
         assert self.lib.hpsi_selftest_memory(self.H.ctx, room, oom) == 0
 
     def state(self):
-        out = (C.c_longlong * 4)()
+        out = (C.c_longlong * 5)()
         assert self.lib.hpsi_selftest_memory_state(self.H.ctx, out) == 0
         return list(out)
 
