@@ -558,6 +558,7 @@ static int d64_begin(hpsi_ctx* c, KSlot& s, int M, int nb, size_t expand_ws, D64
     d->ops = ws + cv.off;
     *ok = true;
     c->d64_ran = true;
+    c->d64_stream = st;
     return d64_scale(c, s, M > s.P, &d->sc, st);
 }
 
@@ -615,6 +616,7 @@ static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const
     if (!ws || c->d64_size < o_ops + d64_proj_ws(nb, nb, s.npw)) return HPSI_OK;
     *done = true;
     c->d64_ran = true;
+    c->d64_stream = st;
     double2* part = reinterpret_cast<double2*>(ws + o_part);
     int* ex = reinterpret_cast<int*>(ws + o_exp);
     const D64Scale sc{ex, ex + s.npw};
@@ -735,6 +737,23 @@ static size_t local_ws(const hpsi_ctx* c, const KSlot& s, int nb, size_t csize)
     Carver cv;
     cv.take<unsigned char>((size_t)ch * s.nxs * c->n2 * c->n3 * csize);
     return cv.off;
+}
+
+// End of a synchronising call: wait for st, and report a bounded wait of the
+// tensor-core kernels that gave up in it (tc: it ran such kernels) or in an earlier
+// FP64 call on st that did not synchronise.
+static int finish(hpsi_ctx* c, cudaStream_t st, bool tc)
+{
+    CUDA_TRY(c, cudaStreamSynchronize(st));
+    if (!tc && !c->d64_ran) return HPSI_OK;
+    if (c->d64_stream == st) c->d64_ran = false;
+    int v = 0;
+    CUDA_TRY(c, cudaMemcpy(&v, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (v) {
+        cudaMemset(c->d_err, 0, sizeof(int));
+        return fail(c, HPSI_ERR_TIMEOUT, "tensor-core GEMM: a bounded pipeline wait gave up (site %d)", v);
+    }
+    return HPSI_OK;
 }
 
 static int check_call(hpsi_ctx* c, int kid, int nb, KSlot** sp, int flags)
@@ -990,19 +1009,6 @@ static int tc_grad_nonlocal(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, d
     return HPSI_OK;
 }
 
-// After a synchronising call: report a bounded-wait timeout of the tensor-core kernels.
-static int check_device_flag(hpsi_ctx* c)
-{
-    int v = 0;
-    c->d64_ran = false;
-    CUDA_TRY(c, cudaMemcpy(&v, c->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (v) {
-        cudaMemset(c->d_err, 0, sizeof(int));
-        return fail(c, HPSI_ERR_TIMEOUT, "tensor-core GEMM: a bounded pipeline wait gave up (site %d)", v);
-    }
-    return HPSI_OK;
-}
-
 // d_a += K_a psi, or with SET d_a = K_a psi
 template <bool SET>
 __global__ void grad_kinetic_kernel(int npw, int nb, const double* __restrict__ kvec, const double2* __restrict__ psi,
@@ -1120,8 +1126,10 @@ static bool fork_fp32(const KSlot& s, int nb)
     return work > 0.8e6 && work < 250e6;
 }
 
-// workspace of one H|psi> on device pointers
-static size_t apply_ws_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int prec, bool energy = false)
+// workspace of one H|psi> on device pointers; fork: the projection chain may run
+// beside the FFT passes (never on the server's lanes)
+static size_t apply_ws_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int prec, bool energy = false,
+                             bool fork = true)
 {
     const bool fp64 = prec == HPSI_PREC_FP64;
     size_t wl = local_ws(c, s, nb, fp64 ? sizeof(double2) : sizeof(float2));
@@ -1132,7 +1140,8 @@ static size_t apply_ws_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int prec
         return wl + tc_ws(s, nb, energy) + (s.P > 0 ? cv.off : 0);
     }
     if (fp64) return std::max(wl, nonlocal_ws<double2, double2>(s, nb, 1));
-    return wl + nonlocal_ws<float2, float2>(s, nb, 1);  // disjoint: they run concurrently
+    const size_t wn = nonlocal_ws<float2, float2>(s, nb, 1);
+    return fork && fork_fp32(s, nb) ? wl + wn : std::max(wl, wn);  // disjoint where they run concurrently
 }
 
 // hpsi += H psi on device pointers with an explicit workspace (prepare_slot first)
@@ -1527,10 +1536,7 @@ extern "C" int hpsi_apply(hpsi_ctx* c, int kid, int nb, const double* psi_, doub
     } else if (!dev) {
         CUDA_TRY(c, cudaMemcpyAsync(hpsi_, hpsi, nel * sizeof(double2), cudaMemcpyDeviceToHost, st));
     }
-    if (!dev || (flags & HPSI_SYNC)) {
-        CUDA_TRY(c, cudaStreamSynchronize(st));
-        if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
-    }
+    if (!dev || (flags & HPSI_SYNC)) return finish(c, st, is_tc(prec));
     return HPSI_OK;
 }
 
@@ -1576,10 +1582,7 @@ extern "C" int hpsi_apply_energies(hpsi_ctx* c, int kid, int nb, const double* p
         CUDA_TRY(c, cudaMemcpyAsync(hpsi_, hpsi, nel * sizeof(double2), cudaMemcpyDeviceToHost, st));
         CUDA_TRY(c, cudaMemcpyAsync(eout, e, nb * sizeof(double), cudaMemcpyDeviceToHost, st));
     }
-    if (!dev || (flags & HPSI_SYNC)) {
-        CUDA_TRY(c, cudaStreamSynchronize(st));
-        if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
-    }
+    if (!dev || (flags & HPSI_SYNC)) return finish(c, st, is_tc(prec));
     return HPSI_OK;
 }
 
@@ -1719,8 +1722,7 @@ extern "C" int hpsi_sternheimer(hpsi_ctx* c, int kid, int nv, const double* psi_
     if (residual)
         for (int b = 0; b < nv; ++b) residual[b] = hb[b] > 0.0 ? std::sqrt(hr[b] / hb[b]) : 0.0;
     if (!dev) CUDA_TRY(c, cudaMemcpyAsync(x_, x, nel * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(c, cudaStreamSynchronize(st));
-    if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
+    if ((rc = finish(c, st, is_tc(prec)))) return rc;
     if (n_active > 0)
         return fail(c, HPSI_ERR_TIMEOUT, "Sternheimer CG: %d of %d bands above tol after %d iterations", n_active, nv,
                     it);
@@ -2045,7 +2047,7 @@ extern "C" int hpsi_hess_apply(hpsi_ctx* c, int kid, int nb, const double* psi_,
     if (!dev)
         for (int k = 0; k < 6; ++k)
             if (out[k]) CUDA_TRY(c, cudaMemcpyAsync(o_[k], out[k], nel * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    if (!dev || (flags & HPSI_SYNC)) CUDA_TRY(c, cudaStreamSynchronize(st));
+    if (!dev || (flags & HPSI_SYNC)) return finish(c, st, false);
     return HPSI_OK;
 }
 
@@ -2088,7 +2090,7 @@ extern "C" int hpsi_density(hpsi_ctx* c, int kid, int nb, const double* psi_, co
               : density_apply<float2>(c, *s, nb, psi, occ, rho, c->ws + o_work, c->d_tw32, st);
     if (rc) return rc;
     if (!dev) CUDA_TRY(c, cudaMemcpyAsync(rho_, rho, N * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (!dev || (flags & HPSI_SYNC)) CUDA_TRY(c, cudaStreamSynchronize(st));
+    if (!dev || (flags & HPSI_SYNC)) return finish(c, st, false);
     return HPSI_OK;
 }
 
@@ -2176,10 +2178,7 @@ extern "C" int hpsi_grad_apply(hpsi_ctx* c, int kid, int nb, const double* psi_,
     if (!dev)
         for (int a = 0; a < 3; ++a)
             if (outs[a]) CUDA_TRY(c, cudaMemcpyAsync(outs[a], d[a], nel * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    if (!dev || (flags & HPSI_SYNC)) {
-        CUDA_TRY(c, cudaStreamSynchronize(st));
-        if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
-    }
+    if (!dev || (flags & HPSI_SYNC)) return finish(c, st, is_tc(prec));
     return HPSI_OK;
 }
 
@@ -2216,10 +2215,7 @@ extern "C" int hpsi_velocity_matrix(hpsi_ctx* c, int kid, int nb, const double* 
     }
     if ((rc = velocity_dev(c, *s, nb, psi, m, prec, c->ws + o_work, st))) return rc;
     if (!dev) CUDA_TRY(c, cudaMemcpyAsync(m_, m, nm * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    if (!dev || (flags & HPSI_SYNC)) {
-        CUDA_TRY(c, cudaStreamSynchronize(st));
-        if ((is_tc(prec) || c->d64_ran) && (rc = check_device_flag(c))) return rc;
-    }
+    if (!dev || (flags & HPSI_SYNC)) return finish(c, st, is_tc(prec));
     return HPSI_OK;
 }
 
@@ -2419,7 +2415,7 @@ extern "C" int hpsi_apply_noalloc(hpsi_ctx* c, int kid, int nb, const double* ps
               : apply_noalloc_impl<float2, float2, float>(c, *s, nb, psi, hpsi, s->pr32, c->d_v32, c->d_tw32, scratch,
                                                            st);
     if (rc) return rc;
-    if (flags & HPSI_SYNC) CUDA_TRY(c, cudaStreamSynchronize(st));
+    if (flags & HPSI_SYNC) return finish(c, st, false);
     return HPSI_OK;
 }
 
@@ -2609,7 +2605,7 @@ static int srv_job_bytes(hpsi_server* S, const hpsi_job& j, size_t* bytes, std::
     if (j.nb < 0 || (j.nb > 0 && (!j.psi || !j.hpsi))) { *why = "job psi/hpsi NULL or nb < 0"; return HPSI_ERR_BAD_ARG; }
     const KSlot& s = it->second;
     const size_t nel = (size_t)j.nb * s.npw;
-    size_t ws = apply_ws_bytes(c, s, j.nb, S->prec), m = 0;
+    size_t ws = apply_ws_bytes(c, s, j.nb, S->prec, false, false), m = 0;
     if (j.vel) {
         m = (size_t)3 * j.nb * j.nb * sizeof(double2);
         ws = std::max(ws, vel_ws_bytes(s, j.nb, S->prec));
