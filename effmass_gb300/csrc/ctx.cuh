@@ -164,7 +164,10 @@ struct hpsi_ctx {
     size_t test_d64_room = SIZE_MAX;
     int test_oom = 0;
     long d64_tries = 0;
-    bool d64_ran = false;         // d_err is checked at the next synchronising call
+    // tensor-core work of an FP64 call whose outcome (d_err) no call has read yet, and
+    // its stream: every call that synchronises that stream reads it (finish)
+    bool d64_ran = false;
+    cudaStream_t d64_stream = nullptr;
     Prof prof;
     int* d_err = nullptr;         // device-side error flag of the bounded waits (tcgen05 GEMMs)
     // side stream of the FP64 and tensor-core H|psi>: the projection chain runs there

@@ -43,6 +43,8 @@
  * Threading: one context per host thread; calls on one context are serialised
  * by the caller.  All device work of a call is queued on `stream` (NULL = the
  * legacy default stream); with HPSI_SYNC the call returns after it finished.
+ * HPSI_ERR_TIMEOUT of a call that did not synchronise comes from the next call
+ * on the context that does (with HPSI_SYNC or host buffers).
  */
 #ifndef HPSI_GB300_H
 #define HPSI_GB300_H
