@@ -167,7 +167,7 @@ __global__ void col_exp_kernel(int M, int K, const double2* __restrict__ A, size
 __global__ void row_exp_kernel(int K, const double2* __restrict__ A, size_t lda, const int* __restrict__ ek, int kper,
                                int* fm)
 {
-    const int m = blockIdx.y, k0 = blockIdx.x * kper, k1 = min(K, k0 + kper);
+    const int m = blockIdx.x, k0 = blockIdx.y * kper, k1 = min(K, k0 + kper);
     int f = 0;
     for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
         const int e = exp_of(A[(size_t)m * lda + k]);
@@ -730,7 +730,8 @@ cudaError_t d64_scales(int M, int K, const double2* A, size_t lda, D64Scale s, c
     const int mper = ceil_div(M, gy);
     col_exp_kernel<<<dim3(gx, ceil_div(M, mper)), 128, 0, st>>>(M, K, A, lda, mper, s.ek);
     const int kper = 8192;
-    row_exp_kernel<<<dim3(ceil_div(K, kper), M), 256, 0, st>>>(K, A, lda, s.ek, kper, s.fm);
+    // rows in x: a gradient of many projectors has more of them than y can hold
+    row_exp_kernel<<<dim3(M, ceil_div(K, kper)), 256, 0, st>>>(K, A, lda, s.ek, kper, s.fm);
     return cudaGetLastError();
 }
 
