@@ -22,7 +22,10 @@
 // projectors decay as exp(-q^2 rc^2/4) over the G-sphere, bands grow or decay
 // independently of that.  Error against 80-bit sums on the 8- and 16-atom cells
 // (projection / expansion, 2-norm): 4e-16 / 1e-16, where the FP64 SIMT GEMMs
-// have 1e-15 / 4e-16.
+// have 1e-15 / 4e-16.  The pair matrix of the velocities has bands for rows, which say
+// nothing about one another: a column scale would be that of the largest band, so
+// its columns are not scaled, and an entry is right to 2^-53 of the product of its
+// own bands' norms.
 //
 // What bounds it: the tensor pipe on large cells (64-atom cell, 128 bands: 80% of
 // the measured bf16 rate in the GEMMs).  The seven slices of a B tile lie one
@@ -171,7 +174,7 @@ __global__ void row_exp_kernel(int K, const double2* __restrict__ A, size_t lda,
     int f = 0;
     for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
         const int e = exp_of(A[(size_t)m * lda + k]);
-        if (e >= 0) f = max(f, e == 0x7ff ? F_BAD : e - ek[k] + F_BIAS);
+        if (e >= 0) f = max(f, e == 0x7ff ? F_BAD : e - (ek ? ek[k] : 1022) + F_BIAS);
     }
     f = __reduce_max_sync(0xffffffffu, f);
     if ((threadIdx.x & 31) == 0 && f) atomicMax(fm + m, f);
@@ -202,6 +205,9 @@ struct SplitArgs {
     KMap map[3];
 };
 
+// biased exponent that column k of A is divided by
+__device__ __forceinline__ int col_exp(const int* ek, int k) { return ek ? ek[k] : 1022; }
+
 // One stage holds 8 complex K values.  TRANS = false: the projection (A row r is
 // A[r][.], scales fm and ek; B row b is B[b][.]); TRANS = true: the expansion (A row
 // r is column r of A, scales ek and fm; band b is column b of W).
@@ -228,10 +234,10 @@ __device__ __forceinline__ void split_a(const SplitArgs& s, int g, int block)
         if (r < s.R && k < s.K) {
             const int ka = TRANS ? map.a(k) : k;
             v[i] = TRANS ? s.A[(size_t)ka * s.lda + r] : s.A[(size_t)r * s.lda + ka];
-            sk[i] = TRANS ? -clean(s.fm[ka]) : 1022 - s.ek[ka];
+            sk[i] = TRANS ? -clean(s.fm[ka]) : 1022 - col_exp(s.ek, ka);
         }
     }
-    const int sr = FIX + (r < s.R ? (TRANS ? 1022 - s.ek[r] : -clean(s.fm[r])) : 0);
+    const int sr = FIX + (r < s.R ? (TRANS ? 1022 - col_exp(s.ek, r) : -clean(s.fm[r])) : 0);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         u[2 * i] = fixed_digits(v[i].x, sr + sk[i]);
@@ -246,7 +252,7 @@ __device__ __forceinline__ int band_exp(const SplitArgs& s, const KMap& map, int
 {
     const double2 v = TRANS ? s.B[(size_t)map.w(k) * s.ldb + b] : s.B[(size_t)b * s.ldb + k];
     const int e = exp_of(v);
-    return e < 0 ? 0 : e == 0x7ff ? F_BAD : e - 1022 + (TRANS ? clean(s.fm[map.a(k)]) : s.ek[k] - 1022) + F_BIAS;
+    return e < 0 ? 0 : e == 0x7ff ? F_BAD : e - 1022 + (TRANS ? clean(s.fm[map.a(k)]) : col_exp(s.ek, k) - 1022) + F_BIAS;
 }
 
 // Exponents fb of the bands of long K, over blocks of B_SEG values
@@ -304,7 +310,7 @@ __device__ __forceinline__ void split_b(const SplitArgs& s, int g, int block)
             int sh = 0;
             if (b < s.nb && k < s.K) {
                 v = TRANS ? s.B[(size_t)map.w(k) * s.ldb + b] : s.B[(size_t)b * s.ldb + k];
-                sh = FIX - f + (TRANS ? clean(s.fm[map.a(k)]) : s.ek[k] - 1022);
+                sh = FIX - f + (TRANS ? clean(s.fm[map.a(k)]) : col_exp(s.ek, k) - 1022);
             }
             const unsigned long long x = fixed_digits(v.x, sh), y = fixed_digits(v.y, sh);
             re[2 * i] = x;
@@ -725,10 +731,11 @@ cudaError_t d64_scales(int M, int K, const double2* A, size_t lda, D64Scale s, c
 {
     if (M == 0 || K == 0) return cudaSuccess;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(s.ek, 0, ((size_t)K + M) * sizeof(int), st))) return e;
+    if ((e = cudaMemsetAsync(s.fm, 0, M * sizeof(int), st))) return e;
+    if (s.ek && (e = cudaMemsetAsync(s.ek, 0, K * sizeof(int), st))) return e;
     const int gx = ceil_div(K, 128), gy = std::max(1, std::min(ceil_div(M, 8), ceil_div(16 * sms(), gx)));
     const int mper = ceil_div(M, gy);
-    col_exp_kernel<<<dim3(gx, ceil_div(M, mper)), 128, 0, st>>>(M, K, A, lda, mper, s.ek);
+    if (s.ek) col_exp_kernel<<<dim3(gx, ceil_div(M, mper)), 128, 0, st>>>(M, K, A, lda, mper, s.ek);
     const int kper = 8192;
     // rows in x: a gradient of many projectors has more of them than y can hold
     row_exp_kernel<<<dim3(M, ceil_div(K, kper)), 256, 0, st>>>(K, A, lda, s.ek, kper, s.fm);

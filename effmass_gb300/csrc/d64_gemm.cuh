@@ -5,10 +5,11 @@
 
 // Power-of-two exponents of a complex128 matrix A [M][K] that the digit split
 // divides out: ek[k] the largest biased exponent of column k, fm[m] the (biased)
-// exponent of row m after the columns are scaled to below one.
+// exponent of row m after the columns are scaled to below one.  Without ek the columns
+// are not scaled.
 struct D64Scale {
     int* ek = nullptr;  // [K]
-    int* fm = nullptr;  // [M]; d64_scales needs it to follow ek
+    int* fm = nullptr;  // [M]
 };
 
 cudaError_t d64_scales(int M, int K, const double2* A, size_t lda, D64Scale s, cudaStream_t st);

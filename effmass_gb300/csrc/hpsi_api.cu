@@ -598,7 +598,7 @@ static size_t d64_velocity_bytes(const KSlot& s, int nb, int prec)
     if (prec != HPSI_PREC_FP64 || nb == 0) return 0;
     Carver cv;
     cv.take<double2>((size_t)d64_proj_splits(nb, nb, s.npw) * nb * nb);
-    cv.take<int>((size_t)s.npw + nb);
+    cv.take<int>((size_t)nb);
     return std::max(cv.off + d64_proj_ws(nb, nb, s.npw), d64_grad_bytes(s, nb, 3, prec));
 }
 
@@ -610,7 +610,7 @@ static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const
     const int nz = d64_proj_splits(nb, nb, s.npw);
     Carver cv;
     const size_t o_part = cv.take<double2>((size_t)nz * nb * nb);
-    const size_t o_exp = cv.take<int>((size_t)s.npw + nb);
+    const size_t o_exp = cv.take<int>((size_t)nb);
     const size_t o_ops = cv.off;
     unsigned char* ws = c->d64_ws;
     if (!ws || c->d64_size < o_ops + d64_proj_ws(nb, nb, s.npw)) return HPSI_OK;
@@ -618,8 +618,7 @@ static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const
     c->d64_ran = true;
     c->d64_stream = st;
     double2* part = reinterpret_cast<double2*>(ws + o_part);
-    int* ex = reinterpret_cast<int*>(ws + o_exp);
-    const D64Scale sc{ex, ex + s.npw};
+    const D64Scale sc{nullptr, reinterpret_cast<int*>(ws + o_exp)};
     const size_t npw = (size_t)s.npw;
     int h = c->prof.open(PH_OTHER, st);
     CUDA_TRY(c, d64_scales(nb, s.npw, psi, npw, sc, st));
