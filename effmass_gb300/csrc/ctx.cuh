@@ -51,8 +51,8 @@ struct KSlot {
     // derivative rows behind them (filled on first use: pr*_grad)
     double2* pr64 = nullptr;
     bool pr64_built = false, pr64_grad = false;  // rows [0, P) and the derivative rows hold their values
-    // exponents of pr64's columns and rows for the digit split, of the first P rows
-    // (H) and of all 4 P (gradient), in pr64's allocation
+    // exponents of pr64 for the digit split (d64_scale_at), of the first P rows (H) and
+    // of all 4 P (gradient), in pr64's allocation
     int* d64_exp[2] = {nullptr, nullptr};
     bool d64_exp_set[2] = {false, false};
     float2* pr32 = nullptr;
@@ -140,6 +140,8 @@ struct hpsi_ctx {
     // that every radial table covers
     std::vector<ProjRow> proj_rows;
     std::vector<double> proj_lam;
+    D64Rows proj_groups;          // their groups by radial function (arrays in d_groups)
+    int* d_groups = nullptr;
     double q_safe = 0;
     unsigned char* stage = nullptr;  // pinned staging of hpsi_set_kpoint
     size_t stage_size = 0;

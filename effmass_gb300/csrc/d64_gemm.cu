@@ -17,15 +17,24 @@
 //
 // Scales: the columns of A (one per K index) are divided by a power of two to
 // at most one and B multiplied by it, then every row of A and of B is divided by
-// its own power of two.  The digits of an element are thus relative to the
-// largest *term* of the sums it enters, not to the largest element of its row:
-// projectors decay as exp(-q^2 rc^2/4) over the G-sphere, bands grow or decay
-// independently of that.  Error against 80-bit sums on the 8- and 16-atom cells
-// (projection / expansion, 2-norm): 4e-16 / 1e-16, where the FP64 SIMT GEMMs
-// have 1e-15 / 4e-16.  The pair matrix of the velocities has bands for rows, which say
-// nothing about one another: a column scale would be that of the largest band, so
-// its columns are not scaled, and an entry is right to 2^-53 of the product of its
-// own bands' norms.
+// its own power of two.  So the digits of an element are relative to the largest
+// scaled element of its row, of A and of B: projectors decay as
+// exp(-q^2 rc^2/4) over the G-sphere, bands grow or decay independently of that.
+// Where both rows are large at the same K, that is relative to the largest term of
+// the sum; error against 80-bit sums on the 8- and 16-atom cells (projection /
+// expansion, 2-norm): 4e-16 / 1e-16, where the FP64 SIMT GEMMs have 1e-15 / 4e-16.
+//
+// Guard: where they are large at different K (a wide projector, and a band where
+// only the narrow ones have not decayed), the digits lose the bits between.  The
+// largest term of a group of rows with one radial function is known from exponents
+// alone, eg[g][k] of the group's columns and those of the band, so the loss is too:
+// sums that lose more than LOSS_MAX bits are formed in FP64 instead (projection: in
+// d64_reduce; expansion: at the store).  Silicon-like cells with two projectors per l
+// lose 0 to 4 bits, 5 in one of a hundred sums of a gradient.  Two radii, 0.8 and 1.8,
+// and a band beyond q = 5 lose 13: without the guard the wide projector's sums were
+// off by 3e-12 of their terms.  The pair matrix of the velocities has no groups: its rows are
+// bands, which say nothing about one another, so their columns are not scaled, and
+// an entry is right to 2^-53 of the product of its bands' norms.
 //
 // What bounds it: the tensor pipe on large cells (64-atom cell, 128 bands: 80% of
 // the measured bf16 rate in the GEMMs).  The seven slices of a B tile lie one
@@ -71,6 +80,10 @@ constexpr int THREADS = 64 + 32 * DRAIN_WARPS;
 constexpr uint32_t TMEM_ALL = 512;
 constexpr size_t A_CAP = 1536ull << 20;    // bytes of A slices resident at once
 constexpr int N_CAP = 256;                // bands per pass
+constexpr int LOSS_MAX = 4;               // bits that a sum may lose to the scales
+constexpr int G_CHUNK = 8;                // groups per guard block of a projection
+constexpr int G_BANDS = 16;               // its bands
+constexpr int G_SEGS = 32;                // K segments of a projection's guard at most
 
 // Row and band exponents are stored with a bias, so that 0 means "no nonzero element".
 constexpr int F_BIAS = 8192;
@@ -151,33 +164,52 @@ __device__ __forceinline__ void store_slices(unsigned char* at, size_t stride, c
 // ---- scales -----------------------------------------------------------------
 __device__ __forceinline__ int ceil_div_d(int a, int b) { return (a + b - 1) / b; }
 
-__global__ void col_exp_kernel(int M, int K, const double2* __restrict__ A, size_t lda, int mper, int* ek)
+// exponents of the columns of A: eg over a group of rows (blockIdx.y), ek over all
+__global__ void col_exp_kernel(D64Rows rows, int K, const double2* __restrict__ A, size_t lda, int* eg, int* ek)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= K) return;
-    const int m0 = blockIdx.y * mper, m1 = min(M, m0 + mper);
+    const int g = blockIdx.y, set = g / rows.ng, r = g - set * rows.ng, i1 = rows.off[r + 1];
     int e = 0;
 #pragma unroll 4
-    for (int m = m0; m < m1; ++m) {
-        const double2 v = A[(size_t)m * lda + k];
+    for (int i = rows.off[r] + blockIdx.z; i < i1; i += gridDim.z) {
+        const double2 v = A[((size_t)set * rows.P + rows.order[i]) * lda + k];
         const int x = exp_of(v.x), y = exp_of(v.y);
         if (x != 0x7ff) e = max(e, x);
         if (y != 0x7ff) e = max(e, y);
     }
-    atomicMax(ek + k, e);
+    if (e == 0) return;
+    atomicMax(eg + (size_t)g * K + k, e);
+    atomicMax(ek + k, e << 16 | g);
+}
+
+// ed: per column the largest of the values and of one derivative
+__global__ void dir_exp_kernel(int ng, int K, const int* __restrict__ eg, int* ed)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, a = blockIdx.y;
+    if (k >= K) return;
+    int e = 0;
+    for (int g = 0; g < ng; ++g) {
+        e = max(e, eg[(size_t)g * K + k] << 16 | g);
+        e = max(e, eg[(size_t)((a + 1) * ng + g) * K + k] << 16 | (ng + g));
+    }
+    ed[(size_t)a * K + k] = e;
 }
 
 __global__ void row_exp_kernel(int K, const double2* __restrict__ A, size_t lda, const int* __restrict__ ek, int kper,
-                               int* fm)
+                               int* fm, D64Rows rows, int* fg)
 {
     const int m = blockIdx.x, k0 = blockIdx.y * kper, k1 = min(K, k0 + kper);
     int f = 0;
     for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
         const int e = exp_of(A[(size_t)m * lda + k]);
-        if (e >= 0) f = max(f, e == 0x7ff ? F_BAD : e - (ek ? ek[k] : 1022) + F_BIAS);
+        if (e >= 0) f = max(f, e == 0x7ff ? F_BAD : e - (ek ? ek[k] >> 16 : 1022) + F_BIAS);
     }
     f = __reduce_max_sync(0xffffffffu, f);
-    if ((threadIdx.x & 31) == 0 && f) atomicMax(fm + m, f);
+    if ((threadIdx.x & 31) == 0 && f) {
+        atomicMax(fm + m, f);
+        if (fg && f < F_BAD) atomicMax(fg + m / rows.P * rows.ng + rows.gid[m % rows.P], f);
+    }
 }
 
 // ---- slices -----------------------------------------------------------------
@@ -195,6 +227,13 @@ struct SplitArgs {
     const double2 *A, *B;
     size_t lda, ldb;
     const int *ek, *fm;     // exponents of A's columns and rows
+    const int *eg, *fg;     // and per group
+    D64Rows rows;
+    int sets;               // blocks of A's rows that take part
+    int g_blocks;           // guard blocks per GEMM
+    int* gt;                // projection: largest terms [segments][groups + 1][ngt], the last over all rows
+    int ngt, kpt, b_bands;  // bands of the projection; K per thread of a segment; bands padded to tiles
+    int* wg;                // expansion: [nd][sets ng][bands padded] exponents of W by group, + 1
     int R, row0;            // rows of the GEMM's A operand; first of this chunk
     int nb, K, KT;          // bands, complex K, stages
     int a_x, a_blocks;      // A blocks per row of blocks, per GEMM
@@ -206,7 +245,7 @@ struct SplitArgs {
 };
 
 // biased exponent that column k of A is divided by
-__device__ __forceinline__ int col_exp(const int* ek, int k) { return ek ? ek[k] : 1022; }
+__device__ __forceinline__ int col_exp(const int* ek, int k) { return ek ? ek[k] >> 16 : 1022; }
 
 // One stage holds 8 complex K values.  TRANS = false: the projection (A row r is
 // A[r][.], scales fm and ek; B row b is B[b][.]); TRANS = true: the expansion (A row
@@ -324,13 +363,87 @@ __device__ __forceinline__ void split_b(const SplitArgs& s, int g, int block)
     }
 }
 
+// Guard of a projection, for one K segment, G_BANDS bands and G_CHUNK groups of rows:
+// the terms of group g's sums are below 2^t, t = max_k eg[g][k] + e(B[b][k]); the same
+// with ek for all rows.  Stored + 1, so that 0 means no term.
+__device__ __forceinline__ void guard_proj(const SplitArgs& s, int block)
+{
+    __shared__ int red[8][G_BANDS][G_CHUNK + 1];
+    const int groups = s.sets * s.rows.ng, gc = ceil_div_d(groups, G_CHUNK), bc = ceil_div_d(s.nb, G_BANDS);
+    const int g0 = block % gc * G_CHUNK, b0 = block / gc % bc * G_BANDS, seg = block / (gc * bc);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int x[G_CHUNK + 1];
+    for (int j = 0; j < s.kpt; ++j) {
+        const int k = (seg * s.kpt + j) * 256 + threadIdx.x;
+        if (k < s.K) x[G_CHUNK] = col_exp(s.ek, k) + 1;
+#pragma unroll
+        for (int g = 0; g < G_CHUNK; ++g) {
+            const int e = k < s.K && g0 + g < groups ? s.eg[(size_t)(g0 + g) * s.K + k] : 0;
+            x[g] = e > 0 ? e + 1 : -4096;
+        }
+#pragma unroll 4
+        for (int b = 0; b < G_BANDS; ++b) {
+            int e = -8192;
+            if (k < s.K && b0 + b < s.nb) {
+                e = exp_of(s.B[(size_t)(b0 + b) * s.ldb + k]);
+                if (e < 0 || e == 0x7ff) e = -8192;
+            }
+#pragma unroll
+            for (int g = 0; g <= G_CHUNK; ++g) {
+                const int t = __reduce_max_sync(0xffffffffu, e < 0 ? 0 : max(0, e + x[g]));
+                if (lane == g) red[w][b][g] = j ? max(red[w][b][g], t) : t;
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < G_BANDS * (G_CHUNK + 1); i += 256) {
+        const int g = i / G_BANDS, b = i - g * G_BANDS;
+        if (b0 + b >= s.nb) continue;
+        int t = 0;
+#pragma unroll
+        for (int y = 0; y < 8; ++y) t = max(t, red[y][b][g]);
+        const int row = g == G_CHUNK ? groups : g0 + g;
+        if (g == G_CHUNK ? g0 == 0 : row < groups) s.gt[((size_t)seg * (groups + 1) + row) * s.ngt + b0 + b] = t;
+    }
+}
+
+// Guard of an expansion: the exponents of W over one group of rows, for 32 bands
+__device__ __forceinline__ void guard_expand(const SplitArgs& s, int g, int block)
+{
+    __shared__ int red[8][32];
+    const int ng = s.rows.ng, q = block % (s.sets * ng), set = q / ng, r = q - set * ng;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, b = block / (s.sets * ng) * 32 + lane;
+    const KMap map = s.map[g];
+    int x = 0;
+    if (b < s.nb) {
+#pragma unroll 4
+        for (int i = s.rows.off[r] + w; i < s.rows.off[r + 1]; i += 8) {
+            const int e = exp_of(s.B[(size_t)map.w(set * s.rows.P + s.rows.order[i]) * s.ldb + b]);
+            if (e != 0x7ff) x = max(x, e + 1);
+        }
+    }
+    red[w][lane] = x;
+    __syncthreads();
+    if (w) return;
+#pragma unroll
+    for (int y = 1; y < 8; ++y) x = max(x, red[y][lane]);
+    const int bands = s.b_bands;
+    if (b < bands) s.wg[((size_t)g * s.sets * ng + q) * bands + b] = x;
+}
+
 // both operands of a GEMM in one launch, B's blocks first (they take longest)
 template <bool TRANS>
 __global__ void __launch_bounds__(256) split_kernel(SplitArgs s)
 {
     const int block = blockIdx.x, g = blockIdx.y;
-    if (block < s.b_blocks) split_b<TRANS>(s, g, block);
-    else split_a<TRANS>(s, g, block - s.b_blocks);
+    if (block < s.b_blocks) {
+        split_b<TRANS>(s, g, block);
+    } else if (block < s.b_blocks + s.g_blocks) {
+        if (TRANS) guard_expand(s, g, block - s.b_blocks);
+        else guard_proj(s, block - s.b_blocks);
+    } else {
+        split_a<TRANS>(s, g, block - s.b_blocks - s.g_blocks);
+    }
 }
 
 // ---- GEMM -------------------------------------------------------------------
@@ -349,10 +462,46 @@ struct D64Out {
     size_t ldo;
     size_t a_bytes, b_bytes;  // operands of one GEMM
     int bands;       // column exponents of one GEMM
-    const int* er;   // row exponents (fm, or ek with bias)
+    const int* er;   // row exponents (fm, or ek)
     const int* fb;   // column exponents
     int M, N, row0;  // result rows and bands; first row of this launch's A chunk
+    // guard of an expansion
+    const int *eg, *ed, *wg;  // exponents of A (by group, by direction) and of W by group
+    int ng, sets, K, dir[3];  // sets of ng groups (set 1: block dir of A's rows); row stride of eg
+    int rows_P;               // rows of a set
+    const double2 *A, *W;
+    size_t lda, ldw;
+    KMap map[3];
 };
+
+// one output of an expansion in FP64
+__device__ __noinline__ double2 expand_exact(const double2* A, size_t lda, int row, const double2* W, size_t ldw, int n,
+                                             int K, KMap map)
+{
+    double re = 0.0, im = 0.0;
+    for (int k = 0; k < K; ++k) {
+        const double2 a = A[(size_t)map.a(k) * lda + row], w = W[(size_t)map.w(k) * ldw + n];
+        re += a.x * w.x - a.y * w.y;
+        im += a.x * w.y + a.y * w.x;
+    }
+    return make_double2(re, im);
+}
+
+// Output (row, n) of GEMM g, v unless the scales cost it more than LOSS_MAX bits; f: the
+// band's exponent, e: that of the row's column of A
+__device__ __noinline__ double2 expand_guarded(const D64Out& o, int g, int row, int n, int f, int e, double2 v)
+{
+    const int* wg = o.wg + (size_t)g * o.sets * o.ng * o.bands + n;
+    int t = 0;
+    for (int s = 0; s < o.sets; ++s)
+        for (int r = 0; r < o.ng; ++r) {
+            const int x = wg[(size_t)(s * o.ng + r) * o.bands];
+            const int a = o.eg[((size_t)(s ? o.dir[g] : 0) * o.ng + r) * o.K + row];
+            if (x > 0 && a > 0) t = max(t, a + x);
+        }
+    if (t == 0 || e + f - (t - 1023) <= LOSS_MAX) return v;
+    return expand_exact(o.A, o.lda, row, o.W, o.ldw, n, o.sets * o.rows_P, o.map[g]);
+}
 
 __device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t (&r)[4])
 {
@@ -495,6 +644,22 @@ __global__ void __launch_bounds__(THREADS, 1)
         // ---- read-out: warp w holds TMEM lanes 32 (w % 4) .. +31 (rows) and
         // bands sub BPW .. +BPW-1 of the tile, real and imaginary columns
         const int q = warp & 3, sub = (warp - 2) >> 2;
+        const int row = o.row0 + blockIdx.y * TM + q * 32 + lane;
+        // Bands whose output may lose more than LOSS_MAX bits: those where the group of A's
+        // rows that has the column's largest element has a small W.  (Loaded here, under
+        // the first copies.)
+        unsigned slow = 0;
+        if (EXPAND && row < o.M) {
+            const int e = o.er[row], b = (o.sets > 1 ? o.ed[(size_t)(o.dir[gemm] - 1) * o.K + row] : e);
+            const int n0 = blockIdx.x * BT + sub * BPW;
+            const int4 x = *reinterpret_cast<const int4*>(
+                o.wg + ((size_t)gemm * o.sets * o.ng + (b & 0xffff)) * o.bands + n0);
+            const int4 f = *reinterpret_cast<const int4*>(o.fb + (size_t)gemm * o.bands + n0);
+            auto loses = [&](int f, int x) {
+                return f != 0 && f < F_BAD && (x == 0 || (e >> 16) - (b >> 16) + f - F_BIAS - (x - 1023) > LOSS_MAX);
+            };
+            slow = loses(f.x, x.x) | loses(f.y, x.y) << 1 | loses(f.z, x.z) << 2 | loses(f.w, x.w) << 3;
+        }
         long long h[2 * BPW], l[2 * BPW];
 #pragma unroll
         for (int i = 0; i < 2 * BPW; ++i) h[i] = l[i] = 0;
@@ -533,13 +698,12 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
             }
         }
-        const int row = o.row0 + blockIdx.y * TM + q * 32 + lane;
         double2* out = gemm == 0 ? o.out[0] : gemm == 1 ? o.out[1] : o.out[2];
         if (go && row < o.M) {
             // h counts diagonal 3, l diagonal 6: weights 2^(72 - 110) and 2^(48 - 110)
             const int fr = o.er[row];
             const bool bad = !EXPAND && fr >= F_BAD;
-            const int er = (EXPAND ? fr - 1022 : clean(fr)) - 62;
+            const int er = (EXPAND ? (fr >> 16) - 1022 : clean(fr)) - 62;
 #pragma unroll
             for (int i = 0; i < BPW; ++i) {
                 const int n = blockIdx.x * BT + sub * BPW + i;
@@ -548,6 +712,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     double2 v = make_double2(round_sum(h[i], l[i], e), round_sum(h[BPW + i], l[BPW + i], e));
                     if (bad || f >= F_BAD) v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
                     if (EXPAND) {
+                        if (slow >> i & 1) v = expand_guarded(o, gemm, row, n, clean(f), fr >> 16, v);
                         double2* at = out + (size_t)n * o.ldo + row;
                         double2 x = *at;
                         x.x += v.x;
@@ -600,9 +765,12 @@ struct Plan {
     int cps, nz;            // chunks per split, splits
     size_t a_bytes, b_bytes, fb_bytes;
     int ng;                 // GEMMs run together
+    int kpt, segs;          // guard of a projection: K per thread, segments
+    size_t guard_bytes;     // gt of a projection; wg of an expansion
 };
 
-Plan plan(int R, int N, int K, bool split_k, int ng)
+// groups: of the rows that take part (both sets of a gradient's expansion)
+Plan plan(int R, int N, int K, bool split_k, int ng, int groups)
 {
     Plan p;
     p.n_pass = std::min(N, N_CAP);
@@ -629,31 +797,50 @@ Plan plan(int R, int N, int K, bool split_k, int ng)
     p.b_bytes = (size_t)p.tiles_n * p.KT * B_STAGE;
     p.fb_bytes = ((size_t)p.tiles_n * BT * sizeof(int) + 255) / 256 * 256;
     p.ng = ng;
+    p.kpt = ceil_div(K, 256 * G_SEGS);
+    p.segs = ceil_div(K, 256 * p.kpt);
+    p.guard_bytes = split_k ? (groups ? (size_t)p.segs * (groups + 1) * N * sizeof(int) : 0) : (size_t)ng * groups * p.tiles_n * BT * sizeof(int);
+    p.guard_bytes = (p.guard_bytes + 255) / 256 * 256;
     return p;
 }
 
-size_t plan_bytes(const Plan& p) { return p.ng * (p.a_bytes + p.b_bytes + p.fb_bytes); }
+size_t plan_bytes(const Plan& p) { return p.ng * (p.a_bytes + p.b_bytes + p.fb_bytes) + p.guard_bytes; }
+int* plan_guard(const Plan& p, unsigned char* ws)
+{
+    return reinterpret_cast<int*>(ws + p.ng * (p.a_bytes + p.b_bytes + p.fb_bytes));
+}
 
 // The GEMMs of an expansion run together when their A slices fit the cap.
-Plan expand_plan(int M, int N, int K, int ng)
+Plan expand_plan(int M, int N, int K, int ng, int groups)
 {
-    const Plan p = plan(K, N, M, false, ng);
-    return ng > 1 && ng * p.a_bytes > A_CAP ? plan(K, N, M, false, 1) : p;
+    const Plan p = plan(K, N, M, false, ng, groups);
+    return ng > 1 && ng * p.a_bytes > A_CAP ? plan(K, N, M, false, 1, groups) : p;
+}
+
+Plan proj_plan(int M, int N, int K, const D64Rows& rows)
+{
+    return plan(M, N, K, true, 1, rows.ng ? M / rows.P * rows.ng : 0);
 }
 
 // rows of A in chunks against all bands, the bands in passes of N_CAP
 template <bool EXPAND>
 cudaError_t run(const Plan& p, int R, int N, int K, const double2* A, size_t lda, D64Scale sc, const double2* B,
-                size_t ldb, double2* part, const KMap* maps, double2* const* out, size_t ldo, unsigned char* ws,
-                int* err, cudaStream_t st)
+                size_t ldb, double2* part, const KMap* maps, const int* dirs, double2* const* out, size_t ldo,
+                unsigned char* ws, int* err, cudaStream_t st)
 {
     SplitArgs s{};
-    s.A = A; s.lda = lda; s.ldb = ldb; s.ek = sc.ek; s.fm = sc.fm;
+    s.A = A; s.lda = lda; s.ldb = ldb; s.ek = sc.ek; s.fm = sc.fm; s.eg = sc.eg; s.fg = sc.fg; s.rows = sc.rows;
+    const int groups = sc.rows.ng;
+    s.sets = groups ? (EXPAND ? K : R) / sc.rows.P : 0;
+    s.ngt = N;
+    s.kpt = p.kpt;
     s.R = R; s.K = K; s.KT = p.KT;
     s.a = ws; s.b = ws + p.ng * p.a_bytes;
     s.a_bytes = p.a_bytes; s.b_bytes = p.b_bytes;
     s.fb = reinterpret_cast<int*>(s.b + p.ng * p.b_bytes);
     const int bands = p.tiles_n * BT;
+    s.b_bands = bands;
+    s.wg = plan_guard(p, ws);
     s.b_seg = K > 2 * B_SEG ? ceil_div(p.KT, B_SEG / 8) : 1;
     s.a_x = ceil_div(p.KT, 2);
     for (int g = 0; g < p.ng; ++g) s.map[g] = maps[g];
@@ -669,9 +856,12 @@ cudaError_t run(const Plan& p, int R, int N, int K, const double2* A, size_t lda
             const int mt = std::min(p.mt_chunk, p.mt - m);
             s.row0 = m * TM;
             s.b_blocks = m == 0 ? bands * s.b_seg : 0;
+            s.gt = plan_guard(p, ws) + n0;
+            s.g_blocks = m > 0 || !groups ? 0 : EXPAND ? s.sets * groups * ceil_div(s.nb, 32)
+                         : p.segs * ceil_div(s.nb, G_BANDS) * ceil_div(s.sets * groups, G_CHUNK);
             s.a_blocks = n0 == 0 || p.mt > p.mt_chunk ? s.a_x * 2 * mt : 0;
             if (s.a_blocks + s.b_blocks)
-                split_kernel<EXPAND><<<dim3(s.a_blocks + s.b_blocks, p.ng), 256, 0, st>>>(s);
+                split_kernel<EXPAND><<<dim3(s.a_blocks + s.b_blocks + s.g_blocks, p.ng), 256, 0, st>>>(s);
             D64Out o{};
             o.part = EXPAND ? nullptr : part + n0;
             o.ldn = N;
@@ -681,6 +871,11 @@ cudaError_t run(const Plan& p, int R, int N, int K, const double2* A, size_t lda
             o.er = EXPAND ? sc.ek : sc.fm;
             o.fb = s.fb;
             o.M = R; o.N = s.nb; o.row0 = s.row0;
+            if (EXPAND) {
+                o.eg = sc.eg; o.ed = sc.ed; o.wg = s.wg; o.ng = groups; o.sets = s.sets; o.K = R; o.rows_P = sc.rows.P;
+                o.A = A; o.lda = lda; o.W = s.B; o.ldw = ldb;
+                for (int g = 0; g < p.ng; ++g) { o.map[g] = maps[g]; o.dir[g] = dirs[g]; }
+            }
             const cudaError_t e = launch_gemm<EXPAND>(dim3(p.tiles_n, mt, EXPAND ? p.ng : p.nz), s.a, s.b, o, p.KT,
                                                       p.cps, err, st);
             if (e) return e;
@@ -689,18 +884,42 @@ cudaError_t run(const Plan& p, int R, int N, int K, const double2* A, size_t lda
     return cudaGetLastError();
 }
 
+// Sums of a projection that the digits do not hold (guard), and their operands
+struct Guard {
+    const int* gt;     // largest terms [segs][groups + 1][N], null: no guard
+    const int* fg;
+    int segs, groups;
+    D64Rows rows;
+    const double2 *A, *B;
+    size_t lda, ldb;
+    int K;
+};
+
 // W[m][n] = scale[m % period] sum_z part[z][m][n]: 32 outputs per block, the splits
-// in SL slices that are added in order
+// in SL slices that are added in order; flagged sums by the whole block in FP64
 template <int SL>
-__global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total, int nz,
-                                                             const double2* __restrict__ part,
+__global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total, int nz, double2* __restrict__ part,
                                                              const double* __restrict__ scale, int period,
-                                                             double2* __restrict__ W)
+                                                             double2* __restrict__ W, Guard gd, bool keep)
 {
     __shared__ double2 sum[SL][32];
+    __shared__ int2 tf[SL][32];
+    __shared__ unsigned todo;
     const size_t i = (size_t)blockIdx.x * 32 + threadIdx.x;
     const int per = ceil_div_d(nz, SL), z1 = min(nz, (int)(threadIdx.y + 1) * per);
     double re = 0.0, im = 0.0;
+    int t = 0, f = 0, fg = 0;
+    if (gd.gt && i < total) {
+        const int m = (int)(i / N), n = (int)(i - (size_t)m * N), set = m / gd.rows.P;
+        const int g = set * gd.rows.ng + gd.rows.gid[m - set * gd.rows.P];
+        fg = clean(gd.fg[g]);
+#pragma unroll 4
+        for (int q = threadIdx.y; q < gd.segs; q += SL) {
+            const int* at = gd.gt + (size_t)q * (gd.groups + 1) * N + n;
+            t = max(t, at[(size_t)g * N]);
+            f = max(f, at[(size_t)gd.groups * N]);
+        }
+    }
     if (i < total) {
 #pragma unroll 4
         for (int z = threadIdx.y * per; z < z1; ++z) {
@@ -709,63 +928,130 @@ __global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total
             im += v.y;
         }
     }
-    if (SL > 1) {
-        sum[threadIdx.y][threadIdx.x] = make_double2(re, im);
-        __syncthreads();
-        if (threadIdx.y) return;
+    sum[threadIdx.y][threadIdx.x] = make_double2(re, im);
+    tf[threadIdx.y][threadIdx.x] = make_int2(t, f);
+    __syncthreads();
+    if (threadIdx.y == 0) {
 #pragma unroll
         for (int y = 1; y < SL; ++y) {
             re += sum[y][threadIdx.x].x;
             im += sum[y][threadIdx.x].y;
+            t = max(t, tf[y][threadIdx.x].x);
+            f = max(f, tf[y][threadIdx.x].y);
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, t > 0 && fg + f - t > LOSS_MAX);
+        if (threadIdx.x == 0) todo = b;
+    }
+    if (gd.gt) __syncthreads();
+    for (unsigned left = gd.gt ? todo : 0u; left; left &= left - 1) {
+        const int j = __ffs((int)left) - 1;
+        const size_t at = (size_t)blockIdx.x * 32 + j;
+        const int m = (int)(at / N), n = (int)(at - (size_t)m * N);
+        const double2 *a = gd.A + (size_t)m * gd.lda, *b = gd.B + (size_t)n * gd.ldb;
+        double x = 0.0, y = 0.0;
+#pragma unroll 4
+        for (int k = threadIdx.y * 32 + threadIdx.x; k < gd.K; k += 32 * SL) {
+            const double2 u = a[k], v = b[k];
+            x += u.x * v.x + u.y * v.y;
+            y += u.x * v.y - u.y * v.x;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            x += __shfl_xor_sync(0xffffffffu, x, o);
+            y += __shfl_xor_sync(0xffffffffu, y, o);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) sum[threadIdx.y][0] = make_double2(x, y);
+        __syncthreads();
+        if (threadIdx.y == 0 && threadIdx.x == j) {
+            re = im = 0.0;
+#pragma unroll
+            for (int q = 0; q < SL; ++q) {
+                re += sum[q][0].x;
+                im += sum[q][0].y;
+            }
         }
     }
-    if (i < total) {
+    if (threadIdx.y == 0 && i < total) {
         const double f = scale ? scale[(int)(i / N) % period] : 1.0;
         W[i] = make_double2(f * re, f * im);
+        if (keep) part[i] = make_double2(re, im);
     }
 }
 
 }  // namespace
 
+size_t d64_scale_ints(int M, int K, const D64Rows& rows)
+{
+    const size_t groups = rows.ng ? (size_t)(M / rows.P) * rows.ng : 0;
+    return (size_t)(groups ? K : 0) + M + groups * K + groups + (groups && M > rows.P ? 3 * (size_t)K : 0);
+}
+
+D64Scale d64_scale_at(int* at, int M, int K, const D64Rows& rows)
+{
+    D64Scale s;
+    s.rows = rows;
+    if (!rows.ng) {
+        s.fm = at;
+        return s;
+    }
+    s.ek = at;
+    s.fm = s.ek + K;
+    s.eg = s.fm + M;
+    const int groups = M / rows.P * rows.ng;
+    s.fg = s.eg + (size_t)groups * K;
+    if (M > rows.P) s.ed = s.fg + groups;
+    return s;
+}
+
 cudaError_t d64_scales(int M, int K, const double2* A, size_t lda, D64Scale s, cudaStream_t st)
 {
     if (M == 0 || K == 0) return cudaSuccess;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(s.fm, 0, M * sizeof(int), st))) return e;
-    if (s.ek && (e = cudaMemsetAsync(s.ek, 0, K * sizeof(int), st))) return e;
-    const int gx = ceil_div(K, 128), gy = std::max(1, std::min(ceil_div(M, 8), ceil_div(16 * sms(), gx)));
-    const int mper = ceil_div(M, gy);
-    if (s.ek) col_exp_kernel<<<dim3(gx, ceil_div(M, mper)), 128, 0, st>>>(M, K, A, lda, mper, s.ek);
+    if ((e = cudaMemsetAsync(s.ek ? s.ek : s.fm, 0, d64_scale_ints(M, K, s.rows) * sizeof(int), st))) return e;
+    if (s.ek) {
+        const int groups = M / s.rows.P * s.rows.ng, gx = ceil_div(K, 128);
+        const int gz = std::max(1, std::min(ceil_div(M, groups), ceil_div(16 * sms(), gx * groups)));
+        col_exp_kernel<<<dim3(gx, groups, gz), 128, 0, st>>>(s.rows, K, A, lda, s.eg, s.ek);
+        if (s.ed) dir_exp_kernel<<<dim3(gx, 3), 128, 0, st>>>(s.rows.ng, K, s.eg, s.ed);
+    }
     const int kper = 8192;
     // rows in x: a gradient of many projectors has more of them than y can hold
-    row_exp_kernel<<<dim3(M, ceil_div(K, kper)), 256, 0, st>>>(K, A, lda, s.ek, kper, s.fm);
+    row_exp_kernel<<<dim3(M, ceil_div(K, kper)), 256, 0, st>>>(K, A, lda, s.ek, kper, s.fm, s.rows, s.fg);
     return cudaGetLastError();
 }
 
-int d64_proj_splits(int M, int N, int K) { return plan(M, N, K, true, 1).nz; }
+int d64_proj_splits(int M, int N, int K) { return plan(M, N, K, true, 1, 0).nz; }
 
-size_t d64_proj_ws(int M, int N, int K) { return plan_bytes(plan(M, N, K, true, 1)); }
+size_t d64_proj_ws(int M, int N, int K, const D64Rows& rows) { return plan_bytes(proj_plan(M, N, K, rows)); }
 
-size_t d64_expand_ws(int M, int N, int K) { return plan_bytes(expand_plan(M, N, K, 1)); }
+size_t d64_expand_ws(int M, int N, int K, const D64Rows& rows) { return plan_bytes(expand_plan(M, N, K, 1, rows.ng)); }
 
-size_t d64_expand_grad_ws(int P, int N, int K, int nd) { return plan_bytes(expand_plan(2 * P, N, K, nd)); }
+size_t d64_expand_grad_ws(int P, int N, int K, int nd, const D64Rows& rows)
+{
+    return plan_bytes(expand_plan(2 * P, N, K, nd, 2 * rows.ng));
+}
 
 cudaError_t d64_proj(int M, int N, int K, const double2* A, size_t lda, D64Scale s, const double2* B, size_t ldb,
                      double2* part, unsigned char* ws, int* err, cudaStream_t st)
 {
     if (M == 0 || N == 0 || K == 0) return cudaSuccess;
     const KMap map{K, 0, 0, 0};
-    return run<false>(plan(M, N, K, true, 1), M, N, K, A, lda, s, B, ldb, part, &map, nullptr, 0, ws, err, st);
+    return run<false>(proj_plan(M, N, K, s.rows), M, N, K, A, lda, s, B, ldb, part, &map, nullptr, nullptr, 0, ws, err,
+                      st);
 }
 
-cudaError_t d64_reduce(int M, int N, int nz, const double2* part, const double* scale, int period, double2* W,
-                       cudaStream_t st)
+cudaError_t d64_reduce(int M, int N, int K, int nz, double2* part, const double* scale, int period, double2* W,
+                       const double2* A, size_t lda, D64Scale s, const double2* B, size_t ldb, unsigned char* ws,
+                       bool keep, cudaStream_t st)
 {
     const size_t total = (size_t)M * N;
     if (total == 0) return cudaSuccess;
+    const Plan p = proj_plan(M, N, K, s.rows);
+    const Guard g{s.rows.ng ? plan_guard(p, ws) : nullptr, s.fg, p.segs, s.rows.ng ? M / s.rows.P * s.rows.ng : 0,
+                  s.rows, A, B, lda, ldb, K};
     const int blocks = ceil_div((long)total, 32);
-    if (nz >= 16) d64_reduce_kernel<8><<<blocks, dim3(32, 8), 0, st>>>(N, total, nz, part, scale, period, W);
-    else d64_reduce_kernel<1><<<blocks, dim3(32, 1), 0, st>>>(N, total, nz, part, scale, period, W);
+    if (nz >= 16) d64_reduce_kernel<8><<<blocks, dim3(32, 8), 0, st>>>(N, total, nz, part, scale, period, W, g, keep);
+    else d64_reduce_kernel<1><<<blocks, dim3(32, 1), 0, st>>>(N, total, nz, part, scale, period, W, g, keep);
     return cudaGetLastError();
 }
 
@@ -774,7 +1060,9 @@ cudaError_t d64_expand(int M, int N, int K, const double2* W, size_t ldw, const 
 {
     if (M == 0 || N == 0 || K == 0) return cudaSuccess;
     const KMap map{M, 0, 0, 0};
-    return run<true>(expand_plan(M, N, K, 1), K, N, M, A, lda, s, W, ldw, nullptr, &map, &out, ldo, ws, err, st);
+    const int dir = 0;
+    return run<true>(expand_plan(M, N, K, 1, s.rows.ng), K, N, M, A, lda, s, W, ldw, nullptr, &map, &dir, &out, ldo, ws,
+                     err, st);
 }
 
 cudaError_t d64_expand_grad(int P, int N, int K, const double2* W, size_t ldw, const double2* A, size_t lda, D64Scale s,
@@ -783,17 +1071,18 @@ cudaError_t d64_expand_grad(int P, int N, int K, const double2* W, size_t ldw, c
     if (P == 0 || N == 0 || K == 0) return cudaSuccess;
     KMap map[3];
     double2* to[3];
-    int nd = 0;
+    int nd = 0, dir[3];
     for (int a = 0; a < 3; ++a)
         if (out[a]) {
+            dir[nd] = a + 1;
             map[nd] = KMap{P, a * P, (a + 1) * P, -P};
             to[nd++] = out[a];
         }
     if (nd == 0) return cudaSuccess;
-    const Plan p = expand_plan(2 * P, N, K, nd);
+    const Plan p = expand_plan(2 * P, N, K, nd, 2 * s.rows.ng);
     for (int g = 0; g < nd; g += p.ng) {
         const cudaError_t e =
-            run<true>(p, K, N, 2 * P, A, lda, s, W, ldw, nullptr, map + g, to + g, ldo, ws, err, st);
+            run<true>(p, K, N, 2 * P, A, lda, s, W, ldw, nullptr, map + g, dir + g, to + g, ldo, ws, err, st);
         if (e) return e;
     }
     return cudaSuccess;

@@ -38,7 +38,7 @@ extern "C" int hpsi_ctx_destroy(hpsi_ctx* c)
     cudaSetDevice(c->dev);
     for (auto& kv : c->slots) slot_free(kv.second);
     dfree(c->d_tables); dfree(c->d_rad_nq); dfree(c->d_rad_dq); dfree(c->d_tau); dfree(c->d_v64); dfree(c->d_v32); dfree(c->d_dv32);
-    dfree(c->d_tw64); dfree(c->d_tw32); dfree(c->d_err); dfree(c->d_hess);
+    dfree(c->d_tw64); dfree(c->d_tw32); dfree(c->d_err); dfree(c->d_hess); dfree(c->d_groups);
     if (c->ws != c->ws_first) cudaFree(c->ws);
     if (c->ws_first) cudaFree(c->ws_first);
     release_optional(c);
@@ -162,6 +162,25 @@ static int ctx_init(hpsi_ctx* c, const hpsi_system* s)
     // the workspace of a small cell's calls, so that the first one does not wait for it
     int rc = ws_reserve(c, 4u << 20);
     if (rc) return rc;
+    if (!c->proj_rows.empty()) {
+        // rows by radial function: order [P], first of each group [ng + 1], group of a row [P]
+        const int P = (int)c->proj_rows.size();
+        std::vector<std::vector<int>> by((size_t)c->nrad);
+        for (int p = 0; p < P; ++p) by[(size_t)c->proj_rows[(size_t)p].rad].push_back(p);
+        std::vector<int> order, off{0}, gid((size_t)P);
+        for (const std::vector<int>& rows : by) {
+            if (rows.empty()) continue;
+            for (int p : rows) gid[(size_t)p] = (int)off.size() - 1;
+            order.insert(order.end(), rows.begin(), rows.end());
+            off.push_back((int)order.size());
+        }
+        const int ng = (int)off.size() - 1;
+        order.insert(order.end(), off.begin(), off.end());
+        order.insert(order.end(), gid.begin(), gid.end());
+        CUDA_TRY(c, dalloc(&c->d_groups, order.size()));
+        CUDA_TRY(c, cudaMemcpy(c->d_groups, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice));
+        c->proj_groups = D64Rows{P, ng, c->d_groups, c->d_groups + P, c->d_groups + P + ng + 1};
+    }
     CUDA_TRY(c, dalloc(&c->d_err, (size_t)1));
     CUDA_TRY(c, cudaMemset(c->d_err, 0, sizeof(int)));
     const size_t N = (size_t)c->n1 * c->n2 * c->n3;
@@ -427,7 +446,8 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
     if (!pr) {
         const size_t rows = (size_t)(c->have_dbeta ? 4 : 1) * s.P;
         // FP64: the digit split's exponents behind the matrix (d64_scale)
-        const size_t n_exp = f64 ? 2 * (size_t)s.npw + s.P + rows : 0;
+        const size_t n1 = d64_scale_ints(s.P, s.npw, c->proj_groups);
+        const size_t n_exp = f64 ? n1 + (c->have_dbeta ? d64_scale_ints(4 * s.P, s.npw, c->proj_groups) : 0) : 0;
         size_t bytes = rows * s.npw * sizeof(C) + n_exp * sizeof(int);
         const int k = f64 ? 0 : 1;
         // a spare would let a capture record a build that it otherwise refuses
@@ -436,7 +456,7 @@ static int ensure_proj(hpsi_ctx* c, KSlot& s, bool grad, cudaStream_t st)
         s.pr_bytes[k] = bytes;
         if (f64) {
             s.d64_exp[0] = reinterpret_cast<int*>(pr + rows * s.npw);
-            s.d64_exp[1] = s.d64_exp[0] + s.npw + s.P;
+            s.d64_exp[1] = s.d64_exp[0] + n1;
             s.d64_exp_set[0] = s.d64_exp_set[1] = false;
         }
     }
@@ -504,10 +524,11 @@ static int nonlocal_apply(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, dou
 // The exponents of the first P rows of slot s's projector matrix, or of all 4 P, once.
 static int d64_scale(hpsi_ctx* c, KSlot& s, bool all, D64Scale* out, cudaStream_t st)
 {
-    *out = D64Scale{s.d64_exp[all], s.d64_exp[all] + s.npw};
+    const int M = (all ? 4 : 1) * s.P;
+    *out = d64_scale_at(s.d64_exp[all], M, s.npw, c->proj_groups);
     if (s.d64_exp_set[all]) return HPSI_OK;
     int h = c->prof.open(PH_BUILD, st);
-    CUDA_TRY(c, d64_scales((all ? 4 : 1) * s.P, s.npw, s.pr64, (size_t)s.npw, *out, st));
+    CUDA_TRY(c, d64_scales(M, s.npw, s.pr64, (size_t)s.npw, *out, st));
     c->prof.close(h, st, 2);
     s.d64_exp_set[all] = !capturing(st);
     return HPSI_OK;
@@ -522,21 +543,27 @@ struct D64Call {
 };
 
 // Workspace of a call that projects M rows and expands with expand_ws bytes of operands
-static size_t d64_bytes(const KSlot& s, int M, int nb, size_t expand_ws)
+static size_t d64_bytes(const hpsi_ctx* c, const KSlot& s, int M, int nb, size_t expand_ws)
 {
     if (s.P == 0 || nb == 0) return 0;
     Carver cv;
     cv.take<double2>((size_t)d64_proj_splits(M, nb, s.npw) * M * nb);
     cv.take<double2>((size_t)M * nb);
-    return cv.off + std::max(d64_proj_ws(M, nb, s.npw), expand_ws);
+    return cv.off + std::max(d64_proj_ws(M, nb, s.npw, c->proj_groups), expand_ws);
 }
-static size_t d64_apply_bytes(const KSlot& s, int nb, int prec)
+static size_t d64_expand_bytes(const hpsi_ctx* c, const KSlot& s, int nb)
 {
-    return prec == HPSI_PREC_FP64 ? d64_bytes(s, s.P, nb, d64_expand_ws(s.P, nb, s.npw)) : 0;
+    return d64_expand_ws(s.P, nb, s.npw, c->proj_groups);
 }
-static size_t d64_grad_bytes(const KSlot& s, int nb, int nd, int prec)
+static size_t d64_apply_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int prec)
 {
-    return prec == HPSI_PREC_FP64 ? d64_bytes(s, 4 * s.P, nb, d64_expand_grad_ws(s.P, nb, s.npw, nd)) : 0;
+    return prec == HPSI_PREC_FP64 ? d64_bytes(c, s, s.P, nb, d64_expand_bytes(c, s, nb)) : 0;
+}
+static size_t d64_grad_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int nd, int prec)
+{
+    return prec == HPSI_PREC_FP64
+               ? d64_bytes(c, s, 4 * s.P, nb, d64_expand_grad_ws(s.P, nb, s.npw, nd, c->proj_groups))
+               : 0;
 }
 
 // Plan a call that projects M rows and expands with expand_ws bytes of operands.
@@ -552,7 +579,7 @@ static int d64_begin(hpsi_ctx* c, KSlot& s, int M, int nb, size_t expand_ws, D64
     Carver cv;
     const size_t o_part = cv.take<double2>((size_t)d->nz * M * nb), o_w = cv.take<double2>((size_t)M * nb);
     unsigned char* ws = c->d64_ws;
-    if (!ws || c->d64_size < d64_bytes(s, M, nb, expand_ws)) return HPSI_OK;
+    if (!ws || c->d64_size < d64_bytes(c, s, M, nb, expand_ws)) return HPSI_OK;
     d->part = reinterpret_cast<double2*>(ws + o_part);
     d->W = reinterpret_cast<double2*>(ws + o_w);
     d->ops = ws + cv.off;
@@ -570,10 +597,11 @@ static int d64_project(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const 
     int h = c->prof.open(PH_PROJ, st);
     CUDA_TRY(c, d64_proj(d.M, nb, s.npw, s.pr64, npw, d.sc, psi, npw, d.part, d.ops, c->d_err, st));
     c->prof.close(h, st, 2);
-    if (e_nl) CUDA_TRY(c, launch_nl_energy<double2>(s.P, nb, d.nz, d.part, s.d_lam, e_nl, st));
     h = c->prof.open(PH_REDUCE, st);
-    CUDA_TRY(c, d64_reduce(d.M, nb, d.nz, d.part, s.d_lam, s.P, d.W, st));
+    CUDA_TRY(c, d64_reduce(d.M, nb, s.npw, d.nz, d.part, s.d_lam, s.P, d.W, s.pr64, npw, d.sc, psi, npw, d.ops,
+                           e_nl != nullptr, st));
     c->prof.close(h, st);
+    if (e_nl) CUDA_TRY(c, launch_nl_energy<double2>(s.P, nb, 1, d.part, s.d_lam, e_nl, st));
     return HPSI_OK;
 }
 
@@ -584,7 +612,7 @@ static int grad_nonlocal_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, 
     const int nd = (d[0] != nullptr) + (d[1] != nullptr) + (d[2] != nullptr);
     const size_t npw = (size_t)s.npw;
     D64Call k;
-    int rc = d64_begin(c, s, 4 * s.P, nb, d64_expand_grad_ws(s.P, nb, s.npw, nd), &k, done, st);
+    int rc = d64_begin(c, s, 4 * s.P, nb, d64_expand_grad_ws(s.P, nb, s.npw, nd, c->proj_groups), &k, done, st);
     if (rc || !*done) return rc;
     if ((rc = d64_project(c, s, nb, psi, k, nullptr, st))) return rc;
     int h = c->prof.open(PH_EXPAND, st);
@@ -593,13 +621,13 @@ static int grad_nonlocal_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, 
     return HPSI_OK;
 }
 
-static size_t d64_velocity_bytes(const KSlot& s, int nb, int prec)
+static size_t d64_velocity_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int prec)
 {
     if (prec != HPSI_PREC_FP64 || nb == 0) return 0;
     Carver cv;
     cv.take<double2>((size_t)d64_proj_splits(nb, nb, s.npw) * nb * nb);
     cv.take<int>((size_t)nb);
-    return std::max(cv.off + d64_proj_ws(nb, nb, s.npw), d64_grad_bytes(s, nb, 3, prec));
+    return std::max(cv.off + d64_proj_ws(nb, nb, s.npw, D64Rows{}), d64_grad_bytes(c, s, nb, 3, prec));
 }
 
 // m[a][i][j] = sum_G conj(psi_i) g_a,j for the three directions (g: [3][nb][npw]); *done as above.
@@ -613,18 +641,19 @@ static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const
     const size_t o_exp = cv.take<int>((size_t)nb);
     const size_t o_ops = cv.off;
     unsigned char* ws = c->d64_ws;
-    if (!ws || c->d64_size < o_ops + d64_proj_ws(nb, nb, s.npw)) return HPSI_OK;
+    if (!ws || c->d64_size < o_ops + d64_proj_ws(nb, nb, s.npw, D64Rows{})) return HPSI_OK;
     *done = true;
     c->d64_ran = true;
     c->d64_stream = st;
     double2* part = reinterpret_cast<double2*>(ws + o_part);
-    const D64Scale sc{nullptr, reinterpret_cast<int*>(ws + o_exp)};
+    const D64Scale sc = d64_scale_at(reinterpret_cast<int*>(ws + o_exp), nb, s.npw, D64Rows{});
     const size_t npw = (size_t)s.npw;
     int h = c->prof.open(PH_OTHER, st);
     CUDA_TRY(c, d64_scales(nb, s.npw, psi, npw, sc, st));
     for (int a = 0; a < 3; ++a) {
         CUDA_TRY(c, d64_proj(nb, nb, s.npw, psi, npw, sc, g + (size_t)a * nb * npw, npw, part, ws + o_ops, c->d_err, st));
-        CUDA_TRY(c, d64_reduce(nb, nb, nz, part, nullptr, nb, m + (size_t)a * nb * nb, st));
+        CUDA_TRY(c, d64_reduce(nb, nb, s.npw, nz, part, nullptr, nb, m + (size_t)a * nb * nb, psi, npw, sc,
+                               g + (size_t)a * nb * npw, npw, ws + o_ops, false, st));
     }
     c->prof.close(h, st, 11);
     return HPSI_OK;
@@ -1172,7 +1201,7 @@ static int apply_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, double2*
         // cores against the integer pipes); the expansion joins after both
         D64Call k;
         bool ok = false;
-        if (d64 && (rc = d64_begin(c, s, s.P, nb, d64_expand_ws(s.P, nb, s.npw), &k, &ok, st))) return rc;
+        if (d64 && (rc = d64_begin(c, s, s.P, nb, d64_expand_bytes(c, s, nb), &k, &ok, st))) return rc;
         if (ok && fork) {
             CUDA_TRY(c, cudaEventRecord(c->ev_fork, st));
             CUDA_TRY(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
@@ -1462,7 +1491,7 @@ extern "C" int hpsi_apply(hpsi_ctx* c, int kid, int nb, const double* psi_, doub
     size_t o_psi = dev ? 0 : cv.take<double2>(nel);
     size_t o_hpsi = dev ? 0 : cv.take<double2>(nel);
     size_t o_work = cv.off;
-    if ((rc = ws_reserve_d64(c, o_work + apply_ws_bytes(c, *s, nb, prec), d64_apply_bytes(*s, nb, prec),
+    if ((rc = ws_reserve_d64(c, o_work + apply_ws_bytes(c, *s, nb, prec), d64_apply_bytes(c, *s, nb, prec),
                              st)))
         return rc;
     const double2* psi = (const double2*)psi_;
@@ -1563,7 +1592,7 @@ extern "C" int hpsi_apply_energies(hpsi_ctx* c, int kid, int nb, const double* p
     size_t o_work = cv.off;
     const EnergyWs w = energy_layout(c, nb, prec);
     if ((rc = ws_reserve_d64(c, o_work + w.work + apply_ws_bytes(c, *s, nb, prec, true),
-                             d64_apply_bytes(*s, nb, prec), st)))
+                             d64_apply_bytes(c, *s, nb, prec), st)))
         return rc;
     const double2* psi = (const double2*)psi_;
     double2* hpsi = (double2*)hpsi_;
@@ -1635,7 +1664,7 @@ extern "C" int hpsi_sternheimer(hpsi_ctx* c, int kid, int nv, const double* psi_
     const size_t o_act = cv.take<int>((size_t)nv);
     const size_t o_work = cv.off;
     const size_t work = std::max(apply_ws_bytes(c, *s, nv, prec), grad_ws_bytes(*s, nv, prec));
-    const size_t d64 = std::max(d64_apply_bytes(*s, nv, prec), d64_grad_bytes(*s, nv, 1, prec));
+    const size_t d64 = std::max(d64_apply_bytes(c, *s, nv, prec), d64_grad_bytes(c, *s, nv, 1, prec));
     if ((rc = ws_reserve_d64(c, o_work + work, d64, st))) return rc;
     unsigned char* ws = c->ws;
     const double2* psi = dev ? (const double2*)psi_ : reinterpret_cast<const double2*>(ws + o_psi);
@@ -2160,7 +2189,7 @@ extern "C" int hpsi_grad_apply(hpsi_ctx* c, int kid, int nb, const double* psi_,
         if (!dev && outs[a]) o_out[a] = cv.take<double2>(nel);
     size_t o_work = cv.off;
     const int nd = (dx != nullptr) + (dy != nullptr) + (dz != nullptr);
-    if ((rc = ws_reserve_d64(c, o_work + grad_ws_bytes(*s, nb, prec), d64_grad_bytes(*s, nb, nd, prec), st)))
+    if ((rc = ws_reserve_d64(c, o_work + grad_ws_bytes(*s, nb, prec), d64_grad_bytes(c, *s, nb, nd, prec), st)))
         return rc;
     const double2* psi = (const double2*)psi_;
     double2* d[3] = {(double2*)dx, (double2*)dy, (double2*)dz};
@@ -2203,7 +2232,7 @@ extern "C" int hpsi_velocity_matrix(hpsi_ctx* c, int kid, int nb, const double* 
     size_t o_psi = dev ? 0 : cv.take<double2>(nel);
     size_t o_m = dev ? 0 : cv.take<double2>(nm);
     size_t o_work = cv.off;
-    if ((rc = ws_reserve_d64(c, o_work + vel_ws_bytes(*s, nb, prec), d64_velocity_bytes(*s, nb, prec), st)))
+    if ((rc = ws_reserve_d64(c, o_work + vel_ws_bytes(*s, nb, prec), d64_velocity_bytes(c, *s, nb, prec), st)))
         return rc;
     const double2* psi = (const double2*)psi_;
     double2* m = (double2*)m_;
