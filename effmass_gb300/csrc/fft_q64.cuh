@@ -9,7 +9,10 @@
 // every partial sum stays below n sqrt(2) 2^FB < 2^62).  Rounding errors are then
 // absolute, about three units per output, where the largest input is 2^55 units
 // for n = 72: against long double transforms the 3-D round trip of the 8-atom
-// cell is 6e-17 off in the 2-norm, the complex128 one 5e-16.
+// cell is 6e-17 off in the 2-norm, the complex128 one 5e-16.  A bound by n wastes bits
+// that lines of more than LONG points cannot spare (a few large elements of 500: 3e-15
+// off, where complex128 is 5e-16), so these take their unit from the sum of their
+// elements' magnitudes, which bounds every partial sum too.
 //
 // Twiddles are Q62 constants, each as two signed words (l, h): value
 // (h 2^32 + l) 2^-62.  A product drops the l x l term (below one unit).
@@ -76,6 +79,33 @@ HPSI_D int bits_of(longlong2 v)
     const int a = (int)(v.x >> 32), b = (int)(v.y >> 32);
     const unsigned o = (unsigned)(a ^ (a >> 31)) | (unsigned)(b ^ (b >> 31));
     return 64 - __clz(o);
+}
+
+// Lines that take their unit from the sum of their magnitudes: below, the bound by n
+// leaves 54 bits or more to the largest element, the level of complex128.
+constexpr int LONG = 181;
+
+// |re| + |im| in units of 2^(e - 20) (e: the line's exponent), rounded up.  Integers, so
+// that a sum does not depend on its order.
+HPSI_D unsigned magnitude(double2 v, int e)
+{
+    if (e <= EXP_NONE || e >= EXP_BAD / 2) return 0u;
+    return 1u + (unsigned)(scalbn(fabs(v.x), 20 - e) + scalbn(fabs(v.y), 20 - e));
+}
+// the same of v 2^u, v an integer of the transforms
+HPSI_D unsigned magnitude(longlong2 v, int u, int e)
+{
+    if (e <= EXP_NONE || e >= EXP_BAD / 2) return 0u;
+    const int a = (int)(v.x >> 32), b = (int)(v.y >> 32);
+    const long long t = (long long)(a ^ (a >> 31)) + (b ^ (b >> 31)) + 2;  // the magnitude is below t 2^(32 + u)
+    const int s = 52 + u - e;
+    return s >= 0 ? (unsigned)(t << min(s, 31)) : 1u + (unsigned)(t >> min(-s, 63));
+}
+
+// bits of the largest element where the magnitudes add up to sum (in units of 2^(e - 20))
+HPSI_D int headroom(int n, unsigned sum)
+{
+    return sum ? max(headroom(n), min(60, 62 - (12 - __clz((int)sum)))) : headroom(n);
 }
 
 // unit of a line whose components are below 2^e, for fb bits

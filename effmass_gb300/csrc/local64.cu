@@ -28,6 +28,10 @@ using q64::RowLines;
 struct BigPlane { static constexpr int threads = 640, blocks = 1; };
 struct SmallPlane { static constexpr int threads = 192, blocks = 3; };
 constexpr int X_THREADS = 288;
+// Kernels by grid: radices to 9 and axes to LONG; axes beyond it; an axis with a
+// factor of 7, 11 or 13.  (The sums of long lines cost the plain kernels registers: 64
+// atoms, 128 bands 5.48 -> 5.94 ms in one kernel for all.)
+enum Kind { PLAIN, LONG_AXIS, WIDE_RADIX };
 
 // rows of a plane that hold sphere points (PlaneRows of local.cu)
 struct Rows {
@@ -149,14 +153,26 @@ struct PlaneSmem {
     }
 };
 
-// units of n lines from their exponents (callers synchronise before and after)
-HPSI_D void take_units(int n, const int* e, int* u, int fb)
+// Units of `lines` lines of n points from their exponents (callers synchronise before
+// and after).  Long lines need the sums of their magnitudes: mag(L, i) of element i < m.
+template <int R, typename M>
+HPSI_D void take_units(int lines, int n, const int* e, int* u, int m, const M& mag)
 {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) u[i] = q64::unit_of(e[i], fb);
+    if (R != PLAIN && n > q64::LONG) {
+        unsigned* sum = reinterpret_cast<unsigned*>(u);
+        for (int i = threadIdx.x; i < lines; i += blockDim.x) sum[i] = 0u;
+        __syncthreads();
+        for (int t = threadIdx.x; t < lines * m; t += blockDim.x) atomicAdd(sum + t % lines, mag(t % lines, t / lines));
+        __syncthreads();
+        for (int i = threadIdx.x; i < lines; i += blockDim.x) u[i] = q64::unit_of(e[i], q64::headroom(n, sum[i]));
+    } else {
+        const int fb = q64::headroom(n);
+        for (int i = threadIdx.x; i < lines; i += blockDim.x) u[i] = q64::unit_of(e[i], fb);
+    }
 }
 
-template <typename SZ, bool WIDE>
-__global__ void __launch_bounds__(SZ::threads, WIDE ? 1 : SZ::blocks)
+template <typename SZ, int R>
+__global__ void __launch_bounds__(SZ::threads, R == WIDE_RADIX ? 1 : SZ::blocks)
     g2r64(LocalArgs a, const double2* __restrict__ psi_, double2* __restrict__ T, const int4* __restrict__ twy_g,
           const int4* __restrict__ twz_g, int tw_smem)
 {
@@ -179,10 +195,10 @@ __global__ void __launch_bounds__(SZ::threads, WIDE ? 1 : SZ::blocks)
         atomicMax(s.re + j, q64::exp_of(v));
     }
     __syncthreads();
-    take_units(n2, s.re, s.ru, q64::headroom(n3));
+    take_units<R>(n2, n3, s.re, s.ru, n3, [&](int j, int k) { return q64::magnitude(grid[j * n3p + k], s.re[j]); });
     __syncthreads();
     // z: rows in use, b0 -> b1 (-> b0 ...)
-    const bool zb = q64::transform<WIDE, +1>(LoadRows{grid, s.ru, n3p, rows}, RowLines{s.b1, n3p, rows.jr, rows.gap},
+    const bool zb = q64::transform<R == WIDE_RADIX, +1>(LoadRows{grid, s.ru, n3p, rows}, RowLines{s.b1, n3p, rows.jr, rows.gap},
                                              RowLines{s.b0, n3p, rows.jr, rows.gap}, a.Lz, rows.count, s.twz);
     longlong2 *z = zb ? s.b0 : s.b1, *o = zb ? s.b1 : s.b0;
     // columns' exponents: thread = (column, slice of rows)
@@ -198,9 +214,12 @@ __global__ void __launch_bounds__(SZ::threads, WIDE ? 1 : SZ::blocks)
         atomicMax(s.ce + k, e);
     }
     __syncthreads();
-    take_units(n3, s.ce, s.cu, q64::headroom(n2));
+    take_units<R>(n3, n2, s.ce, s.cu, rows.count, [&](int k, int L) {
+        const int j = rows.row(L);
+        return s.re[j] == q64::EXP_NONE ? 0u : q64::magnitude(z[j * n3p + k], s.ru[j], s.ce[k]);
+    });
     __syncthreads();
-    const bool yb = q64::transform<WIDE, +1>(ColsFromRows{z, s.ru, s.cu, n3p, rows}, Lines{o, 1, n3p},
+    const bool yb = q64::transform<R == WIDE_RADIX, +1>(ColsFromRows{z, s.ru, s.cu, n3p, rows}, Lines{o, 1, n3p},
                                              Lines{z, 1, n3p}, a.Ly, n3, s.twy);
     const longlong2* y = yb ? z : o;
     double2* Tp = T + B.t0 + (size_t)p * n23;
@@ -211,8 +230,8 @@ __global__ void __launch_bounds__(SZ::threads, WIDE ? 1 : SZ::blocks)
     }
 }
 
-template <typename SZ, bool WIDE>
-__global__ void __launch_bounds__(SZ::threads, WIDE ? 1 : SZ::blocks)
+template <typename SZ, int R>
+__global__ void __launch_bounds__(SZ::threads, R == WIDE_RADIX ? 1 : SZ::blocks)
     r2g64(LocalArgs a, const double2* __restrict__ T, const double2* __restrict__ psi_, double2* __restrict__ hpsi_,
           const double* __restrict__ kinetic_, const int4* __restrict__ twy_g, const int4* __restrict__ twz_g,
           int tw_smem)
@@ -239,9 +258,9 @@ __global__ void __launch_bounds__(SZ::threads, WIDE ? 1 : SZ::blocks)
         atomicMax(s.ce + k, e);
     }
     __syncthreads();
-    take_units(n3, s.ce, s.cu, q64::headroom(n2));
+    take_units<R>(n3, n2, s.ce, s.cu, n2, [&](int k, int j) { return q64::magnitude(grid[j * n3p + k], s.ce[k]); });
     __syncthreads();
-    const bool yb = q64::transform<WIDE, -1>(LoadCols{grid, s.cu, n3p}, Lines{s.b1, 1, n3p}, Lines{s.b0, 1, n3p}, a.Ly,
+    const bool yb = q64::transform<R == WIDE_RADIX, -1>(LoadCols{grid, s.cu, n3p}, Lines{s.b1, 1, n3p}, Lines{s.b0, 1, n3p}, a.Ly,
                                              n3, s.twy);
     longlong2 *y = yb ? s.b0 : s.b1, *o = yb ? s.b1 : s.b0;
     // rows' exponents: one warp per row in use
@@ -255,9 +274,11 @@ __global__ void __launch_bounds__(SZ::threads, WIDE ? 1 : SZ::blocks)
         if ((threadIdx.x & 31) == 0) s.re[j] = e;
     }
     __syncthreads();
-    take_units(n2, s.re, s.ru, q64::headroom(n3));
+    take_units<R>(n2, n3, s.re, s.ru, n3, [&](int j, int k) {
+        return !rows.holds(j) || s.ce[k] == q64::EXP_NONE ? 0u : q64::magnitude(y[j * n3p + k], s.cu[k], s.re[j]);
+    });
     __syncthreads();
-    const bool zb = q64::transform<WIDE, -1>(RowsFromCols{y, s.ru, s.cu, n3p, rows}, RowLines{o, n3p, rows.jr, rows.gap},
+    const bool zb = q64::transform<R == WIDE_RADIX, -1>(RowsFromCols{y, s.ru, s.cu, n3p, rows}, RowLines{o, n3p, rows.jr, rows.gap},
                                              RowLines{y, n3p, rows.jr, rows.gap}, a.Lz, rows.count, s.twz);
     const longlong2* z = zb ? y : o;
     const int e1 = B.plane_off[p + 1];
@@ -359,8 +380,8 @@ HPSI_D void x_load(const XSmem& s, const double2* __restrict__ T, const int* __r
     __syncthreads();
 }
 
-template <bool WIDE, bool ENERGY>
-__global__ void __launch_bounds__(X_THREADS, WIDE ? 1 : 3)
+template <int R, bool ENERGY>
+__global__ void __launch_bounds__(X_THREADS, R == WIDE_RADIX ? 1 : 3)
     xpass64(LocalArgs a, int nb, double2* __restrict__ T, const double* __restrict__ vloc, const int4* __restrict__ tw_g)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -398,10 +419,12 @@ __global__ void __launch_bounds__(X_THREADS, WIDE ? 1 : 3)
     if ((threadIdx.x & 31) == 0) atomicMax(s.ev, ve);
     for (int t = threadIdx.x; t < nxs; t += blockDim.x) s.xpl[plane_x[t]] = t;
     x_load(s, T, plane_x, nxs, plane, base, KT, NL, kt, nbb, bb0);
-    const int fb = q64::headroom(n1);
     const bool vbad = *s.ev >= q64::EXP_BAD;
     const int vu = (*s.ev == q64::EXP_NONE || vbad) ? 0 : *s.ev;  // |V| < 2^vu
-    take_units(NL, s.e, s.u, fb);
+    const auto x_mag = [&](int L, int x) {
+        return s.xpl[x] < 0 ? 0u : q64::magnitude(reinterpret_cast<const double2*>(s.b1)[x * NL + L], s.e[L]);
+    };
+    take_units<R>(NL, n1, s.e, s.u, n1, x_mag);
     for (int t = threadIdx.x; t < n1 * KT; t += blockDim.x) {
         const int2 w = s.vq[t];
         // Q62 of V 2^-vu; 2^62 - 1 at most, so that the high word stays below 2^30
@@ -411,7 +434,7 @@ __global__ void __launch_bounds__(X_THREADS, WIDE ? 1 : 3)
         s.vq[t] = make_int2(l, h);
     }
     __syncthreads();
-    const bool gb = q64::transform<WIDE, +1>(XLoad{reinterpret_cast<const double2*>(s.b1), s.xpl, s.u, NL},
+    const bool gb = q64::transform<R == WIDE_RADIX, +1>(XLoad{reinterpret_cast<const double2*>(s.b1), s.xpl, s.u, NL},
                                              Lines{s.b0, 1, NL}, Lines{s.b1, 1, NL}, a.Lx, NL, s.tw);
     longlong2 *f = gb ? s.b1 : s.b0, *o = gb ? s.b0 : s.b1;
     if constexpr (ENERGY) {
@@ -476,13 +499,20 @@ __global__ void __launch_bounds__(X_THREADS, WIDE ? 1 : 3)
     }
     __syncthreads();
     for (int L = threadIdx.x; L < NL; L += blockDim.x) {
-        // |V psi| < 2^bits units 2^(u + vu): to fb bits
-        const int sh = fb - (64 - __clz(s.mag[L]));
+        // |V psi| < 2^bits units 2^(u + vu): to the line's bits
+        const int bits = 64 - __clz(s.mag[L]);
+        int fb = q64::headroom(n1);
+        if (R != PLAIN && n1 > q64::LONG) {
+            unsigned sum = 0u;
+            for (int x = 0; x < n1; ++x) sum += q64::magnitude(f[x * NL + L], 0, bits);
+            fb = q64::headroom(n1, sum);
+        }
+        const int sh = fb - bits;
         s.mag[L] = (unsigned)sh;
         s.u[L] += vu - sh;
     }
     __syncthreads();
-    const bool rb = q64::transform<WIDE, -1>(XShift{f, reinterpret_cast<const int*>(s.mag), NL}, Lines{o, 1, NL},
+    const bool rb = q64::transform<R == WIDE_RADIX, -1>(XShift{f, reinterpret_cast<const int*>(s.mag), NL}, Lines{o, 1, NL},
                                              Lines{f, 1, NL}, a.Lx, NL, s.tw);
     const longlong2* r = rb ? f : o;
     const int total = nxs * NL;
@@ -494,8 +524,8 @@ __global__ void __launch_bounds__(X_THREADS, WIDE ? 1 : 3)
     }
 }
 
-template <bool WIDE>
-__global__ void __launch_bounds__(X_THREADS, WIDE ? 1 : 3)
+template <int R>
+__global__ void __launch_bounds__(X_THREADS, R == WIDE_RADIX ? 1 : 3)
     xdensity64(LocalArgs a, int nb, const double2* __restrict__ T, const double* __restrict__ occ,
                double* __restrict__ rho, const int4* __restrict__ tw_g)
 {
@@ -516,9 +546,11 @@ __global__ void __launch_bounds__(X_THREADS, WIDE ? 1 : 3)
         for (int t = threadIdx.x; t < NL; t += blockDim.x) s.e[t] = q64::EXP_NONE;
         __syncthreads();
         x_load(s, T, a.plane_x, a.nxs, plane, base, KT, NL, kt, nbb, bb0);
-        take_units(NL, s.e, s.u, q64::headroom(n1));
+        take_units<R>(NL, n1, s.e, s.u, n1, [&](int L, int x) {
+            return s.xpl[x] < 0 ? 0u : q64::magnitude(reinterpret_cast<const double2*>(s.b1)[x * NL + L], s.e[L]);
+        });
         __syncthreads();
-        const bool gb = q64::transform<WIDE, +1>(XLoad{reinterpret_cast<const double2*>(s.b1), s.xpl, s.u, NL},
+        const bool gb = q64::transform<R == WIDE_RADIX, +1>(XLoad{reinterpret_cast<const double2*>(s.b1), s.xpl, s.u, NL},
                                                  Lines{s.b0, 1, NL}, Lines{s.b1, 1, NL}, a.Lx, NL, s.tw);
         const longlong2* f = gb ? s.b1 : s.b0;
         for (int t = threadIdx.x; t < n1 * KT; t += blockDim.x) {
@@ -548,25 +580,30 @@ cudaError_t smem_limit(K kernel, size_t bytes)
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// f(plane size, wide) with the kernel variant of the grid
+// f(plane size, kind) with the kernel variant of the grid
 template <typename F>
 cudaError_t with_variant(const LocalArgs& a, F&& f)
 {
     const bool small = plane_bytes(a, true) * SmallPlane::blocks <= SMEM_MAX;
-    if (wide(a)) return f(BigPlane{}, std::true_type{});
-    return small ? f(SmallPlane{}, std::false_type{}) : f(BigPlane{}, std::false_type{});
+    if (wide(a)) return f(BigPlane{}, std::integral_constant<int, WIDE_RADIX>{});
+    if (std::max({a.n1, a.n2, a.n3}) > q64::LONG) {
+        using R = std::integral_constant<int, LONG_AXIS>;
+        return small ? f(SmallPlane{}, R{}) : f(BigPlane{}, R{});
+    }
+    using R = std::integral_constant<int, PLAIN>;
+    return small ? f(SmallPlane{}, R{}) : f(BigPlane{}, R{});
 }
 
-template <typename SZ, bool WIDE>
+template <typename SZ, int R>
 cudaError_t run_local(const LocalArgs& a, int nb, const double2* psi, double2* hpsi, const double* kinetic, double2* T,
                       const double* vloc, const int4* twx, const int4* twy, const int4* twz, dim3 gp, dim3 gx,
                       cudaStream_t st, Prof* prof)
 {
     const int tw = plane_bytes(a, true) <= SMEM_MAX;
     const size_t sp = plane_bytes(a, tw), sx = xpass_bytes(a);
-    auto g2r = g2r64<SZ, WIDE>;
-    auto r2g = r2g64<SZ, WIDE>;
-    auto xp = a.epart ? xpass64<WIDE, true> : xpass64<WIDE, false>;
+    auto g2r = g2r64<SZ, R>;
+    auto r2g = r2g64<SZ, R>;
+    auto xp = a.epart ? xpass64<R, true> : xpass64<R, false>;
     cudaError_t e;
     if ((e = smem_limit(g2r, sp)) || (e = smem_limit(r2g, sp)) || (e = smem_limit(xp, sx))) return e;
     for (int i = 0; i < 2; ++i)
@@ -627,17 +664,17 @@ cudaError_t launch_local_batch<double2, double>(const LocalArgs& a, int nbands, 
     });
 }
 
-template <typename SZ, bool WIDE>
+template <typename SZ, int R>
 static cudaError_t run_density(const LocalArgs& a, int nb, const double2* psi, const double* occ, double* rho, double2* T,
                                const int4* twx, const int4* twy, const int4* twz, cudaStream_t st)
 {
     const int tw = plane_bytes(a, true) <= SMEM_MAX;
     const size_t sp = plane_bytes(a, tw), sx = xdensity_bytes(a);
-    auto g2r = g2r64<SZ, WIDE>;
+    auto g2r = g2r64<SZ, R>;
     cudaError_t e;
-    if ((e = smem_limit(g2r, sp)) || (e = smem_limit(xdensity64<WIDE>, sx))) return e;
+    if ((e = smem_limit(g2r, sp)) || (e = smem_limit(xdensity64<R>, sx))) return e;
     g2r<<<dim3(a.nxs, nb), SZ::threads, sp, st>>>(a, psi, T, twy, twz, tw);
-    xdensity64<WIDE><<<dim3(ceil_div(a.n3, a.kt), a.n2), X_THREADS, sx, st>>>(a, nb, T, occ, rho, twx);
+    xdensity64<R><<<dim3(ceil_div(a.n3, a.kt), a.n2), X_THREADS, sx, st>>>(a, nb, T, occ, rho, twx);
     return cudaGetLastError();
 }
 

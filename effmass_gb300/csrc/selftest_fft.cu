@@ -111,9 +111,13 @@ __global__ void line_q64_kernel(double2* g, int n, int es, int lines_inner, int 
     longlong2 *b0 = reinterpret_cast<longlong2*>(smem_raw), *b1 = b0 + n;
     int4* tw = reinterpret_cast<int4*>(b1 + n);
     __shared__ int e;
+    __shared__ unsigned sum;
     const int line = blockIdx.x;
     double2* p = g + (size_t)(line % lines_inner) * stride_inner + (size_t)(line / lines_inner) * stride_outer;
-    if (threadIdx.x == 0) e = q64::EXP_NONE;
+    if (threadIdx.x == 0) {
+        e = q64::EXP_NONE;
+        sum = 0u;
+    }
     __syncthreads();
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         const double2 v = p[(size_t)t * es];
@@ -122,7 +126,11 @@ __global__ void line_q64_kernel(double2* g, int n, int es, int lines_inner, int 
         atomicMax(&e, q64::exp_of(v));
     }
     __syncthreads();
-    const int unit = q64::unit_of(e, q64::headroom(n));
+    if (n > q64::LONG)
+        for (int t = threadIdx.x; t < n; t += blockDim.x)
+            atomicAdd(&sum, q64::magnitude(reinterpret_cast<const double2*>(b1)[t], e));
+    __syncthreads();
+    const int unit = q64::unit_of(e, n > q64::LONG ? q64::headroom(n, sum) : q64::headroom(n));
     const bool inb = q64::transform<WIDE, SIGN>(LineDouble{reinterpret_cast<const double2*>(b1), unit},
                                                 q64::Lines{b0, n, 1}, q64::Lines{b1, n, 1}, L, 1, tw);
     const longlong2* r = inb ? b1 : b0;
