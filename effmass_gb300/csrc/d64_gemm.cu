@@ -2,18 +2,18 @@
 //
 // GB300 runs FP64 at 1/64 of the FP32 rate (0.6 T multiply-adds/s on the whole
 // part), so the FP64 projector sums were 94% of an FP64 H|psi> on the 64-atom
-// cell.  Here each operand is written as a sum of S = 7 slices of base-256
+// cell.  Here each operand is written as a sum of S = 8 slices of base-256
 // digits and the products of the slices run as exact integer arithmetic on the
 // tensor cores (the splitting scheme of Ozaki, Ogita, Oishi and Rump,
 // "Error-free transformations of matrix multiplication", Numer. Algorithms 59,
 // 2012):
-//   x 2^-(scales) = sum_i d_i 2^(-7 - 8 i),  i < 7, |d_i| <= 128 (FP16-exact),
-// a fixed-point number of 55 bits.  A slice product is at most 2^14, so FP32
+//   x 2^-(scales) = sum_i d_i 2^(-6 - 8 i),  i < 8, |d_i| <= 128 (FP16-exact),
+// a fixed-point number of 62 bits.  A slice product is at most 2^14, so FP32
 // accumulation of up to 1024 of them is exact; slice pairs (i, j) of one
-// diagonal d = i + j share an accumulator (at most 7 pairs), which is read out
-// every 128 of K.  Diagonals 0..7 are kept (34 of 49 pairs); the dropped ones
-// lie below the 2^-56 rounding of the digits.  The read-outs are added as 64-bit
-// integers and rounded to FP64 once per output.
+// diagonal d = i + j share an accumulator (at most 8 pairs), which is read out
+// every 128 of K.  Diagonals 0..7 are kept (36 of 64 pairs); the largest of the
+// dropped ones is 2^-62 of the product of the scales.  The read-outs are added as
+// 64-bit integers and rounded to FP64 once per output.
 //
 // Scales: the columns of A (one per K index) are divided by a power of two to
 // at most one and B multiplied by it, then every row of A and of B is divided by
@@ -21,8 +21,7 @@
 // scaled element of its row, of A and of B: projectors decay as
 // exp(-q^2 rc^2/4) over the G-sphere, bands grow or decay independently of that.
 // Where both rows are large at the same K, that is relative to the largest term of
-// the sum; error against 80-bit sums on the 8- and 16-atom cells (projection /
-// expansion, 2-norm): 4e-16 / 1e-16, where the FP64 SIMT GEMMs have 1e-15 / 4e-16.
+// the sum.
 //
 // Guard: where they are large at different K (a wide projector, and a band where
 // only the narrow ones have not decayed), the digits lose the bits between.  The
@@ -30,17 +29,20 @@
 // alone, eg[g][k] of the group's columns and those of the band, so the loss is too:
 // sums that lose more than LOSS_MAX bits are formed in FP64 instead (projection: in
 // d64_reduce; expansion: at the store).  Silicon-like cells with two projectors per l
-// lose 0 to 4 bits, 5 in one of a hundred sums of a gradient.  Two radii, 0.8 and 1.8,
-// and a band beyond q = 5 lose 13: without the guard the wide projector's sums were
-// off by 3e-12 of their terms.  The pair matrix of the velocities has no groups: its rows are
-// bands, which say nothing about one another, so their columns are not scaled, and
-// an entry is right to 2^-53 of the product of its bands' norms.
+// lose 0 to 4 bits, 5 or 6 in one of a hundred sums; two radii, 0.8 and 1.8, and a
+// band beyond q = 5 lose 13.  Error of the projections of such cells against 80-bit sums,
+// relative to the 2-norm of a sum's terms, by bits lost (seven slices / eight / FP64
+// sums in chains of 192): 2 bits 9e-16 / 9e-17 / 6e-16, 4 bits 6e-15 / 4e-16 / 6e-16,
+// 6 bits 6e-15 / 4e-16 / 3e-16.  The pair matrix of the velocities has no groups: its
+// rows are bands, which say nothing about one another, so their columns are not
+// scaled, and an entry is right to 2^-59 of the product of its bands' norms (and
+// rounded to FP64).
 //
 // What bounds it: the tensor pipe on large cells (64-atom cell, 128 bands: 80% of
-// the measured bf16 rate in the GEMMs).  The seven slices of a B tile lie one
+// the measured bf16 rate in the GEMMs).  The eight slices of a B tile lie one
 // after the other in shared memory and the eight diagonals in TMEM, so one MMA
-// of up to N = 224 multiplies slice i of A with all its slices of B into their
-// diagonals: 7 MMAs per 16 of K instead of 34, which the issuing thread could not
+// of up to N = 256 multiplies slice i of A with all its slices of B into their
+// diagonals: 8 MMAs per 16 of K instead of 36, which the issuing thread could not
 // feed (70 clocks each).  Tiles of 16 bands (32 rows of B) leave TMEM room for two
 // sets of accumulators, so that one is read out under the next chunk's MMAs;
 // against tiles of 32 bands with one set, H|psi> us before -> now: 8-atom cell,
@@ -52,7 +54,7 @@
 // magic adds in place of F2I, 32 of K per stage (SWIZZLE_64B).
 //
 // Layout: K-major tiles of (rows x 16) FP16 digits, slice after slice: an A tile
-// is 7 x 4 KB and a B tile 7 x NT x 32 bytes of contiguous memory, already in
+// is 8 x 4 KB and a B tile 8 x NT x 32 bytes of contiguous memory, already in
 // the SWIZZLE_32B order of the MMA descriptors, so that a pipeline stage is two
 // bulk copies.
 #include <algorithm>
@@ -63,16 +65,16 @@
 
 namespace {
 
-constexpr int S = 7;                      // slices per operand
+constexpr int S = 8;                      // slices per operand
 constexpr int ND = 8;                     // diagonals kept: i + j < ND
 constexpr int TM = 128;                   // A rows per tile
 constexpr int BT = 16;                    // bands per tile
 constexpr int NT = 2 * BT;                // B rows per tile: two sets of ND accumulators fill TMEM
 constexpr int KB = 16;                    // real K per pipeline stage (one MMA deep)
 constexpr int CHUNK = 8;                  // stages per read-out of the accumulators (128 of K)
-constexpr int FIX = 55;                   // bits of the fixed-point form
-constexpr int A_STAGE = S * TM * KB * 2;  // 28 KB
-constexpr int B_STAGE = S * NT * KB * 2;  // 7 KB
+constexpr int FIX = 62;                   // bits of the fixed-point form
+constexpr int A_STAGE = S * TM * KB * 2;  // 32 KB
+constexpr int B_STAGE = S * NT * KB * 2;  // 8 KB
 constexpr int STAGE = A_STAGE + B_STAGE;
 constexpr int STAGES = 220 * 1024 / STAGE;  // that fit shared memory beside the barriers
 constexpr int DRAIN_WARPS = 16;
@@ -80,7 +82,7 @@ constexpr int THREADS = 64 + 32 * DRAIN_WARPS;
 constexpr uint32_t TMEM_ALL = 512;
 constexpr size_t A_CAP = 1536ull << 20;    // bytes of A slices resident at once
 constexpr int N_CAP = 256;                // bands per pass
-constexpr int LOSS_MAX = 4;               // bits that a sum may lose to the scales
+constexpr int LOSS_MAX = 6;               // bits that a sum may lose to the scales
 constexpr int G_CHUNK = 8;                // groups per guard block of a projection
 constexpr int G_BANDS = 16;               // its bands
 constexpr int G_SEGS = 32;                // K segments of a projection's guard at most
@@ -102,10 +104,10 @@ __device__ __forceinline__ int exp_of(double2 v)
     return max(exp_of(v.x), exp_of(v.y));
 }
 
-constexpr unsigned long long DIGIT_BIAS = 0x80808080808080ull;
+constexpr unsigned long long DIGIT_BIAS = 0x8080808080808080ull;
 
-// rint(x 2^sh) + DIGIT_BIAS for |x 2^sh| < 2^55: byte i of the sum, minus
-// 128, is the base-256 digit of weight 2^(8 i); the top digit takes 9 bits.
+// rint(x 2^sh) + DIGIT_BIAS for |x 2^sh| < 2^62: byte i of the sum, minus
+// 128, is the base-256 digit of weight 2^(8 i); the top digit is at most 64.
 __device__ __forceinline__ unsigned long long fixed_digits(double x, int sh)
 {
     const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
@@ -124,15 +126,9 @@ __device__ __forceinline__ unsigned long long fixed_digits(double x, int sh)
 template <int I>
 __device__ __forceinline__ uint32_t slice_pair(unsigned long long u0, unsigned long long u1)
 {
-    constexpr int b = S - 1 - I;  // byte
-    uint32_t t;
-    if (b == S - 1) {
-        t = __byte_perm((uint32_t)(u0 >> 32), (uint32_t)(u1 >> 32), 0x7632) & 0x01ff01ffu;
-    } else {
-        const uint32_t w0 = b < 4 ? (uint32_t)u0 : (uint32_t)(u0 >> 32), w1 = b < 4 ? (uint32_t)u1 : (uint32_t)(u1 >> 32);
-        constexpr int c = b & 3;
-        t = __byte_perm(w0, w1, c | (c << 4) | ((4 + c) << 8) | ((4 + c) << 12)) & 0x00ff00ffu;
-    }
+    constexpr int b = S - 1 - I, c = b & 3;  // byte
+    const uint32_t w0 = b < 4 ? (uint32_t)u0 : (uint32_t)(u0 >> 32), w1 = b < 4 ? (uint32_t)u1 : (uint32_t)(u1 >> 32);
+    uint32_t t = __byte_perm(w0, w1, c | (c << 4) | ((4 + c) << 8) | ((4 + c) << 12)) & 0x00ff00ffu;
     t |= 0x64006400u;  // FP16 1024 + digit + 128, exact
     const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&t), __floats2half2_rn(1152.f, 1152.f));
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -383,11 +379,9 @@ __device__ __forceinline__ void guard_proj(const SplitArgs& s, int block)
         }
 #pragma unroll 4
         for (int b = 0; b < G_BANDS; ++b) {
-            int e = -8192;
-            if (k < s.K && b0 + b < s.nb) {
-                e = exp_of(s.B[(size_t)(b0 + b) * s.ldb + k]);
-                if (e < 0 || e == 0x7ff) e = -8192;
-            }
+            int e = -1;
+            if (k < s.K && b0 + b < s.nb) e = exp_of(s.B[(size_t)(b0 + b) * s.ldb + k]);
+            if (e == 0x7ff) e = -1;
 #pragma unroll
             for (int g = 0; g <= G_CHUNK; ++g) {
                 const int t = __reduce_max_sync(0xffffffffu, e < 0 ? 0 : max(0, e + x[g]));
@@ -481,8 +475,8 @@ __device__ __noinline__ double2 expand_exact(const double2* A, size_t lda, int r
     double re = 0.0, im = 0.0;
     for (int k = 0; k < K; ++k) {
         const double2 a = A[(size_t)map.a(k) * lda + row], w = W[(size_t)map.w(k) * ldw + n];
-        re += a.x * w.x - a.y * w.y;
-        im += a.x * w.y + a.y * w.x;
+        re = fma(a.x, w.x, fma(-a.y, w.y, re));
+        im = fma(a.x, w.y, fma(a.y, w.x, im));
     }
     return make_double2(re, im);
 }
@@ -510,10 +504,10 @@ __device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t (&r)[4])
                  : "r"(addr));
 }
 
-// (h 2^24 + l) 2^e rounded once to FP64, on the integer pipe
+// (h 2^32 + l) 2^e rounded once to FP64, on the integer pipe
 __device__ __forceinline__ double round_sum(long long h, long long l, int e)
 {
-    const __int128 v = ((__int128)h << 24) + l;
+    const __int128 v = ((__int128)h << 32) + l;
     if (v == 0) return 0.0;
     const bool neg = v < 0;
     const unsigned __int128 a = neg ? (unsigned __int128)-v : (unsigned __int128)v;
@@ -616,23 +610,14 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t st = smem_u32(tiles + s * STAGE);
                 const uint64_t ad = sdesc_sw32(st), bd = sdesc_sw32(st + A_STAGE);
                 const bool first = it == c * CHUNK;
-                // Slice i of A against slices j0 .. j0 + n - 1 of B in one MMA: their
-                // rows follow each other in shared memory, and their diagonals
-                // i + j in TMEM.  The first products of a diagonal (i = 0, and
-                // i = 1 with the last j) overwrite what the last read-out left.
-                auto mma = [&](int i, int j0, int n, bool overwrite) {
-                    tc_mma(acc + (i + j0) * NT, ad + ((i * TM * KB * 2) >> 4), bd + ((j0 * NT * KB * 2) >> 4),
-                           idesc_f16(TM, n * NT, 0), overwrite ? 0u : 1u);
-                };
-                mma(0, 0, S, first);
-                if (first) {
-                    mma(1, 0, ND - 2, false);
-                    mma(1, ND - 2, 1, true);
-                } else {
-                    mma(1, 0, ND - 1, false);
-                }
+                // Slice i of A against slices 0 .. ND - 1 - i of B in one MMA: their rows
+                // follow each other in shared memory, and their diagonals i + j in TMEM.
+                // The first products (i = 0: all diagonals) overwrite what the last
+                // read-out left.
 #pragma unroll
-                for (int i = 2; i < S; ++i) mma(i, 0, ND - i, false);
+                for (int i = 0; i < S; ++i)
+                    tc_mma(acc + i * NT, ad + ((i * TM * KB * 2) >> 4), bd, idesc_f16(TM, (ND - i) * NT, 0),
+                           first && i == 0 ? 0u : 1u);
                 tc_commit(&sh->empty[s]);
             }
             if (!stop) tc_commit(&sh->dfull[buf]);
@@ -687,23 +672,23 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
 #pragma unroll
                 for (int i = 0; i < BPW; ++i) {
-                    // exact integers: |diagonal d| <= 128 (d + 1) 2^14 < 2^24, the sums of
-                    // two adjacent low diagonals within 32 bits
-                    const int t01 = __float2int_rn(__uint_as_float(v[0][i])) * 256 + __float2int_rn(__uint_as_float(v[1][i]));
-                    const int t23 = __float2int_rn(__uint_as_float(v[2][i])) * 256 + __float2int_rn(__uint_as_float(v[3][i]));
-                    const int i4 = __float2int_rn(__uint_as_float(v[4][i])), i5 = __float2int_rn(__uint_as_float(v[5][i]));
-                    const int i67 = __float2int_rn(fmaf(__uint_as_float(v[7][i]), 1.f / 256.f, __uint_as_float(v[6][i])));
+                    // exact integers: |diagonal d| <= 128 (d + 1) 2^14, pairs with a top digit half of
+                    // that, so all are below 2^24 and the sums of two adjacent high ones within 32 bits
+                    int D[ND];
+#pragma unroll
+                    for (int d = 0; d < ND; ++d) D[d] = __float2int_rn(__uint_as_float(v[d][i]));
+                    const int t01 = D[0] * 256 + D[1], t23 = D[2] * 256 + D[3];
                     h[p + i] += (long long)t01 * 65536 + t23;
-                    l[p + i] += (long long)i4 * 65536 + ((long long)i5 * 256 + i67);
+                    l[p + i] += ((long long)D[4] * 16777216 + (long long)D[5] * 65536) + ((long long)D[6] * 256 + D[7]);
                 }
             }
         }
         double2* out = gemm == 0 ? o.out[0] : gemm == 1 ? o.out[1] : o.out[2];
         if (go && row < o.M) {
-            // h counts diagonal 3, l diagonal 6: weights 2^(72 - 110) and 2^(48 - 110)
+            // h counts diagonal 3, l diagonal 7: weights 2^-36 and 2^-68
             const int fr = o.er[row];
             const bool bad = !EXPAND && fr >= F_BAD;
-            const int er = (EXPAND ? (fr >> 16) - 1022 : clean(fr)) - 62;
+            const int er = (EXPAND ? (fr >> 16) - 1022 : clean(fr)) - 68;
 #pragma unroll
             for (int i = 0; i < BPW; ++i) {
                 const int n = blockIdx.x * BT + sub * BPW + i;
@@ -952,8 +937,8 @@ __global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total
 #pragma unroll 4
         for (int k = threadIdx.y * 32 + threadIdx.x; k < gd.K; k += 32 * SL) {
             const double2 u = a[k], v = b[k];
-            x += u.x * v.x + u.y * v.y;
-            y += u.x * v.y - u.y * v.x;
+            x = fma(u.x, v.x, fma(u.y, v.y, x));
+            y = fma(u.x, v.y, fma(-u.y, v.x, y));
         }
         for (int o = 16; o > 0; o >>= 1) {
             x += __shfl_xor_sync(0xffffffffu, x, o);

@@ -7,7 +7,7 @@ The reference is the same call on the SIMT FP64 GEMMs, which the context runs wh
 is granted no room for digits.  V_loc and the kinetic energies are zero, so that the
 nonlocal term stands alone, and results are compared shell by shell in |k+G|, so that
 no component hides behind a larger one.  Tolerance: 1e-13 per sum (test_gpu_fp64_tc.py)
-and the 4 bits that the digits may lose: 16e-13.
+and what the digits may lose, 4 bits of that: 16e-13.
 """
 import numpy as np
 import pytest
