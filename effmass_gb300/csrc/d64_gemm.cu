@@ -35,8 +35,9 @@
 // sums in chains of 192): 2 bits 9e-16 / 9e-17 / 6e-16, 4 bits 6e-15 / 4e-16 / 6e-16,
 // 6 bits 6e-15 / 4e-16 / 3e-16.  The pair matrix of the velocities has no groups: its
 // rows are bands, which say nothing about one another, so their columns are not
-// scaled, and an entry is right to 2^-59 of the product of its bands' norms (and
-// rounded to FP64).
+// scaled, and the largest term of an entry is taken among the largest elements of
+// both rows in 32 segments of K.  That may be too small, which forms a sum in FP64
+// that the digits would have held.
 //
 // What bounds it: the tensor pipe on large cells (64-atom cell, 128 bands: 80% of
 // the measured bf16 rate in the GEMMs).  The eight slices of a B tile lie one
@@ -874,6 +875,7 @@ struct Guard {
     const int* gt;     // largest terms [segs][groups + 1][N], null: no guard
     const int* fg;
     int segs, groups;
+    const int2 *ca, *cb;  // largest elements by segment of A's and B's rows (d64_tops), null: none
     D64Rows rows;
     const double2 *A, *B;
     size_t lda, ldb;
@@ -893,7 +895,8 @@ __global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total
     const size_t i = (size_t)blockIdx.x * 32 + threadIdx.x;
     const int per = ceil_div_d(nz, SL), z1 = min(nz, (int)(threadIdx.y + 1) * per);
     double re = 0.0, im = 0.0;
-    int t = 0, f = 0, fg = 0;
+    int t = 0, f = 0, fg = 0;  // largest term; the scales: f over the columns or of A's row, fg of the other
+    __shared__ int fb[SL][32];
     if (gd.gt && i < total) {
         const int m = (int)(i / N), n = (int)(i - (size_t)m * N), set = m / gd.rows.P;
         const int g = set * gd.rows.ng + gd.rows.gid[m - set * gd.rows.P];
@@ -903,6 +906,24 @@ __global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total
             const int* at = gd.gt + (size_t)q * (gd.groups + 1) * N + n;
             t = max(t, at[(size_t)g * N]);
             f = max(f, at[(size_t)gd.groups * N]);
+        }
+    }
+    if (gd.ca && i < total) {
+        // at least one of the rows' largest elements by segment is near the largest term
+        const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
+#pragma unroll 4
+        for (int q = threadIdx.y; q < D64_TOPS; q += SL) {
+            const int2 a = gd.ca[(size_t)m * D64_TOPS + q], b = gd.cb[(size_t)n * D64_TOPS + q];
+            f = max(f, a.y);
+            fg = max(fg, b.y);
+            if (a.y > 0) {
+                const int e = exp_of(gd.B[(size_t)n * gd.ldb + a.x]);
+                if (e >= 0 && e != 0x7ff) t = max(t, a.y + e + 1);
+            }
+            if (b.y > 0) {
+                const int e = exp_of(gd.A[(size_t)m * gd.lda + b.x]);
+                if (e >= 0 && e != 0x7ff) t = max(t, b.y + e + 1);
+            }
         }
     }
     if (i < total) {
@@ -915,6 +936,7 @@ __global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total
     }
     sum[threadIdx.y][threadIdx.x] = make_double2(re, im);
     tf[threadIdx.y][threadIdx.x] = make_int2(t, f);
+    fb[threadIdx.y][threadIdx.x] = fg;
     __syncthreads();
     if (threadIdx.y == 0) {
 #pragma unroll
@@ -923,12 +945,16 @@ __global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total
             im += sum[y][threadIdx.x].y;
             t = max(t, tf[y][threadIdx.x].x);
             f = max(f, tf[y][threadIdx.x].y);
+            if (gd.ca) fg = max(fg, fb[y][threadIdx.x]);
         }
-        const unsigned b = __ballot_sync(0xffffffffu, t > 0 && fg + f - t > LOSS_MAX);
+        // t = 0: no term among those known; with groups no term at all
+        const unsigned b = __ballot_sync(0xffffffffu, gd.ca ? f > 0 && fg > 0 && fg + f - t > LOSS_MAX
+                                                            : t > 0 && fg + f - t > LOSS_MAX);
         if (threadIdx.x == 0) todo = b;
     }
-    if (gd.gt) __syncthreads();
-    for (unsigned left = gd.gt ? todo : 0u; left; left &= left - 1) {
+    const bool guarded = gd.gt || gd.ca;
+    if (guarded) __syncthreads();
+    for (unsigned left = guarded ? todo : 0u; left; left &= left - 1) {
         const int j = __ffs((int)left) - 1;
         const size_t at = (size_t)blockIdx.x * 32 + j;
         const int m = (int)(at / N), n = (int)(at - (size_t)m * N);
@@ -963,7 +989,36 @@ __global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total
     }
 }
 
+// one block per row, four segments per warp
+__global__ void __launch_bounds__(256) tops_kernel(int K, const double2* __restrict__ x, size_t ld, int2* out)
+{
+    const double2* row = x + (size_t)blockIdx.x * ld;
+    const int lane = threadIdx.x & 31, len = ceil_div_d(K, D64_TOPS);
+    for (int q = threadIdx.x >> 5; q < D64_TOPS; q += 8) {
+        const int k1 = min(K, (q + 1) * len);
+        int e = 0, at = 0;
+#pragma unroll 4
+        for (int k = q * len + lane; k < k1; k += 32) {
+            const int y = exp_of(row[k]) + 1;
+            if (y > e && y != 0x800) {
+                e = y;
+                at = k;
+            }
+        }
+        const int top = __reduce_max_sync(0xffffffffu, e);
+        at = __reduce_max_sync(0xffffffffu, e == top ? at : 0);
+        if (lane == 0) out[(size_t)blockIdx.x * D64_TOPS + q] = make_int2(at, top);
+    }
+}
+
 }  // namespace
+
+cudaError_t d64_tops(int rows, int K, const double2* x, size_t ld, int2* out, cudaStream_t st)
+{
+    if (rows == 0) return cudaSuccess;
+    tops_kernel<<<rows, 256, 0, st>>>(K, x, ld, out);
+    return cudaGetLastError();
+}
 
 size_t d64_scale_ints(int M, int K, const D64Rows& rows)
 {
@@ -1027,13 +1082,13 @@ cudaError_t d64_proj(int M, int N, int K, const double2* A, size_t lda, D64Scale
 
 cudaError_t d64_reduce(int M, int N, int K, int nz, double2* part, const double* scale, int period, double2* W,
                        const double2* A, size_t lda, D64Scale s, const double2* B, size_t ldb, unsigned char* ws,
-                       bool keep, cudaStream_t st)
+                       bool keep, cudaStream_t st, const int2* ca, const int2* cb)
 {
     const size_t total = (size_t)M * N;
     if (total == 0) return cudaSuccess;
     const Plan p = proj_plan(M, N, K, s.rows);
     const Guard g{s.rows.ng ? plan_guard(p, ws) : nullptr, s.fg, p.segs, s.rows.ng ? M / s.rows.P * s.rows.ng : 0,
-                  s.rows, A, B, lda, ldb, K};
+                  ca, cb, s.rows, A, B, lda, ldb, K};
     const int blocks = ceil_div((long)total, 32);
     if (nz >= 16) d64_reduce_kernel<8><<<blocks, dim3(32, 8), 0, st>>>(N, total, nz, part, scale, period, W, g, keep);
     else d64_reduce_kernel<1><<<blocks, dim3(32, 1), 0, st>>>(N, total, nz, part, scale, period, W, g, keep);

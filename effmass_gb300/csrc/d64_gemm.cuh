@@ -38,10 +38,16 @@ cudaError_t d64_proj(int M, int N, int K, const double2* A, size_t lda, D64Scale
 
 // W[m][n] = scale[m % period] sum_z part[z][m][n] (scale null: 1) after d64_proj on the
 // same operands and ws; sums that the digits do not hold well enough are formed
-// in FP64.  The sums without scale are left in part[0] with keep.
+// in FP64.  The sums without scale are left in part[0] with keep.  Without groups the
+// guard needs the largest elements of A's rows (ca) and of B's (cb).
 cudaError_t d64_reduce(int M, int N, int K, int nz, double2* part, const double* scale, int period, double2* W,
                        const double2* A, size_t lda, D64Scale s, const double2* B, size_t ldb, unsigned char* ws,
-                       bool keep, cudaStream_t st);
+                       bool keep, cudaStream_t st, const int2* ca = nullptr, const int2* cb = nullptr);
+
+// out[row][i] = (k, biased exponent + 1) of the largest element of row x[row][.] in
+// the i-th of D64_TOPS segments of K
+constexpr int D64_TOPS = 32;
+cudaError_t d64_tops(int rows, int K, const double2* x, size_t ld, int2* out, cudaStream_t st);
 
 // Expansion: out[n][k] += sum_m W[m][n] A[m][k].  ws: d64_expand_ws bytes.
 size_t d64_expand_ws(int M, int N, int K, const D64Rows& rows);

@@ -627,6 +627,7 @@ static size_t d64_velocity_bytes(const hpsi_ctx* c, const KSlot& s, int nb, int 
     Carver cv;
     cv.take<double2>((size_t)d64_proj_splits(nb, nb, s.npw) * nb * nb);
     cv.take<int>((size_t)nb);
+    cv.take<int2>((size_t)4 * nb * D64_TOPS);
     return std::max(cv.off + d64_proj_ws(nb, nb, s.npw, D64Rows{}), d64_grad_bytes(c, s, nb, 3, prec));
 }
 
@@ -639,6 +640,7 @@ static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const
     Carver cv;
     const size_t o_part = cv.take<double2>((size_t)nz * nb * nb);
     const size_t o_exp = cv.take<int>((size_t)nb);
+    const size_t o_tops = cv.take<int2>((size_t)4 * nb * D64_TOPS);
     const size_t o_ops = cv.off;
     unsigned char* ws = c->d64_ws;
     if (!ws || c->d64_size < o_ops + d64_proj_ws(nb, nb, s.npw, D64Rows{})) return HPSI_OK;
@@ -650,12 +652,16 @@ static int velocity_d64(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, const
     const size_t npw = (size_t)s.npw;
     int h = c->prof.open(PH_OTHER, st);
     CUDA_TRY(c, d64_scales(nb, s.npw, psi, npw, sc, st));
+    int2 *top_psi = reinterpret_cast<int2*>(ws + o_tops), *top_g = top_psi + (size_t)nb * D64_TOPS;
+    CUDA_TRY(c, d64_tops(nb, s.npw, psi, npw, top_psi, st));
+    CUDA_TRY(c, d64_tops(3 * nb, s.npw, g, npw, top_g, st));
     for (int a = 0; a < 3; ++a) {
         CUDA_TRY(c, d64_proj(nb, nb, s.npw, psi, npw, sc, g + (size_t)a * nb * npw, npw, part, ws + o_ops, c->d_err, st));
         CUDA_TRY(c, d64_reduce(nb, nb, s.npw, nz, part, nullptr, nb, m + (size_t)a * nb * nb, psi, npw, sc,
-                               g + (size_t)a * nb * npw, npw, ws + o_ops, false, st));
+                               g + (size_t)a * nb * npw, npw, ws + o_ops, false, st, top_psi,
+                               top_g + (size_t)a * nb * D64_TOPS));
     }
-    c->prof.close(h, st, 11);
+    c->prof.close(h, st, 13);
     return HPSI_OK;
 }
 
