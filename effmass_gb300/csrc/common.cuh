@@ -56,8 +56,16 @@ __device__ __forceinline__ double f2d_bits(float x)
     return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
 
-// to FP64 off the FP64 pipe
-__device__ __forceinline__ double widen(float x) { return f2d_bits(x); }
+// to FP64 off the FP64 pipe, subnormals included
+__device__ __forceinline__ double widen(float x)
+{
+    const uint32_t u = __float_as_uint(x), a = u & 0x7fffffffu;
+    if (a == 0u || a >= 0x00800000u) return f2d_bits(x);
+    const int lz = __clz((int)a);
+    const uint32_t m = a << (lz - 8);  // leading bit at 23: value m 2^(8 - lz - 149)
+    return __hiloint2double((int)((u & 0x80000000u) | (uint32_t)(905 - lz) << 20 | (m & 0x7fffffu) >> 3),
+                            (int)(m << 29));
+}
 __device__ __forceinline__ double widen(double x) { return x; }
 #endif
 
