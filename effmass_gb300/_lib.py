@@ -22,7 +22,7 @@ EXPORTS = ["hpsi_abi_version", "hpsi_ctx_create", "hpsi_ctx_destroy", "hpsi_set_
            "hpsi_batch_buffers", "hpsi_batch_offset", "hpsi_batch_run", "hpsi_batch_apply", "hpsi_batch_info",
            "hpsi_batch_destroy", "hpsi_batch_last_error", "hpsi_selftest_convert", "hpsi_selftest_wait_limit",
            "hpsi_selftest_fft3d", "hpsi_selftest_kpoint_tables", "hpsi_selftest_memory",
-           "hpsi_selftest_memory_state",
+           "hpsi_selftest_memory_state", "hpsi_selftest_sums",
            "hpsi_last_error"]
 
 _lib = None
@@ -74,6 +74,7 @@ def load():
     L.hpsi_profile.argtypes = [ctxp, C.c_int]
     L.hpsi_profile_read.argtypes = [ctxp, dp, C.POINTER(C.c_longlong)]
     L.hpsi_selftest_convert.argtypes = [dp, C.c_long] + [C.c_void_p] * 4
+    L.hpsi_selftest_sums.argtypes = [C.c_void_p, C.c_long, C.c_void_p, C.c_void_p]
     L.hpsi_selftest_wait_limit.argtypes = [C.c_long]
     L.hpsi_selftest_memory.argtypes = [ctxp, C.c_longlong, C.c_int]
     L.hpsi_selftest_memory_state.argtypes = [ctxp, C.POINTER(C.c_longlong)]

@@ -104,6 +104,31 @@ struct Sum2f {
     }
     HPSI_D float value() const { return s + c; }
 };
+
+// Sum of n <= 16 floats as exact as in FP64, on the FP32 pipe: two two-sums in a row,
+// s + c + d with some 70 bits.  A sum that leaves the float range (or holds an infinity
+// or NaN) is taken in FP64.
+template <int N>
+__device__ __forceinline__ double sum_floats(const float (&x)[N], int n = N)
+{
+    static_assert(N <= 16, "d collects errors without compensation");
+    float s = 0.f, c = 0.f, d = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if (i >= n) break;
+        float t = s + x[i], b = t - s;
+        const float e = (s - (t - b)) + (x[i] - b);
+        s = t;
+        t = c + e;
+        b = t - c;
+        d += (c - (t - b)) + (e - b);
+        c = t;
+    }
+    if (fabsf(s) <= 3.4028234e38f) return widen(s) + (widen(c) + widen(d));
+    double r = 0.0;
+    for (int i = 0; i < n; ++i) r += (double)x[i];
+    return r;
+}
 #endif
 
 static inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }

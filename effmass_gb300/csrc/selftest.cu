@@ -22,7 +22,39 @@ __global__ void convert_kernel(const double* __restrict__ x, long n, float* f_bi
     d_hw[i] = (double)h;
 }
 
+__global__ void sum_kernel(const float* __restrict__ x, long rows, double* sum, double* wide)
+{
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rows) return;
+    float a[16];
+    for (int k = 0; k < 16; ++k) {
+        a[k] = x[16 * i + k];
+        wide[16 * i + k] = widen(a[k]);
+    }
+    sum[i] = sum_floats(a);
+}
+
 }  // namespace
+
+// sums of 16 floats each (x [rows][16]) as the band-pair reduction takes them, and
+// every float widened as the FP32 GEMMs widen theirs
+extern "C" int hpsi_selftest_sums(const float* x, long rows, double* sum, double* wide)
+{
+    if (rows < 0 || (rows > 0 && (!x || !sum || !wide))) return HPSI_ERR_BAD_ARG;
+    if (rows == 0) return HPSI_OK;
+    const size_t n = (size_t)rows * 16;
+    unsigned char* m = nullptr;
+    if (cudaMalloc(&m, n * 12 + rows * 8) != cudaSuccess) return HPSI_ERR_OOM;
+    double *dw = reinterpret_cast<double*>(m), *ds = dw + n;
+    float* dx = reinterpret_cast<float*>(ds + rows);
+    cudaError_t e = cudaMemcpy(dx, x, n * sizeof(float), cudaMemcpyHostToDevice);
+    if (!e) sum_kernel<<<(unsigned)((rows + 127) / 128), 128>>>(dx, rows, ds, dw);
+    if (!e) e = cudaGetLastError();
+    if (!e) e = cudaMemcpy(sum, ds, rows * sizeof(double), cudaMemcpyDeviceToHost);
+    if (!e) e = cudaMemcpy(wide, dw, n * sizeof(double), cudaMemcpyDeviceToHost);
+    cudaFree(m);
+    return e ? HPSI_ERR_CUDA : HPSI_OK;
+}
 
 extern "C" int hpsi_selftest_convert(const double* x, long n, float* f_bits, float* f_hw, double* d_bits,
                                      double* d_hw)

@@ -1049,31 +1049,18 @@ __global__ void proj_reduce_kernel(int P, int nb, int N, int nsplit, const float
         }
         return;
     }
-    // complex128: two-float sums of 16 splits, folded in FP64 (an FP64 add per
-    // split was bound by the FP64 pipe: 168 -> 30 us for 256 x 256 over 290 splits)
+    // complex128: 16 splits at a time on the FP32 pipe, added in FP64 (an FP64 add per
+    // split was bound by the FP64 pipe)
     double sr = 0.0, si = 0.0;
     for (int z0 = 0; z0 < nsplit; z0 += 16) {
-        Sum2f re, im;
-        if (z0 + 16 <= nsplit) {
-            float a[16], c[16];
+        float a[16], c[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                a[u] = pre[(z0 + u) * zs];
-                c[u] = pim[(z0 + u) * zs];
-            }
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                re.add(a[u]);
-                im.add(c[u]);
-            }
-        } else {
-            for (int z = z0; z < nsplit; ++z) {
-                re.add(pre[z * zs]);
-                im.add(pim[z * zs]);
-            }
+        for (int u = 0; u < 16; ++u) {
+            a[u] = z0 + u < nsplit ? pre[(z0 + u) * zs] : 0.f;
+            c[u] = z0 + u < nsplit ? pim[(z0 + u) * zs] : 0.f;
         }
-        sr += f2d_bits(re.s) + f2d_bits(re.c);
-        si += f2d_bits(im.s) + f2d_bits(im.c);
+        sr += sum_floats(a);
+        si += sum_floats(c);
     }
     const double f = lam ? lam[p % period] : 1.0;
     W[idx] = from_c128<CW>(make_double2(f * sr, f * si));

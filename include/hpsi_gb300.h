@@ -389,6 +389,10 @@ const char* hpsi_batch_last_error(const hpsi_batch* b);
  * f_hw back to double both ways (d_bits, d_hw).  No reference counterpart. */
 int hpsi_selftest_convert(const double* x, long n, float* f_bits, float* f_hw, double* d_bits, double* d_hw);
 
+/* Device check of the FP64 sums and conversions made on the FP32 and integer pipes:
+ * sum[r] of the 16 floats x[r], and every float to FP64 (host arrays). */
+int hpsi_selftest_sums(const float* x, long rows, double* sum, double* wide);
+
 /* Self-test of the device line transforms (no reference counterpart): the
  * reference's FFT3D (src/math/fft.cppm:60-85) on an n1 x n2 x n3 grid of
  * complex<double> in host memory, transformed in place: dir = +1 G->r
