@@ -1062,18 +1062,26 @@ static auto with_plan(const FftLen& L, F&& f)
     }
     return f(NoPlan{});
 }
-// plane plans (y, z): the same length, or z twice as long (a cell doubled along z:
-// 32 x 64 planes, 128 bands, G->r 50 -> 35 us; H|psi> on the tensor cores 201 -> 177;
-// 30 x 60, 37 bands 145 -> 130; 36 x 72, 37 bands 153 -> 141)
+// Plane plans (y, z) from the radices of both axes: the same length, or one twice the
+// other (a cell doubled along y or z).  Other pairs keep the runtime plans: all 81 would
+// take the compiler minutes.  Cells doubled along z, us: 32 x 64 planes, 128 bands, G->r
+// 50 -> 35, H|psi> on the tensor cores 201 -> 177; 30 x 60, 37 bands 145 -> 130; 36 x 72,
+// 37 bands 153 -> 141.  Along y, FP32 local term of 64 bands: 36 x 72 x 36 88 -> 70,
+// 32 x 64 x 32 72 -> 57, 30 x 60 x 30 95 -> 72.
+template <typename PL> struct PlanLen { static constexpr int n = PL::n; };
+template <> struct PlanLen<NoPlan> { static constexpr int n = 0; };
+constexpr bool plane_pair(int y, int z) { return y > 0 && z > 0 && (y == z || y == 2 * z || 2 * y == z); }
 template <typename F>
 static auto with_planes(const LocalArgs& a, F&& f)
 {
-    if (a.n2 == a.n3) return with_plan(a.Ly, [&](auto pl) { return f(pl, pl); });
-    if (a.n2 == 32 && a.n3 == 64) return f(FftPlan2<8, 4>{}, FftPlan2<8, 8>{});
-    if (a.n2 == 30 && a.n3 == 60) return f(FftPlan3<2, 3, 5>{}, FftPlan3<4, 3, 5>{});
-    if (a.n2 == 36 && a.n3 == 72) return f(FftPlan2<9, 4>{}, FftPlan2<8, 9>{});
-    if (a.n2 == 24 && a.n3 == 48) return f(FftPlan2<8, 3>{}, FftPlan3<8, 2, 3>{});
-    return f(NoPlan{}, NoPlan{});
+    return with_plan(a.Ly, [&](auto py) {
+        using PY = std::decay_t<decltype(py)>;
+        return with_plan(a.Lz, [&](auto pz) {
+            using PZ = std::decay_t<decltype(pz)>;
+            if constexpr (plane_pair(PlanLen<PY>::n, PlanLen<PZ>::n)) return f(PY{}, PZ{});
+            else return f(NoPlan{}, NoPlan{});
+        });
+    });
 }
 template <typename C>
 using G2rFn = void (*)(LocalArgs, const double2*, C*, const C*, const C*);
