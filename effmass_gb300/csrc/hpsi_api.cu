@@ -1346,7 +1346,7 @@ static int energies_dev(hpsi_ctx* c, KSlot& s, int nb, const double2* psi, doubl
         // two G-vectors share a grid point: the Parseval identity does not hold,
         // so the energy is the Rayleigh quotient of the computed H|psi>
         CUDA_TRY(c, launch_band_dot(s.npw, nb, psi, hpsi, dots, st));
-        if ((rc = apply_dev(c, s, nb, psi, hpsi, prec, ws + w.work, st))) return rc;
+        if ((rc = apply_dev(c, s, nb, psi, hpsi, prec, ws + w.work, st, nullptr, nullptr, fork))) return rc;
         CUDA_TRY(c, launch_band_dot(s.npw, nb, psi, hpsi, dots + nb, st));
         CUDA_TRY(c, launch_band_sub(nb, dots + nb, dots, e, st));
         return HPSI_OK;
