@@ -482,20 +482,28 @@ __device__ __noinline__ double2 expand_exact(const double2* A, size_t lda, int r
     return make_double2(re, im);
 }
 
-// Output (row, n) of GEMM g, v unless the scales cost it more than LOSS_MAX bits; f: the
-// band's exponent, e: that of the row's column of A
-__device__ __noinline__ double2 expand_guarded(const D64Out& o, int g, int row, int n, int f, int e, double2 v)
+// bits of the bands n0 .. n0 + 3 whose output at row loses more than LOSS_MAX bits to the
+// scales of GEMM g; f: the bands' exponents (biased), e: that of the row's column of A
+__device__ __noinline__ unsigned expand_loses(const D64Out& o, int g, int row, int n0, int4 f, int e)
 {
-    const int* wg = o.wg + (size_t)g * o.sets * o.ng * o.bands + n;
-    int t = 0;
-    for (int s = 0; s < o.sets; ++s)
+    const int* wg = o.wg + (size_t)g * o.sets * o.ng * o.bands + n0;
+    int4 t = make_int4(0, 0, 0, 0);
+    for (int s = 0; s < o.sets; ++s) {
+        const int* eg = o.eg + (size_t)(s ? o.dir[g] : 0) * o.ng * o.K + row;
+#pragma unroll 4
         for (int r = 0; r < o.ng; ++r) {
-            const int x = wg[(size_t)(s * o.ng + r) * o.bands];
-            const int a = o.eg[((size_t)(s ? o.dir[g] : 0) * o.ng + r) * o.K + row];
-            if (x > 0 && a > 0) t = max(t, a + x);
+            const int4 x = *reinterpret_cast<const int4*>(wg + (size_t)(s * o.ng + r) * o.bands);
+            const int a = eg[(size_t)r * o.K];
+            if (a > 0) {
+                if (x.x > 0) t.x = max(t.x, a + x.x);
+                if (x.y > 0) t.y = max(t.y, a + x.y);
+                if (x.z > 0) t.z = max(t.z, a + x.z);
+                if (x.w > 0) t.w = max(t.w, a + x.w);
+            }
         }
-    if (t == 0 || e + f - (t - 1023) <= LOSS_MAX) return v;
-    return expand_exact(o.A, o.lda, row, o.W, o.ldw, n, o.sets * o.rows_P, o.map[g]);
+    }
+    auto loses = [&](int f, int t) { return f != 0 && f < F_BAD && t > 0 && e + f - F_BIAS - (t - 1023) > LOSS_MAX; };
+    return loses(f.x, t.x) | loses(f.y, t.y) << 1 | loses(f.z, t.z) << 2 | loses(f.w, t.w) << 3;
 }
 
 __device__ __forceinline__ void tmem_ld4(uint32_t addr, uint32_t (&r)[4])
@@ -631,9 +639,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         // bands sub BPW .. +BPW-1 of the tile, real and imaginary columns
         const int q = warp & 3, sub = (warp - 2) >> 2;
         const int row = o.row0 + blockIdx.y * TM + q * 32 + lane;
-        // Bands whose output may lose more than LOSS_MAX bits: those where the group of A's
-        // rows that has the column's largest element has a small W.  (Loaded here, under
-        // the first copies.)
+        // Bands whose output loses more than LOSS_MAX bits: candidates are those where the
+        // group of A's rows that has the column's largest element has a small W.  (Done
+        // here, under the first copies.)
         unsigned slow = 0;
         if (EXPAND && row < o.M) {
             const int e = o.er[row], b = (o.sets > 1 ? o.ed[(size_t)(o.dir[gemm] - 1) * o.K + row] : e);
@@ -645,6 +653,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 return f != 0 && f < F_BAD && (x == 0 || (e >> 16) - (b >> 16) + f - F_BIAS - (x - 1023) > LOSS_MAX);
             };
             slow = loses(f.x, x.x) | loses(f.y, x.y) << 1 | loses(f.z, x.z) << 2 | loses(f.w, x.w) << 3;
+            if (slow) slow &= expand_loses(o, gemm, row, n0, f, e >> 16);
         }
         long long h[2 * BPW], l[2 * BPW];
 #pragma unroll
@@ -698,7 +707,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                     double2 v = make_double2(round_sum(h[i], l[i], e), round_sum(h[BPW + i], l[BPW + i], e));
                     if (bad || f >= F_BAD) v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
                     if (EXPAND) {
-                        if (slow >> i & 1) v = expand_guarded(o, gemm, row, n, clean(f), fr >> 16, v);
+                        if (slow >> i & 1)
+                            v = expand_exact(o.A, o.lda, row, o.W, o.ldw, n, o.sets * o.rows_P, o.map[gemm]);
                         double2* at = out + (size_t)n * o.ldo + row;
                         double2 x = *at;
                         x.x += v.x;
