@@ -36,8 +36,8 @@
 // 6 bits 6e-15 / 4e-16 / 3e-16.  The pair matrix of the velocities has no groups: its
 // rows are bands, which say nothing about one another, so their columns are not
 // scaled, and the largest term of an entry is taken among the largest elements of
-// both rows in 32 segments of K.  That may be too small, which forms a sum in FP64
-// that the digits would have held.
+// both rows in 32 segments of K.  That is 0 to 3 bits too small (8- and 64-atom cells),
+// so entries may seem to lose two bits more.
 //
 // What bounds it: the tensor pipe on large cells (64-atom cell, 128 bands: 80% of
 // the measured bf16 rate in the GEMMs).  The eight slices of a B tile lie one
@@ -46,10 +46,11 @@
 // diagonals: 8 MMAs per 16 of K instead of 36, which the issuing thread could not
 // feed (70 clocks each).  Tiles of 16 bands (32 rows of B) leave TMEM room for two
 // sets of accumulators, so that one is read out under the next chunk's MMAs;
-// against tiles of 32 bands with one set, H|psi> us before -> now: 8-atom cell,
-// 48 bands 187 -> 173; 16 atoms, 37 bands 266 -> 234; 64 atoms, 128 bands
-// 5542 -> 5404; gradient, 8 atoms 129 -> 101.  What is left beside
-// the MMAs is writing the slices of A: 0.66 ms of the 64-atom call, at the rate
+// against tiles of 32 bands with one set, H|psi> us (seven slices, no guard): 8-atom
+// cell, 48 bands 187 -> 173; 16 atoms, 37 bands 266 -> 234; 64 atoms, 128 bands
+// 5542 -> 5404; gradient, 8 atoms 129 -> 101.  The eighth slice and the guard: 64 atoms
+// 5420 -> 5720, 8 atoms 182 -> 187, gradient 103 -> 117.  What is left beside
+// the MMAs is writing the slices of A: 0.7 ms of the 64-atom call, at the rate
 // of the memory.  Tiles of A fetched by half or by a quarter do not change the
 // GEMMs' time, so A is not multicast.  Measured and not kept: integers by FP32
 // magic adds in place of F2I, 32 of K per stage (SWIZZLE_64B).
@@ -84,6 +85,7 @@ constexpr uint32_t TMEM_ALL = 512;
 constexpr size_t A_CAP = 1536ull << 20;    // bytes of A slices resident at once
 constexpr int N_CAP = 256;                // bands per pass
 constexpr int LOSS_MAX = 6;               // bits that a sum may lose to the scales
+constexpr int LOSS_PAIR = 8;              // the same where the largest term is known from below (0 to 3 bits short)
 constexpr int G_CHUNK = 8;                // groups per guard block of a projection
 constexpr int G_BANDS = 16;               // its bands
 constexpr int G_SEGS = 32;                // K segments of a projection's guard at most
@@ -958,7 +960,7 @@ __global__ void __launch_bounds__(32 * SL) d64_reduce_kernel(int N, size_t total
             if (gd.ca) fg = max(fg, fb[y][threadIdx.x]);
         }
         // t = 0: no term among those known; with groups no term at all
-        const unsigned b = __ballot_sync(0xffffffffu, gd.ca ? f > 0 && fg > 0 && fg + f - t > LOSS_MAX
+        const unsigned b = __ballot_sync(0xffffffffu, gd.ca ? f > 0 && fg > 0 && fg + f - t > LOSS_PAIR
                                                             : t > 0 && fg + f - t > LOSS_MAX);
         if (threadIdx.x == 0) todo = b;
     }
@@ -1100,7 +1102,9 @@ cudaError_t d64_reduce(int M, int N, int K, int nz, double2* part, const double*
     const Guard g{s.rows.ng ? plan_guard(p, ws) : nullptr, s.fg, p.segs, s.rows.ng ? M / s.rows.P * s.rows.ng : 0,
                   ca, cb, s.rows, A, B, lda, ldb, K};
     const int blocks = ceil_div((long)total, 32);
-    if (nz >= 16) d64_reduce_kernel<8><<<blocks, dim3(32, 8), 0, st>>>(N, total, nz, part, scale, period, W, g, keep);
+    // eight slices also where sums of many terms may have to be formed
+    if (nz >= 16 || (ca && K > 2048))
+        d64_reduce_kernel<8><<<blocks, dim3(32, 8), 0, st>>>(N, total, nz, part, scale, period, W, g, keep);
     else d64_reduce_kernel<1><<<blocks, dim3(32, 1), 0, st>>>(N, total, nz, part, scale, period, W, g, keep);
     return cudaGetLastError();
 }
