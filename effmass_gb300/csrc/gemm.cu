@@ -13,7 +13,7 @@
 // that shared-memory reads of a warp are bank-conflict free.  What bounds them on
 // the smaller cells is the latency of a block's loads and too few blocks, so the
 // next slice is fetched while one is multiplied, and tiles shrink while blocks do
-// not fill the SMs.  FP32, us before -> now: H|psi> of 2 atoms, 32 bands 41 -> 34;
+// not fill the SMs.  FP32, us before -> now: H|psi> of 2 atoms, 32 bands 41 -> 35..37;
 // 8 atoms, 48 bands 85 -> 58 (projection 26 -> 13, expansion 26 -> 13); 16 atoms,
 // 37 bands 197 -> 156; 64 atoms, 16 bands 878 -> 646; gradient, 8 atoms, 48 bands
 // 194 -> 109.  All sums keep their order: the results are the same bits.
