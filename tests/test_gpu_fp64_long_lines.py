@@ -55,3 +55,23 @@ def test_fp64_local_term_of_long_lines(n):
         if b == 1:
             want = np.abs(r * np.longdouble(np.prod(n))) ** 2
             assert np.sqrt(((rho - want) ** 2).sum() / (want ** 2).sum()) <= 2 * TOL
+
+
+@pytest.mark.parametrize("n", [(128, 4, 4), (4, 128, 4), (4, 4, 128), (160, 3, 4), (4, 176, 4), (180, 4, 4), (4, 4, 144)])
+def test_fp64_local_term_of_middling_lines(n):
+    """Three axes, each rounded to about 2^-53 of its lines' norm: 4e-16."""
+    from effmass_gb300 import build
+    from effmass_gb300.hamiltonian import Hamiltonian
+    build.build()
+    sysm, kp, v, psi = _case(n)
+    at = tuple(kp.g_idx[:, d] % n[d] for d in range(3))
+    out = np.zeros_like(psi)
+    with Hamiltonian(sysm) as H:
+        H.set_kpoint(0, kp)
+        H.apply(0, len(psi), psi, out, "fp64")
+    for b, c in enumerate(psi):
+        grid = np.zeros(n, np.clongdouble)
+        grid[at] = c
+        want = np.fft.fftn(v.astype(np.longdouble) * np.fft.ifftn(grid))[at]
+        err = np.sqrt((np.abs(out[b] - want) ** 2).sum() / (np.abs(want) ** 2).sum())
+        assert err <= 4e-16, (b, float(err))
